@@ -15,6 +15,18 @@ namespace tc {
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// TMA and tcgen05 instructions take their operands from UNIFORM registers.  A role whose loop runs in one lane only
+// (`if (lane == 0)`) keeps them in ordinary registers and moves five or six per instruction across, about 70 clocks for each
+// MMA; so the whole warp walks the loop, on values the compiler can see to be the same in every lane, and one elected
+// lane issues.
+template <typename T>
+__device__ __forceinline__ T warp_uniform(T v) { return __shfl_sync(0xffffffffu, v, 0); }
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r != 0;
+}
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");

@@ -39,8 +39,50 @@ def _ksplit_slices(m: int, n: int, k: int) -> int:
     return sl
 
 
+TC_ROWS = 17            # rows from which the tensor-core GEMM takes over from the decode kernel (which re-reads the weights every 16 rows)
+TC_ROWS_WIDE = 12       # ... and against this many weight rows, where its row tiles alone fill the chip
+TC_WIDE_N = 8192
+TC_MIN_N = 512
+
+
+def _takes_tc(m: int, n: int, k: int) -> bool:
+    """Measured, us, decode kernel / tensor-core GEMM: [4096, 4096] 16 rows 10.9 / 10.1, 24 rows 17.9 / 10.4; [16384, 4096]
+    12 rows 19.8 / 17.9, 9 rows 17.8 / 17.7; [10240, 2560] 12 rows 12.6 / 11.4; [2048, 2048] 16 rows 6.5 / 7.4, 24 rows
+    10.5 / 7.5; [512, 4096] 16 rows 7.8 / 7.8, 24 rows 13.5 / 7.9 (fewer weight rows were not measured)."""
+    return m >= (TC_ROWS_WIDE if n >= TC_WIDE_N else TC_ROWS) and n >= TC_MIN_N and k % 128 == 0
+
+
+def _groupwise_tc(x, packed, scales, zeros):
+    """Group 128, many rows: rwkvq_tc_gemm_int4_group, or None where its alignment rules do not hold.  fp16 and bf16
+    activations go in as they are (the kernel that permutes them also rounds bf16 to fp16)."""
+    n, k = packed.shape[0], packed.shape[1] * 2
+    if packed.stride(1) != 1 or packed.stride(0) % 16 or (packed.data_ptr() | scales.data_ptr() | (0 if zeros is None else zeros.data_ptr())) % 16:
+        return None
+    x2 = x.reshape(-1, k)
+    if x2.dtype not in (torch.float16, torch.bfloat16):
+        x2 = x2.to(torch.float16)
+    x2 = x2.contiguous()
+    if x2.data_ptr() % 16:
+        x2 = x2.clone()
+    abi.require_device()
+    if not x2.is_cuda:
+        raise RuntimeError("rwkvq: INT4 / INT8 projections run on the GPU only (no CPU fallback)")
+    m, dev = x2.shape[0], x2.device
+    out = torch.empty((m, n), dtype=torch.float16, device=dev)
+    ws = torch.empty(int(abi.lib().rwkvq_tc_gemm_wa16_workspace_bytes(m, n, k, 4)), dtype=torch.uint8, device=dev)
+    abi.call("rwkvq_tc_gemm_int4_group", x2.data_ptr(), abi.dtype_code(x2), k, packed.data_ptr(), packed.stride(0), scales.data_ptr(),
+             abi.ptr(zeros), out.data_ptr(), n, m, n, k, ws.data_ptr(), ws.numel(), abi.stream_ptr())
+    abi.after_call()
+    return out
+
+
 def _groupwise_rows(x, packed, scales, zeros, group_size: int) -> torch.Tensor:
     n, k = packed.shape[0], packed.shape[1] * 2
+    if (group_size == 128 and scales.dtype != torch.float16 and x.shape[-1] == k and k and _takes_tc(x.numel() // k, n, k)
+            and os.environ.get("RWKVQ_INT4", "fast") != "generic"):
+        out = _groupwise_tc(x, packed, _f32(scales, x.device), None if zeros is None else _f32(zeros, x.device))
+        if out is not None:
+            return out
     x2 = _rows_f16(x, k)
     dev = x2.device
     scale_f16 = scales.dtype == torch.float16

@@ -27,12 +27,31 @@ def load_int8_weight(z: dict, key: str, dev: str = "cuda"):
     raise KeyError(f"No INT8 weight found for key: {key}")
 
 
+TC_ROWS = 17        # rows from which the tensor-core GEMM takes over (the row kernel takes 16 per pass over the weights)
+TC_MIN_N = 512
+
+
+def _tensor_core(x2, w, scale):
+    abi.require_device()
+    if not x2.is_cuda:
+        raise RuntimeError("rwkvq: INT4 / INT8 projections run on the GPU only (no CPU fallback)")
+    (m, k), n, dev = x2.shape, w.shape[0], x2.device
+    out = torch.empty((m, n), dtype=torch.float16, device=dev)
+    ws = torch.empty(int(abi.lib().rwkvq_tc_gemm_wa16_workspace_bytes(m, n, k, 8)), dtype=torch.uint8, device=dev)
+    abi.call("rwkvq_tc_gemm_int8_w8a16", x2.data_ptr(), k, w.data_ptr(), w.stride(0), scale.data_ptr(), out.data_ptr(), n, m, n, k,
+             ws.data_ptr(), ws.numel(), abi.stream_ptr())
+    abi.after_call()
+    return out
+
+
 def linear_int8_per_tensor(x, weight_info, out_dtype=torch.float16):
     """W8A16 projection: fp16 activations times int8 weights times the scale (int8/int8_ops.py:48-78)."""
     w = weight_info["weight"].contiguous()
     n, k = w.shape
     x2 = _rows_f16(x, k)
     scale = _f32(weight_info["tensor_scale"].reshape(1), x2.device)
+    if x2.shape[0] >= TC_ROWS and n >= TC_MIN_N and k % 16 == 0 and w.data_ptr() % 16 == 0:
+        return _tensor_core(x2, w, scale).to(out_dtype).reshape(*x.shape[:-1], n)
     out = _run_rows(x2, n, lambda xc, oc, m: abi.call(
         "rwkvq_gemv_int8_w8a16", xc.data_ptr(), k, w.data_ptr(), w.stride(0), scale.data_ptr(), oc.data_ptr(), n, m, n, k,
         abi.stream_ptr()))

@@ -74,6 +74,9 @@ SIGNATURES = {
     "rwkvq_gemv_int8_affine": [_p, _i64, _p, _i64, _p, _p, _p, _p, _p, _i64, _i64, _i64, _i64, _p],
     "rwkvq_gemv_int4_group_smem_bytes": [_i64, _i64],
     "rwkvq_gemv_int4_group": [_p, _i64, _p, _i64, _p, _p, _i32, _i32, _p, _i64, _i64, _i64, _i64, _p],
+    "rwkvq_tc_gemm_wa16_workspace_bytes": [_i64, _i64, _i64, _i32],
+    "rwkvq_tc_gemm_int4_group": [_p, _i32, _i64, _p, _i64, _p, _p, _p, _i64, _i64, _i64, _i64, _p, _i64, _p],
+    "rwkvq_tc_gemm_int8_w8a16": [_p, _i64, _p, _i64, _p, _p, _i64, _i64, _i64, _i64, _p, _i64, _p],
     "rwkvq_gemv_int4_ksplit_slices": [_i64, _i64, _i64],
     "rwkvq_gemv_int4_group_ksplit": [_p, _i64, _p, _i64, _p, _p, _p, _i64, _i64, _i64, _i64, _p, _i64, _p],
     "rwkvq_actq_nvfp4": [_p, _i32, _i64, _i64, _i64, _p, _i64, _p, _i64, _p, _p, _p],
@@ -123,7 +126,7 @@ SIGNATURES = {
     "rwkvq_gemv_set_trace": [_p],
     "rwkvq_tc_set_trace": [_p],
 }
-_RESTYPES = {"rwkvq_actq_nvfp4_fused_scratch_bytes": ctypes.c_int64, "rwkvq_gemv_nvfp4_fused_smem_bytes": ctypes.c_int64, "rwkvq_nvfp4_blocked_scale_bytes": ctypes.c_int64, "rwkvq_actq_fp8_fused_scratch_bytes": ctypes.c_int64, "rwkvq_gemv_nvfp4_smem_bytes": ctypes.c_int64, "rwkvq_gemv_int4_group_smem_bytes": ctypes.c_int64, "rwkvq_workspace_bytes": ctypes.c_int64, "rwkvq_last_error_string": ctypes.c_char_p, "rwkvq_launch_count": ctypes.c_int64,
+_RESTYPES = {"rwkvq_tc_gemm_wa16_workspace_bytes": ctypes.c_int64, "rwkvq_actq_nvfp4_fused_scratch_bytes": ctypes.c_int64, "rwkvq_gemv_nvfp4_fused_smem_bytes": ctypes.c_int64, "rwkvq_nvfp4_blocked_scale_bytes": ctypes.c_int64, "rwkvq_actq_fp8_fused_scratch_bytes": ctypes.c_int64, "rwkvq_gemv_nvfp4_smem_bytes": ctypes.c_int64, "rwkvq_gemv_int4_group_smem_bytes": ctypes.c_int64, "rwkvq_workspace_bytes": ctypes.c_int64, "rwkvq_last_error_string": ctypes.c_char_p, "rwkvq_launch_count": ctypes.c_int64,
              "rwkvq_set_wait_limit_us": None, "rwkvq_gemv_set_trace": None, "rwkvq_tc_set_trace": None}
 
 

@@ -1,0 +1,78 @@
+"""GPU parity of the tensor-core weight-only GEMMs (gemm_wa16.cu) against the oracle's dequantized weights in 64 bits.
+
+Bound per element: half an fp16 ulp of the result (2^-11 relative, 2^-25 below the normal range) plus the error of 32-bit
+sums.  A sum of K fp32 terms errs by at most K * 2^-23 times the sum of their magnitudes when every addition truncates;
+roundings of either sign grow with sqrt(K): 2^-16 of the magnitudes covers K = 16384 (sqrt(K) * 2^-23)."""
+import pytest
+import torch
+
+from oracle import rwkvq_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def gen(seed, shape, std=1.0):
+    return torch.randn(shape, generator=torch.Generator().manual_seed(seed)) * std
+
+
+def check(out, x, parts):
+    """parts: weight matrices whose sum is the dequantized weight (their magnitudes bound the intermediate sums)."""
+    xd = x.to(torch.float16).double()
+    ref = sum(xd @ p.double().t() for p in parts)
+    mag = sum(xd.abs() @ p.double().abs().t() for p in parts)
+    err = (out.double().cpu() - ref).abs()
+    bound = ref.abs() * 2.0 ** -11 + 2.0 ** -25 + mag * 2.0 ** -16
+    assert bool((err <= bound).all()), float((err / bound).max())
+
+
+# token tiles of 32 / 64 / 96 / 128 and their remainders, row tiles with a remainder, K slices (few tiles), group counts that
+# are no multiple of 4, one step of K
+@pytest.mark.parametrize("m,n,k", [(17, 512, 128), (33, 640, 768), (64, 520, 4096), (65, 4096, 1152), (129, 1000, 2560),
+                                   (300, 2560, 2560), (1000, 777, 640), (12, 8200, 512), (40, 512, 16384), (257, 16384, 256)])
+@pytest.mark.parametrize("zeros", [True, False])
+def test_int4_group_many_rows(m, n, k, zeros):
+    import rwkvq_abi as abi
+    from int4 import int4_ops, quantize_int4
+    info = quantize_int4.quantize_to_int4_groupwise(gen(n + k, (n, k), k ** -0.5), 128)
+    if not zeros:
+        info["zeros"] = -8.0 * info["scales"]
+    u = O.unpack_int4(info["packed"]).float().reshape(n, k // 128, 128)
+    parts = [(u.double() * info["scales"].double().unsqueeze(2)).reshape(n, k),
+             info["zeros"].double().unsqueeze(2).expand(n, k // 128, 128).reshape(n, k)]
+    d = {a: b.cuda() if torch.is_tensor(b) else b for a, b in info.items()}
+    if not zeros:
+        del d["zeros"]
+    d["qtype"] = "int4_groupwise"
+    for dtype in (torch.float16, torch.bfloat16):
+        x = gen(m, (m, k)).to(dtype)
+        before = abi.launch_count()
+        out = int4_ops.linear_int4(x.cuda(), d)
+        assert abi.launch_count() - before in (2, 3)           # activations, GEMM, sum of the K slices
+        check(out, x, parts)
+        assert torch.equal(out, int4_ops.linear_int4(x.cuda(), d))
+
+
+@pytest.mark.parametrize("m,n,k", [(17, 512, 128), (33, 640, 784), (64, 520, 4096), (65, 4096, 1168), (129, 1000, 16),
+                                   (300, 2560, 2560), (1000, 777, 640), (40, 512, 16384), (257, 16384, 256)])
+def test_int8_w8a16_many_rows(m, n, k):
+    import rwkvq_abi as abi
+    from int8 import int8_ops, quantize_int8
+    q, s = quantize_int8.quantize_to_int8_per_tensor(gen(n + k, (n, k), k ** -0.5))
+    d = {"weight": q.cuda(), "tensor_scale": s.cuda(), "qtype": "int8_per_tensor"}
+    x = gen(m, (m, k)).half()
+    before = abi.launch_count()
+    out = int8_ops.linear_int8(x.cuda(), d)
+    assert abi.launch_count() - before in (1, 2)               # GEMM, sum of the K slices
+    check(out, x, [q.double() * s.double()])
+    assert torch.equal(out, int8_ops.linear_int8(x.cuda(), d))
+
+
+def test_infinite_and_nan_activations_stay_in_their_row():
+    from int8 import int8_ops, quantize_int8
+    q, s = quantize_int8.quantize_to_int8_per_tensor(gen(1, (640, 256), 0.05))
+    x = gen(2, (40, 256)).half()
+    x[3, 7], x[39, 255] = float("inf"), float("nan")
+    out = int8_ops.linear_int8(x.cuda(), {"weight": q.cuda(), "tensor_scale": s.cuda(), "qtype": "int8_per_tensor"}).cpu()
+    ok = [i for i in range(40) if i not in (3, 39)]
+    check(out[ok], x[ok], [q.double() * s.double()])
+    assert not bool(out[3].isfinite().any()) and bool(out[39].isnan().all())
