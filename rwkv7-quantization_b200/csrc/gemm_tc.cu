@@ -273,7 +273,7 @@ __global__ void __launch_bounds__(kTcThreads, SWAP ? 2 : 1) gemm_tc_kernel(const
     __shared__ TcShared s;
     uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const uint32_t stage_bytes = kABytes + (uint32_t)a.NB * kChunk;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_uniform((int)(threadIdx.x >> 5)), lane = threadIdx.x & 31;
     const uint32_t tmem_cols = a.acc_stride * 2 <= 32 ? 32u : (a.acc_stride * 2 <= 64 ? 64u : (a.acc_stride * 2 <= 128 ? 128u : (a.acc_stride * 2 <= 256 ? 256u : 512u)));
 
     griddep_launch_dependents();
@@ -303,87 +303,96 @@ __global__ void __launch_bounds__(kTcThreads, SWAP ? 2 : 1) gemm_tc_kernel(const
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem_base = s.tmem_base;
+    const uint32_t tmem_base = warp_uniform(s.tmem_base);
     if (threadIdx.x == 0) tc_mark(a, 1);
     const volatile int* abort_flag = &s.abort_flag;
 
     if (warp == 0) {
-        // ============================== TMA producer ==============================
-        if (lane == 0) {
-            uint32_t npre = 0;
+        // ============================== TMA producer (the warp walks the loop, one lane issues) ==============================
+        {
+            const bool leader = elect_one();
+            int npre = 0;
             if constexpr (!FUSED) {
                 // The weights do not depend on the previous kernel: the first pass over the ring loads them before the
                 // dependency wait (each stage's barrier already expects the whole stage), so under programmatic
                 // dependent launch a ring of weights is on its way while the activation quantizer still runs.
                 PartIter<SWAP> pre(a);
                 Part q;
-                while (npre < (uint32_t)a.stages && pre.next(q))
-                    for (int kc = q.kc0; kc < q.kc1 && npre < (uint32_t)a.stages; ++kc, ++npre) {
+                while (npre < a.stages && pre.next(q))
+                    for (int kc = q.kc0; kc < q.kc1 && npre < a.stages; ++kc, ++npre) {
                         uint8_t* dst = ring + (size_t)npre * stage_bytes;
-                        mbar_expect_tx(&s.full[npre], stage_bytes);
-                        if constexpr (SWAP) tma_load_2d(dst, &maps.w[q.mat], kc * kChunk, q.prow, &s.full[npre]);
-                        else tma_load_2d(dst + kABytes, &maps.w[q.mat], kc * kChunk, q.qrow, &s.full[npre]);
+                        if (leader) {
+                            mbar_expect_tx(&s.full[npre], stage_bytes);
+                            if constexpr (SWAP) tma_load_2d(dst, &maps.w[q.mat], kc * kChunk, q.prow, &s.full[npre]);
+                            else tma_load_2d(dst + kABytes, &maps.w[q.mat], kc * kChunk, q.qrow, &s.full[npre]);
+                        }
                     }
-                tc_mark(a, 2);
+                if (leader) tc_mark(a, 2);
                 griddep_wait();                         // activation codes are written by the previous kernel
             }
             PartIter<SWAP> it(a);
             Part p;
-            uint32_t n = 0;
+            RingPos rp;
             bool ok = true;
             while (ok && it.next(p)) {
-                for (int kc = p.kc0; kc < p.kc1 && ok; ++kc, ++n) {
-                    const int st = n % a.stages;
+                for (int kc = p.kc0; kc < p.kc1; ++kc, rp.next(a.stages)) {
+                    const int st = rp.i;
                     uint8_t* dst = ring + (size_t)st * stage_bytes;
-                    if (FUSED || n >= npre) {
-                        const uint32_t ph = (n / a.stages) & 1;
-                        if (!mbar_wait(&s.empty[st], ph ^ 1, abort_flag, a.wait_ns)) { tc_abort(s, a); ok = false; break; }
-                        mbar_expect_tx(&s.full[st], FUSED ? kABytes : stage_bytes);
-                        if constexpr (SWAP) tma_load_2d(dst, &maps.w[p.mat], kc * kChunk, p.prow, &s.full[st]);
-                        else tma_load_2d(dst + kABytes, &maps.w[p.mat], kc * kChunk, p.qrow, &s.full[st]);
+                    const bool refill = FUSED || --npre < 0;
+                    if (refill) ok = mbar_wait(&s.empty[st], rp.phase ^ 1, abort_flag, a.wait_ns);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) { tc_abort(s, a); break; }
+                    if (leader) {
+                        if (refill) {
+                            mbar_expect_tx(&s.full[st], FUSED ? kABytes : stage_bytes);
+                            if constexpr (SWAP) tma_load_2d(dst, &maps.w[p.mat], kc * kChunk, p.prow, &s.full[st]);
+                            else tma_load_2d(dst + kABytes, &maps.w[p.mat], kc * kChunk, p.qrow, &s.full[st]);
+                        }
+                        if constexpr (!FUSED) {
+                            if constexpr (SWAP) tma_load_2d(dst + kABytes, &maps.a[p.mat], kc * kChunk, p.qrow, &s.full[st]);
+                            else tma_load_2d(dst, &maps.a[p.mat], kc * kChunk, p.prow, &s.full[st]);
+                        }
                     }
-                    if constexpr (!FUSED) {
-                        if constexpr (SWAP) tma_load_2d(dst + kABytes, &maps.a[p.mat], kc * kChunk, p.qrow, &s.full[st]);
-                        else tma_load_2d(dst, &maps.a[p.mat], kc * kChunk, p.prow, &s.full[st]);
-                    }
-                    if (FUSED && n == 0) tc_mark(a, 2);
                 }
             }
-            tc_mark(a, 10);
+            if (leader) tc_mark(a, 10);
             if (!ok) {   // give copies already in flight a bounded time to land before the CTA's memory is released
                 const unsigned long long t0 = global_ns();
                 while (global_ns() - t0 < 2000000ull) {}
             }
         }
     } else if (warp == 1) {
-        // ============================== MMA issuer ==============================
-        if (lane == 0) {
-            const uint32_t idesc = umma_idesc(KIND, kTileP, a.NB);
+        // ============================== MMA issuer (the warp walks the loop, one lane issues) ==============================
+        {
+            const bool leader = elect_one();
+            const uint32_t idesc = umma_idesc(KIND, kTileP, a.NB), ring_addr = warp_uniform(smem_u32(ring));
             PartIter<SWAP> it(a);
             Part p;
-            uint32_t n = 0, pc = 0;
+            RingPos rp, fp;                             // ring stage, accumulator
             bool ok = true;
             while (ok && it.next(p)) {
-                const int buf = pc & 1;
-                if (!mbar_wait(&s.tempty[buf], ((pc >> 1) & 1) ^ 1, abort_flag, a.wait_ns)) { tc_abort(s, a); break; }
+                ok = __all_sync(0xffffffffu, mbar_wait(&s.tempty[fp.i], fp.phase ^ 1, abort_flag, a.wait_ns));
+                if (!ok) { tc_abort(s, a); break; }
                 tc_fence_after_sync();
-                const uint32_t d = tmem_base + (uint32_t)(buf * a.acc_stride);
-                for (int kc = p.kc0; kc < p.kc1; ++kc, ++n) {
-                    const int st = n % a.stages;
-                    if (!mbar_wait(&s.full[st], (n / a.stages) & 1, abort_flag, a.wait_ns)) { tc_abort(s, a); ok = false; break; }
+                const uint32_t d = tmem_base + (uint32_t)(fp.i * a.acc_stride);
+                for (int kc = p.kc0; kc < p.kc1; ++kc, rp.next(a.stages)) {
+                    const int st = rp.i;
+                    ok = __all_sync(0xffffffffu, mbar_wait(&s.full[st], rp.phase, abort_flag, a.wait_ns));
+                    if (!ok) { tc_abort(s, a); break; }
                     tc_fence_after_sync();
-                    if (n == 0) tc_mark(a, 5);
-                    const uint32_t sa = smem_u32(ring + (size_t)st * stage_bytes);
+                    const uint32_t sa = ring_addr + (uint32_t)st * stage_bytes;
                     const uint64_t da = umma_desc_sw128(sa), db = umma_desc_sw128(sa + kABytes);
+                    if (leader) {
 #pragma unroll
-                    for (int k = 0; k < kChunk / 32; ++k)
-                        tc_mma<KIND>(d, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kc > p.kc0 || k > 0) ? 1u : 0u);
-                    tc_commit(&s.empty[st]);            // the stage may be refilled once these MMAs have read it
+                        for (int k = 0; k < kChunk / 32; ++k)
+                            tc_mma<KIND>(d, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kc > p.kc0 || k > 0) ? 1u : 0u);
+                        tc_commit(&s.empty[st]);        // the stage may be refilled once these MMAs have read it
+                        if (kc == p.kc1 - 1) tc_commit(&s.tfull[fp.i]);
+                    }
                 }
-                if (ok) tc_commit(&s.tfull[buf]);
-                ++pc;
+                fp.next(2);
             }
-            tc_mark(a, 6);
+            if (leader) tc_mark(a, 6);
         }
     } else if (warp < 6) {
         // ============================== epilogue ==============================

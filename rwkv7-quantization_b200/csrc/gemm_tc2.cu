@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(kT2Threads, 1) gemm_tc2_kernel(const __grid_co
     extern __shared__ uint8_t smem_raw[];
     __shared__ Tc2Shared s;
     uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_uniform((int)(threadIdx.x >> 5)), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();          // 0 = leader of the pair
     const int pair = (int)(blockIdx.x >> 1), npairs = (int)(gridDim.x >> 1);
     const int total = a.ptiles * a.qtiles;
@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(kT2Threads, 1) gemm_tc2_kernel(const __grid_co
     __syncthreads();
     cluster_sync_all();                               // the peer's barriers exist before anything signals them
     tc_fence_after_sync();
-    const uint32_t tmem_base = s.tmem_base;
+    const uint32_t tmem_base = warp_uniform(s.tmem_base);
     const volatile int* abort_flag = &s.abort_flag;
 
     auto tile_rows = [&](int t, int& mrow, int& nrow) {       // token tiles fastest: the pairs running together share weight tiles
@@ -156,22 +156,26 @@ __global__ void __launch_bounds__(kT2Threads, 1) gemm_tc2_kernel(const __grid_co
     };
 
     if (warp == 0) {
-        // ============================== TMA producer (both CTAs) ==============================
-        if (lane == 0) {
+        // ============================== TMA producer (both CTAs; the warp walks the loop, one lane issues) ==============================
+        {
+            const bool issuer = elect_one();
             griddep_wait();                           // the activation codes come from the previous kernel
-            uint32_t n = 0;
+            RingPos rp;
             bool ok = true;
             for (int t = pair; t < total && ok; t += npairs) {
                 int mrow, nrow;
                 tile_rows(t, mrow, nrow);
-                for (int kc = 0; kc < a.kchunks; ++kc, ++n) {
-                    const int st = n % a.stages;
-                    if (!mbar_wait(&s.empty[st], ((n / a.stages) & 1) ^ 1, abort_flag, a.wait_ns)) { t2_abort(s, a); ok = false; break; }
+                for (int kc = 0; kc < a.kchunks; ++kc, rp.next(a.stages)) {
+                    const int st = rp.i;
+                    ok = __all_sync(0xffffffffu, mbar_wait(&s.empty[st], rp.phase ^ 1, abort_flag, a.wait_ns));
+                    if (!ok) { t2_abort(s, a); break; }
                     uint8_t* dst = ring + (size_t)st * kT2StageBytes;
-                    if (rank == 0) mbar_expect_tx(&s.full[st], 2 * kT2StageBytes);          // the four tiles of the pair
-                    const uint32_t leader_bar = smem_u32(&s.full[st]) & 0xFEFFFFFFu;         // the barrier of the even CTA
-                    tma_load_2d_pair(dst, &maps.a, kc * kT2Chunk, mrow + (int)rank * kT2Rows, leader_bar);
-                    tma_load_2d_pair(dst + kT2TileBytes, &maps.w, kc * kT2Chunk, nrow + (int)rank * kT2Rows, leader_bar);
+                    if (issuer) {
+                        if (rank == 0) mbar_expect_tx(&s.full[st], 2 * kT2StageBytes);          // the four tiles of the pair
+                        const uint32_t leader_bar = smem_u32(&s.full[st]) & 0xFEFFFFFFu;         // the barrier of the even CTA
+                        tma_load_2d_pair(dst, &maps.a, kc * kT2Chunk, mrow + (int)rank * kT2Rows, leader_bar);
+                        tma_load_2d_pair(dst + kT2TileBytes, &maps.w, kc * kT2Chunk, nrow + (int)rank * kT2Rows, leader_bar);
+                    }
                 }
             }
             if (!ok) {      // give copies already in flight a bounded time to land before the CTA's memory is released
@@ -181,27 +185,31 @@ __global__ void __launch_bounds__(kT2Threads, 1) gemm_tc2_kernel(const __grid_co
         }
     } else if (warp == 1) {
         // ============================== MMA issuer (leader CTA only) ==============================
-        if (lane == 0 && rank == 0) {
-            const uint32_t idesc = umma_idesc(KIND, 256, kT2N);
-            uint32_t n = 0, pc = 0;
+        if (rank == 0) {
+            const bool issuer = elect_one();
+            const uint32_t idesc = umma_idesc(KIND, 256, kT2N), ring_addr = warp_uniform(smem_u32(ring));
+            RingPos rp, fp;                                // ring stage, accumulator
             bool ok = true;
-            for (int t = pair; t < total && ok; t += npairs, ++pc) {
-                const int buf = pc & 1;
-                if (!mbar_wait(&s.tempty[buf], ((pc >> 1) & 1) ^ 1, abort_flag, a.wait_ns)) { t2_abort(s, a); break; }
+            for (int t = pair; t < total && ok; t += npairs, fp.next(2)) {
+                ok = __all_sync(0xffffffffu, mbar_wait(&s.tempty[fp.i], fp.phase ^ 1, abort_flag, a.wait_ns));
+                if (!ok) { t2_abort(s, a); break; }
                 tc_fence_after_sync();
-                const uint32_t d = tmem_base + (uint32_t)(buf * kT2N);
-                for (int kc = 0; kc < a.kchunks; ++kc, ++n) {
-                    const int st = n % a.stages;
-                    if (!mbar_wait(&s.full[st], (n / a.stages) & 1, abort_flag, a.wait_ns)) { t2_abort(s, a); ok = false; break; }
+                const uint32_t d = tmem_base + (uint32_t)(fp.i * kT2N);
+                for (int kc = 0; kc < a.kchunks; ++kc, rp.next(a.stages)) {
+                    const int st = rp.i;
+                    ok = __all_sync(0xffffffffu, mbar_wait(&s.full[st], rp.phase, abort_flag, a.wait_ns));
+                    if (!ok) { t2_abort(s, a); break; }
                     tc_fence_after_sync();
-                    const uint32_t sa = smem_u32(ring + (size_t)st * kT2StageBytes);
+                    const uint32_t sa = ring_addr + (uint32_t)st * kT2StageBytes;
                     const uint64_t da = umma_desc_sw128(sa), db = umma_desc_sw128(sa + kT2TileBytes);
+                    if (issuer) {
 #pragma unroll
-                    for (int k = 0; k < kT2Chunk / 32; ++k)
-                        tc_mma_pair<KIND>(d, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kc > 0 || k > 0) ? 1u : 0u);
-                    tc_commit_pair(&s.empty[st]);          // both CTAs may refill the stage once these MMAs have read it
+                        for (int k = 0; k < kT2Chunk / 32; ++k)
+                            tc_mma_pair<KIND>(d, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kc > 0 || k > 0) ? 1u : 0u);
+                        tc_commit_pair(&s.empty[st]);      // both CTAs may refill the stage once these MMAs have read it
+                        if (kc == a.kchunks - 1) tc_commit_pair(&s.tfull[fp.i]);     // both CTAs' epilogues
+                    }
                 }
-                if (ok) tc_commit_pair(&s.tfull[buf]);     // both CTAs' epilogues
             }
         }
     } else if (warp < 6) {

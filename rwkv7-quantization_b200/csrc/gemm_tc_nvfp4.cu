@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(kNfThreads, 1) gemm_tc_nvfp4_kernel(const __gr
     extern __shared__ uint8_t smem_raw[];
     __shared__ NfShared s;
     uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_uniform((int)(threadIdx.x >> 5)), lane = threadIdx.x & 31;
 
     griddep_launch_dependents();
     if (threadIdx.x == 0) {
@@ -99,20 +99,23 @@ __global__ void __launch_bounds__(kNfThreads, 1) gemm_tc_nvfp4_kernel(const __gr
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem_base = s.tmem_base;
+    const uint32_t tmem_base = warp_uniform(s.tmem_base);
     const volatile int* abort_flag = &s.abort_flag;
     const int tiles = a.mtiles * a.ntiles;
     const int64_t k64 = a.K >> 6;
 
     if (warp == 0) {
-        // ============================== producer ==============================
-        if (lane == 0) {
+        // ============================== producer (the warp walks the loop, one lane issues) ==============================
+        {
+            const bool leader = elect_one();
+            RingPos rp;
             // first pass over the ring: the weights and their scales do not depend on the kernels in front, so they are
             // requested BEFORE the dependency wait of programmatic dependent launch
-            uint32_t npre = 0;
-            for (; npre < (uint32_t)a.stages; ++npre) {
-                const int t = blockIdx.x + (int)(npre / (uint32_t)a.kstages) * (int)gridDim.x, kc = (int)(npre % (uint32_t)a.kstages);
+            int npre = 0;
+            for (; npre < a.stages; ++npre) {
+                const int t = blockIdx.x + (npre / a.kstages) * (int)gridDim.x, kc = npre % a.kstages;
                 if (t >= tiles) break;
+                if (!leader) continue;
                 const int nt = t / a.mtiles;
                 uint8_t* dst = ring + (size_t)npre * kStage;
                 mbar_expect_tx(&s.full[npre], kStage);
@@ -123,16 +126,19 @@ __global__ void __launch_bounds__(kNfThreads, 1) gemm_tc_nvfp4_kernel(const __gr
                     bulk_load_1d(sf + kNfSfStage * (1 + h), a.sfw + ((int64_t)(nt * NH + h) * k64 + kc * 4) * kNfSfChunk, kNfSfStage, &s.full[npre]);
             }
             griddep_wait();                     // activation codes and scales come from the previous kernels
-            uint32_t n = 0;
             bool ok = true;
             for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
                 const int mt = t % a.mtiles, nt = t / a.mtiles;
-                for (int kc = 0; kc < a.kstages; ++kc, ++n) {
-                    const int st = n % a.stages;
+                for (int kc = 0; kc < a.kstages; ++kc, rp.next(a.stages)) {
+                    const int st = rp.i;
                     uint8_t* dst = ring + (size_t)st * kStage;
                     uint8_t* sf = dst + kNfABytes + kBBytes;
-                    if (n >= npre) {
-                        if (!mbar_wait(&s.empty[st], ((n / a.stages) & 1) ^ 1, abort_flag, a.wait_ns)) { nf_abort(s, a); ok = false; break; }
+                    const bool refill = --npre < 0;
+                    if (refill) ok = mbar_wait(&s.empty[st], rp.phase ^ 1, abort_flag, a.wait_ns);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) { nf_abort(s, a); break; }
+                    if (!leader) continue;
+                    if (refill) {
                         mbar_expect_tx(&s.full[st], kStage);
                         tma_load_2d(dst + kNfABytes, &maps.w, kc * (int)kNfRowBytes, nt * BN, &s.full[st]);
 #pragma unroll
@@ -150,26 +156,30 @@ __global__ void __launch_bounds__(kNfThreads, 1) gemm_tc_nvfp4_kernel(const __gr
             }
         }
     } else if (warp == 1) {
-        // ============================== MMA issuer ==============================
-        if (lane == 0) {
-            const uint32_t idesc = nvfp4_idesc(BN);
-            uint32_t n = 0, pc = 0;
+        // ============================== MMA issuer (the warp walks the loop, one lane issues) ==============================
+        {
+            const bool leader = elect_one();
+            const uint32_t idesc = nvfp4_idesc(BN), ring_addr = warp_uniform(smem_u32(ring));
+            RingPos rp, fp;                             // ring stage, accumulator
+            uint32_t n = 0;
             bool ok = true;
-            for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++pc) {
-                const int buf = pc % NACC;
-                if (!mbar_wait(&s.tempty[buf], ((pc / NACC) & 1) ^ 1, abort_flag, a.wait_ns)) { nf_abort(s, a); break; }
+            for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, fp.next(NACC)) {
+                ok = __all_sync(0xffffffffu, mbar_wait(&s.tempty[fp.i], fp.phase ^ 1, abort_flag, a.wait_ns));
+                if (!ok) { nf_abort(s, a); break; }
                 tc_fence_after_sync();
-                const uint32_t d = tmem_base + (uint32_t)(buf * BN);
-                for (int kc = 0; kc < a.kstages; ++kc, ++n) {
-                    const int st = n % a.stages;
-                    if (!mbar_wait(&s.full[st], (n / a.stages) & 1, abort_flag, a.wait_ns)) { nf_abort(s, a); ok = false; break; }
+                const uint32_t d = tmem_base + (uint32_t)(fp.i * BN);
+                for (int kc = 0; kc < a.kstages; ++kc, ++n, rp.next(a.stages)) {
+                    const int st = rp.i;
+                    ok = __all_sync(0xffffffffu, mbar_wait(&s.full[st], rp.phase, abort_flag, a.wait_ns));
+                    if (!ok) { nf_abort(s, a); break; }
                     tc_fence_after_sync();
-                    const uint32_t sa = smem_u32(ring + (size_t)st * kStage);
+                    const uint32_t sa = ring_addr + (uint32_t)st * kStage;
                     const uint32_t ssf = sa + kNfABytes + kBBytes;
                     // scale factors of this stage: two alternating column sets, so a copy never lands in columns
                     // the previous stage's MMAs may still be reading
                     const uint32_t tsfa = tmem_base + kNfSfCol + (n & 1) * 64;
                     const uint32_t tsfb = tsfa + 16;
+                    if (!leader) continue;
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
                         tc_cp_sf(tsfa + k * 4, sf_desc(ssf + k * kNfSfChunk));
@@ -183,8 +193,8 @@ __global__ void __launch_bounds__(kNfThreads, 1) gemm_tc_nvfp4_kernel(const __gr
                         tc_mma_nvfp4(d, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, tsfa + k * 4, tsfb + k * (4 * NH),
                                      (kc > 0 || k > 0) ? 1u : 0u);
                     tc_commit(&s.empty[st]);            // the stage may be refilled once these MMAs have read it
+                    if (kc == a.kstages - 1) tc_commit(&s.tfull[fp.i]);
                 }
-                if (ok) tc_commit(&s.tfull[buf]);
             }
         }
     } else {

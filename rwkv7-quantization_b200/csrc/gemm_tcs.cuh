@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(kTcsThreads, 2) gemm_tcs_kernel(const __grid_c
     const uint32_t stage_bytes = kABytes + (uint32_t)a.NB * kChunk + kSfBytes;
     const uint32_t sf_off = kABytes + (uint32_t)a.NB * kChunk;
     T* rxbuf = reinterpret_cast<T*>(ring + (size_t)a.stages * stage_bytes);        // [C][Mt][R]: partial sums per source CTA, token, row
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_uniform((int)(threadIdx.x >> 5)), lane = threadIdx.x & 31;
     const int C = a.qtiles, R = kTileP / C;
     const int rank = (int)tcs_ctarank();
     const int cid = (int)blockIdx.x / C;                     // cluster = (token tile, row tile), row tiles fastest
@@ -143,31 +143,39 @@ __global__ void __launch_bounds__(kTcsThreads, 2) gemm_tcs_kernel(const __grid_c
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem_base = s.tmem_base;
+    const uint32_t tmem_base = warp_uniform(s.tmem_base);
     tcs_cluster_arrive();            // this CTA's barriers exist; the matching wait comes just before the exchange
     if (threadIdx.x == 0) tc_mark(a, 1);
 
     if (warp == 0) {
-        // ============================== TMA producer ==============================
-        if (lane == 0) {
+        // ============================== TMA producer (the warp walks the loop, one lane issues) ==============================
+        {
+            const bool leader = elect_one();
             const int npre = min(total, a.stages);
             const int64_t k64 = (int64_t)a.kchunks * 4;          // NVFP4: 512-byte scale chunks (128 rows x 64 k) per row tile
             for (int n = 0; n < npre; ++n) {           // weights first: they do not depend on the previous kernel
                 const int mat = n / nk, kc = kc0 + (n - mat * nk);
+                if (!leader) continue;
                 mbar_expect_tx(&s.full[n], stage_bytes);
                 tma_load_2d(ring + (size_t)n * stage_bytes, &maps.w[mat], kc * kChunk, prow, &s.full[n]);
                 if constexpr (KIND == KIND_NF4)
                     bulk_load_1d(ring + (size_t)n * stage_bytes + sf_off, a.sfw + ((int64_t)(prow / kTileP) * k64 + kc * 4) * kNfSfChunk, kNfSfStage, &s.full[n]);
             }
-            tc_mark(a, 2);
+            if (leader) tc_mark(a, 2);
             griddep_wait();                            // the activation codes are written by the previous kernel
-            tc_mark(a, 3);
-            for (int n = 0; n < total; ++n) {
-                const int st = n % a.stages;
-                const int mat = n / nk, kc = kc0 + (n - mat * nk);
+            if (leader) tc_mark(a, 3);
+            RingPos rp;
+            int mat = 0, kc = kc0;
+            bool ok = true;
+            for (int n = 0; n < total; ++n, rp.next(a.stages), ++kc) {
+                if (kc == kc1) { kc = kc0; ++mat; }
+                const int st = rp.i;
                 uint8_t* dst = ring + (size_t)st * stage_bytes;
+                if (n >= npre) ok = mbar_wait(&s.empty[st], rp.phase ^ 1, abort_flag, a.wait_ns);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) { tcs_abort(s, a); break; }
+                if (!leader) continue;
                 if (n >= npre) {
-                    if (!mbar_wait(&s.empty[st], ((n / a.stages) & 1) ^ 1, abort_flag, a.wait_ns)) { tcs_abort(s, a); break; }
                     mbar_expect_tx(&s.full[st], stage_bytes);
                     tma_load_2d(dst, &maps.w[mat], kc * kChunk, prow, &s.full[st]);
                     if constexpr (KIND == KIND_NF4)
@@ -177,18 +185,23 @@ __global__ void __launch_bounds__(kTcsThreads, 2) gemm_tcs_kernel(const __grid_c
                 if constexpr (KIND == KIND_NF4)
                     bulk_load_1d(dst + sf_off + kNfSfStage, a.sfa + ((int64_t)(m0 / kNfTileM) * k64 + kc * 4) * kNfSfChunk, kNfSfStage, &s.full[st]);
             }
-            tc_mark(a, 10);
+            if (leader) tc_mark(a, 10);
         }
     } else if (warp == 1) {
-        // ============================== MMA issuer ==============================
-        if (lane == 0) {
-            const uint32_t idesc = KIND == KIND_NF4 ? nvfp4_idesc(a.NB) : umma_idesc(KIND, kTileP, a.NB);
-            for (int n = 0; n < total; ++n) {
-                const int st = n % a.stages;
-                const int mat = n / nk, i = n - mat * nk;
-                if (!mbar_wait(&s.full[st], (n / a.stages) & 1, abort_flag, a.wait_ns)) { tcs_abort(s, a); break; }
+        // ============================== MMA issuer (the warp walks the loop, one lane issues) ==============================
+        {
+            const bool leader = elect_one();
+            const uint32_t idesc = KIND == KIND_NF4 ? nvfp4_idesc(a.NB) : umma_idesc(KIND, kTileP, a.NB), ring_addr = warp_uniform(smem_u32(ring));
+            RingPos rp;
+            int mat = 0, i = 0;
+            for (int n = 0; n < total; ++n, rp.next(a.stages), ++i) {
+                if (i == nk) { i = 0; ++mat; }
+                const int st = rp.i;
+                const bool ok = __all_sync(0xffffffffu, mbar_wait(&s.full[st], rp.phase, abort_flag, a.wait_ns));
+                if (!ok) { tcs_abort(s, a); break; }
                 tc_fence_after_sync();
-                const uint32_t sa = smem_u32(ring + (size_t)st * stage_bytes);
+                if (!leader) continue;
+                const uint32_t sa = ring_addr + (uint32_t)st * stage_bytes;
                 const uint64_t da = umma_desc_sw128(sa), db = umma_desc_sw128(sa + kABytes);
                 const uint32_t d = tmem_base + (uint32_t)(mat * a.acc_stride);
                 if constexpr (KIND == KIND_NF4) {
@@ -213,10 +226,10 @@ __global__ void __launch_bounds__(kTcsThreads, 2) gemm_tcs_kernel(const __grid_c
                 if (i == nk - 1) tc_commit(&s.tfull[mat]);
                 if (n == 0) tc_mark(a, 5);
             }
-            tc_mark(a, 6);
+            if (leader) tc_mark(a, 6);
         }
     }
-    __syncwarp();                    // single-lane roles: the other lanes wait here for their lane 0
+    __syncwarp();
     tcs_cluster_wait();              // every CTA of the cluster has initialised its barriers
     if (warp < 2) tcs_cluster_arrive();      // these warps never touch a peer's shared memory (the epilogue warps arrive after their last store)
 

@@ -158,17 +158,6 @@ struct W16Tile {
     static_assert(kSmem <= kW16SmemBudget, "ring");
 };
 
-// place in a ring of S slots and the parity of its current round.  Counted, not computed: a division by a run-time
-// stage count costs each role 250 clocks a step, as much as a third of the step's MMAs.
-template <int S>
-struct RingPos {
-    int i = 0;
-    uint32_t phase = 0;
-    __device__ __forceinline__ void next() {
-        if (++i == S) { i = 0; phase ^= 1; }
-    }
-};
-
 template <int FMT, int NB>
 __global__ void __launch_bounds__(kW16Threads, 1) gemm_wa16_kernel(const __grid_constant__ W16Maps maps, const W16Args a) {
     using TL = W16Tile<FMT, NB>;
@@ -239,12 +228,12 @@ __global__ void __launch_bounds__(kW16Threads, 1) gemm_wa16_kernel(const __grid_
             }
             griddep_wait();
             bool ok = true;
-            RingPos<TL::kS> rp;
-            RingPos<TL::kXS> xp;
+            RingPos rp;
+            RingPos xp;
             for (int t = blockIdx.x; t < items && ok; t += gridDim.x) {
                 const Item it = item_of(t);
                 const float* xsrc = kGroup ? a.xsum + ((int64_t)it.mt * a.groups + it.k0) * NB : nullptr;
-                for (int k = it.k0; k < it.k1; ++k, rp.next(), xp.next()) {
+                for (int k = it.k0; k < it.k1; ++k, rp.next(TL::kS), xp.next(TL::kXS)) {
                     const int st = rp.i;
                     uint8_t* dst = ring + (size_t)st * TL::kStage;
                     const bool refill = --npre < 0;
@@ -272,13 +261,13 @@ __global__ void __launch_bounds__(kW16Threads, 1) gemm_wa16_kernel(const __grid_
         {
             const bool leader = elect_one();
             const uint32_t idesc = (1u << 4) | ((uint32_t)(NB >> 3) << 17) | (8u << 24);      // f32 += f16 * f16, both K-major, M = 128
-            RingPos<TL::kS> rp;
-            RingPos<2> fp;                          // accumulator fill
+            RingPos rp;
+            RingPos fp;                          // accumulator fill
             const uint32_t ring_addr = warp_uniform(smem_u32(ring));
             bool ok = true;
             for (int t = blockIdx.x; t < items && ok; t += gridDim.x) {
                 const Item it = item_of(t);
-                for (int k = it.k0; k < it.k1; ++k, rp.next()) {
+                for (int k = it.k0; k < it.k1; ++k, rp.next(TL::kS)) {
                     const int st = rp.i;
                     const bool fresh = kGroup || k == it.k0;
                     ok = (!fresh || mbar_wait(&s.dempty[fp.i], fp.phase ^ 1, abort_flag, a.wait_ns)) && mbar_wait(&s.full[st], rp.phase, abort_flag, a.wait_ns) &&
@@ -297,7 +286,7 @@ __global__ void __launch_bounds__(kW16Threads, 1) gemm_wa16_kernel(const __grid_
                         tc_commit(&s.empty[st]);
                         if (last) tc_commit(&s.dfull[fp.i]);
                     }
-                    if (last) fp.next();
+                    if (last) fp.next(2);
                 }
             }
         }
@@ -307,11 +296,11 @@ __global__ void __launch_bounds__(kW16Threads, 1) gemm_wa16_kernel(const __grid_
         // ============================== weights: packed -> fp16 in tensor memory ==============================
         const uint32_t lane_addr = tmem_base + TL::kACol + ((uint32_t)(warp * 32) << 16);
         const int row = warp * 32 + lane;
-        RingPos<TL::kS> rp;
+        RingPos rp;
         bool ok = true;
         for (int t = blockIdx.x; t < items && ok; t += gridDim.x) {
             const Item it = item_of(t);
-            for (int k = it.k0; k < it.k1; ++k, rp.next()) {
+            for (int k = it.k0; k < it.k1; ++k, rp.next(TL::kS)) {
                 const int st = rp.i;
                 ok = mbar_wait(&s.full[st], rp.phase, abort_flag, a.wait_ns);
                 ok = __all_sync(0xffffffffu, ok);           // the tensor-memory stores are warp-wide
@@ -356,8 +345,8 @@ __global__ void __launch_bounds__(kW16Threads, 1) gemm_wa16_kernel(const __grid_
         constexpr int CH = NH % 32 == 0 ? 32 : 16;       // tensor-memory columns per load
         const int q = warp & 3, half = (warp - 4) >> 2;
         const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16) + half * NH;
-        RingPos<TL::kXS> xp;
-        RingPos<2> fp;
+        RingPos xp;
+        RingPos fp;
         bool ok = true;
         for (int t = blockIdx.x; t < items && ok; t += gridDim.x) {
             const Item it = item_of(t);
@@ -387,7 +376,7 @@ __global__ void __launch_bounds__(kW16Threads, 1) gemm_wa16_kernel(const __grid_
                 };
                 load4(it.k0, s4n, z4n);
 #pragma unroll 1
-                for (int k = it.k0; k < it.k1; ++k, xp.next(), fp.next()) {
+                for (int k = it.k0; k < it.k1; ++k, xp.next(TL::kXS), fp.next(2)) {
                     const int j4 = k & 3;                // k0 is a multiple of 4
                     if (j4 == 0) {
                         s4 = s4n;
@@ -440,7 +429,7 @@ __global__ void __launch_bounds__(kW16Threads, 1) gemm_wa16_kernel(const __grid_
                 tc_fence_before_sync();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&s.dempty[fp.i]);
-                fp.next();
+                fp.next(2);
             }
             // a warp's 32 lanes are 32 neighbouring weight rows: 64 (fp16) or 128 (fp32) contiguous bytes per token
             if (row < a.N) {

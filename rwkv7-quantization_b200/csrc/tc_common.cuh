@@ -27,6 +27,16 @@ __device__ __forceinline__ bool elect_one() {
     return r != 0;
 }
 
+// Place in a ring and the parity of its current round.  Counted, not computed: `n % stages` and `n / stages` with a stage
+// count known at run time only cost each role about 250 clocks a step, as much as half of a step's MMAs.
+struct RingPos {
+    int i = 0;
+    uint32_t phase = 0;
+    __device__ __forceinline__ void next(int slots) {
+        if (++i == slots) { i = 0; phase ^= 1; }
+    }
+};
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
