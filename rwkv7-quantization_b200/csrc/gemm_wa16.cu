@@ -96,10 +96,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
         : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ uint32_t h2_sub(uint32_t v, uint32_t c) {
-    const __half2 r = __hsub2(*reinterpret_cast<const __half2*>(&v), *reinterpret_cast<const __half2*>(&c));
-    return *reinterpret_cast<const uint32_t*>(&r);
-}
 // 8 nibbles of a word -> four fp16 pairs (n0,n4) * 2^-24, (n1,n5) * 2^-20, (n2,n6) * 2^-24, (n3,n7) * 2^-20
 __device__ __forceinline__ void widen_nibbles(uint32_t w, uint32_t* o) {
     const uint32_t h = w >> 8;
@@ -107,12 +103,6 @@ __device__ __forceinline__ void widen_nibbles(uint32_t w, uint32_t* o) {
     o[1] = w & 0x00F000F0u;
     o[2] = h & 0x000F000Fu;
     o[3] = h & 0x00F000F0u;
-}
-// 4 signed bytes -> two fp16 pairs in order: byte ^ 0x80 = b + 128 in the mantissa of 1024, minus 1152
-__device__ __forceinline__ void widen_bytes(uint32_t w, uint32_t* o) {
-    const uint32_t u = w ^ 0x80808080u;
-    o[0] = h2_sub(__byte_perm(u, 0x64646464u, 0x4140), 0x64806480u);
-    o[1] = h2_sub(__byte_perm(u, 0x64646464u, 0x4342), 0x64806480u);
 }
 __device__ __forceinline__ uint64_t pack2(float lo, float hi) {
     uint64_t r;
@@ -323,10 +313,10 @@ __global__ void __launch_bounds__(kW16Threads, 1) gemm_wa16_kernel(const __grid_
 #pragma unroll
                         for (int c = 0; c < 4; ++c) {        // 128-byte swizzle: piece p at p ^ (r % 8)
                             const uint4 v = *reinterpret_cast<const uint4*>(wrow + (((h * 4 + c) ^ (row & 7)) << 4));
-                            widen_bytes(v.x, r + c * 8);
-                            widen_bytes(v.y, r + c * 8 + 2);
-                            widen_bytes(v.z, r + c * 8 + 4);
-                            widen_bytes(v.w, r + c * 8 + 6);
+                            s8x4_to_f16x4(v.x, r + c * 8);
+                            s8x4_to_f16x4(v.y, r + c * 8 + 2);
+                            s8x4_to_f16x4(v.z, r + c * 8 + 4);
+                            s8x4_to_f16x4(v.w, r + c * 8 + 6);
                         }
                     }
                     tmem_st32(lane_addr + (uint32_t)st * 64 + h * 32, r);

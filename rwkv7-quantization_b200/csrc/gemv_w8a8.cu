@@ -71,10 +71,13 @@ __device__ __forceinline__ void issue_slots(uint32_t dst, const uint8_t* src0, c
 // registers are consecutive pairs of two 128-bit loads.  INT8: two m16n8k32 per unit, B from one 128-bit load.
 // FP8 on pre-quantized codes (WIDE = false): the tile holds the e4m3 codes as they come (1 byte each), a lane's 16 codes of
 // a unit arrive with one 128-bit load and are widened here (8 conversions per token tile and unit).
+// int8 weights and fp16 activations: units at and beyond `nv` are skipped -- their weights are zeros, but the activations
+// behind them belong to other k or other tokens, and zero times an infinity would be a NaN.
 template <int QT, bool WIDE, int NT, int D, typename T>
-__device__ __forceinline__ void chunk_body(const uint8_t* st, const uint8_t* const (&xb)[NT], T (&c)[NT][4], T (&c2)[NT][4]) {
+__device__ __forceinline__ void chunk_body(const uint8_t* st, const uint8_t* const (&xb)[NT], T (&c)[NT][4], T (&c2)[NT][4], int nv) {
 #pragma unroll
     for (int j = 0; j < D; ++j) {
+        if (QT == QT_W8F16 && j >= nv) break;
         const uint4 wg = *reinterpret_cast<const uint4*>(st + j * 1024);
         const uint4 wh = *reinterpret_cast<const uint4*>(st + j * 1024 + 512);
         if constexpr (QT == QT_FP8) {
@@ -95,6 +98,22 @@ __device__ __forceinline__ void chunk_body(const uint8_t* st, const uint8_t* con
                 mma_f16(c2[i], g01.z, h01.z, g01.w, h01.w, b0.z, b0.w);
                 mma_f16(c[i], g23.x, h23.x, g23.y, h23.y, b1.x, b1.y);
                 mma_f16(c2[i], g23.z, h23.z, g23.w, h23.w, b1.z, b1.w);
+            }
+        } else if constexpr (QT == QT_W8F16) {
+            const uint32_t wgw[4] = {wg.x, wg.y, wg.z, wg.w}, whw[4] = {wh.x, wh.y, wh.z, wh.w};
+            uint32_t gf[8], hf[8];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                s8x4_to_f16x4(wgw[q], gf + 2 * q);
+                s8x4_to_f16x4(whw[q], hf + 2 * q);
+            }
+#pragma unroll
+            for (int i = 0; i < NT; ++i) {
+                const uint4 b0 = *reinterpret_cast<const uint4*>(xb[i] + j * 128), b1 = *reinterpret_cast<const uint4*>(xb[i] + j * 128 + 16);
+                mma_f16(c[i], gf[0], hf[0], gf[1], hf[1], b0.x, b0.y);
+                mma_f16(c2[i], gf[2], hf[2], gf[3], hf[3], b0.z, b0.w);
+                mma_f16(c[i], gf[4], hf[4], gf[5], hf[5], b1.x, b1.y);
+                mma_f16(c2[i], gf[6], hf[6], gf[7], hf[7], b1.z, b1.w);
             }
         } else {
 #pragma unroll
@@ -126,7 +145,7 @@ __device__ __forceinline__ void store_tile(const W8Args& a, int mat, int n0, int
             const int m = i * 8 + 2 * t + (j & 1), n = n0 + g + ((j & 2) ? 8 : 0);
             if (m >= a.M || n >= a.N) continue;
             float f;
-            if constexpr (QT == QT_FP8) {
+            if constexpr (QT != QT_INT8) {
                 f = c[i][j] * ((j & 2) ? out_hi : out_lo);
             } else {
                 if (a.acc[mat]) a.acc[mat][(int64_t)m * a.ldacc + n] = c[i][j];
@@ -161,7 +180,7 @@ __global__ void __launch_bounds__(kThr, 2) gemv_w8a8_kernel(const W8Args a) {
     using T = typename Acc<QT>::T;
     constexpr int D = kGemvD;
     constexpr bool WIDE = !PRE;
-    constexpr int AB = (QT == QT_FP8 && WIDE) ? 2 : 1;          // bytes per activation in the shared-memory tile
+    constexpr int AB = (QT != QT_INT8 && WIDE) ? 2 : 1;          // bytes per activation in the shared-memory tile
     extern __shared__ __align__(128) uint8_t smem[];
     // layout: red[kWarps][NT*4][32] | xs[32] | sh[8] | xbar + pad (96 B) | ring[kWarps][S][D][2][32 lanes] x 16 B | xq[M][pitch] + 512 B
     T* red = reinterpret_cast<T*>(smem);
@@ -235,7 +254,7 @@ __global__ void __launch_bounds__(kThr, 2) gemv_w8a8_kernel(const W8Args a) {
     for (int i = 0; i < NT; ++i) xb0[i] = xq + min(i * 8 + g, a.M - 1) * a.pitch + kbeg * AB;
     const float wscale = a.ws[mat][0];       // weights and their scale are never written by a kernel
 
-    if ((QT == QT_FP8 || PRE) && threadIdx.x == 0) {
+    if ((QT != QT_INT8 || PRE) && threadIdx.x == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((uint32_t)__cvta_generic_to_shared(xbar)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -261,6 +280,22 @@ __global__ void __launch_bounds__(kThr, 2) gemv_w8a8_kernel(const W8Args a) {
         } else {
             if ((int)threadIdx.x < a.M) xs[threadIdx.x] = a.ascale[mat][threadIdx.x];
         }
+        if (!w8_staged_or_report(xbar, a.status, a.wait_ns)) {     // reported: drain the weight ring and stop
+            cp_async_wait<0>();
+            return;
+        }
+    } else if constexpr (QT == QT_W8F16) {
+        // nothing to quantize: the fp16 rows go into the tile as they are
+        if (threadIdx.x == 0) {
+            const uint32_t b = (uint32_t)__cvta_generic_to_shared(xbar);
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"((uint32_t)(a.M * a.K * 2)) : "memory");
+#pragma unroll 1
+            for (int r = 0; r < a.M; ++r)
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                             ::"r"((uint32_t)__cvta_generic_to_shared(xq + (size_t)r * a.pitch)),
+                               "l"(reinterpret_cast<const char*>(a.x[mat]) + (int64_t)r * a.ldx * 2), "r"((uint32_t)(a.K * 2)), "r"(b) : "memory");
+        }
+        out_scale = 1.f;
         if (!w8_staged_or_report(xbar, a.status, a.wait_ns)) {     // reported: drain the weight ring and stop
             cp_async_wait<0>();
             return;
@@ -306,7 +341,7 @@ __global__ void __launch_bounds__(kThr, 2) gemv_w8a8_kernel(const W8Args a) {
             for (int ch = 0; ch < nch; ++ch) {
                 issue();                       // keep S-1 chunks in flight
                 cp_async_wait<S - 1>();        // this lane's copies of the current chunk have landed
-                chunk_body<QT, WIDE, NT, D>(my_ring + stage * (D * 1024), xb, c, c2);
+                chunk_body<QT, WIDE, NT, D>(my_ring + stage * (D * 1024), xb, c, c2, ue - ub - ch * D);
 #pragma unroll
                 for (int i = 0; i < NT; ++i) xb[i] += D * 64 * AB;
                 if (++stage == S) stage = 0;
@@ -468,6 +503,16 @@ static int32_t dispatch_mt(const W8Args& a, cudaStream_t st) {
 
 static int pitch_codes(int K) { return ((K + 127) / 128) * 128 + 64; }     // 1 byte per code
 static int pitch_wide(int K) { return ((2 * K + 127) / 128) * 128 + 16; }  // f16 values of the e4m3 codes
+
+bool gemv_w8f16_fits(int M, int K) {
+    return M > 0 && M <= 16 && K > 0 && K % 16 == 0 && smem_bytes(M <= 8 ? 1 : 2, M, pitch_wide(K), 2) <= kFusedSmemMax;
+}
+int32_t gemv_w8f16_run(W8Args a, cudaStream_t st, const char* who) {
+    RWKVQ_REQUIRE(gemv_w8f16_fits(a.M, a.K), RWKVQ_E_SHAPE, "%s: M=%d K=%d do not fit the decode kernel", who, a.M, a.K);
+    a.nmat = 1;
+    a.pitch = pitch_wide(a.K);
+    return a.M <= 8 ? dispatch_s<QT_W8F16, RWKVQ_F16, 1, false>(a, st) : dispatch_s<QT_W8F16, RWKVQ_F16, 2, false>(a, st);
+}
 
 bool gemv_codes_fits(int M, int K) {
     const int NT = M <= 8 ? 1 : (M <= 16 ? 2 : 4);

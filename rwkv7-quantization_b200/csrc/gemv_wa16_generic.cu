@@ -1,9 +1,9 @@
 // Weight-only quantized GEMV (fp16 activations, M <= 16 rows) for every stand-alone INT4 / INT8 layout of the
-// reference: one warp per output row, 8 weights per lane and step (one 32-bit load of nibbles or one 64-bit load
+// reference (per-tensor INT8 rows of 16-byte vectors go to the streaming decode kernel instead): one warp per output row, 8 weights per lane and step (one 32-bit load of nibbles or one 64-bit load
 // of bytes), weights dequantized in registers exactly as the reference kernels spell it, fp32 accumulation,
 // warp-shuffle reduction.  This is the general kernel (any group size, affine layouts, padded K); the group-wise
 // INT4 decode path of the 7.2B shapes has its own tensor-core kernel in gemv_int4.cu and is cross-checked by this.
-#include "common.cuh"
+#include "w8a8.cuh"
 
 namespace rwkvq {
 
@@ -157,8 +157,23 @@ int32_t rwkvq_gemv_int4_group_generic(const void* x_f16, int64_t ldx, const uint
     return run_wa16(a, WA_INT4_GROUP, (cudaStream_t)stream, "gemv_int4_group_generic");
 }
 
+int32_t rwkvq_gemv_int8_w8a16_streams(int64_t M, int64_t K) {
+    return M > 0 && M <= kWaMaxM && K > 0 && K < (int64_t(1) << 30) && gemv_w8f16_fits((int)M, (int)K) ? 1 : 0;
+}
+
 int32_t rwkvq_gemv_int8_w8a16(const void* x_f16, int64_t ldx, const int8_t* w, int64_t ldw, const float* scale,
                               void* out_f16, int64_t ldo, int64_t M, int64_t N, int64_t K, void* stream) {
+    // Rows that are 16-byte vectors take the decode kernel of the W8A8 path (weights streamed through per-warp cp.async
+    // rings, widened to fp16 for mma.sync); the row kernel below, one 64-bit load in flight per lane, keeps the others.
+    // Bound by HBM.  Measured, us (graph, rotated weights), row kernel -> here: [2560, 2560] 3 rows 19 -> 3.5, [10240, 2560]
+    // 40 -> 7.5, [2560, 10240] 66 -> 8.2; [16384, 4096] 1 row 14.9 (4.5 TB/s), 16 rows 17.2; [4096, 4096] 8 rows 5.4.
+    if (x_f16 && w && scale && out_f16 && N > 0 && N < (int64_t(1) << 30) && rwkvq_gemv_int8_w8a16_streams(M, K) &&
+        ldw % 16 == 0 && ldw >= K && aligned16(w) && aligned16(x_f16) && ldx % 8 == 0 && ldx >= K && ldo >= N) {
+        W8Args b{};
+        b.x[0] = x_f16; b.w[0] = (const uint8_t*)w; b.ws[0] = scale; b.out[0] = (__half*)out_f16;
+        b.ldx = ldx; b.ldw = ldw; b.ldo = ldo; b.M = (int)M; b.N = (int)N; b.K = (int)K;
+        return gemv_w8f16_run(b, (cudaStream_t)stream, "gemv_int8_w8a16");
+    }
     WaArgs a{};
     a.x = (const __half*)x_f16; a.w = (const uint8_t*)w; a.scales = scale; a.out = (__half*)out_f16;
     a.ldx = ldx; a.ldw = ldw; a.ldo = ldo; a.M = (int)M; a.N = (int)N; a.K = (int)K;

@@ -9,7 +9,7 @@ constexpr int kWarps = 8;
 constexpr int kThr = kWarps * 32;
 constexpr int kUnroll = 4;   // any-M kernel: 64-byte units in flight per lane
 
-enum { QT_FP8 = 0, QT_INT8 = 1 };
+enum { QT_FP8 = 0, QT_INT8 = 1, QT_W8F16 = 2 };    // QT_W8F16: int8 weights, fp16 activations taken as they are
 
 // Programmatic dependent launch: a kernel may start while its predecessor in the stream drains.  Everything
 // before griddep_wait() may only touch data no earlier kernel writes (here: the weights).
@@ -414,6 +414,23 @@ __device__ void quantize_int8_to_smem(const W8Args& a, int mat, uint8_t* xq, flo
         }
     }
 }
+
+// 4 signed bytes -> two fp16 pairs in order, exact: byte ^ 0x80 = b + 128 in the low mantissa bits of 1024, minus 1152
+__device__ __forceinline__ void s8x4_to_f16x4(uint32_t w, uint32_t* o) {
+    constexpr uint32_t k1152 = 0x64806480u;
+    const uint32_t u = w ^ 0x80808080u;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const uint32_t v = __byte_perm(u, 0x64646464u, i ? 0x4342 : 0x4140);
+        const __half2 r = __hsub2(*reinterpret_cast<const __half2*>(&v), *reinterpret_cast<const __half2*>(&k1152));
+        o[i] = *reinterpret_cast<const uint32_t*>(&r);
+    }
+}
+
+// int8 weights times fp16 activations on the same kernel: a.x[0], a.w[0], a.ws[0], a.out[0], M <= 16.  gemv_w8f16_fits: the
+// activation tile has room beside a weight ring.
+bool gemv_w8f16_fits(int M, int K);
+int32_t gemv_w8f16_run(W8Args a, cudaStream_t st, const char* who);
 
 // The decode GEMV on pre-quantized codes (gemv_w8a8.cu): a.codes / a.ascale / a.w / a.ws / a.out filled for a.nmat
 // matrices, M <= 32.  Returns RWKVQ_E_SHAPE without launching when the code tile does not fit shared memory.

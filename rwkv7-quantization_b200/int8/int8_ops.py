@@ -27,8 +27,23 @@ def load_int8_weight(z: dict, key: str, dev: str = "cuda"):
     raise KeyError(f"No INT8 weight found for key: {key}")
 
 
-TC_ROWS = 17        # rows from which the tensor-core GEMM takes over (the row kernel takes 16 per pass over the weights)
+TC_ROWS = 17        # rows from which the tensor-core GEMM takes over (the decode kernel takes 16 per pass over the weights)
 TC_MIN_N = 512
+_streams: dict = {}
+
+
+def _takes_tc(m: int, n: int, k: int) -> bool:
+    """Measured, us, decode kernel / tensor-core GEMM: [4096, 4096] 16 rows 6.5 / 9.9, [16384, 4096] 16 rows 17.2 / 19.3,
+    [512, 4096] 16 rows 4.3 / 6.6.  Blocks too large for the decode kernel's shared memory ([2560, 10240] from 7 rows,
+    [4096, 16384] from 5) run the GEMM, 11.7 and 20.4, not the row kernel, 94 and 117."""
+    if n < TC_MIN_N or k % 16:
+        return False
+    if m >= TC_ROWS:
+        return True
+    fits = _streams.get((m, k))
+    if fits is None:
+        fits = _streams[(m, k)] = m < 1 or bool(abi.lib().rwkvq_gemv_int8_w8a16_streams(m, k))
+    return not fits
 
 
 def _tensor_core(x2, w, scale):
@@ -50,7 +65,7 @@ def linear_int8_per_tensor(x, weight_info, out_dtype=torch.float16):
     n, k = w.shape
     x2 = _rows_f16(x, k)
     scale = _f32(weight_info["tensor_scale"].reshape(1), x2.device)
-    if x2.shape[0] >= TC_ROWS and n >= TC_MIN_N and k % 16 == 0 and w.data_ptr() % 16 == 0:
+    if w.data_ptr() % 16 == 0 and _takes_tc(x2.shape[0], n, k):
         return _tensor_core(x2, w, scale).to(out_dtype).reshape(*x.shape[:-1], n)
     out = _run_rows(x2, n, lambda xc, oc, m: abi.call(
         "rwkvq_gemv_int8_w8a16", xc.data_ptr(), k, w.data_ptr(), w.stride(0), scale.data_ptr(), oc.data_ptr(), n, m, n, k,

@@ -70,6 +70,7 @@ SIGNATURES = {
     "rwkvq_gemv_int4_tensor": [_p, _i64, _p, _i64, _p, _p, _i64, _i64, _i64, _i64, _p],
     "rwkvq_gemv_int4_affine": [_p, _i64, _p, _i64, _p, _p, _p, _p, _p, _i64, _i64, _i64, _i64, _p],
     "rwkvq_gemv_int4_group_generic": [_p, _i64, _p, _i64, _p, _p, _i32, _i32, _p, _i64, _i64, _i64, _i64, _p],
+    "rwkvq_gemv_int8_w8a16_streams": [_i64, _i64],
     "rwkvq_gemv_int8_w8a16": [_p, _i64, _p, _i64, _p, _p, _i64, _i64, _i64, _i64, _p],
     "rwkvq_gemv_int8_affine": [_p, _i64, _p, _i64, _p, _p, _p, _p, _p, _i64, _i64, _i64, _i64, _p],
     "rwkvq_gemv_int4_group_smem_bytes": [_i64, _i64],

@@ -67,12 +67,27 @@ def test_int8_w8a16_many_rows(m, n, k):
     assert torch.equal(out, int8_ops.linear_int8(x.cuda(), d))
 
 
-def test_infinite_and_nan_activations_stay_in_their_row():
+# the streaming decode kernel: token tiles of 8 and their remainders, K ranges of a warp that end inside a chunk (K = 2560,
+# 2320) and inside a 64-byte unit (K = 16, 336), row tiles with a remainder, blocks that no longer fit (tensor-core GEMM)
+@pytest.mark.parametrize("m,n,k", [(1, 16384, 4096), (1, 40, 16), (3, 2560, 2560), (8, 1000, 336), (9, 777, 2320), (16, 4096, 4096),
+                                   (6, 512, 10240), (7, 512, 10240), (5, 520, 16384)])
+def test_int8_w8a16_few_rows(m, n, k):
     from int8 import int8_ops, quantize_int8
-    q, s = quantize_int8.quantize_to_int8_per_tensor(gen(1, (640, 256), 0.05))
-    x = gen(2, (40, 256)).half()
-    x[3, 7], x[39, 255] = float("inf"), float("nan")
+    q, s = quantize_int8.quantize_to_int8_per_tensor(gen(n + k, (n, k), k ** -0.5))
+    d = {"weight": q.cuda(), "tensor_scale": s.cuda(), "qtype": "int8_per_tensor"}
+    x = gen(m, (m, k)).half()
+    out = int8_ops.linear_int8(x.cuda(), d)
+    check(out, x, [q.double() * s.double()])
+    assert torch.equal(out, int8_ops.linear_int8(x.cuda(), d))
+
+
+@pytest.mark.parametrize("m,k", [(40, 256), (6, 2320), (16, 336)])
+def test_infinite_and_nan_activations_stay_in_their_row(m, k):
+    from int8 import int8_ops, quantize_int8
+    q, s = quantize_int8.quantize_to_int8_per_tensor(gen(1, (640, k), 0.05))
+    x = gen(2, (m, k)).half()
+    x[3, 0], x[m - 1, k - 1] = float("inf"), float("nan")
     out = int8_ops.linear_int8(x.cuda(), {"weight": q.cuda(), "tensor_scale": s.cuda(), "qtype": "int8_per_tensor"}).cpu()
-    ok = [i for i in range(40) if i not in (3, 39)]
+    ok = [i for i in range(m) if i not in (3, m - 1)]
     check(out[ok], x[ok], [q.double() * s.double()])
-    assert not bool(out[3].isfinite().any()) and bool(out[39].isnan().all())
+    assert not bool(out[3].isfinite().any()) and bool(out[m - 1].isnan().all())
