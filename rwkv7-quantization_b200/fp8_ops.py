@@ -42,12 +42,16 @@ def linear_fp8(x, weight_info, out_dtype=torch.float16, push=None):
     m, k = x2.shape
     n = w.shape[0]
     dev = x2.device
+    out = abi.new_out(m, n, dev)
+    if push is None and f.ROUTE != "mma" and f._ACTQ_FUSED and k % 8 == 0 and m > 0:
+        # inv = 448/amax and scale = amax/448 the way torch evaluates them on a GPU in prep_x_fp8 (DIV_TORCH)
+        f._linear(abi.LINEAR_FP8, (x2,), (f._u8(w),), (w_ts,), (out.data_ptr(),), out.stride(0), m, n, k, 0, abi.DIV_TORCH, abi.DIV_IEEE,
+                  abi.FLAG_AMAX_AFTER_BF16 | abi.FLAG_QUANT_FROM_BF16, abi.FLAG_OUT_VIA_BF16 | f._wscale_flag(w_ts, n), 1)
+        return f._finish(out, x.shape[:-1], n, out_dtype)
     codes = torch.empty((m, k), dtype=torch.uint8, device=dev)
     amax = torch.empty(1, dtype=torch.float32, device=dev)
     scale = torch.empty(1, dtype=torch.float32, device=dev)
-    out = abi.new_out(m, n, dev)
     st = abi.stream_ptr()
-    # inv = 448/amax and scale = amax/448 the way torch evaluates them on a GPU in prep_x_fp8 (DIV_TORCH)
     f._actq_fp8(x2, codes, amax, scale, abi.DIV_TORCH, abi.FLAG_AMAX_AFTER_BF16 | abi.FLAG_QUANT_FROM_BF16, st)
     gflags = abi.FLAG_OUT_VIA_BF16 | f._wscale_flag(w_ts, n)
     if push is not None:

@@ -84,7 +84,7 @@ def _codes_gemv_fits(m: int, k: int, n=None) -> bool:
 # --------------------------------------------------------------------------- helpers
 def _rows16(x: torch.Tensor) -> torch.Tensor:
     """[..., K] -> contiguous [M, K] in fp16/bf16 (other dtypes become bf16), as the reference wrappers do."""
-    x2 = x.reshape(-1, x.shape[-1])
+    x2 = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])
     if x2.dtype not in (torch.float16, torch.bfloat16):
         x2 = x2.to(torch.bfloat16)
     if x2.stride(-1) != 1 or (x2.shape[0] > 1 and x2.stride(0) != x2.shape[1]) or x2.data_ptr() % 16:
@@ -244,6 +244,40 @@ def _actq_fp8(x2, codes, amax, scale, div, flags, st):
                  abi.ptr(scale), div, flags, st)
 
 
+def _linear(kind, xs, ws_, scales, outs, ldo, m, n, k, decode, act_div, gemm_div, act_flags, gemm_flags, by_scale=0):
+    """Quantizer and GEMM of one projection (or r, k, v) in one call (rwkvq_linear).  xs, ws_, scales: one or three tensors;
+    outs: their result pointers."""
+    x0, w0 = xs[0], ws_[0]
+    dev = x0.device
+    nmat = len(xs)
+    if kind == abi.LINEAR_FP8:
+        need = nmat * abi.up256(m * k) + 256
+        sc = abi.actq_scratch(dev)
+        sc_ptr, sc_bytes = sc.data_ptr(), sc.numel() * 4
+    else:
+        need = nmat * (abi.up256(m * k) + abi.up256(4 * m))
+        sc_ptr = sc_bytes = 0
+    scratch = torch.empty(need, dtype=torch.uint8, device=dev)
+    ws = None if decode else abi.workspace(min(m, 128), n, k, nmat, dev)
+    if nmat == 1:
+        ptrs = (x0.data_ptr(), 0, 0, w0.data_ptr(), 0, 0, scales[0].data_ptr(), 0, 0, outs[0], 0, 0)
+    else:
+        ptrs = (*(t.data_ptr() for t in xs), *(t.data_ptr() for t in ws_), *(t.data_ptr() for t in scales), *outs)
+    abi.call("rwkvq_linear", abi.LINEAR_DESC.pack(
+        *ptrs, x0.stride(0) if m > 1 else k, w0.stride(0), ldo, m, n, k, kind, abi.dtype_code(x0), nmat, decode, act_div, gemm_div, act_flags,
+        gemm_flags, by_scale, 0, scratch.data_ptr(), need, sc_ptr, sc_bytes, 0 if ws is None else ws.data_ptr(), 0 if ws is None else ws.numel(),
+        abi.stream_ptr()))
+    abi.after_call(ws)
+
+
+def _linear3(kind, xs, ws_, scales, m, n, k, decode, act_flags, gemm_flags):
+    """r, k, v through _linear: one quantization launch for the three inputs, one GEMM launch for the three projections."""
+    outs = torch.empty((3, m, n), dtype=torch.float16, device=xs[0].device)
+    o0, step = outs.data_ptr(), m * n * 2
+    _linear(kind, xs, ws_, scales, (o0, o0 + step, o0 + 2 * step), n, m, n, k, decode, abi.DEFAULT_DIV, abi.DEFAULT_DIV, act_flags, gemm_flags)
+    return outs.unbind(0)
+
+
 def can_push(m: int, n: int, k: int) -> bool:
     """True if an FP8 projection of m rows runs the GEMM that can carry the all-gather of a column-split projection."""
     return ROUTE != "mma" and _ACTQ_FUSED and m > 0 and k % 16 == 0 and bool(abi.lib().rwkvq_tc_gemm_can_push(m, n, k))
@@ -254,11 +288,14 @@ def _fp8_codes_gemm(x2, w, w_ts, act_flags, gemm_flags=0, push=None):
     GEMM also stores its result into the peers' buffers and signals them (rwkvq_dist.PeerGather.push_targets)."""
     m, k = x2.shape
     n = w.shape[0]
+    gemm_flags |= _wscale_flag(w_ts, n)
+    out = abi.new_out(m, n, x2.device)
+    if push is None and ROUTE != "mma" and _ACTQ_FUSED and k % 8 == 0 and m > 0:
+        _linear(abi.LINEAR_FP8, (x2,), (w,), (w_ts,), (out.data_ptr(),), out.stride(0), m, n, k, 0, abi.DEFAULT_DIV, abi.DEFAULT_DIV, act_flags, gemm_flags)
+        return out
     codes = torch.empty((m, k), dtype=torch.uint8, device=x2.device)
     amax = torch.empty(1, dtype=torch.float32, device=x2.device)
-    out = abi.new_out(m, n, x2.device)
     st = abi.stream_ptr()
-    gemm_flags |= _wscale_flag(w_ts, n)
     _actq_fp8(x2, codes, amax, None, abi.DEFAULT_DIV, act_flags, st)
     if push is not None:
         ws = abi.workspace(min(m, 128), n, k, 1, x2.device)
@@ -310,64 +347,22 @@ def _fp8_cluster_gemv(x2, w, w_ts):
 
 
 def _fp8_codes_gemv(x2, w, w_ts):
-    """9..32 rows: quantize once (one cooperative launch), then the weight-streaming decode kernel on the codes."""
+    """9..32 rows: quantize once, then the weight-streaming decode kernel on the codes."""
     m, k = x2.shape
     n = w.shape[0]
-    dev = x2.device
-    codes = torch.empty((m, k), dtype=torch.uint8, device=dev)
-    amax = torch.empty(1, dtype=torch.float32, device=dev)
-    out = abi.new_out(m, n, dev)
-    st = abi.stream_ptr()
-    _actq_fp8(x2, codes, amax, None, abi.DEFAULT_DIV, abi.FLAG_QUANT_FROM_BF16, st)
-    abi.call("rwkvq_gemm_fp8", codes.data_ptr(), k, amax.data_ptr(), 1, w.data_ptr(), w.stride(0), w_ts.data_ptr(),
-             out.data_ptr(), out.stride(0), m, n, k, abi.DEFAULT_DIV, _wscale_flag(w_ts, n), st)
-    abi.after_call()
+    out = abi.new_out(m, n, x2.device)
+    _linear(abi.LINEAR_FP8, (x2,), (w,), (w_ts,), (out.data_ptr(),), out.stride(0), m, n, k, 1, abi.DEFAULT_DIV, abi.DEFAULT_DIV,
+            abi.FLAG_QUANT_FROM_BF16, _wscale_flag(w_ts, n))
     return out
 
 
-def _fp8_codes_gemv_rkv(xs, ws_, scales):
-    """r, k, v with 9..32 rows: ONE quantization launch for the three inputs, ONE weight-streaming launch on the codes."""
+def _fp8_codes_rkv(xs, ws_, scales, decode):
+    """r, k, v above the one-launch decode kernel's range: ONE quantization launch for the three inputs, then ONE launch of
+    the weight-streaming kernel (decode) or of the tensor-core GEMM on the codes (the reference: prep3_x +
+    fused_rkv_fp8_kernel)."""
     m, k = xs[0].shape
     n = ws_[0].shape[0]
-    dev = xs[0].device
-    codes = torch.empty((3, m, k), dtype=torch.uint8, device=dev)
-    amax = torch.empty(3, dtype=torch.float32, device=dev)
-    outs = torch.empty((3, m, n), dtype=torch.float16, device=dev)
-    st = abi.stream_ptr()
-    scratch = abi.actq_scratch(dev)
-    abi.call("rwkvq_actq_fp8_fused3", xs[0].data_ptr(), xs[1].data_ptr(), xs[2].data_ptr(), abi.dtype_code(xs[0]), m, k, k,
-             codes[0].data_ptr(), codes[1].data_ptr(), codes[2].data_ptr(), k, amax.data_ptr(), scratch.data_ptr(),
-             scratch.numel() * 4, None, abi.DEFAULT_DIV, abi.FLAG_QUANT_FROM_BF16, st)
-    abi.call("rwkvq_gemm_fp8_rkv", codes[0].data_ptr(), codes[1].data_ptr(), codes[2].data_ptr(), k, amax.data_ptr(), 1,
-             ws_[0].data_ptr(), ws_[1].data_ptr(), ws_[2].data_ptr(), ws_[0].stride(0), scales[0].data_ptr(),
-             scales[1].data_ptr(), scales[2].data_ptr(), outs[0].data_ptr(), outs[1].data_ptr(), outs[2].data_ptr(), n,
-             m, n, k, abi.DEFAULT_DIV, _wscale_flag(scales[0], n), st)
-    abi.after_call()
-    return [outs[0], outs[1], outs[2]]
-
-
-def _fp8_codes_gemm_rkv(xs, ws_, scales):
-    """r, k, v above the decode kernel's range: ONE activation-quantization launch for the three inputs and ONE
-    tensor-core GEMM launch for the three projections (the reference: prep3_x + fused_rkv_fp8_kernel)."""
-    m, k = xs[0].shape
-    n = ws_[0].shape[0]
-    dev = xs[0].device
-    codes = torch.empty((3, m, k), dtype=torch.uint8, device=dev)
-    amax = torch.empty(3, dtype=torch.float32, device=dev)
-    outs = torch.empty((3, m, n), dtype=torch.float16, device=dev)
-    st = abi.stream_ptr()
-    scratch = abi.actq_scratch(dev)
-    flags = _wscale_flag(scales[0], n)
-    abi.call("rwkvq_actq_fp8_fused3", xs[0].data_ptr(), xs[1].data_ptr(), xs[2].data_ptr(), abi.dtype_code(xs[0]), m, k, k,
-             codes[0].data_ptr(), codes[1].data_ptr(), codes[2].data_ptr(), k, amax.data_ptr(), scratch.data_ptr(),
-             scratch.numel() * 4, None, abi.DEFAULT_DIV, abi.FLAG_QUANT_FROM_BF16, st)
-    ws = abi.workspace(min(m, 128), n, k, 3, dev)
-    abi.call("rwkvq_tc_gemm_fp8_rkv", codes[0].data_ptr(), codes[1].data_ptr(), codes[2].data_ptr(), k, amax.data_ptr(), 1,
-             ws_[0].data_ptr(), ws_[1].data_ptr(), ws_[2].data_ptr(), ws_[0].stride(0), scales[0].data_ptr(),
-             scales[1].data_ptr(), scales[2].data_ptr(), outs[0].data_ptr(), outs[1].data_ptr(), outs[2].data_ptr(), n,
-             m, n, k, abi.DEFAULT_DIV, flags, ws.data_ptr(), ws.numel(), st)
-    abi.after_call(ws)
-    return [outs[0], outs[1], outs[2]]
+    return _linear3(abi.LINEAR_FP8, xs, ws_, scales, m, n, k, decode, abi.FLAG_QUANT_FROM_BF16, _wscale_flag(scales[0], n))
 
 
 def linear_fp8_m1_fused(x, weight_info, out_dtype=torch.float16):
@@ -470,7 +465,7 @@ def linear_rkv_fused(xr, xk, xv, wr_info, wk_info, wv_info, out_dtype=torch.floa
     f32 = lambda a: None if a is None else a.to(device=dev, dtype=torch.float32).contiguous()
     n_route = n if (awq_r is None and awq_k is None and same_ld) else None      # the cluster kernel runs on plain codes of like matrices
     if (_codes_gemv_fits(m, k, n_route) and _ACTQ_FUSED and same_ld and awq_r is None and awq_k is None and k % 8 == 0):
-        outs = _fp8_codes_gemv_rkv([t.contiguous() for t in xs], ws_, [i["tensor_scale"] for i in (wr_info, wk_info, wv_info)])
+        outs = _fp8_codes_rkv([t.contiguous() for t in xs], ws_, [i["tensor_scale"] for i in (wr_info, wk_info, wv_info)], 1)
     elif _tc_fused_fits(m, k, 3) and same_ld:
         xs = [t.contiguous() for t in xs]
         outs = [torch.empty((m, n), dtype=torch.float16, device=dev) for _ in range(3)]
@@ -493,7 +488,7 @@ def linear_rkv_fused(xr, xk, xv, wr_info, wk_info, wv_info, out_dtype=torch.floa
                  m, n, k, k, abi.DEFAULT_DIV, wflag, abi.stream_ptr())
         abi.after_call()
     elif ROUTE != "mma" and _ACTQ_FUSED and same_ld and awq_r is None and awq_k is None and k % 8 == 0 and m > 0:
-        outs = _fp8_codes_gemm_rkv([t.contiguous() for t in xs], ws_, [i["tensor_scale"] for i in (wr_info, wk_info, wv_info)])
+        outs = _fp8_codes_rkv([t.contiguous() for t in xs], ws_, [i["tensor_scale"] for i in (wr_info, wk_info, wv_info)], 0)
     else:
         outs = []
         for x2, w, info, awq in zip(xs, ws_, (wr_info, wk_info, wv_info), (awq_r, awq_k, None)):
@@ -512,11 +507,30 @@ _ffn_scratch: dict = {}
 def ffn_scratch(device) -> torch.Tensor:
     """64 zeroed bytes per (device, stream) through which the key projection hands max|relu^2| (FP8: one value; INT8: one
     per token row) to the value projection."""
-    key = (torch.device(device).index or 0, torch.cuda.current_stream().cuda_stream)
+    key = (abi.device_index(device), abi.stream_ptr())
     sc = _ffn_scratch.get(key)
     if sc is None:
         sc = _ffn_scratch[key] = torch.zeros(16, dtype=torch.int32, device=device)
     return sc
+
+
+def _ffn_many(kind, x2, wk, sk, wv, sv, act_div, gemm_div, act_flags, key_flags, value_flags, by_scale, ffn):
+    """The four launches of an FFN pair with many rows in one call (rwkvq_ffn_relu2); (hidden activations, result)."""
+    (m, k), f_dim, n, dev = x2.shape, wk.shape[0], wv.shape[0], x2.device
+    fp8 = kind == abi.LINEAR_FP8
+    need = abi.up256(m * k) + abi.up256(m * f_dim) + (256 if fp8 else 2 * abi.up256(4 * m))
+    scratch = torch.empty(need, dtype=torch.uint8, device=dev)
+    hid = torch.empty((m, f_dim), dtype=torch.float16, device=dev)
+    out = abi.new_out(m, n, dev)
+    sc = abi.actq_scratch(dev) if fp8 else None
+    ws = abi.workspace(min(m, 128), max(f_dim, n), max(k, f_dim), 1, dev)
+    abi.call("rwkvq_ffn_relu2", abi.FFN_DESC.pack(
+        x2.data_ptr(), wk.data_ptr(), sk.data_ptr(), wv.data_ptr(), sv.data_ptr(), hid.data_ptr(), out.data_ptr(), x2.stride(0) if m > 1 else k,
+        wk.stride(0), wv.stride(0), out.stride(0), m, k, f_dim, n, kind, abi.dtype_code(x2), act_div, gemm_div, act_flags, key_flags, value_flags,
+        by_scale, scratch.data_ptr(), need, sc.data_ptr() if fp8 else 0, sc.numel() * 4 if fp8 else 0, ws.data_ptr(), ws.numel(), ffn.data_ptr(),
+        abi.stream_ptr()))
+    abi.after_call(ws)
+    return hid, out
 
 
 def ffn_relu2_fp8(x, key_info, value_info, out_dtype=torch.float16, return_hidden=False):
@@ -548,29 +562,10 @@ def ffn_relu2_fp8(x, key_info, value_info, out_dtype=torch.float16, return_hidde
         # rows the two projections have the semantics of linear_fp8_fused, above those of fp8_ops.linear_fp8 (bf16
         # first, torch's scale arithmetic, results through bf16), as the engine's dispatch has them.
         big = m > FUSED_M_MAX
-        dev_, st = x2.device, abi.stream_ptr()
-        div = abi.DIV_TORCH if big else abi.DEFAULT_DIV
-        aflags = abi.FLAG_QUANT_FROM_BF16 | (abi.FLAG_AMAX_AFTER_BF16 if big else 0)
-        gflags = (abi.FLAG_OUT_VIA_BF16 | abi.FLAG_AMAX_AFTER_BF16) if big else 0
-        codes = torch.empty((m, k), dtype=torch.uint8, device=dev_)
-        sc4 = torch.empty(4, dtype=torch.float32, device=dev_)           # amax / scale of x, amax / scale of the hidden
-        hid = torch.empty((m, f_dim), dtype=torch.float16, device=dev_)
-        hcodes = torch.empty((m, f_dim), dtype=torch.uint8, device=dev_)
-        out = abi.new_out(m, n, dev_)
-        ffn = ffn_scratch(dev_)
-        _actq_fp8(x2, codes, sc4[0:1], sc4[1:2], div, aflags, st)
-        ws = abi.workspace(min(m, 128), max(f_dim, n), max(k, f_dim), 1, dev_)
-        a_ptr, is_amax = (sc4[1:2].data_ptr(), 0) if big else (sc4[0:1].data_ptr(), 1)
-        abi.call("rwkvq_tc_gemm_fp8_relu2", codes.data_ptr(), k, a_ptr, is_amax, _u8(wk).data_ptr(), wk.stride(0), sk.data_ptr(),
-                 hid.data_ptr(), f_dim, m, f_dim, k, abi.DIV_IEEE if big else abi.DEFAULT_DIV, gflags | _wscale_flag(sk, f_dim),
-                 ffn.data_ptr(), ws.data_ptr(), ws.numel(), st)
-        abi.call("rwkvq_actq_fp8_given", hid.data_ptr(), abi.F16, m, f_dim, f_dim, hcodes.data_ptr(), f_dim, sc4[2:3].data_ptr(),
-                 sc4[3:4].data_ptr(), ffn.data_ptr(), div, abi.FLAG_QUANT_FROM_BF16, st)
-        h_ptr = sc4[3:4].data_ptr() if big else sc4[2:3].data_ptr()
-        abi.call("rwkvq_tc_gemm_fp8", hcodes.data_ptr(), f_dim, h_ptr, is_amax, _u8(wv).data_ptr(), wv.stride(0), sv.data_ptr(),
-                 out.data_ptr(), out.stride(0), m, n, f_dim, abi.DIV_IEEE if big else abi.DEFAULT_DIV,
-                 (abi.FLAG_OUT_VIA_BF16 if big else 0) | _wscale_flag(sv, n), ws.data_ptr(), ws.numel(), st)
-        abi.after_call(ws)
+        hid, out = _ffn_many(abi.LINEAR_FP8, x2, wk, sk, wv, sv, abi.DIV_TORCH if big else abi.DEFAULT_DIV, abi.DIV_IEEE if big else abi.DEFAULT_DIV,
+                             abi.FLAG_QUANT_FROM_BF16 | (abi.FLAG_AMAX_AFTER_BF16 if big else 0),
+                             ((abi.FLAG_OUT_VIA_BF16 | abi.FLAG_AMAX_AFTER_BF16) if big else 0) | _wscale_flag(sk, f_dim),
+                             (abi.FLAG_OUT_VIA_BF16 if big else 0) | _wscale_flag(sv, n), int(big), ffn_scratch(x2.device))
     else:
         hid = linear_quantized_fused(x2, {"weight": wk, "tensor_scale": sk, "qtype": "fp8"})
         hid = (hid.float().clamp_(min=0.0) ** 2).to(torch.float16)       # relu_square: fp16(max(y, 0)^2), fp32 arithmetic
@@ -585,7 +580,7 @@ _row_max = {}
 def _row_max_scratch(device, rows: int) -> torch.Tensor:
     """Zeroed floats, one per token row, per (device, stream): the key GEMM of the INT8 FFN pair folds the rows' maxima
     into them and the quantizer behind it clears them again."""
-    key = (torch.device(device).index or 0, torch.cuda.current_stream().cuda_stream)
+    key = (abi.device_index(device), abi.stream_ptr())
     buf = _row_max.get(key)
     if buf is None or buf.numel() < rows:
         buf = _row_max[key] = torch.zeros(max(rows, 4096), dtype=torch.float32, device=device)
@@ -617,23 +612,7 @@ def ffn_relu2_int8(x, key_info, value_info, out_dtype=torch.float16, return_hidd
         abi.after_call()
     elif ROUTE == "auto" and m > GEMV_M_MAX and k % 16 == 0 and f_dim % 16 == 0 and can_push(m, f_dim, k):
         # many rows on the tiled GEMM (can_push: neither the weight-streaming nor the cluster form takes these sizes)
-        dev_, st = x2.device, abi.stream_ptr()
-        codes = torch.empty((m, k), dtype=torch.int8, device=dev_)
-        xs = torch.empty(m, dtype=torch.float32, device=dev_)
-        hid = torch.empty((m, f_dim), dtype=torch.float16, device=dev_)
-        hcodes = torch.empty((m, f_dim), dtype=torch.int8, device=dev_)
-        hs = torch.empty(m, dtype=torch.float32, device=dev_)
-        out = abi.new_out(m, n, dev_)
-        rowmax = _row_max_scratch(dev_, m)
-        abi.call("rwkvq_prep_x_int8", x2.data_ptr(), abi.dtype_code(x2), m, k, x2.stride(0), codes.data_ptr(), k, xs.data_ptr(), abi.DEFAULT_DIV, st)
-        ws = abi.workspace(min(m, 128), max(f_dim, n), max(k, f_dim), 1, dev_)
-        abi.call("rwkvq_tc_gemm_int8_relu2", codes.data_ptr(), k, xs.data_ptr(), wk.data_ptr(), wk.stride(0), sk.data_ptr(), hid.data_ptr(), f_dim,
-                 m, f_dim, k, 0, rowmax.data_ptr(), ws.data_ptr(), ws.numel(), st)
-        abi.call("rwkvq_actq_int8_given", hid.data_ptr(), abi.F16, m, f_dim, f_dim, hcodes.data_ptr(), f_dim, hs.data_ptr(), rowmax.data_ptr(),
-                 abi.DEFAULT_DIV, st)
-        abi.call("rwkvq_tc_gemm_int8", hcodes.data_ptr(), f_dim, hs.data_ptr(), wv.data_ptr(), wv.stride(0), sv.data_ptr(), out.data_ptr(),
-                 out.stride(0), None, 0, m, n, f_dim, 0, ws.data_ptr(), ws.numel(), st)
-        abi.after_call(ws)
+        hid, out = _ffn_many(abi.LINEAR_INT8, x2, wk, sk, wv, sv, abi.DEFAULT_DIV, abi.DEFAULT_DIV, 0, 0, 0, 0, _row_max_scratch(x2.device, m))
     else:
         hid = linear_int8_fused(x2, key_info)
         hid = (hid.float().clamp_(min=0.0) ** 2).to(torch.float16)       # relu_square: fp16(max(y, 0)^2), fp32 arithmetic
@@ -661,8 +640,11 @@ def _int8_any(x2, w, w_scale, acc_out=None, push=None):
                  out.data_ptr(), out.stride(0), m, n, k, 0, ws.data_ptr(), ws.numel(), push[0], push[1], push[2], push[3], st)
         abi.after_call(ws)
         return out
-    if _codes_gemv_fits(m, k):
-        # 9..32 rows: quantize the rows once, then the weight-streaming decode kernel on the codes
+    if acc_out is None and ROUTE != "mma" and m > 0 and (_codes_gemv_fits(m, k) or not (_tc_fused_fits(m, k) or _gemv_fits(m, k, fp8=False))):
+        # from 9 rows on: quantize the rows once, then the weight-streaming decode kernel or the tensor-core GEMM on the codes
+        _linear(abi.LINEAR_INT8, (x2,), (w,), (w_scale,), (out.data_ptr(),), out.stride(0), m, n, k, int(_codes_gemv_fits(m, k)), abi.DEFAULT_DIV, 0, 0, 0)
+    elif _codes_gemv_fits(m, k):
+        # the same steps one by one, with the raw accumulators
         codes = torch.empty((m, k), dtype=torch.int8, device=x2.device)
         xs = torch.empty(m, dtype=torch.float32, device=x2.device)
         abi.call("rwkvq_prep_x_int8", x2.data_ptr(), abi.dtype_code(x2), m, k, x2.stride(0) if m > 1 else k,
@@ -715,21 +697,7 @@ def linear_rkv_int8_fused(xr, xk, xv, wr_info, wk_info, wv_info, out_dtype=torch
     scales = [wr_info["tensor_scale"]] * 3 if compat_shared_scale else [i["tensor_scale"] for i in infos]
     same_ld = len({w.stride(0) for w in ws}) == 1 and all(w.shape == ws[0].shape for w in ws)
     if _codes_gemv_fits(m, k) and same_ld:
-        dev = xs[0].device
-        st = abi.stream_ptr()
-        xs = [t.contiguous() for t in xs]
-        codes = torch.empty((3, m, k), dtype=torch.int8, device=dev)
-        xsc = torch.empty((3, m), dtype=torch.float32, device=dev)
-        outs3 = torch.empty((3, m, n), dtype=torch.float16, device=dev)
-        abi.call("rwkvq_prep3_x_int8", xs[0].data_ptr(), xs[1].data_ptr(), xs[2].data_ptr(), abi.dtype_code(xs[0]), m, k, k,
-                 codes[0].data_ptr(), codes[1].data_ptr(), codes[2].data_ptr(), k, xsc[0].data_ptr(), xsc[1].data_ptr(),
-                 xsc[2].data_ptr(), abi.DEFAULT_DIV, st)
-        abi.call("rwkvq_gemm_int8_rkv", codes[0].data_ptr(), codes[1].data_ptr(), codes[2].data_ptr(), k, xsc[0].data_ptr(),
-                 xsc[1].data_ptr(), xsc[2].data_ptr(), ws[0].data_ptr(), ws[1].data_ptr(), ws[2].data_ptr(), ws[0].stride(0),
-                 scales[0].data_ptr(), scales[1].data_ptr(), scales[2].data_ptr(), outs3[0].data_ptr(), outs3[1].data_ptr(),
-                 outs3[2].data_ptr(), n, m, n, k, 0, st)
-        abi.after_call()
-        outs = [outs3[0], outs3[1], outs3[2]]
+        outs = _linear3(abi.LINEAR_INT8, [t.contiguous() for t in xs], ws, scales, m, n, k, 1, 0, 0)
     elif _tc_fused_fits(m, k, 3) and same_ld:
         xs = [t.contiguous() for t in xs]
         outs = [torch.empty((m, n), dtype=torch.float16, device=xs[0].device) for _ in range(3)]
@@ -748,22 +716,7 @@ def linear_rkv_int8_fused(xr, xk, xv, wr_info, wk_info, wv_info, out_dtype=torch
     elif ROUTE != "mma" and same_ld and m > 0:
         # above the decode kernel's range: ONE row-quantization launch and ONE tensor-core GEMM launch for r, k, v
         # (the reference: 3 x _prep_x_int8_kernel + fused_rkv_int8_kernel)
-        dev = xs[0].device
-        st = abi.stream_ptr()
-        xs = [t.contiguous() for t in xs]
-        codes = torch.empty((3, m, k), dtype=torch.int8, device=dev)
-        xsc = torch.empty((3, m), dtype=torch.float32, device=dev)
-        outs3 = torch.empty((3, m, n), dtype=torch.float16, device=dev)
-        abi.call("rwkvq_prep3_x_int8", xs[0].data_ptr(), xs[1].data_ptr(), xs[2].data_ptr(), abi.dtype_code(xs[0]), m, k, k,
-                 codes[0].data_ptr(), codes[1].data_ptr(), codes[2].data_ptr(), k, xsc[0].data_ptr(), xsc[1].data_ptr(),
-                 xsc[2].data_ptr(), abi.DEFAULT_DIV, st)
-        wsp = abi.workspace(min(m, 128), n, k, 3, dev)
-        abi.call("rwkvq_tc_gemm_int8_rkv", codes[0].data_ptr(), codes[1].data_ptr(), codes[2].data_ptr(), k, xsc[0].data_ptr(),
-                 xsc[1].data_ptr(), xsc[2].data_ptr(), ws[0].data_ptr(), ws[1].data_ptr(), ws[2].data_ptr(), ws[0].stride(0),
-                 scales[0].data_ptr(), scales[1].data_ptr(), scales[2].data_ptr(), outs3[0].data_ptr(), outs3[1].data_ptr(),
-                 outs3[2].data_ptr(), n, m, n, k, 0, wsp.data_ptr(), wsp.numel(), st)
-        abi.after_call(wsp)
-        outs = [outs3[0], outs3[1], outs3[2]]
+        outs = _linear3(abi.LINEAR_INT8, [t.contiguous() for t in xs], ws, scales, m, n, k, 0, 0, 0)
     else:
         outs = [_int8_any(x2, w, s) for x2, w, s in zip(xs, ws, scales)]
     return tuple(_finish(o, lead, n, out_dtype) for o in outs)

@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import struct
 
 import torch
 
@@ -100,6 +101,10 @@ SIGNATURES = {
     "rwkvq_tc_gemm_int8_rkv": [_p, _p, _p, _i64, _p, _p, _p, _p, _p, _p, _i64, _p, _p, _p, _p, _p, _p, _i64, _i64, _i64, _i64,
                                _u32, _p, _i64, _p],
     "rwkvq_tc_static_status": [_p],
+    "rwkvq_linear_scratch_bytes": [_i32, _i32, _i64, _i64],
+    "rwkvq_linear": [_p],
+    "rwkvq_ffn_scratch_bytes": [_i32, _i64, _i64, _i64],
+    "rwkvq_ffn_relu2": [_p],
     "rwkvq_gemv_batch": [_p, _i32, _p],
     "rwkvq_tc_gemm_fp8_relu2": [_p, _i64, _p, _i32, _p, _i64, _p, _p, _i64, _i64, _i64, _i64, _i32, _u32, _p, _p, _i64, _p],
     "rwkvq_actq_fp8_given": [_p, _i32, _i64, _i64, _i64, _p, _i64, _p, _p, _p, _i32, _u32, _p],
@@ -127,7 +132,7 @@ SIGNATURES = {
     "rwkvq_gemv_set_trace": [_p],
     "rwkvq_tc_set_trace": [_p],
 }
-_RESTYPES = {"rwkvq_tc_gemm_wa16_workspace_bytes": ctypes.c_int64, "rwkvq_actq_nvfp4_fused_scratch_bytes": ctypes.c_int64, "rwkvq_gemv_nvfp4_fused_smem_bytes": ctypes.c_int64, "rwkvq_nvfp4_blocked_scale_bytes": ctypes.c_int64, "rwkvq_actq_fp8_fused_scratch_bytes": ctypes.c_int64, "rwkvq_gemv_nvfp4_smem_bytes": ctypes.c_int64, "rwkvq_gemv_int4_group_smem_bytes": ctypes.c_int64, "rwkvq_workspace_bytes": ctypes.c_int64, "rwkvq_last_error_string": ctypes.c_char_p, "rwkvq_launch_count": ctypes.c_int64,
+_RESTYPES = {"rwkvq_linear_scratch_bytes": ctypes.c_int64, "rwkvq_ffn_scratch_bytes": ctypes.c_int64, "rwkvq_tc_gemm_wa16_workspace_bytes": ctypes.c_int64, "rwkvq_actq_nvfp4_fused_scratch_bytes": ctypes.c_int64, "rwkvq_gemv_nvfp4_fused_smem_bytes": ctypes.c_int64, "rwkvq_nvfp4_blocked_scale_bytes": ctypes.c_int64, "rwkvq_actq_fp8_fused_scratch_bytes": ctypes.c_int64, "rwkvq_gemv_nvfp4_smem_bytes": ctypes.c_int64, "rwkvq_gemv_int4_group_smem_bytes": ctypes.c_int64, "rwkvq_workspace_bytes": ctypes.c_int64, "rwkvq_last_error_string": ctypes.c_char_p, "rwkvq_launch_count": ctypes.c_int64,
              "rwkvq_set_wait_limit_us": None, "rwkvq_gemv_set_trace": None, "rwkvq_tc_set_trace": None}
 
 
@@ -140,6 +145,17 @@ class ProjDesc(ctypes.Structure):
 
 
 PROJ_FP8, PROJ_FP8_RKV, PROJ_INT8, PROJ_INT8_RKV = 0, 1, 2, 3
+
+# rwkvq_linear_desc and rwkvq_ffn_desc of include/rwkvq.h as struct formats (native alignment): packing one bytes object costs
+# a quarter of marshalling the same values as ctypes arguments
+LINEAR_FP8, LINEAR_INT8 = 0, 1
+LINEAR_DESC = struct.Struct("@12Q6q6i2I2iQqQqQqQ")
+FFN_DESC = struct.Struct("@7Q8q4i3IiQqQqQqQQ")
+
+
+def up256(n: int) -> int:
+    return (n + 255) & ~255
+
 
 _lib = None
 _device_checked = False
@@ -186,6 +202,11 @@ def stream_ptr() -> int:
     if _raw_stream is not None and _raw_device is not None:
         return _raw_stream(_raw_device())
     return torch.cuda.current_stream().cuda_stream
+
+
+def device_index(device) -> int:
+    """Index of a tensor's device (a torch.device costs an attribute read, anything else a constructor)."""
+    return (device if isinstance(device, torch.device) else torch.device(device)).index or 0
 
 
 _fn_cache: dict = {}
@@ -294,7 +315,7 @@ _scratch: dict = {}
 def actq_scratch(device) -> torch.Tensor:
     """Zero-initialised rendezvous scratch of the one-launch activation quantizers, one per (device, stream): calls on
     a stream are ordered, so they share it; the kernels advance its epoch word themselves."""
-    key = (torch.device(device).index or 0, torch.cuda.current_stream().cuda_stream)
+    key = (device_index(device), stream_ptr())
     sc = _scratch.get(key)
     if sc is None:
         need = max(int(lib().rwkvq_actq_fp8_fused_scratch_bytes()), int(lib().rwkvq_actq_nvfp4_fused_scratch_bytes()))
@@ -316,7 +337,7 @@ def workspace(m: int, n: int, k: int, nmat: int, device) -> torch.Tensor:
     need = _ws_need.get((m, n, k, nmat))
     if need is None:
         need = _ws_need[(m, n, k, nmat)] = int(lib().rwkvq_workspace_bytes(m, n, k, nmat))
-    key = (torch.device(device).index or 0, torch.cuda.current_stream().cuda_stream)
+    key = (device_index(device), stream_ptr())
     ws = _workspaces.get(key)
     if ws is None or ws.numel() < need:
         ws = torch.zeros(max(need, 1 << 20), dtype=torch.uint8, device=device)
@@ -330,7 +351,7 @@ _plain: dict = {}
 def plain_scratch(nbytes: int, device) -> torch.Tensor:
     """Uninitialised scratch (partial sums that a kernel writes before another reads them), one per (device, stream),
     grown on demand.  Separate from workspace(): that one must stay zero between launches."""
-    key = (torch.device(device).index or 0, torch.cuda.current_stream().cuda_stream)
+    key = (device_index(device), stream_ptr())
     buf = _plain.get(key)
     if buf is None or buf.numel() < nbytes:
         buf = torch.empty(max(int(nbytes), 1 << 20), dtype=torch.uint8, device=device)

@@ -84,7 +84,7 @@ class DecodeLayer:
         d.x[j] = x.data_ptr()
 
     def _launch(self, first: int, count: int) -> None:
-        rc = self._batch(self._one[first], count, torch.cuda.current_stream().cuda_stream)
+        rc = self._batch(self._one[first], count, abi.stream_ptr())
         if rc != abi.OK:
             raise RuntimeError(f"rwkvq_gemv_batch failed with status {rc}: {abi.last_error()}")
 
@@ -119,7 +119,7 @@ class DecodeLayer:
         self._bind(dk, 0, x, self._k[2])
         if self._ffn_scratch is None:
             self._ffn_scratch = torch.zeros(16, dtype=torch.int32, device=self.device)
-        st, sc = torch.cuda.current_stream().cuda_stream, self._ffn_scratch.data_ptr()
+        st, sc = abi.stream_ptr(), self._ffn_scratch.data_ptr()
         hid, out = self.outs[2][0], self.outs[3][0]
         if self.int8:
             abi.call("rwkvq_gemv_int8_relu2", dk.x[0], dk.x_dtype, dk.w[0], dk.ldw, dk.w_scale[0], hid.data_ptr(), dk.ldo, dk.M, dk.N, dk.K,
