@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(kThreads) quant_fp8_kernel(const void* x, uint
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     float2 f = cvt2<DT>(w[q]);
-                    if (from_bf16) { f.x = bf16_round(f.x); f.y = bf16_round(f.y); }
+                    if (from_bf16) f = bf16_round2(f);
                     c[q] = e4m3x2(clamp448(f.x * inv), clamp448(f.y * inv));
                 }
                 *reinterpret_cast<uint2*>(crow + k) = make_uint2(c[0] | (c[1] << 16), c[2] | (c[3] << 16));
@@ -266,9 +266,10 @@ struct QInt8Args {
     float* scales[3];
 };
 
-// KEEP: decode-sized grids (latency counts, occupancy does not): a separate instantiation, so that the many-row form
-// keeps its small register footprint.
-template <int DT, bool VEC, bool KEEP = false>
+// KEEP = 1, 2, 4, 8: rows of up to KEEP * 2048 elements stay in registers between the abs-max and the codes (KEEP vectors
+// per thread): one read of the row, all loads in flight at once.  Measured against two reads: 2048 rows of 4096 10.4 ->
+// 9.3 us, of 16384 24.8 -> 24.1.  KEEP = 0: longer rows, two reads (the second hits L1 / L2).
+template <int DT, bool VEC, int KEEP = 0>
 __global__ void __launch_bounds__(kThreads) quant_int8_kernel(const QInt8Args qa, int64_t K, int64_t ldx, int64_t ldc, int div_mode) {
     __shared__ float sh[kThreads / 32];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a projection behind this launch may prefetch its weights
@@ -278,18 +279,16 @@ __global__ void __launch_bounds__(kThreads) quant_int8_kernel(const QInt8Args qa
     int8_t* crow = qa.codes[blockIdx.y] + row * ldc;
     float* scales = qa.scales[blockIdx.y];
     float m = 0.f;
-    if (VEC && KEEP && K <= (int64_t)kThreads * 8 * 8) {
-        // rows of up to 16384 elements: a thread's (at most 8) vectors stay in registers between the abs-max and the
-        // codes -- one read of the row, all loads in flight at once
-        uint4 v[8];
+    if constexpr (VEC && KEEP > 0) {
+        uint4 v[KEEP];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        for (int j = 0; j < KEEP; ++j) {
             const int64_t k = ((int64_t)threadIdx.x + j * kThreads) * 8;
             v[j] = make_uint4(0, 0, 0, 0);
             if (k < K) v[j] = *reinterpret_cast<const uint4*>(xrow + k * 2);
         }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        for (int j = 0; j < KEEP; ++j) {
             const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
@@ -301,7 +300,7 @@ __global__ void __launch_bounds__(kThreads) quant_int8_kernel(const QInt8Args qa
         const float s = div_mode_f32(127.f, m, div_mode);
         if (threadIdx.x == 0) scales[row] = div_mode_f32(m, 127.f, div_mode);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        for (int j = 0; j < KEEP; ++j) {
             const int64_t k = ((int64_t)threadIdx.x + j * kThreads) * 8;
             if (k >= K) continue;
             const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
@@ -494,7 +493,7 @@ __global__ void __launch_bounds__(kFusedThreads, 2) actq_fp8_fused_kernel(const 
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             float2 f = cvt2<DT>(w[q]);
-            if (DT == RWKVQ_F16 && from_bf16) { f.x = bf16_round(f.x); f.y = bf16_round(f.y); }
+            if (DT == RWKVQ_F16 && from_bf16) f = bf16_round2(f);
             c[q] = e4m3x2(f.x * inv, f.y * inv);
         }
         *reinterpret_cast<uint2*>(codes + (int64_t)rj * ldc + (size_t)i * 8) = make_uint2(c[0] | (c[1] << 16), c[2] | (c[3] << 16));
@@ -613,7 +612,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) actq_fp8_small_kernel(const 
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             float2 f = cvt2<DT>(w[q]);
-            if (DT == RWKVQ_F16 && from_bf16) { f.x = bf16_round(f.x); f.y = bf16_round(f.y); }
+            if (DT == RWKVQ_F16 && from_bf16) f = bf16_round2(f);
             c[q] = e4m3x2(f.x * inv, f.y * inv);
         }
         const int r = (int)__umulhi((uint32_t)idx, inv_kv), cc = idx - r * kv;
@@ -736,7 +735,7 @@ __global__ void __launch_bounds__(kTwoThreads) actq_two_codes_kernel(const ActqA
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     float2 f = cvt2<DT>(w[i]);
-                    if (DT == RWKVQ_F16 && from_bf16) { f.x = bf16_round(f.x); f.y = bf16_round(f.y); }
+                    if (DT == RWKVQ_F16 && from_bf16) f = bf16_round2(f);
                     q[i] = e4m3x2(f.x * inv, f.y * inv);
                 }
                 *reinterpret_cast<uint2*>(crow + (int64_t)(c0 + j * cstep) * 8) = make_uint2(q[0] | (q[1] << 16), q[2] | (q[3] << 16));
@@ -760,7 +759,7 @@ __global__ void __launch_bounds__(kTwoThreads) actq_two_codes_kernel(const ActqA
 // producer.  amax_out / scale_out are this call's own copies for the GEMM that follows.
 template <int DT>
 __global__ void __launch_bounds__(kThreads) quant_fp8_given_kernel(const void* x, uint8_t* codes, float* amax_out, float* scale_out,
-                                                                   float* ffn, int M, int64_t K, int64_t ldx, int64_t ldc, int div_mode,
+                                                                   float* ffn, int M, int64_t K, int64_t ldx, int64_t ldc, int cpr, int div_mode,
                                                                    int from_bf16) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -770,29 +769,31 @@ __global__ void __launch_bounds__(kThreads) quant_fp8_given_kernel(const void* x
         *amax_out = amax;
         if (scale_out) *scale_out = scale_fwd(amax, 448.f, div_mode);
     }
-    const int64_t kv = K >> 3, nvec = (int64_t)M * kv;
-    for (int64_t i0 = (int64_t)blockIdx.x * kThreads + threadIdx.x; i0 < nvec; i0 += (int64_t)gridDim.x * kThreads * 4) {
-        uint4 v[4];
-        int64_t r[4], c[4];
+    // CTA b takes every cpr-th group of kThreads vectors of row b / cpr and of every (gridDim.x / cpr)-th row after it
+    // (dense blocks come as one long row: no division per vector, no half-filled groups of loads)
+    const int64_t kv = K >> 3, cstep = (int64_t)cpr * kThreads;
+    const int seg = (int)blockIdx.x % cpr, rstep = (int)gridDim.x / cpr;
+    for (int r = (int)blockIdx.x / cpr; r < M; r += rstep) {
+        const char* row = reinterpret_cast<const char*>(x) + (int64_t)r * ldx * 2;
+        uint8_t* crow = codes + (int64_t)r * ldc;
+        for (int64_t c0 = (int64_t)seg * kThreads + threadIdx.x; c0 < kv; c0 += 4 * cstep) {
+            uint4 v[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int64_t idx = i0 + (int64_t)j * gridDim.x * kThreads;
-            r[j] = idx / kv;
-            c[j] = idx - r[j] * kv;
-            if (idx < nvec) v[j] = *reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(x) + (r[j] * ldx + c[j] * 8) * 2);
-        }
+            for (int j = 0; j < 4; ++j)
+                if (c0 + j * cstep < kv) v[j] = *reinterpret_cast<const uint4*>(row + (c0 + j * cstep) * 16);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            if (i0 + (int64_t)j * gridDim.x * kThreads >= nvec) continue;
-            const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
-            uint32_t q[4];
+            for (int j = 0; j < 4; ++j) {
+                if (c0 + j * cstep >= kv) continue;
+                const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+                uint32_t q[4];
 #pragma unroll
-            for (int p = 0; p < 4; ++p) {
-                float2 f = cvt2<DT>(w[p]);
-                if (DT == RWKVQ_F16 && from_bf16) { f.x = bf16_round(f.x); f.y = bf16_round(f.y); }
-                q[p] = e4m3x2(f.x * inv, f.y * inv);
+                for (int p = 0; p < 4; ++p) {
+                    float2 f = cvt2<DT>(w[p]);
+                    if (DT == RWKVQ_F16 && from_bf16) f = bf16_round2(f);
+                    q[p] = e4m3x2(f.x * inv, f.y * inv);
+                }
+                *reinterpret_cast<uint2*>(crow + (c0 + j * cstep) * 8) = make_uint2(q[0] | (q[1] << 16), q[2] | (q[3] << 16));
             }
-            *reinterpret_cast<uint2*>(codes + r[j] * ldc + c[j] * 8) = make_uint2(q[0] | (q[1] << 16), q[2] | (q[3] << 16));
         }
     }
     __syncthreads();                                    // every thread of this CTA has used the amax
@@ -981,10 +982,19 @@ static int32_t launch_quant_int8(const QInt8Args& qa, int nt, int32_t x_dtype, i
     cfg.numAttrs = use_pdl() ? 1 : 0;
     const int dm = div_mode;
     cudaError_t e;
-    const bool keep = vec && K <= (int64_t)kThreads * 8 * 8 && M * nt <= 4 * (int64_t)sm_count();     // few rows: one read, registers
+    const int64_t per = (int64_t)kThreads * 8;           // elements one vector per thread covers
+    const int keep = !vec || K > 8 * per ? 0 : (K <= per ? 1 : (K <= 2 * per ? 2 : (K <= 4 * per ? 4 : 8)));
 #define RWKVQ_Q(DT, V, KP) e = cudaLaunchKernelEx(&cfg, quant_int8_kernel<DT, V, KP>, qa, K, ldx, ldc, dm)
-    if (x_dtype == RWKVQ_F16) { if (keep) RWKVQ_Q(RWKVQ_F16, true, true); else if (vec) RWKVQ_Q(RWKVQ_F16, true, false); else RWKVQ_Q(RWKVQ_F16, false, false); }
-    else                      { if (keep) RWKVQ_Q(RWKVQ_BF16, true, true); else if (vec) RWKVQ_Q(RWKVQ_BF16, true, false); else RWKVQ_Q(RWKVQ_BF16, false, false); }
+#define RWKVQ_QK(DT) \
+    switch (keep) { \
+        case 1: RWKVQ_Q(DT, true, 1); break; \
+        case 2: RWKVQ_Q(DT, true, 2); break; \
+        case 4: RWKVQ_Q(DT, true, 4); break; \
+        case 8: RWKVQ_Q(DT, true, 8); break; \
+        default: if (vec) RWKVQ_Q(DT, true, 0); else RWKVQ_Q(DT, false, 0); \
+    }
+    if (x_dtype == RWKVQ_F16) { RWKVQ_QK(RWKVQ_F16) } else { RWKVQ_QK(RWKVQ_BF16) }
+#undef RWKVQ_QK
 #undef RWKVQ_Q
     if (e != cudaSuccess) {
         g_launches.fetch_add(1, std::memory_order_relaxed);
@@ -1069,7 +1079,15 @@ static int32_t launch_actq_fused(ActqArgs a, int nt, int32_t x_dtype, int64_t M,
         const int kv = (int)(K / 8);
         int cpr = 1;                                     // CTAs per row: about two CTAs per SM in all, 256+ vectors each
         while ((int64_t)M * cpr * nt < 2 * (int64_t)sm_count() && cpr * 2 * kTwoThreads <= kv) cpr <<= 1;
-        const int rows = (int)std::min<int64_t>(M, std::max<int64_t>(1, 4 * (int64_t)sm_count() / (cpr * nt)));
+        int rows = (int)std::min<int64_t>(M, std::max<int64_t>(1, 6 * (int64_t)sm_count() / (cpr * nt)));
+        if (ldx == K && ldc == K && M * K < (int64_t(1) << 30)) {
+            // Dense blocks (what the wrappers pass): both passes are elementwise, so the block is ONE long row.  Row by row a
+            // thread had two vectors of a 4096-element row under way, and 2048 rows on 592 CTAs left a last wave half empty.
+            a.M = 1;
+            a.K = (int)(M * K);
+            rows = 1;
+            cpr = (int)elementwise_ctas(M * (K / 8), 6 * (int64_t)sm_count() / nt);
+        }
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3((unsigned)(rows * cpr), (unsigned)nt);
         cfg.blockDim = dim3(kTwoThreads);
@@ -1132,9 +1150,14 @@ int32_t rwkvq_actq_fp8_given(const void* x, int32_t x_dtype, int64_t M, int64_t 
     RWKVQ_REQUIRE(M > 0 && K > 0 && K % 8 == 0 && M < (1 << 30), RWKVQ_E_SHAPE, "%s: M=%lld K=%lld (K must be a multiple of 8)", who, (long long)M, (long long)K);
     RWKVQ_REQUIRE(aligned16(x) && ldx % 8 == 0 && ldx >= K && ldc % 8 == 0 && ldc >= K && ((uintptr_t)codes & 7) == 0 && ((uintptr_t)ffn_scratch & 7) == 0,
                   RWKVQ_E_ALIGN, "%s: rows must be 16-byte (x) / 8-byte (codes, scratch) aligned", who);
-    const int64_t nvec = M * (K / 8);
+    if (ldx == K && ldc == K) {                          // dense: one long row
+        K *= M;
+        M = ldx = ldc = 1;
+    }
+    const int64_t most = 8 * (int64_t)sm_count();
+    const int cpr = (int)elementwise_ctas(K / 8, std::max<int64_t>(1, most / std::min(M, most)));
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)std::min<int64_t>((nvec + kThreads * 4 - 1) / (kThreads * 4), 8 * (int64_t)sm_count()));
+    cfg.gridDim = dim3((unsigned)(std::min(M, std::max<int64_t>(1, most / cpr)) * cpr));
     cfg.blockDim = dim3(kThreads);
     cfg.stream = (cudaStream_t)stream;
     cudaLaunchAttribute attr[1];
@@ -1145,8 +1168,8 @@ int32_t rwkvq_actq_fp8_given(const void* x, int32_t x_dtype, int64_t M, int64_t 
     const int m = (int)M, dm = div_mode, fb = (flags & RWKVQ_FLAG_QUANT_FROM_BF16) ? 1 : 0;
     float* ffn = reinterpret_cast<float*>(ffn_scratch);
     const cudaError_t e = x_dtype == RWKVQ_F16
-        ? cudaLaunchKernelEx(&cfg, quant_fp8_given_kernel<RWKVQ_F16>, x, codes, amax_out, scale_out, ffn, m, K, ldx, ldc, dm, fb)
-        : cudaLaunchKernelEx(&cfg, quant_fp8_given_kernel<RWKVQ_BF16>, x, codes, amax_out, scale_out, ffn, m, K, ldx, ldc, dm, fb);
+        ? cudaLaunchKernelEx(&cfg, quant_fp8_given_kernel<RWKVQ_F16>, x, codes, amax_out, scale_out, ffn, m, K, ldx, ldc, cpr, dm, fb)
+        : cudaLaunchKernelEx(&cfg, quant_fp8_given_kernel<RWKVQ_BF16>, x, codes, amax_out, scale_out, ffn, m, K, ldx, ldc, cpr, dm, fb);
     if (e != cudaSuccess) {
         g_launches.fetch_add(1, std::memory_order_relaxed);
         return fail(RWKVQ_E_LAUNCH, "%s: %s", who, cudaGetErrorString(e));

@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
@@ -34,6 +35,13 @@ bool use_pdl();
 // The library's per-device status word (device address): kernels whose entry points take no status pointer set it to
 // RWKVQ_E_TIMEOUT when a bounded wait gives up; rwkvq_device_status reads it.  Null if the lookup failed.
 int* device_status_ptr();
+
+// CTAs of an elementwise pass over `vecs` vectors by 256-thread CTAs that load four vectors per thread at a time: enough for
+// two per SM where the block allows it, then four vectors per thread, at most `most`.  (One vector per thread and one CTA per
+// 256: 717 rows of 4096 took 8.7 instead of 5.3 us, the CTAs' arrivals on one counter queueing up.)
+inline int64_t elementwise_ctas(int64_t vecs, int64_t most) {
+    return std::max<int64_t>(1, std::min((vecs + 255) / 256, std::min(most, std::max<int64_t>(2 * (int64_t)sm_count(), (vecs + 1023) / 1024))));
+}
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
@@ -78,6 +86,10 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
     __nv_bfloat162 p = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&p);
 }
+__device__ __forceinline__ float2 bf16_round2(float2 f) {   // both in one conversion
+    const uint32_t p = pack_bf16x2(f.x, f.y);
+    return make_float2(__uint_as_float(p << 16), __uint_as_float(p & 0xffff0000u));
+}
 // two fp32 -> two e4m3 bytes (lo in bits 0-7), round-to-nearest-even, saturating.  One hardware instruction
 // (written as PTX: the cuda_fp8.h helper may pick its software path, hundreds of instructions per pair).
 __device__ __forceinline__ uint32_t e4m3x2(float lo, float hi) {
@@ -109,6 +121,55 @@ __device__ __forceinline__ uint32_t e2m1x2_to_f16x2(uint32_t byte) {
 __device__ __forceinline__ float e4m3_to_float(uint32_t code) {
     const uint32_t h2 = e4m3x2_to_f16x2(code & 0xffu);
     return __half2float(__ushort_as_half((unsigned short)(h2 & 0xffffu)));
+}
+// two fp32 values in a 64-bit register pair, and arithmetic on both halves in one instruction
+__device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 unpack_f32x2(uint64_t v) {
+    float2 f;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+    return f;
+}
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// 1 / bs, correctly rounded, for an e4m3 block scale: the hardware's approximation (within 1 ulp) and one Newton step.  From
+// every start within 1 ulp of every such scale's reciprocal the step ends on the correctly rounded value (all of them
+// enumerated in exact arithmetic), so this is __frcp_rn without its range checks.
+__device__ __forceinline__ float block_scale_rcp(float bs) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(bs));
+    return fmaf(r, fmaf(-bs, r, 1.f), r);
+}
+
+// e2m1 codes of 8 values of one NVFP4 block: e2m1_rn((f * inv_pts) / bs), the quotient correctly rounded, with bs an e4m3
+// block scale (2^-6 ... 448).  The quotient is a product with the reciprocal, its exact remainder and one correction
+// (P. Markstein, IBM J. Res. Dev. 34(1), 1990: with a correctly rounded reciprocal the corrected quotient is correctly
+// rounded; |t| is far from overflow, and where the remainder underflows the code is a zero either way).  t is kept negated,
+// so that the remainder of a zero is +0 and the correction leaves the zero's sign, which the code carries, alone.  The 16
+// values of a block share one reciprocal: a division for each took half of the quantizers' instructions.
+__device__ __forceinline__ uint32_t nvfp4_codes8(const float (&f)[8], float inv_pts, float bs, float rc) {
+    const uint64_t ninv = pack_f32x2(-inv_pts, -inv_pts), nrc = pack_f32x2(-rc, -rc), bs2 = pack_f32x2(bs, bs);
+    uint32_t out = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const uint64_t nt = mul_f32x2(pack_f32x2(f[2 * q], f[2 * q + 1]), ninv);        // -t
+        const uint64_t u = mul_f32x2(nt, nrc);                                          // t * rc
+        const float2 v = unpack_f32x2(fma_f32x2(fma_f32x2(u, bs2, nt), nrc, u));
+        out |= e2m1x2(v.x, v.y) << (8 * q);
+    }
+    return out;
 }
 __device__ __forceinline__ float clamp448(float v) { return fminf(fmaxf(v, -448.f), 448.f); }
 

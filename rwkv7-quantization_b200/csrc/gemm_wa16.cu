@@ -457,40 +457,54 @@ __global__ void __launch_bounds__(kW16Threads, 1) gemm_wa16_kernel(const __grid_
 }
 
 // Activations for the INT4 kernel: fp16 rows with each run of 8 stored as [0,4,1,5,2,6,3,7], odd ones / 16, and the sums of each group of
-// 128 (of the fp16 values), [token tile][group][NB].  16 lanes hold a group; bound by the one read and one write.
+// 128 (of the fp16 values), [token tile][group][NB].  16 lanes hold a group; bound by the one read and one write, so a thread
+// has four vectors under way: 1 << lgP of a row and the same of the next 4 >> lgP of its CTA's rows.
 template <int DT>
-__global__ void __launch_bounds__(256) wa16_prep_kernel(const uint16_t* __restrict__ x, int64_t ldx, int M, int kv, __half* xp, float* xsum, int NB, int groups) {
+__global__ void __launch_bounds__(256) wa16_prep_kernel(const uint16_t* __restrict__ x, int64_t ldx, int M, int kv, __half* xp, float* xsum, int NB, int groups,
+                                                        int cpr, int lgP) {
     griddep_launch_dependents();
+    const int seg = (int)blockIdx.x % cpr, rstep = (int)gridDim.x / cpr, cstep = cpr * 256, P = 1 << lgP;
+    const uint32_t mask = 0xffffu << (threadIdx.x & 16);
+    const __half2 sixteenth = __floats2half2_rn(0.0625f, 0.0625f);
     griddep_wait();
-    const int64_t total = (int64_t)M * kv;             // kv is a multiple of 16: the half-warps are whole groups
-    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < total; i += (int64_t)gridDim.x * 256) {
-        const int m = (int)(i / kv), v8 = (int)(i - (int64_t)m * kv);
-        uint4 v = ldg_l2_16(x + (int64_t)m * ldx + (int64_t)v8 * 8);
-        float2 f[4] = {cvt2<DT>(v.x), cvt2<DT>(v.y), cvt2<DT>(v.z), cvt2<DT>(v.w)};
-        if constexpr (DT == RWKVQ_BF16) {
-            uint32_t h[4];
+    for (int r0 = (int)blockIdx.x / cpr; r0 < M; r0 += rstep << (2 - lgP)) {
+        for (int base = seg * 256; base < kv; base += P * cstep) {
+            uint4 v4[4];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const __half2 hh = __floats2half2_rn(f[q].x, f[q].y);
-                h[q] = *reinterpret_cast<const uint32_t*>(&hh);
-                f[q] = cvt2<RWKVQ_F16>(h[q]);
+            for (int j = 0; j < 4; ++j) {
+                const int m = r0 + (j >> lgP) * rstep, i = base + (j & (P - 1)) * cstep + (int)threadIdx.x;
+                if (m < M && i < kv) v4[j] = ldg_l2_16(x + (int64_t)m * ldx + (int64_t)i * 8);
             }
-            v = make_uint4(h[0], h[1], h[2], h[3]);
-        }
-        uint4 p;
-        p.x = __byte_perm(v.x, v.z, 0x5410);
-        p.y = __byte_perm(v.x, v.z, 0x7632);
-        p.z = __byte_perm(v.y, v.w, 0x5410);
-        p.w = __byte_perm(v.y, v.w, 0x7632);
-        const __half2 sixteenth = __floats2half2_rn(0.0625f, 0.0625f);
-        *reinterpret_cast<__half2*>(&p.y) = __hmul2(*reinterpret_cast<__half2*>(&p.y), sixteenth);
-        *reinterpret_cast<__half2*>(&p.w) = __hmul2(*reinterpret_cast<__half2*>(&p.w), sixteenth);
-        *reinterpret_cast<uint4*>(xp + i * 8) = p;
-        float sum = ((f[0].x + f[0].y) + (f[1].x + f[1].y)) + ((f[2].x + f[2].y) + (f[3].x + f[3].y));
-        const uint32_t mask = 0xffffu << (threadIdx.x & 16);
 #pragma unroll
-        for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(mask, sum, o);
-        if ((threadIdx.x & 15) == 0) xsum[((int64_t)(m / NB) * groups + (v8 >> 4)) * NB + m % NB] = sum;
+            for (int j = 0; j < 4; ++j) {
+                const int m = r0 + (j >> lgP) * rstep, i = base + (j & (P - 1)) * cstep + (int)threadIdx.x;
+                if (m >= M || i >= kv) continue;           // kv is a multiple of 16: the half-warps stay whole
+                uint4 v = v4[j];
+                float2 f[4] = {cvt2<DT>(v.x), cvt2<DT>(v.y), cvt2<DT>(v.z), cvt2<DT>(v.w)};
+                if constexpr (DT == RWKVQ_BF16) {
+                    uint32_t h[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const __half2 hh = __floats2half2_rn(f[q].x, f[q].y);
+                        h[q] = *reinterpret_cast<const uint32_t*>(&hh);
+                        f[q] = cvt2<RWKVQ_F16>(h[q]);
+                    }
+                    v = make_uint4(h[0], h[1], h[2], h[3]);
+                }
+                uint4 p;
+                p.x = __byte_perm(v.x, v.z, 0x5410);
+                p.y = __byte_perm(v.x, v.z, 0x7632);
+                p.z = __byte_perm(v.y, v.w, 0x5410);
+                p.w = __byte_perm(v.y, v.w, 0x7632);
+                *reinterpret_cast<__half2*>(&p.y) = __hmul2(*reinterpret_cast<__half2*>(&p.y), sixteenth);
+                *reinterpret_cast<__half2*>(&p.w) = __hmul2(*reinterpret_cast<__half2*>(&p.w), sixteenth);
+                *reinterpret_cast<uint4*>(xp + ((int64_t)m * kv + i) * 8) = p;
+                float sum = ((f[0].x + f[0].y) + (f[1].x + f[1].y)) + ((f[2].x + f[2].y) + (f[3].x + f[3].y));
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(mask, sum, o);
+                if ((threadIdx.x & 15) == 0) xsum[((int64_t)(m / NB) * groups + (i >> 4)) * NB + m % NB] = sum;
+            }
+        }
     }
 }
 
@@ -666,10 +680,14 @@ static int32_t run_wa16(int fmt, const void* x, int x_dtype, int64_t ldx, const 
         __half* xp = reinterpret_cast<__half*>(base + l.xp);
         float* xsum = reinterpret_cast<float*>(base + l.xsum);
         a.xsum = xsum;
-        const int64_t blocks = (M * (K / 8) + 255) / 256;
+        const int kv = (int)(K / 8);
+        int cpr = 1, lgP = 0;                            // CTAs per row: two CTAs per SM in all, 256+ vectors each
+        while (M * cpr < 2 * (int64_t)sm_count() && cpr * 512 <= kv) cpr <<= 1;
+        while (lgP < 2 && (cpr * 256 << lgP) < kv) ++lgP;
+        const int64_t blocks = std::min<int64_t>(M, std::max<int64_t>(1, 6 * (int64_t)sm_count() / cpr)) * cpr;
         rc = x_dtype == RWKVQ_F16
-                 ? launch_plain(wa16_prep_kernel<RWKVQ_F16>, blocks, st, who, (const uint16_t*)x, ldx, (int)M, (int)(K / 8), xp, xsum, p.NB, a.groups)
-                 : launch_plain(wa16_prep_kernel<RWKVQ_BF16>, blocks, st, who, (const uint16_t*)x, ldx, (int)M, (int)(K / 8), xp, xsum, p.NB, a.groups);
+                 ? launch_plain(wa16_prep_kernel<RWKVQ_F16>, blocks, st, who, (const uint16_t*)x, ldx, (int)M, kv, xp, xsum, p.NB, a.groups, cpr, lgP)
+                 : launch_plain(wa16_prep_kernel<RWKVQ_BF16>, blocks, st, who, (const uint16_t*)x, ldx, (int)M, kv, xp, xsum, p.NB, a.groups, cpr, lgP);
         if (rc != RWKVQ_OK) return rc;
         xb = xp;
         ldxb = K;

@@ -305,31 +305,34 @@ __global__ void __launch_bounds__(kThr, 2) gemv_nvfp4_fused_kernel(const NfFused
         pts = __fdiv_rn(amax, 2688.f);
         const float inv_pts = __fdiv_rn(1.f, pts), k448 = __fdiv_rn(448.f, amax);
         const int nb = a.K >> 4;                                   // 16-blocks per row (a multiple of 32)
+        const uint32_t inv_nb = 0xFFFFFFFFu / (uint32_t)nb + 1u;   // row of a flat block index without a division (M nb <= 2^14)
+        {
 #pragma unroll 1
-        for (int r = 0; r < a.M; ++r) {
-            uint8_t* row = xs + (size_t)r * a.pitch;
-            const char* src = reinterpret_cast<const char*>(row);
-#pragma unroll 1
-            for (int b = threadIdx.x; b < nb; b += kThr) {
+            for (int idx = threadIdx.x; idx < a.M * nb; idx += kThr) {     // nb is a multiple of 32: a warp's blocks are one row's
+                const int r = (int)__umulhi((uint32_t)idx, inv_nb), b = idx - r * nb;
+                uint8_t* row = xs + (size_t)r * a.pitch;
+                const char* src = reinterpret_cast<const char*>(row);
                 const uint4 v0 = *reinterpret_cast<const uint4*>(src + (size_t)b * 32), v1 = *reinterpret_cast<const uint4*>(src + (size_t)b * 32 + 16);
                 const uint32_t wv[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-                float f[16], bm = 0.f;
+                float f[2][8];
+                const float bm = fmaxf(packed_absmax8<DT>(v0), packed_absmax8<DT>(v1));
 #pragma unroll
                 for (int q = 0; q < 8; ++q) {
                     const float2 p = cvt2<DT>(wv[q]);
-                    f[2 * q] = p.x;
-                    f[2 * q + 1] = p.y;
-                    bm = fmaxf(bm, fmaxf(fabsf(p.x), fabsf(p.y)));
+                    f[q >> 2][2 * (q & 3)] = p.x;
+                    f[q >> 2][2 * (q & 3) + 1] = p.y;
                 }
                 const float sb = fminf(fmaxf(bm * k448, 0.015625f), 448.f);
                 const uint32_t sc = e4m3x2(sb, 0.f) & 0xffu;
                 const uint32_t s2 = e4m3x2_to_f16x2(sc);
                 const uint32_t ss = __byte_perm(s2, s2, 0x1010);           // (bs, bs) as fp16
                 const float bs = __half2float(__ushort_as_half((unsigned short)(s2 & 0xffffu)));
+                const float rc = block_scale_rcp(bs);
+                const uint32_t codes[2] = {nvfp4_codes8(f[0], inv_pts, bs, rc), nvfp4_codes8(f[1], inv_pts, bs, rc)};
                 uint32_t h[8];
 #pragma unroll
                 for (int q = 0; q < 8; ++q) {
-                    const uint32_t pair = e2m1x2_to_f16x2(e2m1x2(__fdiv_rn(f[2 * q] * inv_pts, bs), __fdiv_rn(f[2 * q + 1] * inv_pts, bs)));
+                    const uint32_t pair = e2m1x2_to_f16x2((codes[q >> 2] >> (8 * (q & 3))) & 0xffu);
                     const __half2 d = __hmul2(*reinterpret_cast<const __half2*>(&pair), *reinterpret_cast<const __half2*>(&ss));
                     h[q] = *reinterpret_cast<const uint32_t*>(&d);
                 }
@@ -575,21 +578,18 @@ __global__ void __launch_bounds__(kNfQThreads, 2) actq_nvfp4_fused_kernel(const 
             uint4 v = make_uint4(0, 0, 0, 0);
             if (on) v = *reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(a.x) + ((int64_t)r * a.ldx + (int64_t)i * 8) * 2);
             const uint32_t wv[4] = {v.x, v.y, v.z, v.w};
-            float f[8], bm = 0.f;
+            float f[8], bm = packed_absmax8<DT>(v);
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const float2 p = cvt2<DT>(wv[q]);
                 f[2 * q] = p.x;
                 f[2 * q + 1] = p.y;
-                bm = fmaxf(bm, fmaxf(fabsf(p.x), fabsf(p.y)));
             }
             bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 1));
             const float sb = fminf(fmaxf(bm * k448, 0.015625f), 448.f);
             const uint32_t sc = e4m3x2(sb, 0.f) & 0xffu;
             const float bs = e4m3_to_float(sc);
-            uint32_t out = 0;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) out |= e2m1x2(__fdiv_rn(f[2 * q] * inv_pts, bs), __fdiv_rn(f[2 * q + 1] * inv_pts, bs)) << (8 * q);
+            const uint32_t out = nvfp4_codes8(f, inv_pts, bs, block_scale_rcp(bs));
             if (on) {
                 *reinterpret_cast<uint32_t*>(a.codes + (int64_t)r * a.ldc + (int64_t)i * 4) = out;
                 if ((i & 1) == 0) {
@@ -667,21 +667,18 @@ __global__ void __launch_bounds__(kNfSmallThreads, 1) actq_nvfp4_small_kernel(co
         const int idx = first + j * step;
         if (j * step >= nvec) break;                                   // uniform over the cluster
         const uint32_t wv[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
-        float f[8], bm = 0.f;
+        float f[8], bm = packed_absmax8<DT>(v[j]);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const float2 p = cvt2<DT>(wv[q]);
             f[2 * q] = p.x;
             f[2 * q + 1] = p.y;
-            bm = fmaxf(bm, fmaxf(fabsf(p.x), fabsf(p.y)));
         }
         bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 1));
         const float sb = fminf(fmaxf(bm * k448, 0.015625f), 448.f);
         const uint32_t sc = e4m3x2(sb, 0.f) & 0xffu;
         const float bs = e4m3_to_float(sc);
-        uint32_t out = 0;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) out |= e2m1x2(__fdiv_rn(f[2 * q] * inv_pts, bs), __fdiv_rn(f[2 * q + 1] * inv_pts, bs)) << (8 * q);
+        const uint32_t out = nvfp4_codes8(f, inv_pts, bs, block_scale_rcp(bs));
         if (idx < nvec) {
             const int r = (int)__umulhi((uint32_t)idx, inv_kv), i = idx - r * kv;
             *reinterpret_cast<uint32_t*>(a.codes + (int64_t)r * a.ldc + (int64_t)i * 4) = out;
@@ -703,7 +700,7 @@ __global__ void __launch_bounds__(kNfSmallThreads, 1) actq_nvfp4_small_kernel(co
 // Words: flags[kNfQMaxCtas + 4] = maximum, [+ 7] = CTAs done (the FP8 two-launch quantizer uses the same words of the
 // same scratch in the same way).  Same arithmetic as the cooperative kernel: same bits.
 constexpr int kNfTwoThreads = 256;
-constexpr int64_t kNfTwoMaxVectors = 1 << 19;
+constexpr int64_t kNfTwoMaxVectors = 1 << 23;    // 4096 rows of 16384; larger blocks: one cooperative launch
 
 // grid rows * cpr: CTA b takes every cpr-th group of kNfTwoThreads vectors of row b / cpr and of every
 // (gridDim.x / cpr)-th row after it
@@ -736,56 +733,80 @@ __global__ void __launch_bounds__(kNfTwoThreads) actq_nvfp4_two_amax_kernel(cons
     }
 }
 
+// Codes pass.  A thread takes a whole 16-block (no exchange for its maximum, one scale, one reciprocal, one 8-byte store) and
+// has two under way: two groups of kNfTwoThreads blocks of a row, or the same group of two of its CTA's rows when a row
+// has no more (one = 1).  Four neighbouring scales of a row are one word of the blocked layout: every fourth lane collects
+// and stores them.  Bound by its instructions: with a vector of 8 per thread and a division per element it ran 138
+// instructions a vector at three CTAs an SM (2048 rows of 16384: both passes 54 us, now 32).
 template <int DT>
-__global__ void __launch_bounds__(kNfTwoThreads) actq_nvfp4_two_codes_kernel(const NfQArgs a, int cpr) {
+__global__ void __launch_bounds__(kNfTwoThreads, 4) actq_nvfp4_two_codes_kernel(const NfQArgs a, int cpr, int one) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const int kv = a.K >> 3;
+    const int nb = a.K >> 4, lane = threadIdx.x & 31;
     const int seg = (int)blockIdx.x % cpr, rstep = (int)gridDim.x / cpr, cstep = cpr * kNfTwoThreads;
     int* two = reinterpret_cast<int*>(a.flags) + kNfQMaxCtas + 4;
     const int64_t k64 = a.K >> 6;
+    const bool words = (a.K & 63) == 0 && (reinterpret_cast<uintptr_t>(a.bs_blocked) & 3) == 0;
+    const bool wide = (a.ldc & 7) == 0 && (reinterpret_cast<uintptr_t>(a.codes) & 7) == 0;
     asm volatile("griddepcontrol.wait;" ::: "memory");              // the abs-max pass is complete and visible
     const float amax = fmaxf(__int_as_float(__ldcg(two)), 1e-12f);
     const float pts = __fdiv_rn(amax, 2688.f);
     if (blockIdx.x == 0 && threadIdx.x == 0) *a.pts = pts;
     const float inv_pts = __fdiv_rn(1.f, pts), k448 = __fdiv_rn(448.f, amax);
-    for (int r = (int)blockIdx.x / cpr; r < a.M; r += rstep) {
-        const char* row = reinterpret_cast<const char*>(a.x) + (int64_t)r * a.ldx * 2;
-        // whole warps walk together: kv is even and a 16-block is the vectors of lanes 2j and 2j + 1
-        for (int base = seg * kNfTwoThreads; base < kv; base += 4 * cstep) {
-            uint4 v[4];
+    const int jr = one ? rstep : 0, jc = one ? 0 : cstep;           // where the second block of a thread lies
+    for (int r0 = (int)blockIdx.x / cpr; r0 < a.M; r0 += one ? 2 * rstep : rstep) {
+        for (int base = seg * kNfTwoThreads; base < nb; base += one ? cstep : 2 * cstep) {
+            uint4 v[2][2];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int i = base + j * cstep + (int)threadIdx.x;
-                v[j] = i < kv ? *reinterpret_cast<const uint4*>(row + (int64_t)i * 16) : make_uint4(0, 0, 0, 0);
+            for (int j = 0; j < 2; ++j) {
+                const int r = r0 + j * jr, i = base + j * jc + (int)threadIdx.x;
+                v[j][0] = v[j][1] = make_uint4(0, 0, 0, 0);
+                if (r < a.M && i < nb) {
+                    const uint4* p = reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(a.x) + ((int64_t)r * a.ldx + (int64_t)i * 16) * 2);
+                    v[j][0] = p[0];
+                    v[j][1] = p[1];
+                }
             }
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                if (base + j * cstep >= kv) continue;              // uniform over the CTA
-                const int i = base + j * cstep + (int)threadIdx.x;
-                const uint32_t wv[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
-                float f[8], bm = 0.f;
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const float2 p = cvt2<DT>(wv[q]);
-                    f[2 * q] = p.x;
-                    f[2 * q + 1] = p.y;
-                    bm = fmaxf(bm, fmaxf(fabsf(p.x), fabsf(p.y)));
-                }
-                bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 1));
+            for (int j = 0; j < 2; ++j) {
+                const int r = r0 + j * jr, i = base + j * jc + (int)threadIdx.x;
+                if (r >= a.M || i - (int)threadIdx.x >= nb) continue;      // uniform over the CTA
+                const uint32_t wv[8] = {v[j][0].x, v[j][0].y, v[j][0].z, v[j][0].w, v[j][1].x, v[j][1].y, v[j][1].z, v[j][1].w};
+                const float bm = fmaxf(packed_absmax8<DT>(v[j][0]), packed_absmax8<DT>(v[j][1]));
                 const float sb = fminf(fmaxf(bm * k448, 0.015625f), 448.f);
                 const uint32_t sc = e4m3x2(sb, 0.f) & 0xffu;
-                const float bs = e4m3_to_float(sc);
-                uint32_t out = 0;
+                const float bs = e4m3_to_float(sc), rc = block_scale_rcp(bs);
+                uint32_t out[2];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) out |= e2m1x2(__fdiv_rn(f[2 * q] * inv_pts, bs), __fdiv_rn(f[2 * q + 1] * inv_pts, bs)) << (8 * q);
-                if (i < kv) {
-                    *reinterpret_cast<uint32_t*>(a.codes + (int64_t)r * a.ldc + (int64_t)i * 4) = out;
-                    if ((i & 1) == 0) {
-                        const int b = i >> 1;
-                        if (a.bs_rows) a.bs_rows[(int64_t)r * a.lds + b] = (uint8_t)sc;
-                        if (a.bs_blocked)
-                            a.bs_blocked[((int64_t)(r >> 7) * k64 + (b >> 2)) * 512 + (r & 31) * 16 + ((r & 127) >> 5) * 4 + (b & 3)] = (uint8_t)sc;
+                for (int h = 0; h < 2; ++h) {
+                    float f[8];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const float2 p = cvt2<DT>(wv[4 * h + q]);
+                        f[2 * q] = p.x;
+                        f[2 * q + 1] = p.y;
                     }
+                    out[h] = nvfp4_codes8(f, inv_pts, bs, rc);
+                }
+                uint32_t sc4 = sc;
+                if (words) {
+                    sc4 |= __shfl_down_sync(0xffffffffu, sc, 1) << 8;
+                    sc4 |= __shfl_down_sync(0xffffffffu, sc, 2) << 16;
+                    sc4 |= __shfl_down_sync(0xffffffffu, sc, 3) << 24;
+                }
+                if (i < nb) {
+                    uint32_t* c = reinterpret_cast<uint32_t*>(a.codes + (int64_t)r * a.ldc + (int64_t)i * 8);
+                    if (wide) {
+                        *reinterpret_cast<uint2*>(c) = make_uint2(out[0], out[1]);
+                    } else {
+                        c[0] = out[0];
+                        c[1] = out[1];
+                    }
+                    if (a.bs_blocked) {
+                        uint8_t* blk = a.bs_blocked + ((int64_t)(r >> 7) * k64 + (i >> 2)) * 512 + (r & 31) * 16 + ((r & 127) >> 5) * 4 + (i & 3);
+                        if (!words) *blk = (uint8_t)sc;
+                        else if ((lane & 3) == 0) *reinterpret_cast<uint32_t*>(blk) = sc4;
+                    }
+                    if (a.bs_rows) a.bs_rows[(int64_t)r * a.lds + i] = (uint8_t)sc;
                 }
             }
         }
@@ -933,12 +954,21 @@ int32_t rwkvq_actq_nvfp4_fused(const void* x, int32_t x_dtype, int64_t M, int64_
     const char* two_env = std::getenv("RWKVQ_NVFP4_ACTQ_TWO_MAX");      // read per call: a test switches routes in one process
     const int64_t two_max = two_env ? std::atoll(two_env) : kNfTwoMaxVectors;
     if (M * (K / 8) <= two_max) {
-        const int kv = (int)(K / 8);
-        int cpr = 1;                                     // CTAs per row: about two CTAs per SM in all, 256+ vectors each
-        while ((int64_t)M * cpr < 2 * (int64_t)sm_count() && cpr * 2 * kNfTwoThreads <= kv) cpr <<= 1;
-        const int rows = (int)std::min<int64_t>(M, std::max<int64_t>(1, 4 * (int64_t)sm_count() / cpr));
+        const int nb = (int)(K / 16);
+        int cpr = 1;                                     // CTAs per row: about two CTAs per SM in all, 256+ blocks each
+        while ((int64_t)M * cpr < 2 * (int64_t)sm_count() && cpr * 2 * kNfTwoThreads <= nb) cpr <<= 1;
+        const int one = cpr * kNfTwoThreads >= nb ? 1 : 0;      // a CTA's share of a row is one block per thread
+        const int rows = (int)std::min<int64_t>(M, std::max<int64_t>(1, 8 * (int64_t)sm_count() / cpr));
+        // abs-max of a dense block: one long row, whatever its rows are (no half-filled groups of loads at row ends)
+        NfQArgs m = a;
+        int mcpr = cpr, mgrid = rows * cpr;
+        if (ldx == K && M * K < (int64_t(1) << 30)) {
+            m.M = 1;
+            m.K = (int)(M * K);
+            mcpr = mgrid = (int)elementwise_ctas(M * (K / 8), 6 * (int64_t)sm_count());
+        }
         cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3((unsigned)(rows * cpr));
+        cfg.gridDim = dim3((unsigned)mgrid);
         cfg.blockDim = dim3(kNfTwoThreads);
         cfg.stream = (cudaStream_t)stream;
         cudaLaunchAttribute attr[1];
@@ -946,11 +976,12 @@ int32_t rwkvq_actq_nvfp4_fused(const void* x, int32_t x_dtype, int64_t M, int64_
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = use_pdl() ? 1 : 0;
-        cudaError_t e = x_dtype == RWKVQ_F16 ? cudaLaunchKernelEx(&cfg, actq_nvfp4_two_amax_kernel<RWKVQ_F16>, a, cpr)
-                                             : cudaLaunchKernelEx(&cfg, actq_nvfp4_two_amax_kernel<RWKVQ_BF16>, a, cpr);
+        cudaError_t e = x_dtype == RWKVQ_F16 ? cudaLaunchKernelEx(&cfg, actq_nvfp4_two_amax_kernel<RWKVQ_F16>, m, mcpr)
+                                             : cudaLaunchKernelEx(&cfg, actq_nvfp4_two_amax_kernel<RWKVQ_BF16>, m, mcpr);
+        cfg.gridDim = dim3((unsigned)(rows * cpr));
         if (e == cudaSuccess)
-            e = x_dtype == RWKVQ_F16 ? cudaLaunchKernelEx(&cfg, actq_nvfp4_two_codes_kernel<RWKVQ_F16>, a, cpr)
-                                     : cudaLaunchKernelEx(&cfg, actq_nvfp4_two_codes_kernel<RWKVQ_BF16>, a, cpr);
+            e = x_dtype == RWKVQ_F16 ? cudaLaunchKernelEx(&cfg, actq_nvfp4_two_codes_kernel<RWKVQ_F16>, a, cpr, one)
+                                     : cudaLaunchKernelEx(&cfg, actq_nvfp4_two_codes_kernel<RWKVQ_BF16>, a, cpr, one);
         if (e != cudaSuccess) {
             g_launches.fetch_add(1, std::memory_order_relaxed);
             return fail(RWKVQ_E_LAUNCH, "%s: %s", who, cudaGetErrorString(e));

@@ -128,7 +128,7 @@ __device__ __forceinline__ void fp8_vec_amax(const uint4& v, const float* awq, i
             f.x = div_mode_f32(f.x, awq[k + 2 * q], div_mode);
             f.y = div_mode_f32(f.y, awq[k + 2 * q + 1], div_mode);
         }
-        if (after) { f.x = bf16_round(f.x); f.y = bf16_round(f.y); }
+        if (after) f = bf16_round2(f);
         m = fmaxf(m, fmaxf(fabsf(f.x), fabsf(f.y)));
     }
 }
@@ -144,7 +144,7 @@ __device__ __forceinline__ uint2 fp8_vec_codes(const uint4& v, const float* awq,
             f.x = div_mode_f32(f.x, awq[k + 2 * q], div_mode);
             f.y = div_mode_f32(f.y, awq[k + 2 * q + 1], div_mode);
         }
-        if (DT == RWKVQ_F16 || awq) { f.x = bf16_round(f.x); f.y = bf16_round(f.y); }   // bf16 input is its own rounding
+        if (DT == RWKVQ_F16 || awq) f = bf16_round2(f);   // bf16 input is its own rounding
         c[q] = e4m3x2(f.x * inv, f.y * inv);
     }
     return make_uint2(c[0] | (c[1] << 16), c[2] | (c[3] << 16));

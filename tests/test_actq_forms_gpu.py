@@ -1,0 +1,80 @@
+"""The two-launch activation quantizers against the step-by-step ones (abs-max kernel, then a code kernel that divides each
+element): the same bytes, for dense blocks (walked as one long row) and rows with a pitch, rows that are a few vectors longer
+than a CTA's share, scales whose row length is no multiple of four, zeros of both signs, infinities and NaN."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def block(m, k, pitch, dtype, special):
+    g = torch.Generator().manual_seed(m * 7 + k)
+    x = torch.randn((m, pitch), generator=g) * torch.exp2(torch.randint(-14, 4, (m, pitch // 16 + 1), generator=g).float().repeat_interleave(16, 1)[:, :pitch])
+    x[:, 3::37] = 0.0
+    x[:, 5::41] = -0.0
+    if special:
+        x[m // 2, 17] = float("inf") if special == "inf" else float("nan")
+    return x.to(dtype).cuda()[:, :k]
+
+
+SIZES = [(2048, 128, 128), (70, 1024, 1024), (33, 4112, 4112), (300, 4096, 4352), (17, 16384, 16384), (513, 2064, 2080), (1025, 4096, 4096)]
+
+
+@pytest.mark.parametrize("m,k,pitch", SIZES)
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("special", ["", "inf", "nan"])
+def test_nvfp4(m, k, pitch, dtype, special):
+    import rwkvq_abi as abi
+    x = block(m, k, pitch, dtype, special)
+    dev, st = x.device, abi.stream_ptr()
+    want = torch.empty((m, k // 2), dtype=torch.uint8, device=dev)
+    wbs = torch.empty((m, k // 16), dtype=torch.uint8, device=dev)
+    pts, amax, pts2 = (torch.empty(1, device=dev) for _ in range(3))
+    abi.call("rwkvq_actq_nvfp4", x.data_ptr(), abi.dtype_code(x), m, k, pitch, want.data_ptr(), k // 2, wbs.data_ptr(), k // 16, pts.data_ptr(),
+             amax.data_ptr(), st)
+    sc = abi.actq_scratch(dev)
+    for ldc in (k // 2, k // 2 + 4):                        # code rows on 8- and on 4-byte boundaries
+        got = torch.zeros((m, ldc), dtype=torch.uint8, device=dev)
+        bs = torch.empty_like(wbs)
+        blk = torch.zeros(int(abi.lib().rwkvq_nvfp4_blocked_scale_bytes(m, k)), dtype=torch.uint8, device=dev) if k % 64 == 0 else None
+        abi.call("rwkvq_actq_nvfp4_fused", x.data_ptr(), abi.dtype_code(x), m, k, pitch, got.data_ptr(), ldc, bs.data_ptr(), k // 16, abi.ptr(blk),
+                 pts2.data_ptr(), sc.data_ptr(), sc.numel() * 4, None, st)
+        assert torch.equal(got[:, :k // 2], want) and torch.equal(bs, wbs) and torch.equal(pts.view(torch.int32), pts2.view(torch.int32))
+        if blk is not None:
+            ref = torch.zeros_like(blk)
+            abi.call("rwkvq_nvfp4_pack_scales", wbs.data_ptr(), k // 16, m, k, ref.data_ptr(), st)
+            assert torch.equal(blk, ref)
+
+
+@pytest.mark.parametrize("m,k,pitch", [(2048, 264, 264), (600, 4104, 4104), (600, 4096, 4352), (9, 65536, 65536), (1030, 4096, 4096)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("special", ["", "inf", "nan"])
+def test_fp8_and_int8(m, k, pitch, dtype, special):
+    import rwkvq_abi as abi
+    x = block(m, k, pitch, dtype, special)
+    dev, st = x.device, abi.stream_ptr()
+    want, got = (torch.empty((m, k), dtype=torch.uint8, device=dev) for _ in range(2))
+    a0, a1 = (torch.empty(1, device=dev) for _ in range(2))
+    sc = abi.actq_scratch(dev)
+    fin = x.isfinite()
+    for flags in (abi.FLAG_QUANT_FROM_BF16, abi.FLAG_QUANT_FROM_BF16 | abi.FLAG_AMAX_AFTER_BF16):
+        abi.call("rwkvq_actq_fp8", x.data_ptr(), abi.dtype_code(x), m, k, pitch, want.data_ptr(), k, a0.data_ptr(), None, abi.DIV_FULL, flags, st)
+        abi.call("rwkvq_actq_fp8_fused", x.data_ptr(), abi.dtype_code(x), m, k, pitch, got.data_ptr(), k, a1.data_ptr(), None, sc.data_ptr(),
+                 sc.numel() * 4, None, abi.DIV_FULL, flags, st)
+        # the step-by-step kernel clamps before it converts, which turns the NaN of inf * 0 into a number: finite inputs only
+        assert torch.equal(want[fin], got[fin]) and torch.equal(a0, a1)
+    # the given-amax quantizer with that amax, dense codes and codes with a pitch
+    ffn = torch.zeros(2, dtype=torch.int32, device=dev)
+    for ldc in (k, k + 8):
+        ffn[0] = a0.view(torch.int32)[0]        # the maximum over bf16-rounded values, as the last pass above took it
+        out = torch.zeros((m, ldc), dtype=torch.uint8, device=dev)
+        abi.call("rwkvq_actq_fp8_given", x.data_ptr(), abi.dtype_code(x), m, k, pitch, out.data_ptr(), ldc, a1.data_ptr(), None, ffn.data_ptr(),
+                 abi.DIV_FULL, abi.FLAG_QUANT_FROM_BF16, st)
+        assert torch.equal(out[:, :k], got) and torch.equal(a0, a1) and int(ffn.abs().sum()) == 0
+    # INT8: rows kept in registers (up to 16384) against the formula
+    if k <= 16384 and not special:
+        c = torch.empty((m, k), dtype=torch.int8, device=dev)
+        s = torch.empty(m, device=dev)
+        abi.call("rwkvq_prep_x_int8", x.data_ptr(), abi.dtype_code(x), m, k, pitch, c.data_ptr(), k, s.data_ptr(), abi.DIV_IEEE, st)
+        am = x.float().abs().amax(1).clamp(min=1e-12)
+        assert torch.equal(c, (x.float() * (torch.full_like(am, 127.0) / am)[:, None]).clamp(-128, 127).trunc().to(torch.int8))
