@@ -17,8 +17,9 @@
 //     operand; both come by TMA; 128 x 256 fp32 (or int32) accumulators, double-buffered in tensor memory so the
 //     epilogue of one tile overlaps the MMAs of the next.
 //
-// Roles: warp 0 = TMA producer (one lane), warp 1 = MMA issuer (one lane) and owner of the TMEM allocation,
-// warps 2-5 = epilogue (one TMEM lane quarter each), warps 6-9 = activation quantizer (SWAP+FUSED only).
+// Roles: warp 0 = TMA producer, warp 1 = MMA issuer (one elected lane each) and owner of the TMEM allocation,
+// warps 2-5 = epilogue (one TMEM lane quarter each), warps 6-9 = activation quantizer (SWAP+FUSED) or the epilogue's second
+// half of the columns (GEMM, tc_epilogue.cuh).
 // Every mbarrier wait is bounded; a timeout is reported through the status word and the CTA drains and exits.
 #include <algorithm>
 #include <cstdlib>
@@ -26,6 +27,7 @@
 #include <type_traits>
 
 #include "tc_common.cuh"
+#include "tc_epilogue.cuh"
 #include "tc_host.cuh"
 #include "w8a8.cuh"
 
@@ -276,6 +278,10 @@ __global__ void __launch_bounds__(kTcThreads, SWAP ? 2 : 1) gemm_tc_kernel(const
     const int warp = warp_uniform((int)(threadIdx.x >> 5)), lane = threadIdx.x & 31;
     const uint32_t tmem_cols = a.acc_stride * 2 <= 32 ? 32u : (a.acc_stride * 2 <= 64 ? 64u : (a.acc_stride * 2 <= 128 ? 128u : (a.acc_stride * 2 <= 256 ? 256u : 512u)));
 
+    // epilogue warps: four (one per tensor-memory lane quarter); the tiled form lets eight share a tile, half of the columns
+    // each, unless it pushes its tiles to peers (one staging area per lane quarter)
+    const int nepi = SWAP || a.push.n > 0 ? 4 : 8;
+
     griddep_launch_dependents();
     if (threadIdx.x == 0) tc_mark(a, 0);
 
@@ -286,9 +292,9 @@ __global__ void __launch_bounds__(kTcThreads, SWAP ? 2 : 1) gemm_tc_kernel(const
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(&s.tfull[i], 1);
-            mbar_init(&s.tempty[i], 4);
+            mbar_init(&s.tempty[i], (uint32_t)nepi);
         }
-        mbar_init(&s.done, 4);
+        mbar_init(&s.done, (uint32_t)nepi);
         mbar_init(&s.xbar, 1);
         s.abort_flag = 0;
         s.last_flag = 0;
@@ -394,7 +400,7 @@ __global__ void __launch_bounds__(kTcThreads, SWAP ? 2 : 1) gemm_tc_kernel(const
             }
             if (leader) tc_mark(a, 6);
         }
-    } else if (warp < 6) {
+    } else if (warp < 2 + nepi) {
         // ============================== epilogue ==============================
         griddep_wait();
         if constexpr (SWAP && FUSED) {
@@ -408,12 +414,31 @@ __global__ void __launch_bounds__(kTcThreads, SWAP ? 2 : 1) gemm_tc_kernel(const
         uint32_t pc = 0;
         while (it.next(p)) {
             const int buf = pc & 1;
+            const bool per_row = (a.flags & RWKVQ_FLAG_WSCALE_PER_ROW) != 0;   // one weight scale per output row
+            float wsc = a.ws[p.mat][0];
+            EpiRow e;
+            const int m = p.prow + prow_l;              // tiled form: token row of this thread
+            if constexpr (!SWAP) {
+                // what the tile needs from global memory is fetched while its MMAs still run
+                if constexpr (KIND == KIND_F8) {
+                    const float am = a.a_scale[p.mat][0];
+                    e.actscale = a.amax_is_amax ? div_mode_f32(fmaxf(am, 1e-12f), 448.f, a.div_mode) : am;
+                } else {
+                    e.actscale = m < a.M ? a.a_scale[p.mat][m] : 0.f;
+                }
+                e.ws = a.ws[p.mat];
+                e.rowscale = e.actscale * wsc;
+                e.out = a.out[p.mat] + (int64_t)m * a.ldo;
+                e.acc = KIND == KIND_I8 && a.acc[p.mat] ? a.acc[p.mat] + (int64_t)m * a.ldacc : nullptr;
+                e.N = a.N;
+                e.live = m < a.M;
+                e.vec_ok = (a.ldo % 8 == 0) && ((reinterpret_cast<uintptr_t>(a.out[p.mat]) & 15) == 0);
+                e.flags = a.flags;
+            }
             if (!mbar_wait(&s.tfull[buf], (pc >> 1) & 1, abort_flag, a.wait_ns)) { tc_abort(s, a); break; }
             tc_fence_after_sync();
             if (pc == 0 && et == 0) tc_mark(a, 7);
             const uint32_t taddr = tmem_base + (uint32_t)(buf * a.acc_stride) + ((uint32_t)(q * 32) << 16);
-            const bool per_row = (a.flags & RWKVQ_FLAG_WSCALE_PER_ROW) != 0;   // one weight scale per output row
-            float wsc = a.ws[p.mat][0];
             if constexpr (SWAP) {
                 const int n = p.prow + prow_l;          // weight row
                 if (per_row) wsc = a.ws[p.mat][min(n, a.N - 1)];
@@ -514,64 +539,19 @@ __global__ void __launch_bounds__(kTcThreads, SWAP ? 2 : 1) gemm_tc_kernel(const
                     }
                 }
             } else {
-                const int m = p.prow + prow_l;          // token row
-                float actscale;                         // scale of this thread's token row; the weight scale joins below
-                if constexpr (KIND == KIND_F8) {
-                    const float am = a.a_scale[p.mat][0];
-                    actscale = a.amax_is_amax ? div_mode_f32(fmaxf(am, 1e-12f), 448.f, a.div_mode) : am;
-                } else {
-                    actscale = m < a.M ? a.a_scale[p.mat][m] : 0.f;
-                }
-                const float rowscale = actscale * wsc;
-                const bool vec_ok = (a.ldo % 8 == 0) && ((reinterpret_cast<uintptr_t>(a.out[p.mat]) & 15) == 0);
                 const bool relu2 = (a.flags & RWKVQ_FLAG_RELU2) != 0;
-                const bool hmax_bf16 = (a.flags & RWKVQ_FLAG_AMAX_AFTER_BF16) != 0;
                 float hmax = 0.f;
-                // 16 accumulator columns of this thread's token row -> 8 fp16 pairs (scales, optional bf16 hop, relu^2)
-                auto convert16 = [&](const uint32_t (&r)[16], int n0, uint32_t (&h)[8]) {
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        float s0 = rowscale, s1 = rowscale;
-                        if (per_row) {
-                            s0 = actscale * a.ws[p.mat][min(n0 + 2 * j, a.N - 1)];
-                            s1 = actscale * a.ws[p.mat][min(n0 + 2 * j + 1, a.N - 1)];
-                        }
-                        float f0, f1;
-                        if constexpr (KIND == KIND_F8) {
-                            f0 = __uint_as_float(r[2 * j]) * s0;
-                            f1 = __uint_as_float(r[2 * j + 1]) * s1;
-                        } else {
-                            f0 = (float)(int32_t)r[2 * j] * s0;
-                            f1 = (float)(int32_t)r[2 * j + 1] * s1;
-                        }
-                        if (a.flags & RWKVQ_FLAG_OUT_VIA_BF16) { f0 = bf16_round(f0); f1 = bf16_round(f1); }
-                        __half2 hh = __floats2half2_rn(f0, f1);
-                        if (relu2) {
-                            // the engine's relu_square on the fp16 result, fp32 arithmetic; its maximum (over the bf16-rounded
-                            // values where the consumer takes its amax there) goes to the projection that follows
-                            const float2 y = __half22float2(hh);
-                            const float v0 = fmaxf(y.x, 0.f), v1 = fmaxf(y.y, 0.f);
-                            hh = __floats2half2_rn(v0 * v0, v1 * v1);
-                            if (n0 + 2 * j < a.N) {
-                                const float2 hv = __half22float2(hh);
-                                hmax = fmaxf(hmax, hmax_bf16 ? bf16_round(hv.x) : hv.x);
-                                if (n0 + 2 * j + 1 < a.N) hmax = fmaxf(hmax, hmax_bf16 ? bf16_round(hv.y) : hv.y);
-                            }
-                        }
-                        h[j] = *reinterpret_cast<const uint32_t*>(&hh);
-                    }
-                };
                 if (a.push.n > 0) {
                     // column-split projection with the all-gather riding in this epilogue (TcPush in tc_host.cuh)
                     uint8_t* stg = ring + (size_t)a.stages * stage_bytes + (size_t)(warp - 2) * kTcStgWarp;
-                    const bool vec8 = vec_ok && a.N % 8 == 0;
+                    const bool vec8 = e.vec_ok && a.N % 8 == 0;
                     for (int c0 = 0; c0 < a.NB; c0 += 64) {
 #pragma unroll
                         for (int cc = 0; cc < 4; ++cc) {
                             uint32_t r[16], h[8];
                             tmem_ld16(taddr + c0 + cc * 16, r);
                             tmem_ld_wait();
-                            convert16(r, p.qrow + c0 + cc * 16, h);
+                            epi_convert16<KIND, EPI_ANY>(e, r, p.qrow + c0 + cc * 16, h, hmax);
                             uint4* d = reinterpret_cast<uint4*>(stg + lane * kTcStgRow + cc * 32);
                             d[0] = make_uint4(h[0], h[1], h[2], h[3]);
                             d[1] = make_uint4(h[4], h[5], h[6], h[7]);
@@ -580,32 +560,9 @@ __global__ void __launch_bounds__(kTcThreads, SWAP ? 2 : 1) gemm_tc_kernel(const
                         push_store_rows(a.push, stg, a.out[p.mat], a.ldo, p.prow + q * 32, p.qrow + c0, a.M, a.N, vec8, lane);
                         __syncwarp();
                     }
-                } else
-                for (int c0 = 0; c0 < a.NB; c0 += 16) {
-                    uint32_t r[16];
-                    tmem_ld16(taddr + c0, r);
-                    tmem_ld_wait();
-                    const int n0 = p.qrow + c0;
-                    if (m < a.M && n0 < a.N) {
-                        uint32_t h[8];
-                        convert16(r, n0, h);
-                        __half* o = a.out[p.mat] + (int64_t)m * a.ldo + n0;
-                        if (vec_ok && n0 + 16 <= a.N) {
-                            reinterpret_cast<uint4*>(o)[0] = make_uint4(h[0], h[1], h[2], h[3]);
-                            reinterpret_cast<uint4*>(o)[1] = make_uint4(h[4], h[5], h[6], h[7]);
-                        } else {
-#pragma unroll
-                            for (int j = 0; j < 16; ++j)
-                                if (n0 + j < a.N) o[j] = __ushort_as_half((unsigned short)((h[j >> 1] >> ((j & 1) * 16)) & 0xffff));
-                        }
-                        if constexpr (KIND == KIND_I8) {
-                            if (a.acc[p.mat]) {
-#pragma unroll
-                                for (int j = 0; j < 16; ++j)
-                                    if (n0 + j < a.N) a.acc[p.mat][(int64_t)m * a.ldacc + n0 + j] = (int32_t)r[j];
-                            }
-                        }
-                    }
+                } else {
+                    const int hc = a.NB >> 1, c0 = (warp - 2) >= 4 ? hc : 0;
+                    epi_tile<KIND>(e, taddr + c0, p.qrow + c0, hc, hmax);
                 }
                 tc_fence_before_sync();
                 __syncwarp();
@@ -791,13 +748,18 @@ static int32_t run_tc(TcArgs a, const TcCall& c, cudaStream_t st, const char* wh
         a.status = a.counters + kWsCounterInts;
         a.scratch = reinterpret_cast<float*>(reinterpret_cast<char*>(c.workspace) + kWsHeaderBytes);
     } else {
-        if (!pushing && tc2_eligible(c.kind, a.M, a.N, a.K, a.nmat) && !(c.kind == KIND_I8 && (a.flags & RWKVQ_FLAG_RELU2)))      // many tokens: CTA pairs on 256 x 256 tiles (gemm_tc2.cu)
-            return run_tc2(c.kind, c.codes[0], c.lda, a.a_scale[0], a.amax_is_amax, c.w[0], c.ldw, a.ws[0], a.out[0], a.ldo, a.acc[0], a.ldacc,
-                           a.M, a.N, a.K, a.div_mode, a.flags, a.ffn_amax,
-                           c.workspace ? reinterpret_cast<int*>(c.workspace) + kWsCounterInts : device_status_ptr(), st, who);
         // 256 weight rows per tile; narrower tiles while halving them still leaves no more tiles than SMs
         a.NB = 256;
         while (a.NB > 64 && 2 * (int64_t)a.nmat * ((a.M + kTileP - 1) / kTileP) * ((a.N + a.NB - 1) / a.NB) <= tc_grid()) a.NB >>= 1;
+        if (!pushing && tc2_eligible(c.kind, a.M, a.N, a.K, a.nmat, a.NB)) {      // CTA pairs on 256 x 256 tiles (gemm_tc2.cu)
+            Tc2Call t{};
+            t.kind = c.kind; t.nmat = a.nmat; t.amax_is_amax = a.amax_is_amax; t.M = a.M; t.N = a.N; t.K = a.K; t.div_mode = a.div_mode; t.flags = a.flags;
+            for (int i = 0; i < a.nmat; ++i) {
+                t.codes[i] = c.codes[i]; t.w[i] = c.w[i]; t.a_scale[i] = a.a_scale[i]; t.ws[i] = a.ws[i]; t.out[i] = a.out[i]; t.acc[i] = a.acc[i];
+            }
+            t.ffn_amax = a.ffn_amax; t.lda = c.lda; t.ldw = c.ldw; t.ldo = a.ldo; t.ldacc = a.ldacc;
+            return run_tc2(t, c.workspace ? reinterpret_cast<int*>(c.workspace) + kWsCounterInts : device_status_ptr(), st, who);
+        }
         a.ptiles = (a.M + kTileP - 1) / kTileP;
         a.qtiles = (a.N + a.NB - 1) / a.NB;
         grid = (int)std::min<int64_t>(tc_grid(), (int64_t)a.nmat * a.ptiles * a.qtiles);

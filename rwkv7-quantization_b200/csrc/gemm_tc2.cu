@@ -7,8 +7,8 @@
 // tile from the two CTAs' shared memory and accumulates each CTA's 128 x 256 block in that CTA's own tensor memory.
 // No multicast is involved: every TMA load lands in the shared memory of the CTA that issued it.
 //
-// Roles per CTA as in gemm_tc.cu: warp 0 = TMA producer (one lane), warp 1 = tensor-memory owner and -- in the leader
-// CTA only -- MMA issuer, warps 2-5 = epilogue.  Barriers: full[] lives in the leader (both producers' bytes are
+// Roles per CTA as in gemm_tc.cu: warp 0 = TMA producer, warp 1 = tensor-memory owner and -- in the leader CTA only --
+// MMA issuer (one elected lane each), warps 2-9 = epilogue (tc_epilogue.cuh).  Barriers: full[] lives in the leader (both producers' bytes are
 // counted there: the loads carry .cta_group::2 and name the leader's barrier), empty[] and tfull[] are signalled in both
 // CTAs at once by a multicast tcgen05.commit, tempty[] of the leader collects the arrivals of both CTAs' epilogue warps.
 // Every wait is bounded; the pair meets at a cluster barrier before the tensor memory is released.
@@ -16,6 +16,7 @@
 #include <cstdlib>
 
 #include "tc_common.cuh"
+#include "tc_epilogue.cuh"
 #include "tc_host.cuh"
 #include "w8a8.cuh"
 
@@ -31,20 +32,20 @@ constexpr uint32_t kT2StageBytes = 2 * kT2TileBytes;       // tokens + this CTA'
 constexpr int kT2N = 256;                     // weight rows per pair tile (UMMA N)
 
 struct Tc2Maps {
-    CUtensorMap a;      // activation codes [M, K], box 128 rows x 128 bytes
-    CUtensorMap w;      // weights [N, K], box 128 rows x 128 bytes
+    CUtensorMap a[3];   // activation codes [M, K], box 128 rows x 128 bytes
+    CUtensorMap w[3];   // weights [N, K], box 128 rows x 128 bytes
 };
 
 struct Tc2Args {
-    const float* a_scale;      // FP8 amax-or-scale [1]; INT8 row scales [M]
-    const float* ws;           // weight scale: one value, or N with RWKVQ_FLAG_WSCALE_PER_ROW
-    __half* out;
-    int32_t* acc;              // INT8: optional raw accumulators
-    float* ffn_amax;           // RWKVQ_FLAG_RELU2: maximum of the relu^2 results
+    const float* a_scale[3];   // FP8 amax-or-scale [1]; INT8 row scales [M]
+    const float* ws[3];        // weight scale: one value, or N with RWKVQ_FLAG_WSCALE_PER_ROW
+    __half* out[3];
+    int32_t* acc[3];           // INT8: optional raw accumulators
+    float* ffn_amax;           // RWKVQ_FLAG_RELU2: maximum of the relu^2 results -- FP8: one word; INT8: one per token row
     int* status;
     unsigned long long wait_ns;
     int64_t ldo, ldacc;
-    int M, N, K;
+    int M, N, K, nmat;
     int kchunks, ptiles, qtiles, stages;      // ptiles: 256-token pair tiles, qtiles: 256-row weight tiles
     int div_mode, amax_is_amax;
     uint32_t flags;
@@ -122,7 +123,7 @@ __global__ void __launch_bounds__(kT2Threads, 1) gemm_tc2_kernel(const __grid_co
     const int warp = warp_uniform((int)(threadIdx.x >> 5)), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();          // 0 = leader of the pair
     const int pair = (int)(blockIdx.x >> 1), npairs = (int)(gridDim.x >> 1);
-    const int total = a.ptiles * a.qtiles;
+    const int per_mat = a.ptiles * a.qtiles, total = a.nmat * per_mat;
     constexpr uint32_t kCols = 512;                   // two 256-column accumulators
 
     griddep_launch_dependents();
@@ -133,14 +134,16 @@ __global__ void __launch_bounds__(kT2Threads, 1) gemm_tc2_kernel(const __grid_co
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(&s.tfull[i], 1);
-            mbar_init(&s.tempty[i], 8);               // four epilogue warps of each CTA (used in the leader only)
+            mbar_init(&s.tempty[i], 16);              // eight epilogue warps of each CTA (used in the leader only)
         }
-        mbar_init(&s.done, 4);
+        mbar_init(&s.done, 8);
         s.abort_flag = 0;
         fence_barrier_init();
         fence_proxy_async();
-        prefetch_tmap(&maps.a);
-        prefetch_tmap(&maps.w);
+        for (int i = 0; i < a.nmat; ++i) {
+            prefetch_tmap(&maps.a[i]);
+            prefetch_tmap(&maps.w[i]);
+        }
     }
     if (warp == 1) tmem_alloc_pair(&s.tmem_base, kCols);
     tc_fence_before_sync();
@@ -151,30 +154,50 @@ __global__ void __launch_bounds__(kT2Threads, 1) gemm_tc2_kernel(const __grid_co
     const volatile int* abort_flag = &s.abort_flag;
 
     auto tile_rows = [&](int t, int& mrow, int& nrow) {       // token tiles fastest: the pairs running together share weight tiles
+        const int mat = (t >= per_mat) + (t >= 2 * per_mat);
+        t -= mat * per_mat;
         mrow = (t % a.ptiles) * 256;
         nrow = (t / a.ptiles) * kT2N;
+        return mat;
     };
 
     if (warp == 0) {
         // ============================== TMA producer (both CTAs; the warp walks the loop, one lane issues) ==============================
         {
             const bool issuer = elect_one();
+            // first pass over the ring: the weights do not depend on the kernel in front, so they are requested before the
+            // dependency wait of programmatic dependent launch
+            int npre = 0;
+            for (int t = pair; t < total && npre < a.stages; t += npairs) {
+                int mrow, nrow;
+                const int mat = tile_rows(t, mrow, nrow);
+                for (int kc = 0; kc < a.kchunks && npre < a.stages; ++kc, ++npre) {
+                    if (!issuer) continue;
+                    if (rank == 0) mbar_expect_tx(&s.full[npre], 2 * kT2StageBytes);
+                    tma_load_2d_pair(ring + (size_t)npre * kT2StageBytes + kT2TileBytes, &maps.w[mat], kc * kT2Chunk, nrow + (int)rank * kT2Rows,
+                                     smem_u32(&s.full[npre]) & 0xFEFFFFFFu);
+                }
+            }
             griddep_wait();                           // the activation codes come from the previous kernel
             RingPos rp;
             bool ok = true;
             for (int t = pair; t < total && ok; t += npairs) {
                 int mrow, nrow;
-                tile_rows(t, mrow, nrow);
+                const int mat = tile_rows(t, mrow, nrow);
                 for (int kc = 0; kc < a.kchunks; ++kc, rp.next(a.stages)) {
                     const int st = rp.i;
-                    ok = __all_sync(0xffffffffu, mbar_wait(&s.empty[st], rp.phase ^ 1, abort_flag, a.wait_ns));
+                    const bool refill = --npre < 0;
+                    if (refill) ok = mbar_wait(&s.empty[st], rp.phase ^ 1, abort_flag, a.wait_ns);
+                    ok = __all_sync(0xffffffffu, ok);
                     if (!ok) { t2_abort(s, a); break; }
                     uint8_t* dst = ring + (size_t)st * kT2StageBytes;
                     if (issuer) {
-                        if (rank == 0) mbar_expect_tx(&s.full[st], 2 * kT2StageBytes);          // the four tiles of the pair
                         const uint32_t leader_bar = smem_u32(&s.full[st]) & 0xFEFFFFFFu;         // the barrier of the even CTA
-                        tma_load_2d_pair(dst, &maps.a, kc * kT2Chunk, mrow + (int)rank * kT2Rows, leader_bar);
-                        tma_load_2d_pair(dst + kT2TileBytes, &maps.w, kc * kT2Chunk, nrow + (int)rank * kT2Rows, leader_bar);
+                        if (refill) {
+                            if (rank == 0) mbar_expect_tx(&s.full[st], 2 * kT2StageBytes);      // the four tiles of the pair
+                            tma_load_2d_pair(dst + kT2TileBytes, &maps.w[mat], kc * kT2Chunk, nrow + (int)rank * kT2Rows, leader_bar);
+                        }
+                        tma_load_2d_pair(dst, &maps.a[mat], kc * kT2Chunk, mrow + (int)rank * kT2Rows, leader_bar);
                     }
                 }
             }
@@ -212,95 +235,48 @@ __global__ void __launch_bounds__(kT2Threads, 1) gemm_tc2_kernel(const __grid_co
                 }
             }
         }
-    } else if (warp < 6) {
+    } else {
         // ============================== epilogue (both CTAs, each its own 128 token rows) ==============================
         griddep_wait();
         const int q = warp & 3;                         // tensor-memory lane quarter this warp may read
+        const int half = (warp - 2) >> 2;               // its half of the tile's columns
         const int row_l = q * 32 + lane;
-        const bool per_row = (a.flags & RWKVQ_FLAG_WSCALE_PER_ROW) != 0;
-        const bool relu2 = KIND == KIND_F8 && (a.flags & RWKVQ_FLAG_RELU2) != 0;
-        const bool hmax_bf16 = (a.flags & RWKVQ_FLAG_AMAX_AFTER_BF16) != 0;
-        const float wsc = a.ws[0];
         const uint32_t leader_tempty[2] = {mapa_u32(smem_u32(&s.tempty[0]), 0), mapa_u32(smem_u32(&s.tempty[1]), 0)};
-        const bool vec_ok = (a.ldo % 8 == 0) && ((reinterpret_cast<uintptr_t>(a.out) & 15) == 0);
-        uint32_t pc = 0;
-        for (int t = pair; t < total; t += npairs, ++pc) {
-            const int buf = pc & 1;
-            if (!mbar_wait(&s.tfull[buf], (pc >> 1) & 1, abort_flag, a.wait_ns)) { t2_abort(s, a); break; }
-            tc_fence_after_sync();
+        RingPos fp;
+        for (int t = pair; t < total; t += npairs, fp.next(2)) {
             int mrow, nrow;
-            tile_rows(t, mrow, nrow);
+            const int mat = tile_rows(t, mrow, nrow);
             const int m = mrow + (int)rank * kT2Rows + row_l;
-            const uint32_t taddr = tmem_base + (uint32_t)(buf * kT2N) + ((uint32_t)(q * 32) << 16);
-            float actscale;
+            // what the tile needs from global memory is fetched while its MMAs still run
+            EpiRow e;
             if constexpr (KIND == KIND_F8) {
-                const float am = a.a_scale[0];
-                actscale = a.amax_is_amax ? div_mode_f32(fmaxf(am, 1e-12f), 448.f, a.div_mode) : am;
+                const float am = a.a_scale[mat][0];
+                e.actscale = a.amax_is_amax ? div_mode_f32(fmaxf(am, 1e-12f), 448.f, a.div_mode) : am;
             } else {
-                actscale = m < a.M ? a.a_scale[m] : 0.f;
+                e.actscale = m < a.M ? a.a_scale[mat][m] : 0.f;
             }
-            const float rowscale = actscale * wsc;
+            e.ws = a.ws[mat];
+            e.rowscale = e.actscale * e.ws[0];
+            e.out = a.out[mat] + (int64_t)m * a.ldo;
+            e.acc = KIND == KIND_I8 && a.acc[mat] ? a.acc[mat] + (int64_t)m * a.ldacc : nullptr;
+            e.N = a.N;
+            e.live = m < a.M;
+            e.vec_ok = (a.ldo % 8 == 0) && ((reinterpret_cast<uintptr_t>(a.out[mat]) & 15) == 0);
+            e.flags = a.flags;
+            if (!mbar_wait(&s.tfull[fp.i], fp.phase, abort_flag, a.wait_ns)) { t2_abort(s, a); break; }
+            tc_fence_after_sync();
             float hmax = 0.f;
-            for (int c0 = 0; c0 < kT2N; c0 += 16) {
-                uint32_t r[16];
-                tmem_ld16(taddr + c0, r);
-                tmem_ld_wait();
-                const int n0 = nrow + c0;
-                if (m < a.M && n0 < a.N) {
-                    uint32_t h[8];
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        float s0 = rowscale, s1 = rowscale;
-                        if (per_row) {
-                            s0 = actscale * a.ws[min(n0 + 2 * j, a.N - 1)];
-                            s1 = actscale * a.ws[min(n0 + 2 * j + 1, a.N - 1)];
-                        }
-                        float f0, f1;
-                        if constexpr (KIND == KIND_F8) {
-                            f0 = __uint_as_float(r[2 * j]) * s0;
-                            f1 = __uint_as_float(r[2 * j + 1]) * s1;
-                        } else {
-                            f0 = (float)(int32_t)r[2 * j] * s0;
-                            f1 = (float)(int32_t)r[2 * j + 1] * s1;
-                        }
-                        if (a.flags & RWKVQ_FLAG_OUT_VIA_BF16) { f0 = bf16_round(f0); f1 = bf16_round(f1); }
-                        __half2 hh = __floats2half2_rn(f0, f1);
-                        if (relu2) {        // the engine's relu_square on the fp16 result; its maximum goes to the next projection
-                            const float2 y = __half22float2(hh);
-                            const float v0 = fmaxf(y.x, 0.f), v1 = fmaxf(y.y, 0.f);
-                            hh = __floats2half2_rn(v0 * v0, v1 * v1);
-                            if (n0 + 2 * j < a.N) {
-                                const float2 hv = __half22float2(hh);
-                                hmax = fmaxf(hmax, hmax_bf16 ? bf16_round(hv.x) : hv.x);
-                                if (n0 + 2 * j + 1 < a.N) hmax = fmaxf(hmax, hmax_bf16 ? bf16_round(hv.y) : hv.y);
-                            }
-                        }
-                        h[j] = *reinterpret_cast<const uint32_t*>(&hh);
-                    }
-                    __half* o = a.out + (int64_t)m * a.ldo + n0;
-                    if (vec_ok && n0 + 16 <= a.N) {
-                        reinterpret_cast<uint4*>(o)[0] = make_uint4(h[0], h[1], h[2], h[3]);
-                        reinterpret_cast<uint4*>(o)[1] = make_uint4(h[4], h[5], h[6], h[7]);
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 16; ++j)
-                            if (n0 + j < a.N) o[j] = __ushort_as_half((unsigned short)((h[j >> 1] >> ((j & 1) * 16)) & 0xffff));
-                    }
-                    if constexpr (KIND == KIND_I8) {
-                        if (a.acc) {
-#pragma unroll
-                            for (int j = 0; j < 16; ++j)
-                                if (n0 + j < a.N) a.acc[(int64_t)m * a.ldacc + n0 + j] = (int32_t)r[j];
-                        }
-                    }
-                }
-            }
+            epi_tile<KIND>(e, tmem_base + (uint32_t)(fp.i * kT2N) + ((uint32_t)(q * 32) << 16) + half * (kT2N / 2), nrow + half * (kT2N / 2), kT2N / 2, hmax);
             tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(leader_tempty[buf]);        // this accumulator may be overwritten
-            if (relu2) {
-                hmax = warp_max(hmax);
-                if (lane == 0 && hmax > 0.f) atomic_max_nonneg(a.ffn_amax, hmax);
+            if (lane == 0) mbar_arrive_cluster(leader_tempty[fp.i]);       // this accumulator may be overwritten
+            if (a.flags & RWKVQ_FLAG_RELU2) {
+                if constexpr (KIND == KIND_F8) {
+                    hmax = warp_max(hmax);
+                    if (lane == 0 && hmax > 0.f) atomic_max_nonneg(a.ffn_amax, hmax);
+                } else {                                 // INT8 scales its activations per row
+                    if (m < a.M && hmax > 0.f) atomic_max_nonneg(a.ffn_amax + m, hmax);
+                }
             }
         }
         tc_fence_before_sync();
@@ -328,39 +304,51 @@ static int t2_grid_pairs() { return std::max(1, sm_count() / 2); }
 // tokens on, -2..5 % at 2048 (same number of waves, deeper pipeline to fill) -- so the L2 -> shared-memory traffic it
 // halves is not what limits that kernel (under the 1 kW power cap both run at 2.2-2.5 PFLOP/s).  It is therefore used
 // from RWKVQ_TC2_MIN_M tokens on (default 4096; RWKVQ_TC2=0 switches it off, RWKVQ_TC2_MIN_M=129 uses it wherever it fits).
-bool tc2_eligible(int kind, int64_t M, int64_t N, int64_t K, int nmat) {
+// Pairs or single CTAs?  Both run waves of tiles whose MMAs take as long (256 x 256 on a pair, 128 x 256 on a CTA), but a pair
+// loads 64 KB for a step of its tile, two single CTAs 96 KB, and an SM's intake from L2 bounds the single form.  Measured per
+// 128-byte step of K: 0.385 us on pairs, 0.41 / 0.30 / 0.24 us on single CTAs with 256 / 128 / 64 weight rows per tile (few
+// tiles); a pair launch costs 0.9 us more (cluster set-up, one more barrier).  Measured, us, single / pairs: FP8 [16384, 4096]
+// 384 rows 32.8 / 29.8, 2048 rows 109.3 / 98.8; [4096, 16384] 717 rows 51.7 / 48.5; [4096, 4096] 1024 rows 16.6 / 17.0; [2560, 2560]
+// 1500 rows 12.8 / 13.5, 2048 rows 20.8 / 19.1.  INT8 [16384, 4096] 2048 rows 100.7 / 89.9.
+bool tc2_eligible(int kind, int64_t M, int64_t N, int64_t K, int nmat, int single_nb) {
     static const int64_t min_m = [] {
         const char* off = std::getenv("RWKVQ_TC2");
         if (off && off[0] == '0') return (int64_t)1 << 62;
         const char* e = std::getenv("RWKVQ_TC2_MIN_M");
-        const long long v = e ? std::atoll(e) : 4096;
+        const long long v = e ? std::atoll(e) : 129;
         return (int64_t)std::max<long long>(v, 129);
     }();
-    if (nmat != 1 || M < min_m || N < kT2N || K % 16) return false;
-    const int64_t tiles = ((M + 255) / 256) * ((N + kT2N - 1) / kT2N);
-    return tiles >= t2_grid_pairs() / 2 && (kind == KIND_F8 || kind == KIND_I8);
+    if (M < min_m || N < kT2N || K % 16 || (kind != KIND_F8 && kind != KIND_I8)) return false;
+    const int64_t pairs = t2_grid_pairs(), tiles = nmat * ((M + 255) / 256) * ((N + kT2N - 1) / kT2N);
+    const int64_t single = nmat * ((M + 127) / 128) * ((N + single_nb - 1) / single_nb);
+    const double kc = (double)((K + kT2Chunk - 1) / kT2Chunk), step1 = single_nb > 128 ? 0.41 : (single_nb > 64 ? 0.30 : 0.24);
+    const double t2 = (double)((tiles + pairs - 1) / pairs) * kc * 0.385 + 0.9, t1 = (double)((single + 2 * pairs - 1) / (2 * pairs)) * kc * step1;
+    return t2 <= t1;
 }
 
-int32_t run_tc2(int kind, const void* codes, int64_t lda, const float* a_scale, int amax_is_amax, const void* w, int64_t ldw, const float* ws,
-                __half* out, int64_t ldo, int32_t* acc, int64_t ldacc, int M, int N, int K, int div_mode, uint32_t flags, float* ffn_amax,
-                int* status, cudaStream_t st, const char* who) {
+int32_t run_tc2(const Tc2Call& c, int* status, cudaStream_t st, const char* who) {
     Tc2Args a{};
-    a.a_scale = a_scale; a.ws = ws; a.out = out; a.acc = acc; a.ffn_amax = ffn_amax; a.status = status; a.wait_ns = wait_limit_ns();
-    a.ldo = ldo; a.ldacc = ldacc; a.M = M; a.N = N; a.K = K; a.div_mode = div_mode; a.amax_is_amax = amax_is_amax; a.flags = flags;
-    a.kchunks = (K + kT2Chunk - 1) / kT2Chunk;
-    a.ptiles = (M + 255) / 256;
-    a.qtiles = (N + kT2N - 1) / kT2N;
+    const int kind = c.kind;
+    a.ffn_amax = c.ffn_amax; a.status = status; a.wait_ns = wait_limit_ns();
+    a.ldo = c.ldo; a.ldacc = c.ldacc; a.M = c.M; a.N = c.N; a.K = c.K; a.nmat = c.nmat; a.div_mode = c.div_mode; a.amax_is_amax = c.amax_is_amax; a.flags = c.flags;
+    a.kchunks = (c.K + kT2Chunk - 1) / kT2Chunk;
+    a.ptiles = (c.M + 255) / 256;
+    a.qtiles = (c.N + kT2N - 1) / kT2N;
     a.stages = kT2MaxStages;
     const size_t smem = (size_t)a.stages * kT2StageBytes + 1024;
     Tc2Maps maps;
-    int32_t rc = make_map(&maps.a, codes, M, K, lda, kT2Rows, who);
-    if (rc) return rc;
-    rc = make_map(&maps.w, w, N, K, ldw, kT2Rows, who);
-    if (rc) return rc;
+    int32_t rc;
+    for (int i = 0; i < c.nmat; ++i) {
+        a.a_scale[i] = c.a_scale[i]; a.ws[i] = c.ws[i]; a.out[i] = c.out[i]; a.acc[i] = c.acc[i];
+        rc = make_map(&maps.a[i], c.codes[i], c.M, c.K, c.lda, kT2Rows, who);
+        if (rc) return rc;
+        rc = make_map(&maps.w[i], c.w[i], c.N, c.K, c.ldw, kT2Rows, who);
+        if (rc) return rc;
+    }
     const void* kern = kind == KIND_F8 ? (const void*)gemm_tc2_kernel<KIND_F8> : (const void*)gemm_tc2_kernel<KIND_I8>;
     rc = ensure_smem_optin(kern, (int)smem, who);
     if (rc) return rc;
-    const int pairs = (int)std::min<int64_t>(t2_grid_pairs(), (int64_t)a.ptiles * a.qtiles);
+    const int pairs = (int)std::min<int64_t>(t2_grid_pairs(), (int64_t)a.nmat * a.ptiles * a.qtiles);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)(2 * pairs));
     cfg.blockDim = dim3(kT2Threads);

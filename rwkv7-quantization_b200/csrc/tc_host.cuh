@@ -119,12 +119,22 @@ __device__ __forceinline__ void push_store_rows(const TcPush& p, const uint8_t* 
 }
 #endif
 
-// W8A8 GEMM on CTA pairs (gemm_tc2.cu): eligibility (many tokens, enough 256 x 256 tiles to fill the pairs, not switched
-// off with RWKVQ_TC2=0) and the launch.  kind: tc::KIND_F8 / tc::KIND_I8.
-bool tc2_eligible(int kind, int64_t M, int64_t N, int64_t K, int nmat);
-int32_t run_tc2(int kind, const void* codes, int64_t lda, const float* a_scale, int amax_is_amax, const void* w, int64_t ldw, const float* ws,
-                __half* out, int64_t ldo, int32_t* acc, int64_t ldacc, int M, int N, int K, int div_mode, uint32_t flags, float* ffn_amax,
-                int* status, cudaStream_t st, const char* who);
+// W8A8 GEMM on CTA pairs (gemm_tc2.cu): whether it is the better form (single_nb: weight rows per tile of the single-CTA form
+// for these sizes; RWKVQ_TC2=0 switches it off) and the launch, for one matrix or r, k, v.  kind: tc::KIND_F8 / tc::KIND_I8.
+struct Tc2Call {
+    int kind, nmat, amax_is_amax, M, N, K, div_mode;
+    uint32_t flags;
+    const void* codes[3];
+    const void* w[3];
+    const float* a_scale[3];
+    const float* ws[3];
+    __half* out[3];
+    int32_t* acc[3];
+    float* ffn_amax;
+    int64_t lda, ldw, ldo, ldacc;
+};
+bool tc2_eligible(int kind, int64_t M, int64_t N, int64_t K, int nmat, int single_nb);
+int32_t run_tc2(const Tc2Call& c, int* status, cudaStream_t st, const char* who);
 
 // NVFP4 GEMM for few tokens (up to 256) on the cluster split-K kernel of gemm_tc.cu (gemm_tcs.cuh): weights = the
 // 128-row operand, K split across a thread-block cluster, partial sums through distributed shared memory.
