@@ -12,9 +12,11 @@
 // 2048 contiguous bytes, fetched by one bulk copy onto the same mbarrier as the code tiles.
 //
 // One persistent CTA per SM: warp 0 = producer (one lane), warp 1 = MMA issuer (one lane) and owner of the
-// tensor-memory allocation, warps 2-5 = epilogue (one lane quarter each).  Tile 128 tokens x BN weight rows;
+// tensor-memory allocation, warps 2-9 = epilogue (two per lane quarter).  Tile 128 tokens x BN weight rows;
 // BN = 128 keeps two accumulators in tensor memory so the epilogue of a tile overlaps the MMAs of the next,
-// BN = 256 keeps one.  Every mbarrier wait is bounded; a timeout is reported through the status word.
+// BN = 256 keeps one, whose epilogue is exposed: eight warps read it before they convert and store anything.  Measured,
+// us, one lane walking the loops and four epilogue warps -> here: [4096, 4096] 2048 rows 31.3 -> 20.2, [16384, 4096] 105.3 -> 67.4,
+// [4096, 16384] 101.4 -> 58.5 (4.7 PFLOP/s), [2560, 2560] 512 rows 9.9 -> 7.3.  Every mbarrier wait is bounded; a timeout is reported through the status word.
 //
 // The format is described in the reference's reports (iterations/phase1_nvfp4_exploration/reports/
 // 03_fused_kernel_en.md:22-34, 11_fused_gemm_ops_en.md:20-26); the reference ships no code for it.
@@ -29,7 +31,7 @@
 namespace rwkvq {
 using namespace tc;
 
-constexpr int kNfThreads = 192;
+constexpr int kNfThreads = 320;
 constexpr int kNfMaxStages = 8;
 constexpr uint32_t kNfRowBytes = 128;                       // packed codes of one row per stage (256 values of k)
 constexpr uint32_t kNfABytes = kNfTileM * kNfRowBytes;      // 16 KiB
@@ -71,6 +73,7 @@ template <int BN, bool PUSH = false>
 __global__ void __launch_bounds__(kNfThreads, 1) gemm_tc_nvfp4_kernel(const __grid_constant__ NfMaps maps, const NfArgs a) {
     constexpr int NACC = BN == 128 ? 2 : 1;
     constexpr int NH = BN / 128;                                   // 128-row scale tiles of the B operand
+    constexpr int kEpi = PUSH ? 4 : 8;                             // epilogue warps (PUSH: one staging area per lane quarter)
     constexpr uint32_t kBBytes = BN * kNfRowBytes;
     constexpr uint32_t kStage = kNfABytes + kBBytes + kNfSfStage * (1 + NH);
     extern __shared__ uint8_t smem_raw[];
@@ -86,9 +89,9 @@ __global__ void __launch_bounds__(kNfThreads, 1) gemm_tc_nvfp4_kernel(const __gr
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(&s.tfull[i], 1);
-            mbar_init(&s.tempty[i], 4);
+            mbar_init(&s.tempty[i], kEpi);
         }
-        mbar_init(&s.done, 4);
+        mbar_init(&s.done, kEpi);
         s.abort_flag = 0;
         fence_barrier_init();
         fence_proxy_async();
@@ -197,7 +200,7 @@ __global__ void __launch_bounds__(kNfThreads, 1) gemm_tc_nvfp4_kernel(const __gr
                 }
             }
         }
-    } else {
+    } else if (warp < 2 + kEpi) {
         // ============================== epilogue ==============================
         griddep_wait();
         const int q = warp & 3;                         // tensor-memory lane quarter this warp may read
@@ -236,13 +239,11 @@ __global__ void __launch_bounds__(kNfThreads, 1) gemm_tc_nvfp4_kernel(const __gr
                     __syncwarp();
                 }
             } else {
-#pragma unroll 2
-            for (int c0 = 0; c0 < BN; c0 += 16) {
-                uint32_t r[16];
-                tmem_ld16(taddr + c0, r);
-                tmem_ld_wait();
-                const int n0 = nt * BN + c0;
-                if (m < a.M && n0 < a.N) {
+                // two warps per lane quarter, half of the tile's columns each, two tensor-memory loads under way: with one
+                // accumulator (BN = 256) the next tile's MMAs wait for this
+                const int h0 = (warp - 2) >= 4 ? BN / 2 : 0;
+                auto store16 = [&](const uint32_t (&r)[16], int n0) {
+                    if (m >= a.M || n0 >= a.N) return;
                     uint32_t h[8];
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
@@ -258,12 +259,27 @@ __global__ void __launch_bounds__(kNfThreads, 1) gemm_tc_nvfp4_kernel(const __gr
                         for (int j = 0; j < 16; ++j)
                             if (n0 + j < a.N) o[j] = __ushort_as_half((unsigned short)((h[j >> 1] >> ((j & 1) * 16)) & 0xffff));
                     }
+                };
+#pragma unroll
+                for (int c0 = h0; c0 < h0 + BN / 2; c0 += 64) {
+                    uint32_t r[4][16];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) tmem_ld16(taddr + c0 + i * 16, r[i]);
+                    tmem_ld_wait();
+                    if (c0 + 64 == h0 + BN / 2) {            // the accumulator has been read: the next tile may start
+                        tc_fence_before_sync();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&s.tempty[buf]);
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) store16(r[i], nt * BN + c0 + i * 16);
                 }
             }
+            if constexpr (PUSH) {
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&s.tempty[buf]);
             }
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&s.tempty[buf]);
         }
         if constexpr (PUSH) __threadfence_system();      // this thread's peer stores are ordered before its arrival below
         tc_fence_before_sync();
