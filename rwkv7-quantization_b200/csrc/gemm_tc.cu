@@ -722,9 +722,9 @@ static int32_t run_tc(TcArgs a, const TcCall& c, cudaStream_t st, const char* wh
     a.kchunks = (a.K + kChunk - 1) / kChunk;
     const bool pushing = a.push.n > 0 || a.push.counter != nullptr;
     if (pushing)
-        RWKVQ_REQUIRE(!c.fused && a.nmat == 1 && !swap && !tcs_eligible(a.M, a.N, a.K, a.flags, 1) && !(a.flags & RWKVQ_FLAG_RELU2) && a.acc[0] == nullptr,
+        RWKVQ_REQUIRE(!c.fused && a.nmat == 1 && !swap && !tcs_eligible(KIND_F8, a.M, a.N, a.K, a.flags, 1) && !(a.flags & RWKVQ_FLAG_RELU2) && a.acc[0] == nullptr,
                       RWKVQ_E_SHAPE, "%s: %d rows run a kernel that cannot carry the all-gather (see rwkvq_tc_gemm_can_push)", who, a.M);
-    if (!pushing && !c.fused && tcs_eligible(a.M, a.N, a.K, a.flags, a.nmat)) {
+    if (!pushing && !c.fused && tcs_eligible(c.kind, a.M, a.N, a.K, a.flags, a.nmat)) {
         a.status = nullptr;
         return run_tcs(a, c, st, who);
     }
@@ -800,10 +800,12 @@ bool tcs_nvfp4_eligible(int64_t M, int64_t N, int64_t K) {
     const int min_c = env ? std::atoi(env) : 0;
     static const int on = std::getenv("RWKVQ_TCS") ? std::atoi(std::getenv("RWKVQ_TCS")) : 1;
     if (!on || M < 1 || M > kTcsMaxM || K % 256 || K < 2048) return false;
-    // measured on the 7.2B shapes: with 128 row tiles (N = 16384) a cluster of two wins up to 32 tokens (16 tokens:
-    // 14.7 against 18.5 us) and loses at 64 (23.9 against 22.1 us); from 65 tokens on a cluster of two wins again (FFN
-    // value, 256 tokens: 57 -> 40 us)
-    return tcs_cluster_size(M, N, K / 2) >= (min_c > 0 ? min_c : (M > 32 && M <= 64 ? 4 : 2));
+    // measured, us, cluster / tiled: up to 32 tokens a cluster of two is enough ([16384, 4096] 16 tokens 9.3 / 12.4), at 64 it takes
+    // four ([4096, 4096] 6.7 / 7.4; two: [8192, 2048] 7.2 / 5.4), above that a long K ([4096, 16384] 128 tokens 13.7 / 23.8) or
+    // four again ([4096, 4096] 128 tokens 8.2 / 8.4; two, 256 tokens: 10.3 / 8.7; K = 2048: [2048, 2048] 7.0 / 5.8)
+    const int c = tcs_cluster_size(M, N, K / 2, true);
+    if (min_c > 0) return c >= min_c;
+    return M <= 32 ? c >= 2 : (M <= 64 ? c >= 4 : (c >= 2 && K >= 8192) || (c >= 4 && K >= 4096));
 }
 
 int32_t run_tcs_nvfp4(const uint8_t* a_codes, int64_t lda, const uint8_t* a_scales_blocked, const float* a_pts, const uint8_t* w_codes,
@@ -975,7 +977,7 @@ int32_t rwkvq_tc_cluster_gemv_fp8(const void* x, int32_t x_dtype, int64_t ldx, c
  * take). */
 int32_t rwkvq_tc_gemm_can_push(int64_t M, int64_t N, int64_t K) {
     if (M <= 0 || N <= 0 || K <= 0 || K % 16) return 0;
-    return !takes_swap_route(M, N, K, 1, false) && !tcs_eligible(M, N, K, 0, 1);
+    return !takes_swap_route(M, N, K, 1, false) && !tcs_eligible(KIND_F8, M, N, K, 0, 1);
 }
 
 /* rwkvq_tc_gemm_fp8 fused with the all-gather of a column-split projection: see rwkvq_tc_gemm_nvfp4_push for
@@ -1132,7 +1134,7 @@ int32_t rwkvq_tc_gemm_fp8_static(const uint8_t* a_codes, int64_t lda, const floa
                                  int32_t div_mode, uint32_t flags, void* stream) {
     const char* who = "tc_gemm_fp8_static";
     // only the weight-streaming form (few tokens) keeps partial sums in the scratch; the tiled GEMM uses the status word alone
-    const int64_t need = (M > 0 && N > 0 && K > 0 && takes_swap_route(M, N, K, 1, false) && !tcs_eligible(M, N, K, flags, 1))
+    const int64_t need = (M > 0 && N > 0 && K > 0 && takes_swap_route(M, N, K, 1, false) && !tcs_eligible(KIND_F8, M, N, K, flags, 1))
                              ? rwkvq_workspace_bytes(M, N, K, 1) : kWsHeaderBytes;
     RWKVQ_REQUIRE(need <= (int64_t)kStaticScratchBytes, RWKVQ_E_WORKSPACE, "%s: this shape needs %lld bytes of scratch, the built-in array has %lld",
                   who, (long long)need, (long long)kStaticScratchBytes);

@@ -650,34 +650,51 @@ __global__ void __launch_bounds__(kTcsqThreads, 2) gemm_tcsq_kernel(const __grid
 // up to 64 tokens, one per SM with token tiles of 128 -- at most 8 and at most one per two 128-byte steps of K.  It
 // depends on the shape alone (not on how many matrices a launch carries), so a fused r/k/v launch and three single
 // launches split K alike and give the same bits.
+// Two limits beyond that.  Token tiles of 128: at most 4 -- a CTA fills its SM, and clusters of 8 whole SMs do not all find
+// room in the GPU's processing clusters at once ([2048, 8192], 128 rows: 16.7 us with 8, 10.5 with 4).  NVFP4 up to 64 tokens:
+// ONE CTA per SM, as its two sets of scale columns take half of an SM's tensor memory -- with two the next call's CTAs
+// cannot start beside them and prefetch ([4096, 4096] 8 rows: 8.0 us with 8, 4.9 with 4; [2560, 2560] 6.1 -> 4.2; [8192, 2048] 7.7 with
+// 4, 4.9 with 2) -- unless that leaves no split at all ([16384, 4096] 9.3 with 2, 12.4 tiled) or K is long: then two CTAs an SM
+// hold twice the weights that are prefetched behind the one-launch quantizer ([4096, 16384] 1 to 4 rows, with the quantizer: 11.5 us
+// with 8, 13.6 with 4; behind the two-launch quantizer, from 5 rows, 14.5 to 18.9 with 8 and 15.7 with 4; [2560, 10240], 160 CTAs
+// with 8: 10.3 and 11.5).
+// NVFP4 CTAs also take at least two steps each.
 static int tcs_token_tile(int64_t M) { return M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : 128)); }
-static int tcs_cluster_size(int64_t M, int64_t N, int64_t K) {
+static int tcs_cluster_size(int64_t M, int64_t N, int64_t K, bool nf4 = false) {
     const int64_t ptiles = (N + kTileP - 1) / kTileP, kchunks = (K + kChunk - 1) / kChunk;
     const int nb = tcs_token_tile(M);
-    const int64_t units = ptiles * ((M + nb - 1) / nb), room = (int64_t)sm_count() * (nb <= 64 ? 2 : 1);
-    static const int cmax = std::getenv("RWKVQ_TCS_CMAX") ? std::atoi(std::getenv("RWKVQ_TCS_CMAX")) : 8;
-    int c = 1;
-    while (c < cmax && units * (c * 2) <= room && kchunks >= c * 2) c <<= 1;
-    return c;
+    const int64_t units = ptiles * ((M + nb - 1) / nb);
+    auto widest = [&](int64_t room) {
+        int c = 1;
+        while (c < (nb <= 64 ? 8 : 4) && units * (c * 2) <= room && kchunks >= c * (nf4 ? 4 : 2)) c <<= 1;
+        return c;
+    };
+    const int c1 = widest(nf4 && K >= 4096 && nb <= 64 ? sm_count() * 5 / 4 : sm_count());
+    const bool spread = nf4 && (K < 4096 || M * K > 32768);     // K: bytes of packed codes, two values each
+    if (nb > 64 || (spread && c1 > 1)) return c1;
+    return spread ? std::min(widest(2 * (int64_t)sm_count()), 2) : widest(2 * (int64_t)sm_count());
 }
 
-// Measured on the 7.2B shapes: the cluster kernel wins where a matrix has few row tiles (N = 4096: 32), i.e. where the
-// tiled GEMM form cannot give every SM a tile; with 128 row tiles (N = 16384) the GEMM form is as fast or faster.
-static bool tcs_eligible(int64_t M, int64_t N, int64_t K, uint32_t flags, int nmat) {
-    (void)nmat;                  // the K split and the grid are those of one matrix
+// Where the cluster kernel is the better form (measured, us, cluster / tiled GEMM).  Up to 32 rows where a row tile's K can be
+// shared by four CTAs or more: FP8 [4096, 4096] 24 rows 6.9 / 11.8, [2560, 2560] 4.8 / 6.8.  33 to 64 rows, against a long K ([4096,
+// 16384] 64 rows 18.5 / 31.0, [2560, 10240] 10.7 / 19.3); at K = 4096 one matrix still gains (8.4 / 9.5) but r, k, v in one
+// launch lose more (17.9 / 11.6; [2560, 2560] 15.4 / 7.4), and FP8 has one form for both so that they give the same bits.  INT8 sums
+// are exact: one matrix keeps the cluster, three take the tiled form from 32 rows on (14.6 / 10.7).  (All measured from N = 1024 up; below, a few tiles cannot fill the GPU and
+// the cluster stays.)  65 to 256 rows (token tiles
+// of 128) against a long K ([4096, 16384] 256 rows 28.3 / 33.8).  K = 1024 leaves a CTA one or two steps (r, k, v 8.1 / 4.2).
+static bool tcs_eligible(int kind, int64_t M, int64_t N, int64_t K, uint32_t flags, int nmat) {
     static const int on = std::getenv("RWKVQ_TCS") ? std::atoi(std::getenv("RWKVQ_TCS")) : 1;
     static const int64_t max_m = std::getenv("RWKVQ_TCS_MAX_M") ? std::atoll(std::getenv("RWKVQ_TCS_MAX_M")) : kTcsMaxM;
-    if (!on || M < 1 || M > std::min<int64_t>(max_m, kTcsMaxM) || (flags & RWKVQ_FLAG_RELU2)) return false;
+    if (!on || M < 1 || M > std::min<int64_t>(max_m, kTcsMaxM) || (flags & RWKVQ_FLAG_RELU2) || K < 2048) return false;
     const int c = tcs_cluster_size(M, N, K);
-    // token tiles of 128 (65 ... 256 rows): measured faster than the tiled GEMM form only against a long K (FFN value,
-    // K = 16384: 57 -> 29 us at 96 rows, 61 -> 52 us at 256); at K = 4096 the GEMM form wins from about 160 rows on and
-    // the three-matrix launch everywhere
-    return K >= 1024 && (M <= 64 ? c >= 4 : (c >= 2 && K >= 8192));
+    if (M > 64) return c >= 2 && K >= 8192;
+    if (kind == KIND_I8 && nmat > 1 && M >= 32 && K < 8192 && N >= 1024) return false;
+    return c >= 4 && (M <= 32 || K >= 8192 || N < 1024 || (kind == KIND_I8 && nmat == 1));
 }
 
 static int32_t run_tcs(TcArgs a, const TcCall& c, cudaStream_t st, const char* who) {
     const int64_t kbytes = c.kind == KIND_NF4 ? a.K / 2 : a.K;          // bytes of K per row: two e2m1 values per byte
-    const int C = tcs_cluster_size(a.M, a.N, kbytes);
+    const int C = tcs_cluster_size(a.M, a.N, kbytes, c.kind == KIND_NF4);
     a.NB = tcs_token_tile(a.M);
     a.ptiles = (a.N + kTileP - 1) / kTileP;
     a.qtiles = C;
@@ -726,7 +743,7 @@ static int32_t run_tcs(TcArgs a, const TcCall& c, cudaStream_t st, const char* w
 // one-launch form: FP8, a single matrix, up to 32 rows, the shapes the cluster kernel takes anyway
 static bool tcsq_eligible(int64_t M, int64_t N, int64_t K) {
     static const int on = std::getenv("RWKVQ_TCSQ") ? std::atoi(std::getenv("RWKVQ_TCSQ")) : 1;
-    return on && M >= 1 && M <= kTcsqMaxM && K % 8 == 0 && tcs_eligible(M, N, K, 0, 1);
+    return on && M >= 1 && M <= kTcsqMaxM && K % 8 == 0 && tcs_eligible(KIND_F8, M, N, K, 0, 1);
 }
 
 static int32_t run_tcsq(TcArgs a, const void* w, int64_t ldw, int x_dtype, cudaStream_t st, const char* who) {

@@ -273,14 +273,14 @@ __global__ void __launch_bounds__(kTcsnThreads, 2) gemm_tcsn_kernel(const __grid
 static bool tcsn_eligible(int64_t M, int64_t N, int64_t K) {
     const char* env = std::getenv("RWKVQ_TCSN");                 // read per call: a test switches routes in one process
     if ((env && std::atoi(env) == 0) || M < 1 || M > kTcsnMaxM || K % 256 || K < 2048) return false;
-    const int C = tcs_cluster_size(M, N, K / 2);
+    const int C = tcs_cluster_size(M, N, K / 2, true);
     const int64_t per_cta = (K / 256 + C - 1) / C;
     // a quantizer thread keeps at most kTcsnBlocksPerThread blocks; the token area (4 KB per step) must leave two ring stages
     return C >= 2 && per_cta <= 16 && M * per_cta * 16 <= 128 * kTcsnBlocksPerThread;
 }
 
 static int32_t run_tcsn(TcArgs a, const void* w, int64_t ldw, int x_dtype, cudaStream_t st, const char* who) {
-    const int C = tcs_cluster_size(a.M, a.N, a.K / 2);
+    const int C = tcs_cluster_size(a.M, a.N, a.K / 2, true);
     a.NB = 16;
     a.kchunks = a.K / 256;
     a.ptiles = (a.N + kTileP - 1) / kTileP;

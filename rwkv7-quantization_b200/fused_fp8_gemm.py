@@ -49,21 +49,27 @@ _ACTQ_FUSED = os.environ.get("RWKVQ_ACTQ", "fused") == "fused"   # one cooperati
 CODES_M_MIN = int(os.environ.get("RWKVQ_CODES_M_MIN", "9"))      # rows from which the decode GEMV runs on pre-quantized codes
 TC_M_MIN = int(os.environ.get("RWKVQ_TC_M_MIN", "33"))          # rows from which the tensor-memory kernels take over from the decode GEMVs (never below 9)
 CODES_MK_MIN = 49152       # ... and already from 3 rows when the block is this large (long rows: K = 16384); measured
-# FP8, rows from which the cluster split-K tensor-core kernel takes over from the codes GEMV where it applies (matrices
-# with few 128-row tiles, e.g. N = 4096).  Measured on [4096, 4096]: 16 rows 8.7 (GEMV) against 9.2 us, 20 rows 10.4 against
-# 9.3, 28 rows 10.8 against 9.3; r/k/v: 16 rows 15.5 against 17.9, 20 rows 21.1 against 18.0, 28 rows 22.2 against 19.0
-# (from 17 rows the GEMV works on three token tiles).  With many row tiles (N = 16384) the GEMV stays ahead up to 32 rows.
+# Rows from which the cluster split-K tensor-core kernel takes over from the codes GEMV where it applies (matrices with few
+# 128-row tiles).  Measured with the quantizer in front, us, GEMV / cluster: [4096, 4096] FP8 16 rows 8.9 / 8.7, 20 rows 10.8 / 8.8,
+# r/k/v 16 rows 15.2 / 15.6, 20 rows 21.0 / 16.2 (from 17 rows the GEMV works on three token tiles); INT8 16 rows 7.5 / 7.4,
+# 20 rows 9.4 / 7.7.  Against a long K, where the code tile crowds the GEMV's ring, from fewer: [4096, 16384] FP8 9 rows 19.9 / 18.5,
+# [2560, 10240] FP8 9 rows 11.6 / 10.7, 12 rows 12.7 / 10.8; INT8 [4096, 16384] 9 rows 17.6 / 16.7, 12 rows 25.7 / 17.5, [2560, 10240]
+# 9 rows 9.9 / 9.9, 12 rows 11.1 / 9.9.  With many row tiles (N = 16384) the GEMV stays ahead up to 32 rows.
 CLUSTER_FROM_M = int(os.environ.get("RWKVQ_CLUSTER_FROM_M", "17"))
+CLUSTER_LONG_K = 10240
+CLUSTER_LONG_K_FROM_M = 9
 _decode_route_cache: dict = {}
 _tc_route_cache: dict = {}
 
 
 def _takes_tc(m: int, k: int, n=None) -> bool:
-    """Do `m` rows go to the tensor-memory kernels instead of the decode GEMVs?  Always from TC_M_MIN rows; FP8 callers
-    that pass the matrix's row count `n` also from CLUSTER_FROM_M rows where the cluster split-K kernel applies."""
+    """Do `m` rows go to the tensor-memory kernels instead of the decode GEMVs?  Always from TC_M_MIN rows; callers that
+    pass the matrix's row count `n` also from CLUSTER_FROM_M rows (long K: CLUSTER_LONG_K_FROM_M) where the cluster
+    split-K kernel applies."""
     if m >= TC_M_MIN and m > 8:
         return True
-    if n is None or m < max(CLUSTER_FROM_M, 9) or m > GEMV_M_MAX or ROUTE != "auto" or k % 16 or not _ACTQ_FUSED:
+    first = CLUSTER_FROM_M if k < CLUSTER_LONG_K else min(CLUSTER_FROM_M, CLUSTER_LONG_K_FROM_M)
+    if n is None or m < max(first, 9) or m > GEMV_M_MAX or ROUTE != "auto" or k % 16 or not _ACTQ_FUSED:
         return False
     hit = _tc_route_cache.get((m, n, k))
     if hit is None:
@@ -640,10 +646,11 @@ def _int8_any(x2, w, w_scale, acc_out=None, push=None):
                  out.data_ptr(), out.stride(0), m, n, k, 0, ws.data_ptr(), ws.numel(), push[0], push[1], push[2], push[3], st)
         abi.after_call(ws)
         return out
-    if acc_out is None and ROUTE != "mma" and m > 0 and (_codes_gemv_fits(m, k) or not (_tc_fused_fits(m, k) or _gemv_fits(m, k, fp8=False))):
+    decode = _codes_gemv_fits(m, k, n if acc_out is None else None)
+    if acc_out is None and ROUTE != "mma" and m > 0 and (decode or not (_tc_fused_fits(m, k) or _gemv_fits(m, k, fp8=False, n=n))):
         # from 9 rows on: quantize the rows once, then the weight-streaming decode kernel or the tensor-core GEMM on the codes
-        _linear(abi.LINEAR_INT8, (x2,), (w,), (w_scale,), (out.data_ptr(),), out.stride(0), m, n, k, int(_codes_gemv_fits(m, k)), abi.DEFAULT_DIV, 0, 0, 0)
-    elif _codes_gemv_fits(m, k):
+        _linear(abi.LINEAR_INT8, (x2,), (w,), (w_scale,), (out.data_ptr(),), out.stride(0), m, n, k, int(decode), abi.DEFAULT_DIV, 0, 0, 0)
+    elif decode:
         # the same steps one by one, with the raw accumulators
         codes = torch.empty((m, k), dtype=torch.int8, device=x2.device)
         xs = torch.empty(m, dtype=torch.float32, device=x2.device)
@@ -696,7 +703,12 @@ def linear_rkv_int8_fused(xr, xk, xv, wr_info, wk_info, wv_info, out_dtype=torch
     n = ws[0].shape[0]
     scales = [wr_info["tensor_scale"]] * 3 if compat_shared_scale else [i["tensor_scale"] for i in infos]
     same_ld = len({w.stride(0) for w in ws}) == 1 and all(w.shape == ws[0].shape for w in ws)
-    if _codes_gemv_fits(m, k) and same_ld:
+    # r, k, v in one launch: the tensor-core forms from 17 rows of wide matrices on (us, GEMV / tensor core: [4096, 4096] 20 rows 16.7 /
+    # 15.0; [2560, 2560] 10.9 / 12.0), from 32 rows on always (17.4 / 13.3, 12.1 / 11.8).  INT8 sums are exact: any form, same bits.
+    n_route = n if same_ld and (n >= 4096 or m >= 32) else None
+    if m >= 32 and m <= GEMV_M_MAX and ROUTE == "auto" and same_ld and k % 16 == 0:
+        outs = _linear3(abi.LINEAR_INT8, [t.contiguous() for t in xs], ws, scales, m, n, k, 0, 0, 0)
+    elif _codes_gemv_fits(m, k, n_route) and same_ld:
         outs = _linear3(abi.LINEAR_INT8, [t.contiguous() for t in xs], ws, scales, m, n, k, 1, 0, 0)
     elif _tc_fused_fits(m, k, 3) and same_ld:
         xs = [t.contiguous() for t in xs]
@@ -706,7 +718,7 @@ def linear_rkv_int8_fused(xr, xk, xv, wr_info, wk_info, wv_info, out_dtype=torch
                  ws[0].data_ptr(), ws[1].data_ptr(), ws[2].data_ptr(), ws[0].stride(0), scales[0].data_ptr(),
                  scales[1].data_ptr(), scales[2].data_ptr(), outs[0].data_ptr(), outs[1].data_ptr(),
                  outs[2].data_ptr(), n, m, n, k, k, abi.DEFAULT_DIV, 0, wsp.data_ptr(), wsp.numel(), abi.stream_ptr())
-    elif _gemv_fits(m, k, fp8=False) and same_ld:
+    elif _gemv_fits(m, k, fp8=False, n=n_route) and same_ld:
         xs = [t.contiguous() for t in xs]
         outs = [torch.empty((m, n), dtype=torch.float16, device=xs[0].device) for _ in range(3)]
         abi.call("rwkvq_gemv_int8_rkv", xs[0].data_ptr(), xs[1].data_ptr(), xs[2].data_ptr(), abi.dtype_code(xs[0]),
