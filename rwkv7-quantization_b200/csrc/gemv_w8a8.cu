@@ -156,7 +156,7 @@ __device__ __forceinline__ void store_tile(const W8Args& a, int mat, int n0, int
             if constexpr (RELU2) {
                 // the engine's relu_square on the fp16 result: fp16(max(y, 0)^2) in fp32 arithmetic; its maximum (over the
                 // bf16-rounded values where the consumer takes its amax there) is published for the projection that follows
-                const float v = fmaxf(__half2float(y), 0.f);
+                const float yf = __half2float(y), v = yf < 0.f ? 0.f : yf;          // NaN stays NaN, as in a relu of its own
                 y = __float2half_rn(v * v);
                 const float hv = __half2float(y);
                 if constexpr (QT == QT_FP8) hmax[0] = fmaxf(hmax[0], (a.flags & RWKVQ_FLAG_AMAX_AFTER_BF16) ? bf16_round(hv) : hv);

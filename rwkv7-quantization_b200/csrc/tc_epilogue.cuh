@@ -48,7 +48,7 @@ __device__ __forceinline__ void epi_convert16(const EpiRow& e, const uint32_t (&
             // the engine's relu_square on the fp16 result, fp32 arithmetic; its maximum (over the bf16-rounded values where the
             // consumer takes its amax there) goes to the projection that follows
             const float2 y = __half22float2(hh);
-            const float v0 = fmaxf(y.x, 0.f), v1 = fmaxf(y.y, 0.f);
+            const float v0 = y.x < 0.f ? 0.f : y.x, v1 = y.y < 0.f ? 0.f : y.y;      // NaN stays NaN, as in a relu of its own
             hh = __floats2half2_rn(v0 * v0, v1 * v1);
             float2 hv = __half22float2(hh);
             if (hmax_bf16) hv = bf16_round2(hv);

@@ -65,6 +65,29 @@ def results():
     return [t.cpu() for t in out]
 
 
+@pytest.mark.parametrize("scheme", ["fp8", "int8"])
+@pytest.mark.parametrize("m,k,f,n", [(9, 1024, 4096, 1024), (13, 4096, 16384, 4096), (32, 768, 3072, 768), (20, 2560, 10240, 2560), (5, 4096, 16384, 4096),
+                                     (40, 2048, 8192, 512), (200, 1024, 4096, 1024), (1, 1024, 4096, 1024), (6, 768, 3072, 768)])
+def test_ffn_pair_equals_its_three_steps(scheme, m, k, f, n):
+    """The FFN pair (relu_square in an epilogue or in the quantizer that follows) equals its three steps bit for bit, NaN and infinity included."""
+    import fused_fp8_gemm as ff
+    g = torch.Generator(device="cuda").manual_seed(m + k)
+    mk = lambda a, b: (torch.randn((a, b), generator=g, device="cuda") * b ** -0.5 * 100).round().clamp(-127, 127)  # noqa: E731
+    dt = torch.float8_e4m3fn if scheme == "fp8" else torch.int8
+    info = [{"weight": mk(a, b).to(dt), "tensor_scale": torch.tensor(0.01, device="cuda"), "qtype": scheme} for a, b in ((f, k), (n, f))]
+    pair = ff.ffn_relu2_fp8 if scheme == "fp8" else ff.ffn_relu2_int8
+    for special in (None, float("inf"), float("nan")):
+        x = torch.randn((m, k), generator=g, device="cuda").half()
+        if special is not None:
+            x[m // 2, 3] = special
+        hid = ff.linear_quantized_fused(x, info[0])
+        hid = (hid.float().clamp_(min=0.0) ** 2).to(torch.float16)
+        want = ff.linear_quantized_fused(hid, info[1])
+        got = pair(x, info[0], info[1])
+        assert torch.equal(got.view(torch.int16), want.view(torch.int16)), special
+        assert torch.equal(pair(x, info[0], info[1], return_hidden=True)[0].view(torch.int16), want.view(torch.int16))
+
+
 def test_pairs_and_single_ctas_give_the_same_bits(tmp_path):
     f = str(tmp_path / "single.pt")
     code = f"import sys; sys.path[:0] = [{os.path.join(ROOT, 'rwkv7-quantization_b200')!r}, {os.path.join(ROOT, 'tests')!r}]\n" \
