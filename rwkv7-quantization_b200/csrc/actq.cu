@@ -269,7 +269,8 @@ struct QInt8Args {
 // KEEP = 1, 2, 4, 8: rows of up to KEEP * 2048 elements stay in registers between the abs-max and the codes (KEEP vectors
 // per thread): one read of the row, all loads in flight at once.  Measured against two reads: 2048 rows of 4096 10.4 ->
 // 9.3 us, of 16384 24.8 -> 24.1.  KEEP = 0: longer rows, two reads (the second hits L1 / L2).
-template <int DT, bool VEC, int KEEP = 0>
+// RELU2 (fp16 only, KEEP > 0): the row goes through relu_square on its way in.
+template <int DT, bool VEC, int KEEP = 0, bool RELU2 = false>
 __global__ void __launch_bounds__(kThreads) quant_int8_kernel(const QInt8Args qa, int64_t K, int64_t ldx, int64_t ldc, int div_mode) {
     __shared__ float sh[kThreads / 32];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a projection behind this launch may prefetch its weights
@@ -289,6 +290,7 @@ __global__ void __launch_bounds__(kThreads) quant_int8_kernel(const QInt8Args qa
         }
 #pragma unroll
         for (int j = 0; j < KEEP; ++j) {
+            if constexpr (RELU2) v[j] = relu2_f16x8(v[j]);
             const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
@@ -534,7 +536,11 @@ constexpr int kSmallThreads = 1024;
 constexpr int kSmallThreadsLight = 256;
 constexpr int kSmallKeep = 8;
 
-template <int DT>
+// RELU2 (fp16 only): x is the FFN key projection's result and goes through relu_square on its way in.  The FFN pair of 9-32
+// rows ran relu_square as four elementwise launches of its own (about 8 us of a 68 us pass of four projections at width
+// 4096, 13 rows; the pass is 60.7 us without them).  A relu_square in the key projection's own epilogue would save no
+// further launch: the cluster forms hold a share of the sum each and publish no maximum.
+template <int DT, bool RELU2 = false>
 __global__ void __launch_bounds__(kSmallThreads, 1) actq_fp8_small_kernel(const ActqArgs a) {
     __shared__ float sh[kSmallThreads / 32];
     __shared__ float s_part[8];           // maxima of the cluster's CTAs (each CTA writes its slot in every CTA)
@@ -585,7 +591,10 @@ __global__ void __launch_bounds__(kSmallThreads, 1) actq_fp8_small_kernel(const 
             if (i0 + j * step < nvec) v[j] = *reinterpret_cast<const uint4*>(vec_ptr(i0 + j * step));
 #pragma unroll
         for (int j = 0; j < kSmallKeep; ++j)
-            if (i0 + j * step < nvec) m = vec_max(v[j], m);
+            if (i0 + j * step < nvec) {
+                if constexpr (RELU2) v[j] = relu2_f16x8(v[j]);
+                m = vec_max(v[j], m);
+            }
     }
     m = warp_max(m);
     if (lane == 0) sh[warp] = m;
@@ -630,7 +639,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) actq_fp8_small_kernel(const 
                 if (i0 + j * step < nvec) v[j] = *reinterpret_cast<const uint4*>(vec_ptr(i0 + j * step));
 #pragma unroll
             for (int j = 0; j < kSmallKeep; ++j)
-                if (i0 + j * step < nvec) vec_codes(v[j], i0 + j * step);
+                if (i0 + j * step < nvec) vec_codes(RELU2 ? relu2_f16x8(v[j]) : v[j], i0 + j * step);
         }
     }
 }
@@ -961,7 +970,7 @@ int32_t rwkvq_prep_x_fp8(const void* x, int32_t x_dtype, int64_t M, int64_t K, i
 }
 
 static int32_t launch_quant_int8(const QInt8Args& qa, int nt, int32_t x_dtype, int64_t M, int64_t K, int64_t ldx, int64_t ldc,
-                                 int32_t div_mode, cudaStream_t st, const char* who) {
+                                 int32_t div_mode, cudaStream_t st, const char* who, bool relu2 = false) {
     RWKVQ_REQUIRE(x_dtype == RWKVQ_F16 || x_dtype == RWKVQ_BF16, RWKVQ_E_BADARG, "%s: x_dtype %d", who, x_dtype);
     RWKVQ_REQUIRE(div_mode == RWKVQ_DIV_IEEE || div_mode == RWKVQ_DIV_FULL, RWKVQ_E_BADARG, "%s: div_mode %d", who, div_mode);
     RWKVQ_REQUIRE(M >= 0 && K >= 0 && ldx >= K && ldc >= K, RWKVQ_E_SHAPE, "%s: M=%lld K=%lld", who, (long long)M, (long long)K);
@@ -993,7 +1002,15 @@ static int32_t launch_quant_int8(const QInt8Args& qa, int nt, int32_t x_dtype, i
         case 8: RWKVQ_Q(DT, true, 8); break; \
         default: if (vec) RWKVQ_Q(DT, true, 0); else RWKVQ_Q(DT, false, 0); \
     }
-    if (x_dtype == RWKVQ_F16) { RWKVQ_QK(RWKVQ_F16) } else { RWKVQ_QK(RWKVQ_BF16) }
+    if (relu2) {
+        RWKVQ_REQUIRE(keep > 0 && x_dtype == RWKVQ_F16, RWKVQ_E_SHAPE, "%s: fp16 rows of at most %lld elements, 16-byte aligned", who, (long long)(8 * per));
+        switch (keep) {
+            case 1: e = cudaLaunchKernelEx(&cfg, quant_int8_kernel<RWKVQ_F16, true, 1, true>, qa, K, ldx, ldc, dm); break;
+            case 2: e = cudaLaunchKernelEx(&cfg, quant_int8_kernel<RWKVQ_F16, true, 2, true>, qa, K, ldx, ldc, dm); break;
+            case 4: e = cudaLaunchKernelEx(&cfg, quant_int8_kernel<RWKVQ_F16, true, 4, true>, qa, K, ldx, ldc, dm); break;
+            default: e = cudaLaunchKernelEx(&cfg, quant_int8_kernel<RWKVQ_F16, true, 8, true>, qa, K, ldx, ldc, dm);
+        }
+    } else if (x_dtype == RWKVQ_F16) { RWKVQ_QK(RWKVQ_F16) } else { RWKVQ_QK(RWKVQ_BF16) }
 #undef RWKVQ_QK
 #undef RWKVQ_Q
     if (e != cudaSuccess) {
@@ -1010,6 +1027,13 @@ int32_t rwkvq_prep_x_int8(const void* x, int32_t x_dtype, int64_t M, int64_t K, 
     return launch_quant_int8(qa, 1, x_dtype, M, K, ldx, ldc, div_mode, (cudaStream_t)stream, "prep_x_int8");
 }
 
+int32_t rwkvq_prep_x_int8_relu2(const void* y_f16, int64_t M, int64_t K, int64_t ldx, int8_t* codes, int64_t ldc, float* scales, int32_t div_mode,
+                                void* stream) {
+    QInt8Args qa{};
+    qa.x[0] = y_f16; qa.codes[0] = codes; qa.scales[0] = scales;
+    return launch_quant_int8(qa, 1, RWKVQ_F16, M, K, ldx, ldc, div_mode, (cudaStream_t)stream, "prep_x_int8_relu2", true);
+}
+
 int32_t rwkvq_prep3_x_int8(const void* xr, const void* xk, const void* xv, int32_t x_dtype, int64_t M, int64_t K, int64_t ldx,
                            int8_t* codes_r, int8_t* codes_k, int8_t* codes_v, int64_t ldc, float* scales_r, float* scales_k,
                            float* scales_v, int32_t div_mode, void* stream) {
@@ -1021,9 +1045,13 @@ int32_t rwkvq_prep3_x_int8(const void* xr, const void* xk, const void* xv, int32
 
 int64_t rwkvq_actq_fp8_fused_scratch_bytes(void) { return (kFusedEpochWord + 32) * 4; }
 
+// largest block of the one-launch cluster quantizer: eight CTAs of 1024 threads with eight vectors each in registers
+constexpr int64_t kSmallMaxVectors = (int64_t)8 * 8 * kSmallThreads;
+
 static int32_t launch_actq_fused(ActqArgs a, int nt, int32_t x_dtype, int64_t M, int64_t K, int64_t ldx, int64_t ldc, void* scratch,
-                                 int64_t scratch_bytes, int32_t* status, int32_t div_mode, uint32_t flags, cudaStream_t st, const char* who) {
-    RWKVQ_REQUIRE(scratch != nullptr && a.amax_out != nullptr, RWKVQ_E_BADARG, "%s: null pointer", who);
+                                 int64_t scratch_bytes, int32_t* status, int32_t div_mode, uint32_t flags, cudaStream_t st, const char* who,
+                                 bool relu2 = false) {
+    RWKVQ_REQUIRE((scratch != nullptr || relu2) && a.amax_out != nullptr, RWKVQ_E_BADARG, "%s: null pointer", who);
     for (int t = 0; t < nt; ++t) {
         RWKVQ_REQUIRE(a.x[t] && a.codes[t], RWKVQ_E_BADARG, "%s: null pointer (tensor %d)", who, t);
         RWKVQ_REQUIRE(aligned16(a.x[t]) && ((uintptr_t)a.codes[t] & 7) == 0, RWKVQ_E_ALIGN, "%s: rows must be 16-byte (x) / 8-byte (codes) aligned", who);
@@ -1032,8 +1060,12 @@ static int32_t launch_actq_fused(ActqArgs a, int nt, int32_t x_dtype, int64_t M,
     RWKVQ_REQUIRE(div_mode == RWKVQ_DIV_IEEE || div_mode == RWKVQ_DIV_FULL || div_mode == RWKVQ_DIV_TORCH, RWKVQ_E_BADARG, "%s: div_mode %d", who, div_mode);
     RWKVQ_REQUIRE(M > 0 && K > 0 && K % 8 == 0 && M < (1 << 30), RWKVQ_E_SHAPE, "%s: M=%lld K=%lld (K must be a multiple of 8)", who, (long long)M, (long long)K);
     RWKVQ_REQUIRE(ldx % 8 == 0 && ldx >= K && ldc % 8 == 0 && ldc >= K, RWKVQ_E_ALIGN, "%s: rows must be 16-byte (x) / 8-byte (codes) aligned", who);
-    RWKVQ_REQUIRE(scratch_bytes >= rwkvq_actq_fp8_fused_scratch_bytes() && ((uintptr_t)scratch & 3) == 0, RWKVQ_E_WORKSPACE,
-                  "%s: scratch of %lld bytes needed", who, (long long)rwkvq_actq_fp8_fused_scratch_bytes());
+    if (relu2)
+        RWKVQ_REQUIRE(x_dtype == RWKVQ_F16 && nt == 1 && M * (K / 8) <= kSmallMaxVectors && K / 8 < 65536, RWKVQ_E_SHAPE,
+                      "%s: fp16 rows, at most %lld elements in all", who, (long long)kSmallMaxVectors * 8);
+    else
+        RWKVQ_REQUIRE(scratch_bytes >= rwkvq_actq_fp8_fused_scratch_bytes() && ((uintptr_t)scratch & 3) == 0, RWKVQ_E_WORKSPACE,
+                      "%s: scratch of %lld bytes needed", who, (long long)rwkvq_actq_fp8_fused_scratch_bytes());
     a.nt = nt;
     a.cpt = (int)std::min<int64_t>(M, std::min<int64_t>(kFusedMaxCtas, 2 * (int64_t)sm_count()) / nt);
     a.after_bf16 = (flags & RWKVQ_FLAG_AMAX_AFTER_BF16) ? 1 : 0;
@@ -1043,8 +1075,8 @@ static int32_t launch_actq_fused(ActqArgs a, int nt, int32_t x_dtype, int64_t M,
     a.flags = reinterpret_cast<uint32_t*>(scratch) + kFusedMaxCtas;
     a.wait_ns = wait_limit_ns();
     const char* small_env = std::getenv("RWKVQ_ACTQ_SMALL_MAX");         // read per call: a test switches forms in one process
-    const int64_t small_max = small_env ? std::atoll(small_env) : (int64_t)8 * 8 * kSmallThreads;
-    if (M * (K / 8) <= std::min<int64_t>(small_max, (int64_t)8 * 8 * kSmallThreads) && K / 8 < 65536) {
+    const int64_t small_max = small_env && !relu2 ? std::atoll(small_env) : kSmallMaxVectors;
+    if (M * (K / 8) <= std::min<int64_t>(small_max, kSmallMaxVectors) && K / 8 < 65536) {
         // decode-sized block: a cluster of CTAs per tensor (about 4 vectors per thread), no grid rendezvous, programmatic
         // dependent launch (the scratch is not touched)
         static const int64_t light_max = std::getenv("RWKVQ_ACTQ_LIGHT_MAX") ? std::atoll(std::getenv("RWKVQ_ACTQ_LIGHT_MAX")) : 8 * 8 * kSmallThreadsLight;
@@ -1064,7 +1096,8 @@ static int32_t launch_actq_fused(ActqArgs a, int nt, int32_t x_dtype, int64_t M,
         attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = use_pdl() ? 2 : 1;
-        const cudaError_t e = x_dtype == RWKVQ_F16 ? cudaLaunchKernelEx(&cfg, actq_fp8_small_kernel<RWKVQ_F16>, a)
+        const cudaError_t e = relu2                ? cudaLaunchKernelEx(&cfg, actq_fp8_small_kernel<RWKVQ_F16, true>, a)
+                              : x_dtype == RWKVQ_F16 ? cudaLaunchKernelEx(&cfg, actq_fp8_small_kernel<RWKVQ_F16>, a)
                                                    : cudaLaunchKernelEx(&cfg, actq_fp8_small_kernel<RWKVQ_BF16>, a);
         if (e != cudaSuccess) {
             g_launches.fetch_add(1, std::memory_order_relaxed);
@@ -1128,6 +1161,13 @@ int32_t rwkvq_actq_fp8_fused(const void* x, int32_t x_dtype, int64_t M, int64_t 
     ActqArgs a{};
     a.x[0] = x; a.codes[0] = codes; a.amax_out = amax; a.scale_out[0] = scale;
     return launch_actq_fused(a, 1, x_dtype, M, K, ldx, ldc, scratch, scratch_bytes, status, div_mode, flags, (cudaStream_t)stream, "actq_fp8_fused");
+}
+
+int32_t rwkvq_actq_fp8_relu2(const void* y_f16, int64_t M, int64_t K, int64_t ldx, uint8_t* codes, int64_t ldc, float* amax, float* scale, int32_t div_mode,
+                             uint32_t flags, void* stream) {
+    ActqArgs a{};
+    a.x[0] = y_f16; a.codes[0] = codes; a.amax_out = amax; a.scale_out[0] = scale;
+    return launch_actq_fused(a, 1, RWKVQ_F16, M, K, ldx, ldc, nullptr, 0, nullptr, div_mode, flags, (cudaStream_t)stream, "actq_fp8_relu2", true);
 }
 
 int32_t rwkvq_actq_fp8_fused3(const void* xr, const void* xk, const void* xv, int32_t x_dtype, int64_t M, int64_t K, int64_t ldx,

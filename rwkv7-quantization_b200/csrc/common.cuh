@@ -144,6 +144,21 @@ __device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c
     return r;
 }
 
+// the engine's relu_square of 8 fp16 values: fp16(max(y, 0)^2) in fp32 arithmetic, NaN kept
+__device__ __forceinline__ uint4 relu2_f16x8(const uint4& v) {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    uint32_t h[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        float2 f = cvt2<RWKVQ_F16>(w[q]);
+        f.x = f.x < 0.f ? 0.f : f.x;
+        f.y = f.y < 0.f ? 0.f : f.y;
+        const __half2 r = __floats2half2_rn(f.x * f.x, f.y * f.y);
+        h[q] = *reinterpret_cast<const uint32_t*>(&r);
+    }
+    return make_uint4(h[0], h[1], h[2], h[3]);
+}
+
 // 1 / bs, correctly rounded, for an e4m3 block scale: the hardware's approximation (within 1 ulp) and one Newton step.  From
 // every start within 1 ulp of every such scale's reciprocal the step ends on the correctly rounded value (all of them
 // enumerated in exact arithmetic), so this is __frcp_rn without its range checks.

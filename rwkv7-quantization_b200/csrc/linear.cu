@@ -30,6 +30,7 @@ int32_t rwkvq_linear(const rwkvq_linear_desc* d) {
                   (long long)d->M, (long long)d->K);
     RWKVQ_REQUIRE(d->scratch && ((uintptr_t)d->scratch & 255) == 0 && d->scratch_bytes >= rwkvq_linear_scratch_bytes(d->kind, d->nmat, d->M, d->K),
                   RWKVQ_E_WORKSPACE, "%s: %lld bytes of 256-byte aligned scratch needed", who, (long long)rwkvq_linear_scratch_bytes(d->kind, d->nmat, d->M, d->K));
+    RWKVQ_REQUIRE(!d->relu2 || (d->nmat == 1 && d->x_dtype == RWKVQ_F16), RWKVQ_E_BADARG, "%s: relu2 takes one matrix and fp16 rows", who);
     uint8_t* c[3] = {nullptr, nullptr, nullptr};
     const int64_t M = d->M, N = d->N, K = d->K, cb = up256(M * K);
     for (int i = 0; i < d->nmat; ++i) c[i] = reinterpret_cast<uint8_t*>(d->scratch) + i * cb;
@@ -40,8 +41,9 @@ int32_t rwkvq_linear(const rwkvq_linear_desc* d) {
         const float* a = d->by_scale ? sc + 4 : sc;
         const int32_t is_amax = d->by_scale ? 0 : 1;
         if (d->nmat == 1) {
-            rc = rwkvq_actq_fp8_fused(d->x[0], d->x_dtype, M, K, d->ldx, c[0], K, sc, scale, d->actq_scratch, d->actq_scratch_bytes, nullptr, d->act_div,
-                                      d->act_flags, d->stream);
+            rc = d->relu2 ? rwkvq_actq_fp8_relu2(d->x[0], M, K, d->ldx, c[0], K, sc, scale, d->act_div, d->act_flags, d->stream)
+                          : rwkvq_actq_fp8_fused(d->x[0], d->x_dtype, M, K, d->ldx, c[0], K, sc, scale, d->actq_scratch, d->actq_scratch_bytes, nullptr,
+                                                 d->act_div, d->act_flags, d->stream);
             if (rc != RWKVQ_OK) return rc;
             const uint8_t* w = (const uint8_t*)d->w[0];
             return d->decode ? rwkvq_gemm_fp8(c[0], K, a, is_amax, w, d->ldw, d->w_scale[0], d->out[0], d->ldo, M, N, K, d->gemm_div, d->gemm_flags, d->stream)
@@ -63,7 +65,8 @@ int32_t rwkvq_linear(const rwkvq_linear_desc* d) {
     int8_t* q[3] = {(int8_t*)c[0], (int8_t*)c[1], (int8_t*)c[2]};
     const int8_t *w0 = (const int8_t*)d->w[0], *w1 = (const int8_t*)d->w[1], *w2 = (const int8_t*)d->w[2];
     if (d->nmat == 1) {
-        rc = rwkvq_prep_x_int8(d->x[0], d->x_dtype, M, K, d->ldx, q[0], K, s[0], d->act_div, d->stream);
+        rc = d->relu2 ? rwkvq_prep_x_int8_relu2(d->x[0], M, K, d->ldx, q[0], K, s[0], d->act_div, d->stream)
+                      : rwkvq_prep_x_int8(d->x[0], d->x_dtype, M, K, d->ldx, q[0], K, s[0], d->act_div, d->stream);
         if (rc != RWKVQ_OK) return rc;
         return d->decode ? rwkvq_gemm_int8(q[0], K, s[0], w0, d->ldw, d->w_scale[0], d->out[0], d->ldo, nullptr, N, M, N, K, d->gemm_flags, d->stream)
                          : rwkvq_tc_gemm_int8(q[0], K, s[0], w0, d->ldw, d->w_scale[0], d->out[0], d->ldo, nullptr, N, M, N, K, d->gemm_flags, d->workspace,

@@ -250,7 +250,7 @@ def _actq_fp8(x2, codes, amax, scale, div, flags, st):
                  abi.ptr(scale), div, flags, st)
 
 
-def _linear(kind, xs, ws_, scales, outs, ldo, m, n, k, decode, act_div, gemm_div, act_flags, gemm_flags, by_scale=0):
+def _linear(kind, xs, ws_, scales, outs, ldo, m, n, k, decode, act_div, gemm_div, act_flags, gemm_flags, by_scale=0, relu2=0):
     """Quantizer and GEMM of one projection (or r, k, v) in one call (rwkvq_linear).  xs, ws_, scales: one or three tensors;
     outs: their result pointers."""
     x0, w0 = xs[0], ws_[0]
@@ -271,7 +271,7 @@ def _linear(kind, xs, ws_, scales, outs, ldo, m, n, k, decode, act_div, gemm_div
         ptrs = (*(t.data_ptr() for t in xs), *(t.data_ptr() for t in ws_), *(t.data_ptr() for t in scales), *outs)
     abi.call("rwkvq_linear", abi.LINEAR_DESC.pack(
         *ptrs, x0.stride(0) if m > 1 else k, w0.stride(0), ldo, m, n, k, kind, abi.dtype_code(x0), nmat, decode, act_div, gemm_div, act_flags,
-        gemm_flags, by_scale, 0, scratch.data_ptr(), need, sc_ptr, sc_bytes, 0 if ws is None else ws.data_ptr(), 0 if ws is None else ws.numel(),
+        gemm_flags, by_scale, relu2, scratch.data_ptr(), need, sc_ptr, sc_bytes, 0 if ws is None else ws.data_ptr(), 0 if ws is None else ws.numel(),
         abi.stream_ptr()))
     abi.after_call(ws)
 
@@ -507,6 +507,8 @@ def linear_rkv_fused(xr, xk, xv, wr_info, wk_info, wv_info, out_dtype=torch.floa
     return tuple(_finish(o, lead, n, out_dtype) for o in outs)
 
 
+RELU2_FP8_MAX = 65536 * 8            # elements the quantizer with relu_square on its input takes (rwkvq_actq_fp8_relu2)
+RELU2_INT8_MAX_ROW = 16384           # elements per row of its INT8 form (rwkvq_prep_x_int8_relu2)
 _ffn_scratch: dict = {}
 
 
@@ -572,6 +574,14 @@ def ffn_relu2_fp8(x, key_info, value_info, out_dtype=torch.float16, return_hidde
                              abi.FLAG_QUANT_FROM_BF16 | (abi.FLAG_AMAX_AFTER_BF16 if big else 0),
                              ((abi.FLAG_OUT_VIA_BF16 | abi.FLAG_AMAX_AFTER_BF16) if big else 0) | _wscale_flag(sk, f_dim),
                              (abi.FLAG_OUT_VIA_BF16 if big else 0) | _wscale_flag(sv, n), int(big), ffn_scratch(x2.device))
+    elif (not return_hidden and m > 1 and ROUTE == "auto" and _ACTQ_FUSED and not _CLUSTER_FIRST and not abi._out_override and m <= FUSED_M_MAX
+          and f_dim % 8 == 0 and m * f_dim <= RELU2_FP8_MAX and not (_gemv_fits(m, f_dim, n=n) and not _codes_gemv_fits(m, f_dim, n))):
+        # rows between the two fused pairs: relu_square rides in the quantizer of the value projection (the routes are those
+        # of the separate calls: codes GEMV where it fits, else the tensor-core forms)
+        hid = linear_quantized_fused(x2, {"weight": wk, "tensor_scale": sk, "qtype": "fp8"})
+        out = torch.empty((m, n), dtype=torch.float16, device=x2.device)
+        _linear(abi.LINEAR_FP8, (hid,), (_u8(wv),), (sv,), (out.data_ptr(),), n, m, n, f_dim, int(_codes_gemv_fits(m, f_dim, n)), abi.DEFAULT_DIV,
+                abi.DEFAULT_DIV, abi.FLAG_QUANT_FROM_BF16, _wscale_flag(sv, n), 0, 1)
     else:
         hid = linear_quantized_fused(x2, {"weight": wk, "tensor_scale": sk, "qtype": "fp8"})
         hid = (hid.float().clamp_(min=0.0) ** 2).to(torch.float16)       # relu_square: fp16(max(y, 0)^2), fp32 arithmetic
@@ -619,6 +629,11 @@ def ffn_relu2_int8(x, key_info, value_info, out_dtype=torch.float16, return_hidd
     elif ROUTE == "auto" and m > GEMV_M_MAX and k % 16 == 0 and f_dim % 16 == 0 and can_push(m, f_dim, k):
         # many rows on the tiled GEMM (can_push: neither the weight-streaming nor the cluster form takes these sizes)
         hid, out = _ffn_many(abi.LINEAR_INT8, x2, wk, sk, wv, sv, abi.DEFAULT_DIV, abi.DEFAULT_DIV, 0, 0, 0, 0, _row_max_scratch(x2.device, m))
+    elif (not return_hidden and m > 0 and ROUTE == "auto" and not abi._out_override and f_dim % 16 == 0 and f_dim <= RELU2_INT8_MAX_ROW
+          and not (_gemv_fits(m, f_dim, fp8=False, n=n) and not _codes_gemv_fits(m, f_dim, n))):
+        hid = linear_int8_fused(x2, key_info)            # relu_square rides in the quantizer of the value projection
+        out = torch.empty((m, n), dtype=torch.float16, device=x2.device)
+        _linear(abi.LINEAR_INT8, (hid,), (wv,), (sv,), (out.data_ptr(),), n, m, n, f_dim, int(_codes_gemv_fits(m, f_dim, n)), abi.DEFAULT_DIV, 0, 0, 0, 0, 1)
     else:
         hid = linear_int8_fused(x2, key_info)
         hid = (hid.float().clamp_(min=0.0) ** 2).to(torch.float16)       # relu_square: fp16(max(y, 0)^2), fp32 arithmetic

@@ -101,6 +101,8 @@ SIGNATURES = {
     "rwkvq_tc_gemm_int8_rkv": [_p, _p, _p, _i64, _p, _p, _p, _p, _p, _p, _i64, _p, _p, _p, _p, _p, _p, _i64, _i64, _i64, _i64,
                                _u32, _p, _i64, _p],
     "rwkvq_tc_static_status": [_p],
+    "rwkvq_actq_fp8_relu2": [_p, _i64, _i64, _i64, _p, _i64, _p, _p, _i32, _u32, _p],
+    "rwkvq_prep_x_int8_relu2": [_p, _i64, _i64, _i64, _p, _i64, _p, _i32, _p],
     "rwkvq_linear_scratch_bytes": [_i32, _i32, _i64, _i64],
     "rwkvq_linear": [_p],
     "rwkvq_ffn_scratch_bytes": [_i32, _i64, _i64, _i64],
