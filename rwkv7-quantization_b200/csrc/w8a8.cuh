@@ -309,6 +309,52 @@ __device__ __forceinline__ uint2 int8_vec_codes(const uint4& v, float s) {
                       pack_s8x4(__float2int_rz(f2.x * s), __float2int_rz(f2.y * s), __float2int_rz(f3.x * s), __float2int_rz(f3.y * s)));
 }
 
+// 2-8 rows whose length is a multiple of a warp's 32 vectors, at most KEEP such chunks per warp: each warp takes an equal run
+// of the block's chunks and keeps them in registers; a chunk's maximum joins its row's in shared memory.
+// The prologue is a chain of dependent latencies that every CTA repeats, so what counts is one read and few steps: a row at a
+// time cost a reduction over the CTA per row (3-4 rows), a warp per row left warps idle and read its row twice (5-8 rows).
+// [4096, 4096], whole kernel: 3 rows 7.0 -> 5.9 us, 4 rows 8.0 -> 6.2, 5 and 6 rows 7.2 -> 6.7; [2560, 2560] 5 rows
+// 5.0 -> 4.2.  KEEP is 8 or 12 and no more: the code runs once on a cold instruction cache, 16 vectors cost 0.7 us more in
+// every launch than 8, and a loop over batches of 8 that reads the earlier ones again 1.7 us.
+template <int DT, int KEEP>
+__device__ __forceinline__ void quantize_int8_chunks(const W8Args& a, const char* x, uint8_t* xq, float* xs, float* sh, int per) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nc = a.K >> 8, total = a.M * nc, c0 = warp * per, c1 = min(c0 + per, total);
+    const uint32_t inv_nc = 0xFFFFFFFFu / (uint32_t)nc + 1u;              // row of a chunk index without a division
+    uint32_t* const rowmax = reinterpret_cast<uint32_t*>(sh);             // maxima as bits: non-negative floats order like integers
+    uint4 v[KEEP];
+    if (c0 < c1) {
+#pragma unroll
+        for (int j = 0; j < KEEP; ++j) {
+            const int c = min(c0 + j, c1 - 1), r = (int)__umulhi((uint32_t)c, inv_nc);
+            v[j] = ldg_l2_16(x + ((int64_t)r * a.ldx + (int64_t)(c - r * nc) * 256 + lane * 8) * 2);
+        }
+    }
+    if (threadIdx.x < 8) rowmax[threadIdx.x] = 0u;
+    __syncthreads();
+    if (c0 < c1) {
+#pragma unroll
+        for (int j = 0; j < KEEP; ++j) {
+            const uint32_t m = __reduce_max_sync(0xffffffffu, __float_as_uint(int8_vec_amax<DT>(v[j], 0.f)));
+            if (lane == 0) atomicMax(rowmax + __umulhi((uint32_t)min(c0 + j, c1 - 1), inv_nc), m);
+        }
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < a.M) {
+        const float m = fmaxf(sh[threadIdx.x], 1e-12f);
+        xs[threadIdx.x] = div_mode_f32(m, 127.f, a.div_mode);
+        sh[threadIdx.x] = div_mode_f32(127.f, m, a.div_mode);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < KEEP; ++j) {
+        const int c = c0 + j;
+        if (c >= c1) break;
+        const int r = (int)__umulhi((uint32_t)c, inv_nc);
+        *reinterpret_cast<uint2*>(xq + (size_t)r * a.pitch + (size_t)(c - r * nc) * 256 + lane * 8) = int8_vec_codes<DT>(v[j], sh[r]);
+    }
+}
+
 // GIVEN: the rows' maxima come from a.ffn_amax[2 + r] (published by the kernel that produced x, the FFN key projection
 // with relu^2 in its epilogue): no abs-max pass; the CTA's threads walk all rows' vectors, eight loads in flight each.
 template <int DT, bool GIVEN = false>
@@ -340,6 +386,13 @@ __device__ void quantize_int8_to_smem(const W8Args& a, int mat, uint8_t* xq, flo
                 if (i0 + j * kThr < nvec) *reinterpret_cast<uint2*>(xq + (size_t)rr[j] * a.pitch + (size_t)cc[j] * 8) = int8_vec_codes<DT>(v[j], sh[rr[j]]);
         }
         return;
+    }
+    // (2 rows: only from K = 4096, below it the row at a time is level or quicker, r/k/v of 1024: 3.6 against 3.9 us; 5-8 rows:
+    // only from K = 2048, below it a warp holds its whole row anyway, 3.0 against 3.1 us)
+    if (a.M >= 2 && a.M <= 8 && (a.K & 255) == 0 && a.K >= (a.M == 2 ? 4096 : a.M <= 4 ? 512 : 2048)) {
+        const int per = (a.M * (a.K >> 8) + kWarps - 1) / kWarps;
+        if (per <= 8) { quantize_int8_chunks<DT, 8>(a, x, xq, xs, sh, per); return; }
+        if (per <= 12) { quantize_int8_chunks<DT, 12>(a, x, xq, xs, sh, per); return; }
     }
     if (a.M <= 4 && a.K > 2 * kThr * 8 && a.K <= 8 * kThr * 8) {
         // long rows: the whole CTA works on one row at a time and keeps it in registers between amax and codes

@@ -78,3 +78,23 @@ def test_fp8_and_int8(m, k, pitch, dtype, special):
         abi.call("rwkvq_prep_x_int8", x.data_ptr(), abi.dtype_code(x), m, k, pitch, c.data_ptr(), k, s.data_ptr(), abi.DIV_IEEE, st)
         am = x.float().abs().amax(1).clamp(min=1e-12)
         assert torch.equal(c, (x.float() * (torch.full_like(am, 127.0) / am)[:, None]).clamp(-128, 127).trunc().to(torch.int8))
+
+
+@pytest.mark.parametrize("k", [512, 768, 1024, 1536, 2048, 2304, 2560, 4096, 5120, 8192, 16384])
+@pytest.mark.parametrize("m", [2, 3, 4, 5, 6, 7, 8])
+def test_int8_rows_quantized_inside_the_gemv(m, k):
+    """Every form of the INT8 prologue of 2-8 rows gives the codes and scales of the row quantizer: the same bits come out of the GEMM on its codes."""
+    import rwkvq_abi as abi
+    g = torch.Generator(device="cuda").manual_seed(k + m)
+    n, ld = 192, k + 8
+    w = torch.randint(-127, 128, (n, k), generator=g, device="cuda", dtype=torch.int8)
+    x = (torch.randn((m, ld), generator=g, device="cuda") * torch.logspace(-3, 1, m, device="cuda")[:, None]).bfloat16()
+    x[1] = 0
+    ws, xs = torch.full((1,), 0.01, device="cuda"), torch.empty(m, device="cuda")
+    codes = torch.empty((m, k), dtype=torch.int8, device="cuda")
+    out = torch.empty((2, m, n), dtype=torch.float16, device="cuda")
+    st = abi.stream_ptr()
+    abi.call("rwkvq_gemv_int8", x.data_ptr(), abi.BF16, w.data_ptr(), k, ws.data_ptr(), out[0].data_ptr(), n, None, 0, m, n, k, ld, abi.DEFAULT_DIV, 0, st)
+    abi.call("rwkvq_prep_x_int8", x.data_ptr(), abi.BF16, m, k, ld, codes.data_ptr(), k, xs.data_ptr(), abi.DEFAULT_DIV, st)
+    abi.call("rwkvq_gemm_int8", codes.data_ptr(), k, xs.data_ptr(), w.data_ptr(), k, ws.data_ptr(), out[1].data_ptr(), n, None, 0, m, n, k, 0, st)
+    assert torch.equal(out[0].view(torch.int16), out[1].view(torch.int16))
