@@ -300,10 +300,7 @@ __global__ void __launch_bounds__(kT2Threads, 1) gemm_tc2_kernel(const __grid_co
 // ------------------------------------------------------------------------------------------------ host side
 static int t2_grid_pairs() { return std::max(1, sm_count() / 2); }
 
-// Measured on B200 (7.2B shapes, FP8 and INT8): the pair kernel is level with the single-CTA kernel -- +1..3 % from 4096
-// tokens on, -2..5 % at 2048 (same number of waves, deeper pipeline to fill) -- so the L2 -> shared-memory traffic it
-// halves is not what limits that kernel (under the 1 kW power cap both run at 2.2-2.5 PFLOP/s).  It is therefore used
-// from RWKVQ_TC2_MIN_M tokens on (default 4096; RWKVQ_TC2=0 switches it off, RWKVQ_TC2_MIN_M=129 uses it wherever it fits).
+// RWKVQ_TC2=0 switches the pairs off, RWKVQ_TC2_MIN_M raises their first row count (129: below it a pair tile is half empty).
 // Pairs or single CTAs?  Both run waves of tiles whose MMAs take as long (256 x 256 on a pair, 128 x 256 on a CTA), but a pair
 // loads 64 KB for a step of its tile, two single CTAs 96 KB, and an SM's intake from L2 bounds the single form.  Measured per
 // 128-byte step of K: 0.385 us on pairs, 0.41 / 0.30 / 0.24 us on single CTAs with 256 / 128 / 64 weight rows per tile (few

@@ -692,8 +692,8 @@ __global__ void __launch_bounds__(kNfSmallThreads, 1) actq_nvfp4_small_kernel(co
     }
 }
 
-// The same quantization as TWO plain launches chained by programmatic dependent launch, for blocks of up to 2^19
-// vectors (few tokens): a cooperative launch costs about 6 us more than a plain one and gives a 16-row block 16 CTAs;
+// The same quantization as TWO plain launches chained by programmatic dependent launch, for blocks of up to 2^23
+// vectors: a cooperative launch costs about 6 us more than a plain one and gives a 16-row block 16 CTAs;
 // here the abs-max pass and the code pass each spread the block over two CTAs per SM.  The maximum travels through a
 // scratch word (atomic max of the float's bits: the values are non-negative); the last CTA of the code pass clears
 // it, so the words are zero again before the next launch on the stream can reach them and a captured graph replays.

@@ -19,10 +19,11 @@ Routing by M = rows of the flattened activation:
                 block -- with many rows the per-CTA quantization (bound by the SMs' conversion throughput) costs more
                 than the weight stream it precedes.  RWKVQ_CODES_M_MIN moves the boundary; shapes whose code tile
                 does not fit shared memory fall to the routes around
-    larger M    activation-quantization kernel, then the tcgen05 GEMM on the codes: tokens as the 128-row operand,
-                128 x 256 tiles (narrower while there are fewer tiles than SMs); only a long K against few weight rows
-                (FFN value) with at most 48 tokens, or a call whose activations do not fit the GEMV's shared memory,
-                takes the weight-streaming form (weights as the 128-row operand, stream-K over the SMs)
+    larger M    activation-quantization kernel, then a tcgen05 GEMM on the codes: the cluster split-K kernel for matrices
+                with few row tiles (from 17 rows; up to 256 against a long K), else tokens as the 128-row operand with
+                128 x 256 tiles (narrower while there are fewer tiles than SMs), on CTA pairs with 256 x 256 tiles from
+                129 rows where their waves are cheaper
+From 9 rows on the quantizer and the GEMM are one call into the library with one scratch buffer.
 RWKVQ_ROUTE=tc  sends M <= 4 to the tensor-memory kernel with the quantization fused into it as well;
 RWKVQ_ROUTE=mma keeps everything on the mma.sync kernels (M <= 32 fused, codes GEMM above).  All routes compute the
 same results (INT8 bit for bit) and cross-check each other in the tests.
