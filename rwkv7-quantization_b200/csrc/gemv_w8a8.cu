@@ -175,7 +175,9 @@ __device__ __forceinline__ void store_tile(const W8Args& a, int mat, int n0, int
 // one bulk copy per row into the tile -- no arithmetic, M*K bytes per CTA; otherwise the prologue quantizes x itself.
 // FFN: 0 = plain projection; 1 = relu^2 in the epilogue and its maximum published (rwkvq_gemv_fp8_relu2); 2 = quantize with
 // the published amax (rwkvq_gemv_fp8_preamax).  Separate instantiations: the plain kernel carries none of that code.
-template <int QT, int DT, int NT, int S, bool PRE, int FFN = 0>
+// KEEP > 0: the INT8 prologue of 2-8 rows that keeps KEEP vectors per thread (int8_keep says when); as a branch of the plain
+// kernel its code cost every other row count 0.2-0.5 us per launch (width 768, two layers: 28.7 -> 30.8 us at one row).
+template <int QT, int DT, int NT, int S, bool PRE, int FFN = 0, int KEEP = 0>
 __global__ void __launch_bounds__(kThr, 2) gemv_w8a8_kernel(const W8Args a) {
     using T = typename Acc<QT>::T;
     constexpr int D = kGemvD;
@@ -308,7 +310,8 @@ __global__ void __launch_bounds__(kThr, 2) gemv_w8a8_kernel(const W8Args a) {
         }
         out_scale = div_mode_f32(amax, 448.f, a.div_mode);
     } else {
-        quantize_int8_to_smem<DT, FFN == 2>(a, mat, xq, xs, sh);
+        if constexpr (KEEP > 0) quantize_int8_chunks<DT, KEEP>(a, reinterpret_cast<const char*>(a.x[mat]), xq, xs, sh, (a.M * (a.K >> 8) + kWarps - 1) / kWarps);
+        else quantize_int8_to_smem<DT, FFN == 2>(a, mat, xq, xs, sh);
     }
     __syncthreads();
     w8_mark(a, 3);
@@ -418,9 +421,9 @@ static size_t smem_bytes(int NT, int M, int pitch, int S) {
 
 constexpr size_t kFusedSmemMax = 224 * 1024;    // of the 227 KB a CTA may opt in to
 
-template <int QT, int DT, int NT, int S, bool PRE, int FFN = 0>
+template <int QT, int DT, int NT, int S, bool PRE, int FFN = 0, int KEEP = 0>
 static int32_t launch_one(W8Args a, size_t smem, cudaStream_t st) {
-    auto kern = gemv_w8a8_kernel<QT, DT, NT, S, PRE, FFN>;
+    auto kern = gemv_w8a8_kernel<QT, DT, NT, S, PRE, FFN, KEEP>;
     // per instantiation and device: opt in to large dynamic shared memory and ask how many CTAs fit on an SM
     static thread_local int cfg_dev = -1;
     static thread_local size_t cfg_smem = ~size_t(0);
@@ -474,22 +477,42 @@ constexpr size_t kTwoPerSm = 110 * 1024;     // shared memory per CTA that still
 // Ring depth: the deepest ring (5, 4, 3 stages) that leaves room for two CTAs per SM; failing that, one CTA per SM with
 // the deepest ring that fits beside the activation tile (long rows, many tokens) -- one CTA with a deep ring measured
 // faster than two CTAs with two stages.
-template <int QT, int DT, int NT, bool PRE, int FFN = 0>
+template <int QT, int DT, int NT, bool PRE, int FFN = 0, int KEEP = 0>
 static int32_t dispatch_s(const W8Args& a, cudaStream_t st) {
     const size_t s5 = smem_bytes(NT, a.M, a.pitch, 5), s4 = smem_bytes(NT, a.M, a.pitch, 4), s3 = smem_bytes(NT, a.M, a.pitch, 3),
                  s2 = smem_bytes(NT, a.M, a.pitch, 2);
-    if (s5 <= kTwoPerSm) return launch_one<QT, DT, NT, 5, PRE, FFN>(a, s5, st);
-    if (s4 <= kTwoPerSm) return launch_one<QT, DT, NT, 4, PRE, FFN>(a, s4, st);
-    if (s3 <= kTwoPerSm) return launch_one<QT, DT, NT, 3, PRE, FFN>(a, s3, st);
+    if (s5 <= kTwoPerSm) return launch_one<QT, DT, NT, 5, PRE, FFN, KEEP>(a, s5, st);
+    if (s4 <= kTwoPerSm) return launch_one<QT, DT, NT, 4, PRE, FFN, KEEP>(a, s4, st);
+    if (s3 <= kTwoPerSm) return launch_one<QT, DT, NT, 3, PRE, FFN, KEEP>(a, s3, st);
     RWKVQ_REQUIRE(s2 <= kFusedSmemMax, RWKVQ_E_SHAPE, "gemv_w8a8: M*K = %d*%d does not fit the kernel's shared memory", a.M, a.K);
-    if (s5 <= kFusedSmemMax) return launch_one<QT, DT, NT, 5, PRE, FFN>(a, s5, st);
-    if (s4 <= kFusedSmemMax) return launch_one<QT, DT, NT, 4, PRE, FFN>(a, s4, st);
-    if (s3 <= kFusedSmemMax) return launch_one<QT, DT, NT, 3, PRE, FFN>(a, s3, st);
-    return launch_one<QT, DT, NT, 2, PRE, FFN>(a, s2, st);
+    if (s5 <= kFusedSmemMax) return launch_one<QT, DT, NT, 5, PRE, FFN, KEEP>(a, s5, st);
+    if (s4 <= kFusedSmemMax) return launch_one<QT, DT, NT, 4, PRE, FFN, KEEP>(a, s4, st);
+    if (s3 <= kFusedSmemMax) return launch_one<QT, DT, NT, 3, PRE, FFN, KEEP>(a, s3, st);
+    return launch_one<QT, DT, NT, 2, PRE, FFN, KEEP>(a, s2, st);
+}
+
+// The INT8 prologue that keeps its rows in registers: vectors per thread, or 0 where the older forms are as quick or quicker.
+// Two layers of four projections replayed from a graph, us, older forms / this one: width 768 3 rows 37.0 / 32.7, 4 rows
+// 41.0 / 31.8; 1536 4 rows 47.2 / 39.6; 2560 4 rows 73.8 / 59.5, 5 rows 63.5 / 57.4, 8 rows 63.7 / 61.3; 4096 2 rows 93.1 / 90.5,
+// 4 rows 106 / 90.9, 6 rows 100.4 / 96.7.  2 rows below K = 4096: level or slower (r/k/v of 1024: 3.6 / 3.9 per launch); 5-8
+// rows below K = 2048: a warp holds its whole row anyway (3.0 / 3.1).  More than 12 vectors per thread: slower (see the kernel's
+// prologue).
+static int int8_keep(int M, int K) {
+    if (M < 2 || M > 8 || K % 256 != 0 || K < (M == 2 ? 4096 : (M <= 4 ? 512 : 2048))) return 0;
+    const int per = (M * (K >> 8) + kWarps - 1) / kWarps;
+    return per <= 8 ? 8 : (per <= 12 ? 12 : 0);
 }
 
 template <int QT, int DT, bool PRE>
 static int32_t dispatch_mt(const W8Args& a, cudaStream_t st) {
+    if constexpr (!PRE && QT == QT_INT8) {
+        const int keep = a.flags & RWKVQ_FLAG_AMAX_GIVEN ? 0 : int8_keep(a.M, a.K);
+        const bool relu2 = (a.flags & RWKVQ_FLAG_RELU2) != 0;
+        if (keep && !(relu2 && a.nmat != 1)) {
+            if (relu2) return keep == 8 ? dispatch_s<QT, DT, 1, PRE, 1, 8>(a, st) : dispatch_s<QT, DT, 1, PRE, 1, 12>(a, st);
+            return keep == 8 ? dispatch_s<QT, DT, 1, PRE, 0, 8>(a, st) : dispatch_s<QT, DT, 1, PRE, 0, 12>(a, st);
+        }
+    }
     if constexpr (!PRE) {                       // the FFN pair: up to 8 rows
         if (a.flags & (RWKVQ_FLAG_RELU2 | RWKVQ_FLAG_AMAX_GIVEN)) {
             RWKVQ_REQUIRE(a.M <= 8 && a.nmat == 1, RWKVQ_E_SHAPE, "gemv_fp8 relu2 / preamax: at most 8 rows, got %d", a.M);

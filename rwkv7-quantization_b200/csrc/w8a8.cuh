@@ -314,8 +314,9 @@ __device__ __forceinline__ uint2 int8_vec_codes(const uint4& v, float s) {
 // The prologue is a chain of dependent latencies that every CTA repeats, so what counts is one read and few steps: a row at a
 // time cost a reduction over the CTA per row (3-4 rows), a warp per row left warps idle and read its row twice (5-8 rows).
 // [4096, 4096], whole kernel: 3 rows 7.0 -> 5.9 us, 4 rows 8.0 -> 6.2, 5 and 6 rows 7.2 -> 6.7; [2560, 2560] 5 rows
-// 5.0 -> 4.2.  KEEP is 8 or 12 and no more: the code runs once on a cold instruction cache, 16 vectors cost 0.7 us more in
-// every launch than 8, and a loop over batches of 8 that reads the earlier ones again 1.7 us.
+// 5.0 -> 4.2.  KEEP is 8 or 12 and no more, in an instantiation of its own (gemv_w8a8_kernel): the code runs once on a cold
+// instruction cache, 16 vectors cost 0.7 us more in every launch than 8, and a loop over batches of 8 that reads the earlier
+// ones again 1.7 us.
 template <int DT, int KEEP>
 __device__ __forceinline__ void quantize_int8_chunks(const W8Args& a, const char* x, uint8_t* xq, float* xs, float* sh, int per) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -386,13 +387,6 @@ __device__ void quantize_int8_to_smem(const W8Args& a, int mat, uint8_t* xq, flo
                 if (i0 + j * kThr < nvec) *reinterpret_cast<uint2*>(xq + (size_t)rr[j] * a.pitch + (size_t)cc[j] * 8) = int8_vec_codes<DT>(v[j], sh[rr[j]]);
         }
         return;
-    }
-    // (2 rows: only from K = 4096, below it the row at a time is level or quicker, r/k/v of 1024: 3.6 against 3.9 us; 5-8 rows:
-    // only from K = 2048, below it a warp holds its whole row anyway, 3.0 against 3.1 us)
-    if (a.M >= 2 && a.M <= 8 && (a.K & 255) == 0 && a.K >= (a.M == 2 ? 4096 : a.M <= 4 ? 512 : 2048)) {
-        const int per = (a.M * (a.K >> 8) + kWarps - 1) / kWarps;
-        if (per <= 8) { quantize_int8_chunks<DT, 8>(a, x, xq, xs, sh, per); return; }
-        if (per <= 12) { quantize_int8_chunks<DT, 12>(a, x, xq, xs, sh, per); return; }
     }
     if (a.M <= 4 && a.K > 2 * kThr * 8 && a.K <= 8 * kThr * 8) {
         // long rows: the whole CTA works on one row at a time and keeps it in registers between amax and codes
