@@ -32,18 +32,12 @@
 #include <algorithm>
 #include <cstdlib>
 
-#include "tc_common.cuh"
-#include "tc_host.cuh"
-#include "w8a8.cuh"
+#include "wa16.cuh"
 
 namespace rwkvq {
-using namespace tc;
 
-enum { W16_INT4_GROUP = 0, W16_INT8_TENSOR = 1 };
 constexpr int kW16Threads = 512;                // four warpgroups
 constexpr int kW16MaxStages = 7;
-constexpr int kW16K = 128;                    // k per ring stage = one INT4 group
-constexpr size_t kW16SmemBudget = 225 * 1024;
 
 struct W16Maps {
     CUtensorMap w, x;
@@ -84,60 +78,6 @@ __device__ __forceinline__ void tc_mma_f16_ts_d16(uint32_t d_tmem, uint32_t a_tm
         "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p, 4;\n\t}"
         ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc) : "memory");
 }
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {     // this thread's lane, 32 columns
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
-        "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
-        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-          "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]),
-          "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]),
-          "r"(r[30]), "r"(r[31])
-        : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,"
-        "%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-          "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
-          "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
-          "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// 8 nibbles of a word -> fp16 pairs odd = (n1,n5), (n3,n7) * 2^-20 and even = (n0,n4), (n2,n6) * 2^-24
-__device__ __forceinline__ void widen_nibbles(uint32_t w, uint32_t* odd, uint32_t* even) {
-    const uint32_t h = w >> 8;
-    odd[0] = w & 0x00F000F0u;
-    odd[1] = h & 0x00F000F0u;
-    even[0] = w & 0x000F000Fu;
-    even[1] = h & 0x000F000Fu;
-}
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ uint64_t pack2_loaded(uint32_t lo, uint32_t hi) {
-    uint64_t r;
-    asm volatile("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
-    return r;
-}
-__device__ __forceinline__ float2 unpack2(uint64_t v) {
-    float2 f;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
-    return f;
-}
-// two independent fp32 fused multiply-adds in one instruction
-__device__ __forceinline__ void fma2(uint64_t& acc, uint64_t x, uint64_t y) {
-    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(x), "l"(y));
-}
-// the same on a register pair of a tensor-memory load: volatile, so that it stays behind the load's wait
-__device__ __forceinline__ void fma2_loaded(uint64_t& acc, uint64_t x, uint32_t lo, uint32_t hi) {
-    asm volatile("{\n\t.reg .b64 t;\n\tmov.b64 t, {%2, %3};\n\tfma.rn.f32x2 %0, %1, t, %0;\n\t}" : "+l"(acc) : "l"(x), "r"(lo), "r"(hi));
-}
-
 template <int FMT, int NB>
 struct W16Tile {
     static constexpr bool kGroup = FMT == W16_INT4_GROUP;
@@ -202,8 +142,8 @@ __global__ void __launch_bounds__(kW16Threads, 1) gemm_wa16_kernel(const __grid_
         it.nt = r % a.ntiles;
         it.sl = r / a.ntiles;
         const int q4 = (a.ksteps + 3) >> 2;
-        it.k0 = (int)((int64_t)q4 * it.sl / a.slices) * 4;
-        it.k1 = min((int)((int64_t)q4 * (it.sl + 1) / a.slices) * 4, a.ksteps);
+        it.k0 = (int)((uint32_t)(q4 * it.sl) / (uint32_t)a.slices) * 4;             // below 2^21 * 16
+        it.k1 = min((int)((uint32_t)(q4 * (it.sl + 1)) / (uint32_t)a.slices) * 4, a.ksteps);
         return it;
     };
 
@@ -474,8 +414,8 @@ __global__ void __launch_bounds__(kW16Threads, 1) gemm_wa16_kernel(const __grid_
 // [0,4,2,6, 8,12,10,14, ...], and the sums of each group of 128 (of the fp16 values), [token tile][group][NB].  16 lanes hold a group; bound by the one read and one write, so a thread
 // has four vectors under way: 1 << lgP of a row and the same of the next 4 >> lgP of its CTA's rows.
 template <int DT>
-__global__ void __launch_bounds__(256) wa16_prep_kernel(const uint16_t* __restrict__ x, int64_t ldx, int M, int kv, __half* xp, float* xsum, int NB, int groups,
-                                                        int cpr, int lgP) {
+__global__ void __launch_bounds__(256) wa16_prep_kernel(const uint16_t* __restrict__ x, int64_t ldx, int M, int kv, __half* xp, float* xsum, uint4* xz, int NB,
+                                                        int groups, int cpr, int lgP) {
     griddep_launch_dependents();
     const int seg = (int)blockIdx.x % cpr, rstep = (int)gridDim.x / cpr, cstep = cpr * 256, P = 1 << lgP;
     const uint32_t mask = 0xffffu << (threadIdx.x & 16);
@@ -510,7 +450,14 @@ __global__ void __launch_bounds__(256) wa16_prep_kernel(const uint16_t* __restri
                 float sum = ((f[0].x + f[0].y) + (f[1].x + f[1].y)) + ((f[2].x + f[2].y) + (f[3].x + f[3].y));
 #pragma unroll
                 for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(mask, sum, o);
-                if ((threadIdx.x & 15) == 0) xsum[((int64_t)(m / NB) * groups + (i >> 4)) * NB + m % NB] = sum;
+                if ((threadIdx.x & 15) == 0) {
+                    if (xz) {
+                        const Bf16Parts p = bf16_parts(sum);
+                        xz[(int64_t)m * groups + (i >> 4)] = make_uint4(p.h | (p.m << 16), p.l | (p.h1 << 16), p.m | (p.h1 << 16), 0u);
+                    } else {
+                        xsum[((int64_t)(m / NB) * groups + (i >> 4)) * NB + m % NB] = sum;
+                    }
+                }
             }
         }
     }
@@ -545,14 +492,14 @@ __global__ void __launch_bounds__(256) wa16_reduce_kernel(const float* __restric
 }
 
 // ------------------------------------------------------------------------------------------------ host side
-struct W16Plan { int NB, slices; };
+struct W16Plan { int NB, slices; bool pair; };
 
-// Token tile and K slices: the pair with the least estimated time.  Measured on [4096, 4096], [16384, 4096], [4096, 16384]
-// and [2560, 2560] at 8 to 1000 rows: a step (128 k of a tile) takes 0.40 / 0.52 / 0.65 / 0.79 us with 32 / 64 / 96 / 128
-// tokens (INT4: the widened weights and the accumulators share tensor memory's ports with the MMAs) and 0.40 / 0.43 /
-// 0.48 / 0.57 us (INT8: what an SM takes in from L2); K slices cost 3.4 us for the second launch plus the round trip
-// of the partial sums.  The estimate is within 10 % of every measured pair (INT4, us: [4096, 16384] at 128 rows with
-// 4 x 128 tokens 34.2, with 2 x 64 39.8; [2560, 2560] at 17 rows in 5 slices 8.0, whole 11.1).
+// Form (single CTAs or pairs), token tile and K slices: those with the least estimated time.  Measured on [4096, 4096], [16384, 4096],
+// [4096, 16384], [2560, 2560], [10240, 2560], [2560, 10240], [1024, 1024] and [4096, 1024] at 8 to 2048 rows: a step (128 k of a tile)
+// takes 0.40 / 0.52 / 0.65 / 0.76 us with 32 / 64 / 96 / 128 tokens on one CTA (INT4: the widened weights and the accumulators share
+// tensor memory's ports with the MMAs) and 0.40 / 0.43 / 0.48 / 0.55 us (INT8: what an SM takes in from L2); on a pair, with 256 weight
+// rows, 0.51 / 0.86 us with 128 / 256 tokens (INT4) and 0.73 us with 256 (INT8); K slices cost 3.4 us for the second launch plus
+// the round trip of the partial sums.  Of the forms timed for each size the estimate takes one within 10 % of the best.
 // The register split of the INT4 kernels with 96 and 128 tokens adds up only if a thread starts with 128 registers; a compiler
 // that gives them another number leaves the narrower tiles.  RWKVQ_WA16_MAX_NB lowers the limit (read once).
 template <int NB>
@@ -564,24 +511,29 @@ static bool w16_regs_fit() {
     return fit;
 }
 static int w16_max_tokens(int fmt) {
-    static const int cap = std::getenv("RWKVQ_WA16_MAX_NB") ? std::max(32, std::atoi(std::getenv("RWKVQ_WA16_MAX_NB"))) : 128;
+    static const int cap = std::getenv("RWKVQ_WA16_MAX_NB") ? std::max(32, std::atoi(std::getenv("RWKVQ_WA16_MAX_NB"))) : 256;
     return fmt == W16_INT8_TENSOR || (w16_regs_fit<96>() && w16_regs_fit<128>()) ? cap : std::min(cap, 64);
 }
 static W16Plan wa16_plan(int fmt, int64_t M, int64_t N, int64_t K) {
-    static constexpr double kStep[2][4] = {{400., 520., 650., 790.}, {400., 430., 480., 570.}};      // ns
-    const int64_t ksteps = (K + kW16K - 1) / kW16K, nt = (N + 127) / 128, q4 = (ksteps + 3) / 4;
+    static constexpr double kStep[2][4] = {{400., 520., 650., 760.}, {400., 430., 480., 550.}};      // ns
+    static constexpr double kPairStep[2][2] = {{510., 860.}, {0., 730.}};                            // 0: no such tile
+    // RWKVQ_WA16_PAIR=0 switches the pairs off, =force uses them wherever they are legal (read once)
+    static const char mode = std::getenv("RWKVQ_WA16_PAIR") ? std::getenv("RWKVQ_WA16_PAIR")[0] : 0;
+    const int64_t ksteps = (K + kW16K - 1) / kW16K, q4 = (ksteps + 3) / 4;
     const int max_nb = w16_max_tokens(fmt);
-    W16Plan best{32, 1};
+    W16Plan best{32, 1, false};
     double best_t = 1e30;
-    for (int i = 0; i < 4; ++i) {
-        const int nb = 32 * (i + 1);
-        if (nb > max_nb) break;
-        const int64_t mt = (M + nb - 1) / nb;
+    for (int i = 0; i < 6; ++i) {
+        const bool pair = i >= 4;
+        const int nb = pair ? 128 << (i - 4) : 32 * (i + 1);
+        if (nb > max_nb || (pair && (kPairStep[fmt][i - 4] == 0. || mode == '0' || !wa16_pair_fits(fmt))) || (!pair && mode == 'f')) continue;
+        const int64_t mt = (M + nb - 1) / nb, nt = pair ? (N + 255) / 256 : (N + 127) / 128, units = pair ? sm_count() / 2 : sm_count();
         for (int64_t sl = 1; sl <= 16 && sl <= q4; ++sl) {
-            const int64_t waves = (mt * nt * sl + sm_count() - 1) / sm_count();
-            double t = (double)waves * ((double)std::min((q4 + sl - 1) / sl * 4, ksteps) * kStep[fmt][i] + 300.0);
+            const int64_t waves = (mt * nt * sl + units - 1) / units, len = std::min((q4 + sl - 1) / sl * 4, ksteps);
+            double t = (double)waves * ((double)len * (pair ? kPairStep[fmt][i - 4] : kStep[fmt][i]) + 300.0);
+            if (pair) t += waves * (fmt == W16_INT4_GROUP ? (len + 15) / 16 : 0) * kPairStep[fmt][i - 4] + 500.0;
             if (sl > 1) t += 3400.0 + (double)sl * M * N * 8.0 / 8000.0;
-            if (t < best_t) { best_t = t; best = {nb, (int)sl}; }
+            if (t < best_t) { best_t = t; best = {nb, (int)sl, pair}; }
         }
     }
     return best;
@@ -632,22 +584,6 @@ static int32_t launch_plain(Kern kern, int64_t blocks, cudaStream_t st, const ch
     return check_launch(who);
 }
 
-// byte matrix, tiles of box_rows x box_bytes; 64-byte boxes take the 64-byte swizzle
-static int32_t w16_map(CUtensorMap* m, const void* ptr, int64_t rows, int64_t row_bytes, int64_t ld, int box_rows, int box_bytes, const char* who) {
-    if (box_bytes == 128) return make_map(m, ptr, rows, row_bytes, ld, box_rows, who);
-    EncodeTiledFn fn = encode_fn();
-    RWKVQ_REQUIRE(fn != nullptr, RWKVQ_E_LAUNCH, "%s: cuTensorMapEncodeTiled is not available from the driver", who);
-    RWKVQ_REQUIRE(aligned16(ptr) && ld % 16 == 0 && ld >= row_bytes, RWKVQ_E_ALIGN, "%s: TMA needs a 16-byte aligned base and row pitch", who);
-    const cuuint64_t dims[2] = {(cuuint64_t)row_bytes, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)ld};
-    const cuuint32_t box[2] = {(cuuint32_t)box_bytes, (cuuint32_t)box_rows};
-    const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                          CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    RWKVQ_REQUIRE(r == CUDA_SUCCESS, RWKVQ_E_LAUNCH, "%s: cuTensorMapEncodeTiled failed (%d)", who, (int)r);
-    return RWKVQ_OK;
-}
-
 struct W16Layout { int64_t xp, xsum, part, total; };     // byte offsets in the workspace, 256-byte aligned
 static W16Layout wa16_layout(int fmt, int64_t M, int64_t N, int64_t K, const W16Plan& p) {
     auto up = [](int64_t v) { return (v + 255) / 256 * 256; };
@@ -655,7 +591,7 @@ static W16Layout wa16_layout(int fmt, int64_t M, int64_t N, int64_t K, const W16
     int64_t at = 0;
     if (fmt == W16_INT4_GROUP) {
         l.xp = at; at += up(M * K * 2);
-        l.xsum = at; at += up((M + p.NB - 1) / p.NB * p.NB * (K / kW16K) * 4);
+        l.xsum = at; at += up(p.pair ? M * (K / kW16K) * kW16ZSlots * 2 : (M + p.NB - 1) / p.NB * p.NB * (K / kW16K) * 4);
     }
     l.part = at;
     if (p.slices > 1) at += up((int64_t)p.slices * M * N * 4);
@@ -704,24 +640,32 @@ static int32_t run_wa16(int fmt, const void* x, int x_dtype, int64_t ldx, const 
         while (M * cpr < 2 * (int64_t)sm_count() && cpr * 512 <= kv) cpr <<= 1;
         while (lgP < 2 && (cpr * 256 << lgP) < kv) ++lgP;
         const int64_t blocks = std::min<int64_t>(M, std::max<int64_t>(1, 6 * (int64_t)sm_count() / cpr)) * cpr;
+        uint4* xz = p.pair ? reinterpret_cast<uint4*>(xsum) : nullptr;
         rc = x_dtype == RWKVQ_F16
-                 ? launch_plain(wa16_prep_kernel<RWKVQ_F16>, blocks, st, who, (const uint16_t*)x, ldx, (int)M, kv, xp, xsum, p.NB, a.groups, cpr, lgP)
-                 : launch_plain(wa16_prep_kernel<RWKVQ_BF16>, blocks, st, who, (const uint16_t*)x, ldx, (int)M, kv, xp, xsum, p.NB, a.groups, cpr, lgP);
+                 ? launch_plain(wa16_prep_kernel<RWKVQ_F16>, blocks, st, who, (const uint16_t*)x, ldx, (int)M, kv, xp, xsum, xz, p.NB, a.groups, cpr, lgP)
+                 : launch_plain(wa16_prep_kernel<RWKVQ_BF16>, blocks, st, who, (const uint16_t*)x, ldx, (int)M, kv, xp, xsum, xz, p.NB, a.groups, cpr, lgP);
         if (rc != RWKVQ_OK) return rc;
         xb = xp;
         ldxb = K;
     }
-    W16Maps maps;
-    rc = w16_map(&maps.w, w, N, group ? K / 2 : K, ldw, 128, group ? 64 : 128, who);
-    if (rc != RWKVQ_OK) return rc;
-    rc = w16_map(&maps.x, xb, M, K * 2, ldxb * 2, p.NB, 128, who);
-    if (rc != RWKVQ_OK) return rc;
-    if (group) {
-        rc = p.NB == 32 ? launch_wa16<W16_INT4_GROUP, 32>(maps, a, st, who) : p.NB == 64 ? launch_wa16<W16_INT4_GROUP, 64>(maps, a, st, who)
-             : p.NB == 96 ? launch_wa16<W16_INT4_GROUP, 96>(maps, a, st, who) : launch_wa16<W16_INT4_GROUP, 128>(maps, a, st, who);
+    if (p.pair) {
+        W16PairCall c{};
+        c.fmt = fmt; c.NB = p.NB; c.slices = p.slices; c.w = w; c.ldw = ldw; c.x = xb; c.ldx = ldxb; c.xz = a.xsum; c.scales = scales; c.zeros = zeros;
+        c.out = (__half*)out; c.part = a.part; c.ldo = ldo; c.M = M; c.N = N; c.K = K;
+        rc = run_wa16_pair(c, st, who);
     } else {
-        rc = p.NB == 32 ? launch_wa16<W16_INT8_TENSOR, 32>(maps, a, st, who) : p.NB == 64 ? launch_wa16<W16_INT8_TENSOR, 64>(maps, a, st, who)
-             : p.NB == 96 ? launch_wa16<W16_INT8_TENSOR, 96>(maps, a, st, who) : launch_wa16<W16_INT8_TENSOR, 128>(maps, a, st, who);
+        W16Maps maps;
+        rc = w16_map(&maps.w, w, N, group ? K / 2 : K, ldw, 128, group ? 64 : 128, who);
+        if (rc != RWKVQ_OK) return rc;
+        rc = w16_map(&maps.x, xb, M, K * 2, ldxb * 2, p.NB, 128, who);
+        if (rc != RWKVQ_OK) return rc;
+        if (group) {
+            rc = p.NB == 32 ? launch_wa16<W16_INT4_GROUP, 32>(maps, a, st, who) : p.NB == 64 ? launch_wa16<W16_INT4_GROUP, 64>(maps, a, st, who)
+                 : p.NB == 96 ? launch_wa16<W16_INT4_GROUP, 96>(maps, a, st, who) : launch_wa16<W16_INT4_GROUP, 128>(maps, a, st, who);
+        } else {
+            rc = p.NB == 32 ? launch_wa16<W16_INT8_TENSOR, 32>(maps, a, st, who) : p.NB == 64 ? launch_wa16<W16_INT8_TENSOR, 64>(maps, a, st, who)
+                 : p.NB == 96 ? launch_wa16<W16_INT8_TENSOR, 96>(maps, a, st, who) : launch_wa16<W16_INT8_TENSOR, 128>(maps, a, st, who);
+        }
     }
     if (rc != RWKVQ_OK || p.slices == 1) return rc;
     const int64_t per = (N & 3) == 0 ? 1024 : 256;
@@ -734,6 +678,12 @@ static int32_t run_wa16(int fmt, const void* x, int x_dtype, int64_t ldx, const 
 using namespace rwkvq;
 
 extern "C" {
+
+int32_t rwkvq_tc_gemm_wa16_form(int64_t M, int64_t N, int64_t K, int32_t bits) {
+    if (M < 1 || N < 1 || K < 1 || (bits != 4 && bits != 8) || K % (bits == 4 ? kW16K : 16)) return 0;
+    const W16Plan p = wa16_plan(bits == 4 ? W16_INT4_GROUP : W16_INT8_TENSOR, M, N, K);
+    return p.slices * 1000 + (p.pair ? -p.NB : p.NB);
+}
 
 /* Bytes of workspace that the tensor-core weight-only GEMMs need for these sizes (256-byte aligned, contents irrelevant);
  * bits = 4 (group 128) or 8 (per tensor); 0: sizes these kernels do not take. */

@@ -65,22 +65,22 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
     return ok != 0;
 }
 // Waits for the phase with the given parity; false = gave up (time limit) or another role already aborted.
-// Reading %globaltimer costs hundreds of nanoseconds, so the clock is consulted only after a few thousand failed
-// polls (tens of microseconds); short waits never touch it.
+// Reading %globaltimer costs hundreds of nanoseconds, so the clock is consulted only every 1024 failed polls, from the 4096th
+// (tens of microseconds) on; short waits never touch it.  One small loop: this is inlined at every wait of every role, and
+// roles that run different code on one scheduler share its instruction cache.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const volatile int* abort_flag, unsigned long long limit_ns) {
+    unsigned long long t0 = 0;
 #pragma unroll 1
-    for (int i = 0; i < 4096; ++i)
-        if (mbar_try_wait(bar, parity)) return true;
-    const unsigned long long t0 = global_ns();
-    for (;;) {
-#pragma unroll 1
-        for (int i = 0; i < 1024; ++i) {
-            if (mbar_try_wait(bar, parity)) return true;
-            __nanosleep(64);
-        }
-        if (*abort_flag) return false;
-        if (global_ns() - t0 > limit_ns) return false;
+    for (int i = 0; !mbar_try_wait(bar, parity); ++i) {
+        if (i < 4096) continue;
+        __nanosleep(64);
+        if (i & 1023) continue;
+        const unsigned long long now = global_ns();
+        if (t0 == 0) t0 = now;
+        if (*abort_flag || now - t0 > limit_ns) return false;
+        i = 4096;
     }
+    return true;
 }
 
 // ---------------------------------------------------------------- TMA

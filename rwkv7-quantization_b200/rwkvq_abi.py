@@ -79,6 +79,7 @@ SIGNATURES = {
     "rwkvq_gemv_int4_group_smem_bytes": [_i64, _i64],
     "rwkvq_gemv_int4_group": [_p, _i64, _p, _i64, _p, _p, _i32, _i32, _p, _i64, _i64, _i64, _i64, _p],
     "rwkvq_tc_gemm_wa16_workspace_bytes": [_i64, _i64, _i64, _i32],
+    "rwkvq_tc_gemm_wa16_form": [_i64, _i64, _i64, _i32],
     "rwkvq_tc_gemm_int4_group": [_p, _i32, _i64, _p, _i64, _p, _p, _p, _i64, _i64, _i64, _i64, _p, _i64, _p],
     "rwkvq_tc_gemm_int8_w8a16": [_p, _i64, _p, _i64, _p, _p, _i64, _i64, _i64, _i64, _p, _i64, _p],
     "rwkvq_gemv_int4_ksplit_slices": [_i64, _i64, _i64],

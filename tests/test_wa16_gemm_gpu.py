@@ -118,6 +118,50 @@ def test_plans_with_narrower_token_tiles(limit):
     subprocess.run([sys.executable, "-c", code], check=True, env=dict(os.environ, RWKVQ_WA16_MAX_NB=str(limit)), timeout=300)
 
 
+def pair_plans():
+    import rwkvq_abi as abi
+    # remainders of the 256-row and 128- / 256-token tiles, zero points of an odd and of more than 16 groups, K slices, one step
+    for m, n, k in ((17, 512, 128), (127, 769, 640), (129, 1000, 1152), (200, 4096, 4224), (257, 555, 2176), (300, 2560, 2560), (1000, 777, 640), (40, 512, 16384)):
+        for bits in (4, 8):
+            assert abi.lib().rwkvq_tc_gemm_wa16_form(m, n, k, bits) % 1000 in (1000 - 128, 1000 - 256)
+        for zeros in (True, False):
+            test_int4_group_many_rows(m, n, k, zeros)
+        test_int8_w8a16_many_rows(m, n, k)
+    test_int4_group_small_activations(200, 1000, 640, 128)
+    test_int4_infinite_and_nan_activations_stay_in_their_row(200, 640, 1152)
+    test_infinite_and_nan_activations_stay_in_their_row(40, 256)
+    assert abi.device_status() == 0
+
+
+def test_plans_on_cta_pairs():
+    """Pairs wherever they are legal; a process reads the switch once."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    code = f"import sys; sys.path[:0] = [{os.path.join(root, 'rwkv7-quantization_b200')!r}, {root!r}, {os.path.join(root, 'tests')!r}]\n" \
+           "import test_wa16_gemm_gpu as t; t.pair_plans()"
+    subprocess.run([sys.executable, "-c", code], check=True, env=dict(os.environ, RWKVQ_WA16_PAIR="force"), timeout=300)
+
+
+@pytest.mark.parametrize("z", [0.0, 1.0, -2.0 ** -120, 3.0e38, float("inf")])
+def test_int4_zero_points_of_unusual_size_on_pairs(z):
+    """The zero points' three bf16 parts: 0, a value that is one part, a tiny and a huge one, an infinity -- against the form that
+    multiplies them in fp32."""
+    import rwkvq_abi as abi
+    from int4 import int4_ops, quantize_int4
+    m, n, k = 1000, 4096, 256
+    assert abi.lib().rwkvq_tc_gemm_wa16_form(m, n, k, 4) < 1000
+    info = quantize_int4.quantize_to_int4_groupwise(gen(1, (n, k), k ** -0.5), 128)
+    info["zeros"][5, 1] = z
+    d = {a: b.cuda() if torch.is_tensor(b) else b for a, b in info.items()}
+    d["qtype"] = "int4_groupwise"
+    x = gen(2, (m, k)).half()
+    x[:, 128:] = x[:, 128:].abs()                              # sums of one sign
+    y, few = int4_ops.linear_int4(x.cuda(), d), int4_ops.linear_int4(x[:16].cuda(), d)
+    assert torch.equal(y[:16, 5].isinf(), few[:, 5].isinf()) and not bool(y[:, 5].isnan().any())
+    ok = few[:, 5].isfinite()
+    assert bool(((y[:16, 5] - few[:, 5])[ok].abs() <= few[:, 5][ok].abs() * 2.0 ** -10 + 2.0 ** -10).all())
+    assert bool(y[:, :5].isfinite().all()) and bool(y[:, 6:].isfinite().all())
+
+
 # the streaming decode kernel: token tiles of 8 and their remainders, K ranges of a warp that end inside a chunk (K = 2560,
 # 2320) and inside a 64-byte unit (K = 16, 336), row tiles with a remainder, blocks that no longer fit (tensor-core GEMM)
 @pytest.mark.parametrize("m,n,k", [(1, 16384, 4096), (1, 40, 16), (3, 2560, 2560), (8, 1000, 336), (9, 777, 2320), (16, 4096, 4096),
