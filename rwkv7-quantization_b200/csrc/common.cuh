@@ -215,6 +215,25 @@ __device__ __forceinline__ uint4 ldg_stream(const void* p) {
     return r;
 }
 
+// 16 fp16 values of a result row: one 32-byte store where the row allows it (two 16-byte stores of a lane send each sector to
+// L2 twice, as halves), `left` = columns from here to the row's end
+__device__ __forceinline__ void store_f16x16(__half* o, const uint32_t (&h)[8], int left, bool vec16, bool vec32) {
+    if (vec32 && left >= 16) {
+        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                     ::"l"(o), "r"(h[0]), "r"(h[1]), "r"(h[2]), "r"(h[3]), "r"(h[4]), "r"(h[5]), "r"(h[6]), "r"(h[7]) : "memory");
+    } else if (vec16 && left >= 16) {
+        reinterpret_cast<uint4*>(o)[0] = make_uint4(h[0], h[1], h[2], h[3]);
+        reinterpret_cast<uint4*>(o)[1] = make_uint4(h[4], h[5], h[6], h[7]);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+            if (j < left) o[j] = __ushort_as_half((unsigned short)((h[j >> 1] >> ((j & 1) * 16)) & 0xffff));
+    }
+}
+// rows of a result start on 16- / 32-byte boundaries
+__device__ __forceinline__ bool rows_vec16(const void* out, int64_t ldo) { return (ldo % 8 == 0) && ((reinterpret_cast<uintptr_t>(out) & 15) == 0); }
+__device__ __forceinline__ bool rows_vec32(const void* out, int64_t ldo) { return (ldo % 16 == 0) && ((reinterpret_cast<uintptr_t>(out) & 31) == 0); }
+
 __device__ __forceinline__ unsigned long long global_ns() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)::"memory");

@@ -434,7 +434,8 @@ __global__ void __launch_bounds__(kTcThreads, SWAP ? 2 : 1) gemm_tc_kernel(const
                 e.acc = KIND == KIND_I8 && a.acc[p.mat] ? a.acc[p.mat] + (int64_t)m * a.ldacc : nullptr;
                 e.N = a.N;
                 e.live = m < a.M;
-                e.vec_ok = (a.ldo % 8 == 0) && ((reinterpret_cast<uintptr_t>(a.out[p.mat]) & 15) == 0);
+                e.vec_ok = rows_vec16(a.out[p.mat], a.ldo);
+                e.vec32 = rows_vec32(a.out[p.mat], a.ldo);
                 e.flags = a.flags;
             }
             if (!mbar_wait(&s.tfull[buf], (pc >> 1) & 1, abort_flag, a.wait_ns)) { tc_abort(s, a); break; }

@@ -225,7 +225,8 @@ __global__ void __launch_bounds__(kT2Threads, 1) gemm_tc2_kernel(const __grid_co
             e.acc = KIND == KIND_I8 && a.acc[mat] ? a.acc[mat] + (int64_t)m * a.ldacc : nullptr;
             e.N = a.N;
             e.live = m < a.M;
-            e.vec_ok = (a.ldo % 8 == 0) && ((reinterpret_cast<uintptr_t>(a.out[mat]) & 15) == 0);
+            e.vec_ok = rows_vec16(a.out[mat], a.ldo);
+            e.vec32 = rows_vec32(a.out[mat], a.ldo);
             e.flags = a.flags;
             if (!mbar_wait(&s.tfull[fp.i], fp.phase, abort_flag, a.wait_ns)) { t2_abort(s, a); break; }
             tc_fence_after_sync();

@@ -14,9 +14,9 @@
 // One persistent CTA per SM: warp 0 = producer (one lane), warp 1 = MMA issuer (one lane) and owner of the
 // tensor-memory allocation, warps 2-9 = epilogue (two per lane quarter).  Tile 128 tokens x BN weight rows;
 // BN = 128 keeps two accumulators in tensor memory so the epilogue of a tile overlaps the MMAs of the next,
-// BN = 256 keeps one, whose epilogue is exposed: eight warps read it before they convert and store anything.  Measured,
-// us, one lane walking the loops and four epilogue warps -> here: [4096, 4096] 2048 rows 31.3 -> 20.2, [16384, 4096] 105.3 -> 67.4,
-// [4096, 16384] 101.4 -> 58.5 (4.7 PFLOP/s), [2560, 2560] 512 rows 9.9 -> 7.3.  Every mbarrier wait is bounded; a timeout is reported through the status word.
+// BN = 256 keeps one, whose epilogue is exposed: eight warps read it before they convert and store anything.  Results go out in
+// 32-byte stores, whole sectors (as pairs of 16 bytes: [16384, 4096] 2048 rows 68.0 -> 61.4 us, [10240, 2560] 39.6 -> 30.8).  Large
+// prompts run on CTA pairs (gemm_tc2_nvfp4.cu, which has the rule).  Every mbarrier wait is bounded; a timeout is reported through the status word.
 //
 // The format is described in the reference's reports (iterations/phase1_nvfp4_exploration/reports/
 // 03_fused_kernel_en.md:22-34, 11_fused_gemm_ops_en.md:20-26); the reference ships no code for it.
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(kNfThreads, 1) gemm_tc_nvfp4_kernel(const __gr
         griddep_wait();
         const int q = warp & 3;                         // tensor-memory lane quarter this warp may read
         const float scale = a.a_pts[0] * a.w_pts[0];
-        const bool vec_ok = (a.ldo % 8 == 0) && ((reinterpret_cast<uintptr_t>(a.out) & 15) == 0);
+        const bool vec_ok = rows_vec16(a.out, a.ldo), vec32 = rows_vec32(a.out, a.ldo);
         uint32_t pc = 0;
         for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++pc) {
             const int mt = t % a.mtiles, nt = t / a.mtiles;
@@ -250,15 +250,7 @@ __global__ void __launch_bounds__(kNfThreads, 1) gemm_tc_nvfp4_kernel(const __gr
                         const __half2 hh = __floats2half2_rn(__uint_as_float(r[2 * j]) * scale, __uint_as_float(r[2 * j + 1]) * scale);
                         h[j] = *reinterpret_cast<const uint32_t*>(&hh);
                     }
-                    __half* o = a.out + (int64_t)m * a.ldo + n0;
-                    if (vec_ok && n0 + 16 <= a.N) {
-                        reinterpret_cast<uint4*>(o)[0] = make_uint4(h[0], h[1], h[2], h[3]);
-                        reinterpret_cast<uint4*>(o)[1] = make_uint4(h[4], h[5], h[6], h[7]);
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 16; ++j)
-                            if (n0 + j < a.N) o[j] = __ushort_as_half((unsigned short)((h[j >> 1] >> ((j & 1) * 16)) & 0xffff));
-                    }
+                    store_f16x16(a.out + (int64_t)m * a.ldo + n0, h, a.N - n0, vec_ok, vec32);
                 };
 #pragma unroll
                 for (int c0 = h0; c0 < h0 + BN / 2; c0 += 64) {
@@ -381,12 +373,14 @@ static int32_t run_tc_nvfp4(const uint8_t* a_codes, int64_t lda, const uint8_t* 
     if (push == nullptr && tcs_nvfp4_eligible(M, N, K))         // few tokens: K split across a thread-block cluster
         return run_tcs_nvfp4(a_codes, lda, a_scales_blocked, a_pts, w_codes, ldw, w_scales_blocked, w_tscale, (__half*)out_f16, ldo, M, N, K,
                              workspace ? reinterpret_cast<int*>(workspace) + kWsCounterInts : nullptr, (cudaStream_t)stream, who);
-    const char* bn_env = std::getenv("RWKVQ_NF4_BN");          // read per call: a test switches tiles in one process
+    const char* bn_env = std::getenv("RWKVQ_NF4_BN");          // 128, 256 or "pair"; read per call: a test switches tiles in one process
     const int forced_bn = bn_env ? std::atoi(bn_env) : 0;
-    // 256-row weight tiles halve the activation re-reads per flop but keep one accumulator; they pay once there are
-    // enough of them to fill the SMs
-    const int64_t tiles256 = ((M + kNfTileM - 1) / kNfTileM) * ((N + 255) / 256);
-    const int bn = forced_bn == 128 || forced_bn == 256 ? forced_bn : (tiles256 * 4 >= (int64_t)sm_count() * 3 ? 256 : 128);
+    const bool forced_pair = bn_env && bn_env[0] == 'p';
+    const int form = forced_pair ? 0 : (forced_bn == 128 || forced_bn == 256 ? forced_bn : tc_nvfp4_form(M, N, K));
+    if (push == nullptr && form == 0)
+        return run_tc2_nvfp4(a_codes, lda, a_scales_blocked, a_pts, w_codes, ldw, w_scales_blocked, w_tscale, (__half*)out_f16, ldo, M, N, K,
+                             workspace ? reinterpret_cast<int*>(workspace) + kWsCounterInts : nullptr, (cudaStream_t)stream, who);
+    const int bn = form ? form : 256;                          // a pushing call stays on single CTAs
     NfArgs a{};
     if (push) a.push = *push;
     a.wait_ns = wait_limit_ns();

@@ -21,7 +21,7 @@ struct EpiRow {
     __half* out;                   // this token's row of the result
     int32_t* acc;                  // INT8: this token's row of raw accumulators, or null (EPI_ANY only)
     int N;
-    bool live, vec_ok;             // the token exists; 16-byte stores are possible
+    bool live, vec_ok, vec32;      // the token exists; 16- / 32-byte stores are possible
     uint32_t flags;
 };
 
@@ -64,15 +64,7 @@ __device__ __forceinline__ void epi_store16(const EpiRow& e, const uint32_t (&r)
     if (!e.live || n0 >= e.N) return;
     uint32_t h[8];
     epi_convert16<KIND, EPI>(e, r, n0, h, hmax);
-    __half* o = e.out + n0;
-    if (e.vec_ok && n0 + 16 <= e.N) {
-        reinterpret_cast<uint4*>(o)[0] = make_uint4(h[0], h[1], h[2], h[3]);
-        reinterpret_cast<uint4*>(o)[1] = make_uint4(h[4], h[5], h[6], h[7]);
-    } else {
-#pragma unroll
-        for (int j = 0; j < 16; ++j)
-            if (n0 + j < e.N) o[j] = __ushort_as_half((unsigned short)((h[j >> 1] >> ((j & 1) * 16)) & 0xffff));
-    }
+    store_f16x16(e.out + n0, h, e.N - n0, e.vec_ok, e.vec32);
     if constexpr (KIND == tc::KIND_I8 && EPI == EPI_ANY) {
         if (e.acc) {
 #pragma unroll

@@ -136,6 +136,13 @@ struct Tc2Call {
 bool tc2_eligible(int kind, int64_t M, int64_t N, int64_t K, int nmat, int single_nb);
 int32_t run_tc2(const Tc2Call& c, int* status, cudaStream_t st, const char* who);
 
+// NVFP4 GEMM for many tokens on CTA pairs (gemm_tc2_nvfp4.cu), and which tiled form these sizes take (0: pairs, else the weight rows
+// per tile of the single-CTA form).
+int tc_nvfp4_form(int64_t M, int64_t N, int64_t K);
+int32_t run_tc2_nvfp4(const uint8_t* a_codes, int64_t lda, const uint8_t* a_scales_blocked, const float* a_pts, const uint8_t* w_codes, int64_t ldw,
+                      const uint8_t* w_scales_blocked, const float* w_tscale, __half* out, int64_t ldo, int64_t M, int64_t N, int64_t K, int* status,
+                      cudaStream_t st, const char* who);
+
 // NVFP4 GEMM for few tokens (up to 256) on the cluster split-K kernel of gemm_tc.cu (gemm_tcs.cuh): weights = the
 // 128-row operand, K split across a thread-block cluster, partial sums through distributed shared memory.
 bool tcs_nvfp4_eligible(int64_t M, int64_t N, int64_t K);

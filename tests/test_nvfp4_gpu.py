@@ -109,10 +109,10 @@ def test_pack_scales_blocked_order(nf):
     assert got.shape[0] == want.size and (got == want.reshape(-1)).all()
 
 
-@pytest.mark.parametrize("bn", ["128", "256"])
-@pytest.mark.parametrize("m,n,k", [(17, 128, 256), (130, 520, 1024), (300, 384, 2048), (128, 2048, 4096), (513, 1000, 768)])
+@pytest.mark.parametrize("bn", ["128", "256", "pair"])
+@pytest.mark.parametrize("m,n,k", [(17, 128, 256), (130, 520, 1024), (300, 384, 2048), (128, 2048, 4096), (513, 1000, 768), (257, 257, 1536), (1030, 5000, 256)])
 def test_tensor_core_route(nf, monkeypatch, bn, m, n, k):
-    """The tcgen05 block-scaled GEMM (both tile widths) against the oracle and against the GEMV route; ragged M and N."""
+    """The tcgen05 block-scaled GEMM (both tile widths and CTA pairs; few and many tiles per CTA) against the oracle and against the GEMV route; ragged M and N."""
     import rwkvq_abi as abi
     monkeypatch.setenv("RWKVQ_NF4_BN", bn)
     w = gen(n * 3 + k, (n, k), (1.0 / k) ** 0.5)

@@ -109,3 +109,25 @@ def test_pairs_and_single_ctas_give_the_same_bits(tmp_path):
     assert len(here) == len(runs["force"]) == len(runs["0"])
     for a, b, c in zip(here, runs["force"], runs["0"]):
         assert torch.equal(a, b) and torch.equal(a, c)
+
+
+@pytest.mark.parametrize("offset", [8, 16])
+@pytest.mark.parametrize("m,n,k", [(40, 512, 512), (200, 1024, 512), (600, 2048, 512), (1100, 4096, 256)])
+def test_results_in_a_column_range(m, n, k, offset):
+    """Rows that start on 16- and on 32-byte boundaries (the epilogue's store widths) give the same bits as a result of its own, and
+    leave the columns around them alone."""
+    import fused_fp8_gemm as f
+    import nvfp4_ops
+    import rwkvq_abi as abi
+    g = torch.Generator(device="cuda").manual_seed(m)
+    x = torch.randn((m, k), generator=g, device="cuda").half()
+    w = torch.randn((n, k), generator=g, device="cuda") * k ** -0.5
+    s = w.abs().max()
+    for info in ({"weight": (w / s * 448).to(torch.float8_e4m3fn), "tensor_scale": s / 448, "qtype": "fp8"},
+                 {"weight": (w / s * 127).round().to(torch.int8), "tensor_scale": s / 127, "qtype": "int8"}, nvfp4_ops.quantize_to_nvfp4(w)):
+        want = f.linear_quantized_fused(x, info)
+        wide = torch.full((m, n + 32), 7.0, dtype=torch.float16, device="cuda")
+        with abi.output_into(wide[:, offset:offset + n]):
+            f.linear_quantized_fused(x, info)
+        assert torch.equal(wide[:, offset:offset + n], want)
+        assert bool((wide[:, :offset] == 7).all()) and bool((wide[:, offset + n:] == 7).all())
