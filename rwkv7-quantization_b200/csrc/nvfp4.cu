@@ -737,15 +737,15 @@ __global__ void __launch_bounds__(kNfTwoThreads) actq_nvfp4_two_amax_kernel(cons
 }
 
 // Codes pass.  A thread takes a whole 16-block (no exchange for its maximum, one scale, one reciprocal, one 8-byte store) and
-// has two under way: two groups of kNfTwoThreads blocks of a row, or the same group of two of its CTA's rows when a row
-// has no more (one = 1).  Four neighbouring scales of a row are one word of the blocked layout: every fourth lane collects
-// and stores them.  Bound by its instructions: with a vector of 8 per thread and a division per element it ran 138
-// instructions a vector at three CTAs an SM (2048 rows of 16384: both passes 54 us, now 32).
-template <int DT>
-__global__ void __launch_bounds__(kNfTwoThreads, 4) actq_nvfp4_two_codes_kernel(const NfQArgs a, int cpr, int one) {
+// has J under way.  The blocks of all rows are one list, whatever a row's length is: CTAs of whole rows left four fifths of
+// their threads idle at K = 768 and ran two waves at 2048 rows of 4096 (both passes, us: 1000 rows of 768 10.2 -> 5.8, of 4096 11.8 -> 8.2,
+// 2048 rows of 768 12.4 -> 6.7, of 4096 14.5 -> 10.8).  Four neighbouring scales of a row are one word of the blocked layout: every
+// fourth lane collects and stores them.  Block i is in row i * magic >> 40, the exact quotient: i < 2^23 and nb <= 2^16 (host),
+// magic = ceil(2^40 / nb).
+template <int DT, int J>
+__global__ void __launch_bounds__(kNfTwoThreads, 4) actq_nvfp4_two_codes_kernel(const NfQArgs a, int total, unsigned long long magic) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const int nb = a.K >> 4, lane = threadIdx.x & 31;
-    const int seg = (int)blockIdx.x % cpr, rstep = (int)gridDim.x / cpr, cstep = cpr * kNfTwoThreads;
+    const int nb = a.K >> 4, lane = threadIdx.x & 31, step = (int)gridDim.x * kNfTwoThreads;
     int* two = reinterpret_cast<int*>(a.flags) + kNfQMaxCtas + 4;
     const int64_t k64 = a.K >> 6;
     const bool words = (a.K & 63) == 0 && (reinterpret_cast<uintptr_t>(a.bs_blocked) & 3) == 0;
@@ -756,62 +756,61 @@ __global__ void __launch_bounds__(kNfTwoThreads, 4) actq_nvfp4_two_codes_kernel(
     const float pts = __fdiv_rn(amax, 2688.f);
     if (blockIdx.x == 0 && threadIdx.x == 0) *a.pts = pts;
     const float inv_pts = __fdiv_rn(1.f, pts), k448 = __fdiv_rn(448.f, amax);
-    const int jr = one ? rstep : 0, jc = one ? 0 : cstep;           // where the second block of a thread lies
-    for (int r0 = (int)blockIdx.x / cpr; r0 < a.M; r0 += one ? 2 * rstep : rstep) {
-        for (int base = seg * kNfTwoThreads; base < nb; base += one ? cstep : 2 * cstep) {
-            uint4 v[2][2];
+    for (int b0 = (int)blockIdx.x * kNfTwoThreads + (int)threadIdx.x; b0 - lane < total; b0 += J * step) {
+        uint4 v[J][2];
+        int row[J];
 #pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const int r = r0 + j * jr, i = base + j * jc + (int)threadIdx.x;
-                v[j][0] = v[j][1] = make_uint4(0, 0, 0, 0);
-                if (r < a.M && i < nb) {
-                    const uint4* p = reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(a.x) + ((int64_t)r * a.ldx + (int64_t)i * 16) * 2);
-                    v[j][0] = p[0];
-                    v[j][1] = p[1];
-                }
+        for (int j = 0; j < J; ++j) {
+            const int b = b0 + j * step;
+            row[j] = (int)(((unsigned long long)b * magic) >> 40);
+            v[j][0] = v[j][1] = make_uint4(0, 0, 0, 0);
+            if (b < total) {
+                const uint4* p = reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(a.x) + ((int64_t)row[j] * a.ldx + (int64_t)(b - row[j] * nb) * 16) * 2);
+                v[j][0] = p[0];
+                v[j][1] = p[1];
             }
+        }
 #pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const int r = r0 + j * jr, i = base + j * jc + (int)threadIdx.x;
-                if (r >= a.M || i - (int)threadIdx.x >= nb) continue;      // uniform over the CTA
-                const uint32_t wv[8] = {v[j][0].x, v[j][0].y, v[j][0].z, v[j][0].w, v[j][1].x, v[j][1].y, v[j][1].z, v[j][1].w};
-                const float bm = fmaxf(packed_absmax8<DT>(v[j][0]), packed_absmax8<DT>(v[j][1]));
-                const float sb = fminf(fmaxf(bm * k448, 0.015625f), 448.f);
-                const uint32_t sc = e4m3x2(sb, 0.f) & 0xffu;
-                const float bs = e4m3_to_float(sc), rc = block_scale_rcp(sc, eighth);
-                uint32_t out[2];
+        for (int j = 0; j < J; ++j) {
+            const int b = b0 + j * step, r = row[j], i = b - r * nb;
+            if (b - lane >= total) continue;                        // uniform over the warp
+            const uint32_t wv[8] = {v[j][0].x, v[j][0].y, v[j][0].z, v[j][0].w, v[j][1].x, v[j][1].y, v[j][1].z, v[j][1].w};
+            const float bm = fmaxf(packed_absmax8<DT>(v[j][0]), packed_absmax8<DT>(v[j][1]));
+            const float sb = fminf(fmaxf(bm * k448, 0.015625f), 448.f);
+            const uint32_t sc = e4m3x2(sb, 0.f) & 0xffu;
+            const float bs = e4m3_to_float(sc), rc = block_scale_rcp(sc, eighth);
+            uint32_t out[2];
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    float f[8];
+            for (int h = 0; h < 2; ++h) {
+                float f[8];
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const float2 p = cvt2<DT>(wv[4 * h + q]);
-                        f[2 * q] = p.x;
-                        f[2 * q + 1] = p.y;
-                    }
-                    out[h] = nvfp4_codes8(f, inv_pts, bs, rc);
+                for (int q = 0; q < 4; ++q) {
+                    const float2 p = cvt2<DT>(wv[4 * h + q]);
+                    f[2 * q] = p.x;
+                    f[2 * q + 1] = p.y;
                 }
-                uint32_t sc4 = sc;
-                if (words) {
-                    sc4 |= __shfl_down_sync(0xffffffffu, sc, 1) << 8;
-                    sc4 |= __shfl_down_sync(0xffffffffu, sc, 2) << 16;
-                    sc4 |= __shfl_down_sync(0xffffffffu, sc, 3) << 24;
+                out[h] = nvfp4_codes8(f, inv_pts, bs, rc);
+            }
+            uint32_t sc4 = sc;
+            if (words) {                                            // K a multiple of 64: the four lanes are on one row
+                sc4 |= __shfl_down_sync(0xffffffffu, sc, 1) << 8;
+                sc4 |= __shfl_down_sync(0xffffffffu, sc, 2) << 16;
+                sc4 |= __shfl_down_sync(0xffffffffu, sc, 3) << 24;
+            }
+            if (b < total) {
+                uint32_t* c = reinterpret_cast<uint32_t*>(a.codes + (int64_t)r * a.ldc + (int64_t)i * 8);
+                if (wide) {
+                    *reinterpret_cast<uint2*>(c) = make_uint2(out[0], out[1]);
+                } else {
+                    c[0] = out[0];
+                    c[1] = out[1];
                 }
-                if (i < nb) {
-                    uint32_t* c = reinterpret_cast<uint32_t*>(a.codes + (int64_t)r * a.ldc + (int64_t)i * 8);
-                    if (wide) {
-                        *reinterpret_cast<uint2*>(c) = make_uint2(out[0], out[1]);
-                    } else {
-                        c[0] = out[0];
-                        c[1] = out[1];
-                    }
-                    if (a.bs_blocked) {
-                        uint8_t* blk = a.bs_blocked + ((int64_t)(r >> 7) * k64 + (i >> 2)) * 512 + (r & 31) * 16 + ((r & 127) >> 5) * 4 + (i & 3);
-                        if (!words) *blk = (uint8_t)sc;
-                        else if ((lane & 3) == 0) *reinterpret_cast<uint32_t*>(blk) = sc4;
-                    }
-                    if (a.bs_rows) a.bs_rows[(int64_t)r * a.lds + i] = (uint8_t)sc;
+                if (a.bs_blocked) {
+                    uint8_t* blk = a.bs_blocked + ((int64_t)(r >> 7) * k64 + (i >> 2)) * 512 + (r & 31) * 16 + ((r & 127) >> 5) * 4 + (i & 3);
+                    if (!words) *blk = (uint8_t)sc;
+                    else if ((lane & 3) == 0) *reinterpret_cast<uint32_t*>(blk) = sc4;
                 }
+                if (a.bs_rows) a.bs_rows[(int64_t)r * a.lds + i] = (uint8_t)sc;
             }
         }
     }
@@ -957,11 +956,10 @@ int32_t rwkvq_actq_nvfp4_fused(const void* x, int32_t x_dtype, int64_t M, int64_
     }
     const char* two_env = std::getenv("RWKVQ_NVFP4_ACTQ_TWO_MAX");      // read per call: a test switches routes in one process
     const int64_t two_max = two_env ? std::atoll(two_env) : kNfTwoMaxVectors;
-    if (M * (K / 8) <= two_max) {
+    if (M * (K / 8) <= std::min(two_max, (int64_t)1 << 24) && K <= (int64_t)1 << 20) {      // the limits of the codes pass' division
         const int nb = (int)(K / 16);
-        int cpr = 1;                                     // CTAs per row: about two CTAs per SM in all, 256+ blocks each
+        int cpr = 1;                                     // abs-max, CTAs per row: about two CTAs per SM in all, 256+ blocks each
         while ((int64_t)M * cpr < 2 * (int64_t)sm_count() && cpr * 2 * kNfTwoThreads <= nb) cpr <<= 1;
-        const int one = cpr * kNfTwoThreads >= nb ? 1 : 0;      // a CTA's share of a row is one block per thread
         const int rows = (int)std::min<int64_t>(M, std::max<int64_t>(1, 8 * (int64_t)sm_count() / cpr));
         // abs-max of a dense block: one long row, whatever its rows are (no half-filled groups of loads at row ends)
         NfQArgs m = a;
@@ -982,10 +980,19 @@ int32_t rwkvq_actq_nvfp4_fused(const void* x, int32_t x_dtype, int64_t M, int64_
         cfg.numAttrs = use_pdl() ? 1 : 0;
         cudaError_t e = x_dtype == RWKVQ_F16 ? cudaLaunchKernelEx(&cfg, actq_nvfp4_two_amax_kernel<RWKVQ_F16>, m, mcpr)
                                              : cudaLaunchKernelEx(&cfg, actq_nvfp4_two_amax_kernel<RWKVQ_BF16>, m, mcpr);
-        cfg.gridDim = dim3((unsigned)(rows * cpr));
+        // codes: four CTAs an SM are resident.  Four blocks a thread under way where two do not cover the list and one or two
+        // rounds of four do; larger lists are bound by throughput, two a thread and twice the CTAs (both passes, us: 2048 rows of 16384
+        // 32.3, four a thread on the resident CTAs 34.9; 1024 rows of 16384 19.8 and 18.0)
+        const int64_t total = M * nb, per = kNfTwoThreads, res = 4 * (int64_t)sm_count();
+        const bool four = total > 2 * res * per && total <= 7 * res * per;
+        cfg.gridDim = dim3((unsigned)std::min(total > 7 * res * per ? 2 * res : res, (total + per - 1) / per));
+        const unsigned long long magic = ((1ull << 40) + nb - 1) / nb;
+        const int tot = (int)total;
         if (e == cudaSuccess)
-            e = x_dtype == RWKVQ_F16 ? cudaLaunchKernelEx(&cfg, actq_nvfp4_two_codes_kernel<RWKVQ_F16>, a, cpr, one)
-                                     : cudaLaunchKernelEx(&cfg, actq_nvfp4_two_codes_kernel<RWKVQ_BF16>, a, cpr, one);
+            e = x_dtype == RWKVQ_F16 ? (four ? cudaLaunchKernelEx(&cfg, actq_nvfp4_two_codes_kernel<RWKVQ_F16, 4>, a, tot, magic)
+                                             : cudaLaunchKernelEx(&cfg, actq_nvfp4_two_codes_kernel<RWKVQ_F16, 2>, a, tot, magic))
+                                     : (four ? cudaLaunchKernelEx(&cfg, actq_nvfp4_two_codes_kernel<RWKVQ_BF16, 4>, a, tot, magic)
+                                             : cudaLaunchKernelEx(&cfg, actq_nvfp4_two_codes_kernel<RWKVQ_BF16, 2>, a, tot, magic));
         if (e != cudaSuccess) {
             g_launches.fetch_add(1, std::memory_order_relaxed);
             return fail(RWKVQ_E_LAUNCH, "%s: %s", who, cudaGetErrorString(e));

@@ -230,6 +230,26 @@ def test_cluster_splitk_route(nf, monkeypatch, m, n, k):
     assert rel_err(out, O.linear_nvfp4(x, oinfo)) <= 1e-2
 
 
+# the list of blocks of the two-launch form: rows shorter than a CTA, row ends inside a warp, less than one round of the resident
+# CTAs, two and four blocks a thread, more than one round; K no multiple of 64
+@pytest.mark.parametrize("m,k", [(1000, 768), (2100, 2320), (333, 80), (1185, 4096), (2048, 4096), (1200, 16384), (1100, 16400)])
+def test_two_launch_quantizer_covers_every_block(nf, monkeypatch, m, k):
+    monkeypatch.setenv("RWKVQ_NVFP4_ACTQ_SMALL_MAX", "0")
+    for dtype in (torch.bfloat16, torch.float16):
+        x = gen(m * 5 + k, (m, k), 1.0, dtype).cuda()
+        monkeypatch.setenv("RWKVQ_NVFP4_ACTQ", "split")
+        want = nf.quantize_activations_nvfp4(x)
+        monkeypatch.setenv("RWKVQ_NVFP4_ACTQ", "fused")
+        got = nf.quantize_activations_nvfp4(x)
+        assert torch.equal(want[0], got[0]) and torch.equal(want[1].view(torch.uint8), got[1].view(torch.uint8)) and torch.equal(want[2], got[2])
+    if k % 64 == 0:
+        codes, blk, _ = nf.quantize_activations_nvfp4(x, blocked=True)
+        rows = torch.arange(m, device="cuda")[:, None]
+        b = torch.arange(k // 16, device="cuda")[None, :]
+        at = ((rows // 128) * (k // 64) + b // 4) * 512 + (rows % 32) * 16 + ((rows % 128) // 32) * 4 + b % 4
+        assert torch.equal(blk[at], want[1].view(torch.uint8)) and torch.equal(codes, want[0])
+
+
 @pytest.mark.parametrize("form", ["auto", "two", "coop"])
 @pytest.mark.parametrize("m,k", [(1, 512), (130, 1024), (300, 4096), (16, 16384), (5, 4096), (64, 4096), (3, 16448)])
 def test_fused_activation_quantizer_routes_agree(nf, monkeypatch, m, k, form):
