@@ -1,5 +1,7 @@
 // W8A8 GEMM for many tokens on CTA PAIRS: tcgen05.mma.cta_group::2 (two SMs work on one 256 x 256 tile).
 //
+// Tiles: 256 tokens x bn weight rows (below: bn = 256).
+//
 // Why pairs.  With one CTA per 128 x 256 tile (gemm_tc.cu) every 128-byte step of K needs 48 KB of operands from L2
 // per SM for 512 cycles of tensor-core work -- 96 bytes per clock, more than an SM gets from L2, so the tensor pipe
 // idles a third of the time.  In a pair each CTA loads its own 128 token rows and only HALF of the 256 weight rows
@@ -30,11 +32,11 @@ constexpr int kT2Chunk = 128;                 // bytes of K per stage
 constexpr int kT2Rows = 128;                  // rows of each operand tile per CTA
 constexpr uint32_t kT2TileBytes = kT2Rows * kT2Chunk;      // 16 KB
 constexpr uint32_t kT2StageBytes = 2 * kT2TileBytes;       // tokens + this CTA's half of the weight tile
-constexpr int kT2N = 256;                     // weight rows per pair tile (UMMA N)
+constexpr int kT2N = 256;                     // most weight rows per pair tile (UMMA N)
 
 struct Tc2Maps {
     CUtensorMap a[3];   // activation codes [M, K], box 128 rows x 128 bytes
-    CUtensorMap w[3];   // weights [N, K], box 128 rows x 128 bytes
+    CUtensorMap w[3];   // weights [N, K], box bn / 2 rows x 128 bytes
 };
 
 struct Tc2Args {
@@ -47,7 +49,8 @@ struct Tc2Args {
     unsigned long long wait_ns;
     int64_t ldo, ldacc;
     int M, N, K, nmat;
-    int kchunks, ptiles, qtiles, stages;      // ptiles: 256-token pair tiles, qtiles: 256-row weight tiles
+    int bn;                                   // weight rows per tile: a multiple of 16 up to 256
+    int kchunks, ptiles, qtiles, stages;      // ptiles: 256-token pair tiles, qtiles: weight tiles
     int div_mode, amax_is_amax;
     uint32_t flags;
 };
@@ -116,12 +119,14 @@ __global__ void __launch_bounds__(kT2Threads, 1) gemm_tc2_kernel(const __grid_co
     tc_fence_after_sync();
     const uint32_t tmem_base = warp_uniform(s.tmem_base);
     const volatile int* abort_flag = &s.abort_flag;
+    const int wrows = a.bn >> 1;                      // weight rows of a tile that this CTA loads
+    const uint32_t tx = 2 * (kT2TileBytes + (uint32_t)wrows * kT2Chunk);      // the four tiles of the pair
 
     auto tile_rows = [&](int t, int& mrow, int& nrow) {       // token tiles fastest: the pairs running together share weight tiles
         const int mat = (t >= per_mat) + (t >= 2 * per_mat);
         t -= mat * per_mat;
         mrow = (t % a.ptiles) * 256;
-        nrow = (t / a.ptiles) * kT2N;
+        nrow = (t / a.ptiles) * a.bn;
         return mat;
     };
 
@@ -137,8 +142,8 @@ __global__ void __launch_bounds__(kT2Threads, 1) gemm_tc2_kernel(const __grid_co
                 const int mat = tile_rows(t, mrow, nrow);
                 for (int kc = 0; kc < a.kchunks && npre < a.stages; ++kc, ++npre) {
                     if (!issuer) continue;
-                    if (rank == 0) mbar_expect_tx(&s.full[npre], 2 * kT2StageBytes);
-                    tma_load_2d_pair(ring + (size_t)npre * kT2StageBytes + kT2TileBytes, &maps.w[mat], kc * kT2Chunk, nrow + (int)rank * kT2Rows,
+                    if (rank == 0) mbar_expect_tx(&s.full[npre], tx);
+                    tma_load_2d_pair(ring + (size_t)npre * kT2StageBytes + kT2TileBytes, &maps.w[mat], kc * kT2Chunk, nrow + (int)rank * wrows,
                                      smem_u32(&s.full[npre]) & 0xFEFFFFFFu);
                 }
             }
@@ -158,8 +163,8 @@ __global__ void __launch_bounds__(kT2Threads, 1) gemm_tc2_kernel(const __grid_co
                     if (issuer) {
                         const uint32_t leader_bar = smem_u32(&s.full[st]) & 0xFEFFFFFFu;         // the barrier of the even CTA
                         if (refill) {
-                            if (rank == 0) mbar_expect_tx(&s.full[st], 2 * kT2StageBytes);      // the four tiles of the pair
-                            tma_load_2d_pair(dst + kT2TileBytes, &maps.w[mat], kc * kT2Chunk, nrow + (int)rank * kT2Rows, leader_bar);
+                            if (rank == 0) mbar_expect_tx(&s.full[st], tx);
+                            tma_load_2d_pair(dst + kT2TileBytes, &maps.w[mat], kc * kT2Chunk, nrow + (int)rank * wrows, leader_bar);
                         }
                         tma_load_2d_pair(dst, &maps.a[mat], kc * kT2Chunk, mrow + (int)rank * kT2Rows, leader_bar);
                     }
@@ -174,7 +179,7 @@ __global__ void __launch_bounds__(kT2Threads, 1) gemm_tc2_kernel(const __grid_co
         // ============================== MMA issuer (leader CTA only) ==============================
         if (rank == 0) {
             const bool issuer = elect_one();
-            const uint32_t idesc = umma_idesc(KIND, 256, kT2N), ring_addr = warp_uniform(smem_u32(ring));
+            const uint32_t idesc = umma_idesc(KIND, 256, a.bn), ring_addr = warp_uniform(smem_u32(ring));
             RingPos rp, fp;                                // ring stage, accumulator
             bool ok = true;
             for (int t = pair; t < total && ok; t += npairs, fp.next(2)) {
@@ -203,7 +208,7 @@ __global__ void __launch_bounds__(kT2Threads, 1) gemm_tc2_kernel(const __grid_co
         // ============================== epilogue (both CTAs, each its own 128 token rows) ==============================
         griddep_wait();
         const int q = warp & 3;                         // tensor-memory lane quarter this warp may read
-        const int half = (warp - 2) >> 2;               // its half of the tile's columns
+        const int c0 = warp < 6 ? 0 : ((a.bn + 31) >> 5) << 4, cols = warp < 6 ? ((a.bn + 31) >> 5) << 4 : a.bn - c0;     // its columns of the tile
         const int row_l = q * 32 + lane;
         const uint32_t leader_tempty[2] = {mapa_u32(smem_u32(&s.tempty[0]), 0), mapa_u32(smem_u32(&s.tempty[1]), 0)};
         RingPos fp;
@@ -231,7 +236,7 @@ __global__ void __launch_bounds__(kT2Threads, 1) gemm_tc2_kernel(const __grid_co
             if (!mbar_wait(&s.tfull[fp.i], fp.phase, abort_flag, a.wait_ns)) { t2_abort(s, a); break; }
             tc_fence_after_sync();
             float hmax = 0.f;
-            epi_tile<KIND>(e, tmem_base + (uint32_t)(fp.i * kT2N) + ((uint32_t)(q * 32) << 16) + half * (kT2N / 2), nrow + half * (kT2N / 2), kT2N / 2, hmax);
+            epi_tile<KIND>(e, tmem_base + (uint32_t)(fp.i * kT2N) + ((uint32_t)(q * 32) << 16) + c0, nrow + c0, cols, hmax);
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(leader_tempty[fp.i]);       // this accumulator may be overwritten
@@ -265,13 +270,32 @@ __global__ void __launch_bounds__(kT2Threads, 1) gemm_tc2_kernel(const __grid_co
 // ------------------------------------------------------------------------------------------------ host side
 static int t2_grid_pairs() { return std::max(1, sm_count() / 2); }
 
+// Weight rows per pair tile.  A tile of 256 leaves pairs idle wherever the tiles are not a multiple of the pairs: [4096, 4096] at 717
+// rows is 48 tiles for 74 pairs, [2560, 10240] at 2048 rows 80.  Any multiple of 16 is a legal tile, so the one with the least
+// estimated time is taken: a 128-byte step of K takes 0.094 us + 0.00073 a row, a launch 3.2 us + 0.009 a row and up to 1.6 where all
+// SMs store their results.  Measured, us, tiles of 256 / the tile taken: [4096, 4096] 717 rows 15.3 / 12.7 (176), [4096, 16384] 717 rows
+// 45.3 / 35.8, [2560, 10240] 1000 rows 29.3 / 19.5 (144), 2048 rows 49.6 / 35.5, [2560, 2560] 2048 rows 16.2 / 13.5, [16384, 4096] 717 rows 38.7 /
+// 35.8 (224).
+struct T2Tile { int bn; double us; };
+static T2Tile tc2_tile(int64_t M, int64_t N, int64_t K, int nmat) {
+    const char* bn_env = std::getenv("RWKVQ_TC2_BN");          // read per call: a test switches tiles in one process
+    const int forced = bn_env ? std::atoi(bn_env) : 0;
+    const int64_t pairs = t2_grid_pairs(), pt = nmat * ((M + 255) / 256);
+    const double kc = (double)((K + kT2Chunk - 1) / kT2Chunk);
+    T2Tile best{0, 0.};
+    for (int bn = kT2N; bn >= 128; bn -= 16) {
+        if (forced >= 128 && forced <= kT2N && forced % 16 == 0 && bn != forced) continue;
+        const int64_t waves = (pt * ((N + bn - 1) / bn) + pairs - 1) / pairs;
+        const double fill = std::min(1.0, (double)(pt * ((N + bn - 1) / bn)) / (double)pairs);
+        const double us = 3.15 + 0.009 * bn + 1.6 * fill + (double)waves * kc * (0.094 + 0.000731 * bn);
+        if (best.bn == 0 || us < best.us) best = {bn, us};
+    }
+    return best;
+}
 // RWKVQ_TC2=0 switches the pairs off, =force uses them wherever they are legal, RWKVQ_TC2_MIN_M raises their first row count (129: below it a pair tile is half empty).
-// Pairs or single CTAs?  Both run waves of tiles whose MMAs take as long (256 x 256 on a pair, 128 x 256 on a CTA), but a pair
-// loads 64 KB for a step of its tile, two single CTAs 96 KB, and an SM's intake from L2 bounds the single form.  Measured per
-// 128-byte step of K: 0.385 us on pairs, 0.41 / 0.30 / 0.24 us on single CTAs with 256 / 128 / 64 weight rows per tile (few
-// tiles); a pair launch costs 0.9 us more (cluster set-up, one more barrier).  Measured, us, single / pairs: FP8 [16384, 4096]
-// 384 rows 32.8 / 29.8, 2048 rows 109.3 / 98.8; [4096, 16384] 717 rows 51.7 / 48.5; [4096, 4096] 1024 rows 16.6 / 17.0; [2560, 2560]
-// 1500 rows 12.8 / 13.5, 2048 rows 20.8 / 19.1.  INT8 [16384, 4096] 2048 rows 100.7 / 89.9.
+// Pairs or single CTAs?  The estimate above against that of the single form: 3.3 / 4.0 / 3.5 us and 0.37 / 0.22 / 0.19 a step with 256 / 128 /
+// 64 weight rows per tile.  Measured, us, single / pairs: FP8 [16384, 4096] 384 rows 27.4 / 24.5, 2048 rows 100.3 / 91.4; [4096, 16384] 717 rows 48.6 /
+// 38.6; [4096, 4096] 1000 rows 15.6 / 16.3; [8192, 2048] 384 rows 10.2 / 11.3, 2048 rows 28.3 / 25.3; [2560, 2560] 1500 rows 11.5 / 11.9.
 bool tc2_eligible(int kind, int64_t M, int64_t N, int64_t K, int nmat, int single_nb) {
     static const int64_t min_m = [] {
         const char* off = std::getenv("RWKVQ_TC2");
@@ -283,10 +307,10 @@ bool tc2_eligible(int kind, int64_t M, int64_t N, int64_t K, int nmat, int singl
     if (M < min_m || N < kT2N || K % 16 || (kind != KIND_F8 && kind != KIND_I8)) return false;
     static const bool force = std::getenv("RWKVQ_TC2") && std::getenv("RWKVQ_TC2")[0] == 'f';
     if (force) return true;
-    const int64_t pairs = t2_grid_pairs(), tiles = nmat * ((M + 255) / 256) * ((N + kT2N - 1) / kT2N);
+    const int64_t pairs = t2_grid_pairs();
     const int64_t single = nmat * ((M + 127) / 128) * ((N + single_nb - 1) / single_nb);
-    const double kc = (double)((K + kT2Chunk - 1) / kT2Chunk), step1 = single_nb > 128 ? 0.41 : (single_nb > 64 ? 0.30 : 0.24);
-    const double t2 = (double)((tiles + pairs - 1) / pairs) * kc * 0.385 + 0.9, t1 = (double)((single + 2 * pairs - 1) / (2 * pairs)) * kc * step1;
+    const double kc = (double)((K + kT2Chunk - 1) / kT2Chunk), step1 = single_nb > 128 ? 0.369 : (single_nb > 64 ? 0.218 : 0.193);
+    const double t2 = tc2_tile(M, N, K, nmat).us, t1 = (single_nb > 128 ? 3.3 : (single_nb > 64 ? 4.0 : 3.5)) + (double)((single + 2 * pairs - 1) / (2 * pairs)) * kc * step1;
     return t2 <= t1;
 }
 
@@ -296,8 +320,9 @@ int32_t run_tc2(const Tc2Call& c, int* status, cudaStream_t st, const char* who)
     a.ffn_amax = c.ffn_amax; a.status = status; a.wait_ns = wait_limit_ns();
     a.ldo = c.ldo; a.ldacc = c.ldacc; a.M = c.M; a.N = c.N; a.K = c.K; a.nmat = c.nmat; a.div_mode = c.div_mode; a.amax_is_amax = c.amax_is_amax; a.flags = c.flags;
     a.kchunks = (c.K + kT2Chunk - 1) / kT2Chunk;
+    a.bn = tc2_tile(c.M, c.N, c.K, c.nmat).bn;
     a.ptiles = (c.M + 255) / 256;
-    a.qtiles = (c.N + kT2N - 1) / kT2N;
+    a.qtiles = (c.N + a.bn - 1) / a.bn;
     a.stages = kT2MaxStages;
     const size_t smem = (size_t)a.stages * kT2StageBytes + 1024;
     Tc2Maps maps;
@@ -306,7 +331,7 @@ int32_t run_tc2(const Tc2Call& c, int* status, cudaStream_t st, const char* who)
         a.a_scale[i] = c.a_scale[i]; a.ws[i] = c.ws[i]; a.out[i] = c.out[i]; a.acc[i] = c.acc[i];
         rc = make_map(&maps.a[i], c.codes[i], c.M, c.K, c.lda, kT2Rows, who);
         if (rc) return rc;
-        rc = make_map(&maps.w[i], c.w[i], c.N, c.K, c.ldw, kT2Rows, who);
+        rc = make_map(&maps.w[i], c.w[i], c.N, c.K, c.ldw, a.bn / 2, who);
         if (rc) return rc;
     }
     const void* kern = kind == KIND_F8 ? (const void*)gemm_tc2_kernel<KIND_F8> : (const void*)gemm_tc2_kernel<KIND_I8>;

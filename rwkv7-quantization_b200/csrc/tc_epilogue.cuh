@@ -74,17 +74,18 @@ __device__ __forceinline__ void epi_store16(const EpiRow& e, const uint32_t (&r)
     }
 }
 
-// `cols` accumulator columns (a multiple of 32) at taddr, result columns from n0 on
+// `cols` accumulator columns (a multiple of 16) at taddr, result columns from n0 on
 template <int KIND, int EPI>
 __device__ __forceinline__ void epi_cols(const EpiRow& e, uint32_t taddr, int n0, int cols, float& hmax) {
 #pragma unroll 1
     for (int c0 = 0; c0 < cols; c0 += 32) {
         uint32_t r0[16], r1[16];
+        const bool two = c0 + 16 < cols;
         tc::tmem_ld16(taddr + c0, r0);
-        tc::tmem_ld16(taddr + c0 + 16, r1);
+        if (two) tc::tmem_ld16(taddr + c0 + 16, r1);
         tc::tmem_ld_wait();
         epi_store16<KIND, EPI>(e, r0, n0 + c0, hmax);
-        epi_store16<KIND, EPI>(e, r1, n0 + c0 + 16, hmax);
+        if (two) epi_store16<KIND, EPI>(e, r1, n0 + c0 + 16, hmax);
     }
 }
 

@@ -131,3 +131,24 @@ def test_results_in_a_column_range(m, n, k, offset):
             f.linear_quantized_fused(x, info)
         assert torch.equal(wide[:, offset:offset + n], want)
         assert bool((wide[:, :offset] == 7).all()) and bool((wide[:, offset + n:] == 7).all())
+
+
+def tile_widths():
+    """Every width of a pair's tile against the widest: halves of an odd number of 16-column pieces, columns past the last tile."""
+    import rwkvq_abi as abi
+    global SIZES
+    sizes = [(129, 1000, 400), (300, 4104, 1040), (517, 2560, 768)]
+    for SIZES in ([s] for s in sizes):
+        want = None
+        for bn in range(256, 127, -16):
+            os.environ["RWKVQ_TC2_BN"] = str(bn)
+            got = results()
+            want = got if want is None else want
+            assert all(torch.equal(a, b) for a, b in zip(got, want)), (SIZES, bn)
+    assert abi.device_status() == 0
+
+
+def test_pair_tiles_of_every_width():
+    code = f"import sys; sys.path[:0] = [{os.path.join(ROOT, 'rwkv7-quantization_b200')!r}, {os.path.join(ROOT, 'tests')!r}]\n" \
+           "import test_tiled_gemm_gpu as t; t.tile_widths()"
+    subprocess.run([sys.executable, "-c", code], check=True, env=dict(os.environ, RWKVQ_TC2="force"), timeout=300)
