@@ -80,6 +80,29 @@ int32_t rwkvq_linear(const rwkvq_linear_desc* d) {
                                               d->out[1], d->out[2], d->ldo, M, N, K, d->gemm_flags, d->workspace, d->workspace_bytes, d->stream);
 }
 
+int64_t rwkvq_linear_nvfp4_scratch_bytes(int64_t M, int64_t K) {
+    if (M < 0 || K < 0 || K % 64) return 0;
+    return up256(M * (K / 2)) + up256(rwkvq_nvfp4_blocked_scale_bytes(M, K)) + 256;
+}
+
+int32_t rwkvq_linear_nvfp4(const rwkvq_nvfp4_desc* d) {
+    const char* who = "linear_nvfp4";
+    RWKVQ_REQUIRE(d != nullptr, RWKVQ_E_BADARG, "%s: null descriptor", who);
+    const int64_t M = d->M, N = d->N, K = d->K;
+    RWKVQ_REQUIRE(M > 0 && N >= 0 && K > 0 && K % 256 == 0 && M < (int64_t(1) << 30) && K < (int64_t(1) << 30), RWKVQ_E_SHAPE, "%s: M=%lld K=%lld", who,
+                  (long long)M, (long long)K);
+    RWKVQ_REQUIRE(d->scratch && ((uintptr_t)d->scratch & 255) == 0 && d->scratch_bytes >= rwkvq_linear_nvfp4_scratch_bytes(M, K), RWKVQ_E_WORKSPACE,
+                  "%s: %lld bytes of 256-byte aligned scratch needed", who, (long long)rwkvq_linear_nvfp4_scratch_bytes(M, K));
+    uint8_t* codes = reinterpret_cast<uint8_t*>(d->scratch);
+    uint8_t* scales = codes + up256(M * (K / 2));
+    float* pts = reinterpret_cast<float*>(scales + up256(rwkvq_nvfp4_blocked_scale_bytes(M, K)));
+    const int32_t rc = rwkvq_actq_nvfp4_fused(d->x, (int32_t)d->x_dtype, M, K, d->ldx, codes, K / 2, nullptr, K / 16, scales, pts, d->actq_scratch,
+                                              d->actq_scratch_bytes, nullptr, d->stream);
+    if (rc != RWKVQ_OK) return rc;
+    return rwkvq_tc_gemm_nvfp4(codes, K / 2, scales, pts, d->w, d->ldw, d->w_scales_blocked, d->w_tscale, d->out, d->ldo, M, N, K, d->workspace,
+                               d->workspace_bytes, d->stream);
+}
+
 int64_t rwkvq_ffn_scratch_bytes(int32_t kind, int64_t M, int64_t K, int64_t F) {
     if (M < 0 || K < 0 || F < 0 || (kind != RWKVQ_LINEAR_FP8 && kind != RWKVQ_LINEAR_INT8)) return 0;
     return up256(M * K) + up256(M * F) + (kind == RWKVQ_LINEAR_FP8 ? 256 : 2 * up256(4 * M));

@@ -63,7 +63,7 @@ def _groupwise_tc(x, packed, scales, zeros):
     n, k = packed.shape[0], packed.shape[1] * 2
     if packed.stride(1) != 1 or packed.stride(0) % 16 or (packed.data_ptr() | scales.data_ptr() | (0 if zeros is None else zeros.data_ptr())) % 16:
         return None
-    x2 = x.reshape(-1, k)
+    x2 = x if x.dim() == 2 else x.reshape(-1, k)
     if x2.dtype not in (torch.float16, torch.bfloat16):
         x2 = x2.to(torch.float16)
     x2 = x2.contiguous()
@@ -74,7 +74,7 @@ def _groupwise_tc(x, packed, scales, zeros):
         raise RuntimeError("rwkvq: INT4 / INT8 projections run on the GPU only (no CPU fallback)")
     m, dev = x2.shape[0], x2.device
     out = torch.empty((m, n), dtype=torch.float16, device=dev)
-    ws = torch.empty(int(abi.lib().rwkvq_tc_gemm_wa16_workspace_bytes(m, n, k, 4)), dtype=torch.uint8, device=dev)
+    ws = torch.empty(abi.wa16_workspace_bytes(m, n, k, 4), dtype=torch.uint8, device=dev)
     abi.call("rwkvq_tc_gemm_int4_group", x2.data_ptr(), abi.dtype_code(x2), k, packed.data_ptr(), packed.stride(0), scales.data_ptr(),
              abi.ptr(zeros), out.data_ptr(), n, m, n, k, ws.data_ptr(), ws.numel(), abi.stream_ptr())
     abi.after_call()

@@ -46,13 +46,17 @@ def _takes_tc(m: int, n: int, k: int) -> bool:
     return not fits
 
 
+def _shaped(out, x, n: int, out_dtype):
+    return out if x.dim() == 2 and out.dtype is out_dtype else out.to(out_dtype).reshape(*x.shape[:-1], n)
+
+
 def _tensor_core(x2, w, scale):
     abi.require_device()
     if not x2.is_cuda:
         raise RuntimeError("rwkvq: INT4 / INT8 projections run on the GPU only (no CPU fallback)")
     (m, k), n, dev = x2.shape, w.shape[0], x2.device
     out = torch.empty((m, n), dtype=torch.float16, device=dev)
-    ws = torch.empty(int(abi.lib().rwkvq_tc_gemm_wa16_workspace_bytes(m, n, k, 8)), dtype=torch.uint8, device=dev)
+    ws = torch.empty(abi.wa16_workspace_bytes(m, n, k, 8), dtype=torch.uint8, device=dev)
     abi.call("rwkvq_tc_gemm_int8_w8a16", x2.data_ptr(), k, w.data_ptr(), w.stride(0), scale.data_ptr(), out.data_ptr(), n, m, n, k,
              ws.data_ptr(), ws.numel(), abi.stream_ptr())
     abi.after_call()
@@ -69,11 +73,11 @@ def linear_int8_per_tensor(x, weight_info, out_dtype=torch.float16):
     if w is not w0 or scale.data_ptr() != s0.data_ptr():         # copies made just now: in front of the projection
         abi.order_copies((w, w0), (scale, s0))
     if w.data_ptr() % 16 == 0 and _takes_tc(x2.shape[0], n, k):
-        return _tensor_core(x2, w, scale).to(out_dtype).reshape(*x.shape[:-1], n)
+        return _shaped(_tensor_core(x2, w, scale), x, n, out_dtype)
     out = _run_rows(x2, n, lambda xc, oc, m: abi.call(
         "rwkvq_gemv_int8_w8a16", xc.data_ptr(), k, w.data_ptr(), w.stride(0), scale.data_ptr(), oc.data_ptr(), n, m, n, k,
         abi.stream_ptr()))
-    return out.to(out_dtype).reshape(*x.shape[:-1], n)
+    return _shaped(out, x, n, out_dtype)
 
 
 def linear_int8_affine(x, weight_info, out_dtype=torch.float16):

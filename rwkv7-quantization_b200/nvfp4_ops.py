@@ -182,6 +182,19 @@ def linear_nvfp4(x, weight_info, out_dtype=torch.float16, push=None):
                  wts.data_ptr(), out.data_ptr(), out.stride(0), m, n, k, abi.stream_ptr())
         out = out.reshape(*x.shape[:-1], n)
         return out if out_dtype in (None, out.dtype) else out.to(out_dtype)
+    if route == "tc" and push is None and m > 0 and os.environ.get("RWKVQ_NVFP4_ACTQ", "fused") == "fused":
+        # quantizer and GEMM in one call with one scratch buffer
+        dev = x2.device
+        w_blk = _blocked_weight_scales(weight_info, k)
+        need = abi.linear_nvfp4_scratch_bytes(m, k)
+        scratch = torch.empty(need, dtype=torch.uint8, device=dev)
+        out = abi.new_out(m, n, dev)
+        sc, ws = abi.actq_scratch(dev), abi.workspace(1, 1, 1, 1, dev)
+        abi.call("rwkvq_linear_nvfp4", abi.NVFP4_DESC.pack(
+            x2.data_ptr(), w.data_ptr(), w_blk.data_ptr(), wts.data_ptr(), out.data_ptr(), k, w.stride(0), out.stride(0), m, n, k, abi.dtype_code(x2),
+            scratch.data_ptr(), need, sc.data_ptr(), sc.numel() * 4, ws.data_ptr(), ws.numel(), abi.stream_ptr()))
+        out = out if x.dim() == 2 else out.reshape(*x.shape[:-1], n)
+        return out if out_dtype in (None, out.dtype) else out.to(out_dtype)
     codes, bs, pts = quantize_activations_nvfp4(x, blocked=(route == "tc"))
     out = abi.new_out(m, n, codes.device)
     if route == "tc":

@@ -108,6 +108,8 @@ SIGNATURES = {
     "rwkvq_prep_x_int8_relu2": [_p, _i64, _i64, _i64, _p, _i64, _p, _i32, _p],
     "rwkvq_linear_scratch_bytes": [_i32, _i32, _i64, _i64],
     "rwkvq_linear": [_p],
+    "rwkvq_linear_nvfp4_scratch_bytes": [_i64, _i64],
+    "rwkvq_linear_nvfp4": [_p],
     "rwkvq_ffn_scratch_bytes": [_i32, _i64, _i64, _i64],
     "rwkvq_ffn_relu2": [_p],
     "rwkvq_gemv_batch": [_p, _i32, _p],
@@ -137,7 +139,7 @@ SIGNATURES = {
     "rwkvq_gemv_set_trace": [_p],
     "rwkvq_tc_set_trace": [_p],
 }
-_RESTYPES = {"rwkvq_linear_scratch_bytes": ctypes.c_int64, "rwkvq_ffn_scratch_bytes": ctypes.c_int64, "rwkvq_tc_gemm_wa16_workspace_bytes": ctypes.c_int64, "rwkvq_actq_nvfp4_fused_scratch_bytes": ctypes.c_int64, "rwkvq_gemv_nvfp4_fused_smem_bytes": ctypes.c_int64, "rwkvq_nvfp4_blocked_scale_bytes": ctypes.c_int64, "rwkvq_actq_fp8_fused_scratch_bytes": ctypes.c_int64, "rwkvq_gemv_nvfp4_smem_bytes": ctypes.c_int64, "rwkvq_gemv_int4_group_smem_bytes": ctypes.c_int64, "rwkvq_workspace_bytes": ctypes.c_int64, "rwkvq_last_error_string": ctypes.c_char_p, "rwkvq_launch_count": ctypes.c_int64,
+_RESTYPES = {"rwkvq_linear_scratch_bytes": ctypes.c_int64, "rwkvq_linear_nvfp4_scratch_bytes": ctypes.c_int64, "rwkvq_ffn_scratch_bytes": ctypes.c_int64, "rwkvq_tc_gemm_wa16_workspace_bytes": ctypes.c_int64, "rwkvq_actq_nvfp4_fused_scratch_bytes": ctypes.c_int64, "rwkvq_gemv_nvfp4_fused_smem_bytes": ctypes.c_int64, "rwkvq_nvfp4_blocked_scale_bytes": ctypes.c_int64, "rwkvq_actq_fp8_fused_scratch_bytes": ctypes.c_int64, "rwkvq_gemv_nvfp4_smem_bytes": ctypes.c_int64, "rwkvq_gemv_int4_group_smem_bytes": ctypes.c_int64, "rwkvq_workspace_bytes": ctypes.c_int64, "rwkvq_last_error_string": ctypes.c_char_p, "rwkvq_launch_count": ctypes.c_int64,
              "rwkvq_set_wait_limit_us": None, "rwkvq_gemv_set_trace": None, "rwkvq_tc_set_trace": None}
 
 
@@ -159,6 +161,9 @@ LINEAR_DESC = struct.Struct("@12Q6q6i2I2iQqQqQqQ")
 FFN_DESC = struct.Struct("@7Q8q4i3IiQqQqQqQQ")
 
 
+NVFP4_DESC = struct.Struct("@5Q7qQqQqQqQ")
+
+
 def up256(n: int) -> int:
     return (n + 255) & ~255
 
@@ -166,6 +171,11 @@ def up256(n: int) -> int:
 def linear_scratch_bytes(kind: int, nmat: int, m: int, k: int) -> int:
     """rwkvq_linear_scratch_bytes without the boundary crossing (a test holds the two together)."""
     return nmat * up256(m * k) + 256 if kind == LINEAR_FP8 else nmat * (up256(m * k) + up256(4 * m))
+
+
+def linear_nvfp4_scratch_bytes(m: int, k: int) -> int:
+    """rwkvq_linear_nvfp4_scratch_bytes likewise (K a multiple of 64)."""
+    return up256(m * (k // 2)) + (m + 255) // 256 * 16 * k + 256
 
 
 def ffn_scratch_bytes(kind: int, m: int, k: int, f: int) -> int:
@@ -389,6 +399,19 @@ def workspace(m: int, n: int, k: int, nmat: int, device) -> torch.Tensor:
     if ws is None or ws.numel() < need:
         ws = replace_kept(_workspaces, key, need, 1 << 20, torch.zeros, dtype=torch.uint8, device=device)
     return ws
+
+
+_wa16_need: dict = {}
+
+
+def wa16_workspace_bytes(m: int, n: int, k: int, bits: int) -> int:
+    """rwkvq_tc_gemm_wa16_workspace_bytes, asked once per shape (it estimates every form)."""
+    need = _wa16_need.get((m, n, k, bits))
+    if need is None:
+        if len(_wa16_need) >= 4096:
+            _wa16_need.clear()
+        need = _wa16_need[(m, n, k, bits)] = int(lib().rwkvq_tc_gemm_wa16_workspace_bytes(m, n, k, bits))
+    return need
 
 
 _plain: dict = {}

@@ -186,3 +186,7 @@ def test_scratch_sizes_agree_with_the_library():
                 for nmat in (1, 3):
                     assert abi.linear_scratch_bytes(kind, nmat, m, k) == abi.lib().rwkvq_linear_scratch_bytes(kind, nmat, m, k)
                 assert abi.ffn_scratch_bytes(kind, m, k, 4 * k) == abi.lib().rwkvq_ffn_scratch_bytes(kind, m, k, 4 * k)
+    for m in (1, 9, 255, 256, 257, 2048):
+        for k in (256, 768, 2560, 16384):
+            assert abi.linear_nvfp4_scratch_bytes(m, k) == abi.lib().rwkvq_linear_nvfp4_scratch_bytes(m, k)
+    assert abi.lib().rwkvq_linear_nvfp4_scratch_bytes(4, 100) == 0
