@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(kT2Threads, 1) gemm_tc2_kernel(const __grid_co
             if (!mbar_wait(&s.tfull[fp.i], fp.phase, abort_flag, a.wait_ns)) { t2_abort(s, a); break; }
             tc_fence_after_sync();
             float hmax = 0.f;
-            epi_tile<KIND>(e, tmem_base + (uint32_t)(fp.i * kT2N) + ((uint32_t)(q * 32) << 16) + c0, nrow + c0, cols, hmax);
+            epi_tile<KIND, true>(e, tmem_base + (uint32_t)(fp.i * kT2N) + ((uint32_t)(q * 32) << 16) + c0, nrow + c0, cols, hmax);
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(leader_tempty[fp.i]);       // this accumulator may be overwritten

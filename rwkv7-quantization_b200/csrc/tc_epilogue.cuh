@@ -74,13 +74,13 @@ __device__ __forceinline__ void epi_store16(const EpiRow& e, const uint32_t (&r)
     }
 }
 
-// `cols` accumulator columns (a multiple of 16) at taddr, result columns from n0 on
-template <int KIND, int EPI>
+// `cols` accumulator columns (a multiple of 32, with ODD of 16) at taddr, result columns from n0 on
+template <int KIND, int EPI, bool ODD>
 __device__ __forceinline__ void epi_cols(const EpiRow& e, uint32_t taddr, int n0, int cols, float& hmax) {
 #pragma unroll 1
     for (int c0 = 0; c0 < cols; c0 += 32) {
         uint32_t r0[16], r1[16];
-        const bool two = c0 + 16 < cols;
+        const bool two = !ODD || c0 + 16 < cols;
         tc::tmem_ld16(taddr + c0, r0);
         if (two) tc::tmem_ld16(taddr + c0 + 16, r1);
         tc::tmem_ld_wait();
@@ -89,15 +89,15 @@ __device__ __forceinline__ void epi_cols(const EpiRow& e, uint32_t taddr, int n0
     }
 }
 
-template <int KIND>
+template <int KIND, bool ODD = false>
 __device__ __forceinline__ void epi_tile(const EpiRow& e, uint32_t taddr, int n0, int cols, float& hmax) {
     const bool any = (e.flags & RWKVQ_FLAG_WSCALE_PER_ROW) || (KIND == tc::KIND_I8 && e.acc);
     const bool via = (e.flags & RWKVQ_FLAG_OUT_VIA_BF16) != 0, relu2 = (e.flags & RWKVQ_FLAG_RELU2) != 0;
-    if (any) epi_cols<KIND, EPI_ANY>(e, taddr, n0, cols, hmax);
-    else if (relu2 && via) epi_cols<KIND, EPI_RELU2_BF16>(e, taddr, n0, cols, hmax);
-    else if (relu2) epi_cols<KIND, EPI_RELU2>(e, taddr, n0, cols, hmax);
-    else if (via) epi_cols<KIND, EPI_BF16>(e, taddr, n0, cols, hmax);
-    else epi_cols<KIND, EPI_PLAIN>(e, taddr, n0, cols, hmax);
+    if (any) epi_cols<KIND, EPI_ANY, ODD>(e, taddr, n0, cols, hmax);
+    else if (relu2 && via) epi_cols<KIND, EPI_RELU2_BF16, ODD>(e, taddr, n0, cols, hmax);
+    else if (relu2) epi_cols<KIND, EPI_RELU2, ODD>(e, taddr, n0, cols, hmax);
+    else if (via) epi_cols<KIND, EPI_BF16, ODD>(e, taddr, n0, cols, hmax);
+    else epi_cols<KIND, EPI_PLAIN, ODD>(e, taddr, n0, cols, hmax);
 }
 
 }  // namespace rwkvq

@@ -55,11 +55,18 @@ CODES_MK_MIN = 49152       # ... and already from 3 rows when the block is this 
 # r/k/v 16 rows 15.2 / 15.6, 20 rows 21.0 / 16.2 (from 17 rows the GEMV works on three token tiles); INT8 16 rows 7.5 / 7.4,
 # 20 rows 9.4 / 7.7.  Against a long K, where the code tile crowds the GEMV's ring, from fewer: [4096, 16384] FP8 9 rows 19.9 / 18.5,
 # [2560, 10240] FP8 9 rows 11.6 / 10.7, 12 rows 12.7 / 10.8; INT8 [4096, 16384] 9 rows 17.6 / 16.7, 12 rows 25.7 / 17.5, [2560, 10240]
-# 9 rows 9.9 / 9.9, 12 rows 11.1 / 9.9.  Matrices with many row tiles stay on the GEMV up to 32 rows; the line was drawn on an older
-# tiled form, which is ahead from 17 rows now ([10240, 2560] FP8 17 rows 14.5 / 11.1, 32 rows 15.1 / 11.4).
+# 9 rows 9.9 / 9.9, 12 rows 11.1 / 9.9.  Matrices of MANY_ROWS_N weight rows and more, which the cluster kernel does not take, go to the
+# tiled form from as many tokens: GEMV / tiled, 17 and 32 rows: [10240, 2560] FP8 14.2 / 10.9 and 15.2 / 11.1, INT8 10.4 / 10.0 and 11.8 / 10.0;
+# [16384, 4096] FP8 20.8 / 16.7 and 22.0 / 16.9, INT8 16.1 / 15.9 and 18.3 / 16.2; [14336, 3584] FP8 18.6 / 14.3, INT8 14.0 / 13.3; [12288, 3072] FP8
+# 16.5 / 12.5, INT8 12.4 / 11.5 (16 rows, on the stream-K form: FP8 [16384, 4096] 15.9 / 23.5).  In a chain the GEMV overlaps more with its
+# neighbours: whole layers at 24 rows, FP8 of width 2560 / 3072 / 4096 102.3 -> 99.7, 113.4 -> 109.2, 143.0 -> 143.5 (32 rows 155.0 -> 151.8), INT8 80.4
+# -> 76.8, 92.4 -> 88.0, 121.6 -> 135.6: INT8 of K = 4096 stays.  Other K were not measured.
 CLUSTER_FROM_M = int(os.environ.get("RWKVQ_CLUSTER_FROM_M", "17"))
 CLUSTER_LONG_K = 10240
 CLUSTER_LONG_K_FROM_M = 9
+MANY_ROWS_N = 10240
+MANY_ROWS_K = (2560, 4096)
+MANY_ROWS_K_INT8 = 3072
 # Against a short K (a few steps per tile) the tiled tensor-core GEMM takes over.  FP8: from CLUSTER_FROM_M rows at K = 1024 to
 # TILED_SHORT_K, square matrices at K = 1024 only.  Measured with the quantizer, us, GEMV / tiled, 17 and 32 rows: [1024, 1024] 6.9 / 6.7
 # and 7.8 / 6.9, r/k/v 9.6 / 7.3 and 10.3 / 7.4; [4096, 1024] 6.9 / 6.8 and 7.7 / 7.0; [5120, 1280] 8.2 / 7.5 and 9.1 / 7.5; [1280, 1280] 6.8 / 7.3
@@ -84,6 +91,8 @@ def _takes_tc(m: int, k: int, n=None, int8: bool = False) -> bool:
     first = CLUSTER_FROM_M if k < CLUSTER_LONG_K else min(CLUSTER_FROM_M, CLUSTER_LONG_K_FROM_M)
     if n is None or m < max(first, 9) or m > GEMV_M_MAX or ROUTE != "auto" or k % 16 or not _ACTQ_FUSED:
         return False
+    if n >= MANY_ROWS_N and m >= 17 and MANY_ROWS_K[0] <= k <= (MANY_ROWS_K_INT8 if int8 else MANY_ROWS_K[1]):
+        return True
     if int8 and k < 2048:
         return n >= TILED_WIDE_N and (k <= 1024 or m >= TILED_ROWS)
     if 1024 <= k <= (1024 if n == k else TILED_SHORT_K) and n >= TILED_MIN_N:

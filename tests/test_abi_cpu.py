@@ -176,6 +176,9 @@ def test_rows_that_leave_the_decode_kernel_against_a_short_k():
     first = lambda n, k, int8: next((m for m in range(9, 33) if f._takes_tc(m, k, n, int8)), None)  # noqa: E731
     assert [first(n, k, True) for n, k in ((4096, 1024), (6144, 1536), (7168, 1792), (1024, 1024), (1792, 1792))] == [17, 28, 28, None, None]
     assert [first(n, k, False) for n, k in ((1024, 1024), (4096, 1024), (5120, 1280), (1280, 1280), (1024, 512), (512, 1024))] == [17, 17, 17, None, None, None]
+    # many weight rows: from 17 tokens where K was measured
+    many = ((10240, 2560), (12288, 3072), (16384, 4096))
+    assert [first(n, k, False) for n, k in many] == [17, 17, 17] and [first(n, k, True) for n, k in many] == [17, 17, None]
 
 
 def test_scratch_sizes_agree_with_the_library():
