@@ -277,8 +277,12 @@ static int t2_grid_pairs() { return std::max(1, sm_count() / 2); }
 // 45.3 / 35.8, [2560, 10240] 1000 rows 29.3 / 19.5 (144), 2048 rows 49.6 / 35.5, [2560, 2560] 2048 rows 16.2 / 13.5, [16384, 4096] 717 rows 38.7 /
 // 35.8 (224).
 struct T2Tile { int bn; double us; };
+static bool t2_forced() {
+    static const bool force = std::getenv("RWKVQ_TC2") && std::getenv("RWKVQ_TC2")[0] == 'f';
+    return force;
+}
 static T2Tile tc2_tile(int64_t M, int64_t N, int64_t K, int nmat) {
-    const char* bn_env = std::getenv("RWKVQ_TC2_BN");          // read per call: a test switches tiles in one process
+    const char* bn_env = t2_forced() ? std::getenv("RWKVQ_TC2_BN") : nullptr;      // read per call: a test switches tiles in one process
     const int forced = bn_env ? std::atoi(bn_env) : 0;
     const int64_t pairs = t2_grid_pairs(), pt = nmat * ((M + 255) / 256);
     const double kc = (double)((K + kT2Chunk - 1) / kT2Chunk);
@@ -305,8 +309,7 @@ bool tc2_eligible(int kind, int64_t M, int64_t N, int64_t K, int nmat, int singl
         return (int64_t)std::max<long long>(v, 129);
     }();
     if (M < min_m || N < kT2N || K % 16 || (kind != KIND_F8 && kind != KIND_I8)) return false;
-    static const bool force = std::getenv("RWKVQ_TC2") && std::getenv("RWKVQ_TC2")[0] == 'f';
-    if (force) return true;
+    if (t2_forced()) return true;
     const int64_t pairs = t2_grid_pairs();
     const int64_t single = nmat * ((M + 127) / 128) * ((N + single_nb - 1) / single_nb);
     const double kc = (double)((K + kT2Chunk - 1) / kT2Chunk), step1 = single_nb > 128 ? 0.369 : (single_nb > 64 ? 0.218 : 0.193);
