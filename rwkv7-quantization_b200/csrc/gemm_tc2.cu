@@ -285,13 +285,13 @@ static T2Tile tc2_tile(int64_t M, int64_t N, int64_t K, int nmat) {
     const char* bn_env = t2_forced() ? std::getenv("RWKVQ_TC2_BN") : nullptr;      // read per call: a test switches tiles in one process
     const int forced = bn_env ? std::atoi(bn_env) : 0;
     const int64_t pairs = t2_grid_pairs(), pt = nmat * ((M + 255) / 256);
-    const double kc = (double)((K + kT2Chunk - 1) / kT2Chunk);
+    const double kc = (double)((K + kT2Chunk - 1) / kT2Chunk), inv_pairs = 1.0 / (double)pairs;
     T2Tile best{0, 0.};
-    for (int bn = kT2N; bn >= 128; bn -= 16) {
+    for (int bn = kT2N; bn >= 128; bn -= 16) {                 // on the path of every call: one short division a width where all tiles run at once
         if (forced >= 128 && forced <= kT2N && forced % 16 == 0 && bn != forced) continue;
-        const int64_t waves = (pt * ((N + bn - 1) / bn) + pairs - 1) / pairs;
-        const double fill = std::min(1.0, (double)(pt * ((N + bn - 1) / bn)) / (double)pairs);
-        const double us = 3.15 + 0.009 * bn + 1.6 * fill + (double)waves * kc * (0.094 + 0.000731 * bn);
+        const int64_t tiles = pt * (int64_t)(((uint32_t)N + (uint32_t)bn - 1) / (uint32_t)bn);      // N < 2^30
+        const int64_t waves = tiles <= pairs ? 1 : (tiles + pairs - 1) / pairs;
+        const double us = 3.15 + 0.009 * bn + 1.6 * std::min(1.0, (double)tiles * inv_pairs) + (double)waves * kc * (0.094 + 0.000731 * bn);
         if (best.bn == 0 || us < best.us) best = {bn, us};
     }
     return best;
