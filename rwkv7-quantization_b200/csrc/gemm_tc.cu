@@ -1005,6 +1005,11 @@ int32_t rwkvq_tc_gemm_form(int32_t kind, int32_t nmat, int64_t M, int64_t N, int
     return tc_form(kind == RWKVQ_LINEAR_FP8 ? KIND_F8 : KIND_I8, M, N, K, flags, nmat);
 }
 
+int32_t rwkvq_tc_gemm_pair_width(int32_t kind, int32_t nmat, int64_t M, int64_t N, int64_t K) {
+    if ((kind != RWKVQ_LINEAR_FP8 && kind != RWKVQ_LINEAR_INT8) || nmat < 1 || nmat > 3 || M <= 0 || N <= 0 || K <= 0 || K % 16) return RWKVQ_E_BADARG;
+    return tc2_width(kind == RWKVQ_LINEAR_FP8 ? KIND_F8 : KIND_I8, M, N, K, nmat);
+}
+
 /* rwkvq_tc_gemm_fp8 fused with the all-gather of a column-split projection: see rwkvq_tc_gemm_nvfp4_push for
  * peer_out / peer_flag / epoch.  Only shapes for which rwkvq_tc_gemm_can_push() is 1; no RELU2 flag. */
 int32_t rwkvq_tc_gemm_fp8_push(const uint8_t* a_codes, int64_t lda, const float* amax, int32_t amax_is_amax, const uint8_t* w,

@@ -32,7 +32,7 @@ constexpr int kT2Chunk = 128;                 // bytes of K per stage
 constexpr int kT2Rows = 128;                  // rows of each operand tile per CTA
 constexpr uint32_t kT2TileBytes = kT2Rows * kT2Chunk;      // 16 KB
 constexpr uint32_t kT2StageBytes = 2 * kT2TileBytes;       // tokens + this CTA's half of the weight tile
-constexpr int kT2N = 256;                     // most weight rows per pair tile (UMMA N)
+constexpr int kT2N = 256;                     // most weight rows per pair tile (the instruction's N)
 
 struct Tc2Maps {
     CUtensorMap a[3];   // activation codes [M, K], box 128 rows x 128 bytes
@@ -49,7 +49,7 @@ struct Tc2Args {
     unsigned long long wait_ns;
     int64_t ldo, ldacc;
     int M, N, K, nmat;
-    int bn;                                   // weight rows per tile: a multiple of 16 up to 256
+    int bn;                                   // weight rows per tile: a multiple of 16 (FP8) or 32 (INT8) from 128 to 256
     int kchunks, ptiles, qtiles, stages;      // ptiles: 256-token pair tiles, qtiles: weight tiles
     int div_mode, amax_is_amax;
     uint32_t flags;
@@ -271,8 +271,9 @@ __global__ void __launch_bounds__(kT2Threads, 1) gemm_tc2_kernel(const __grid_co
 static int t2_grid_pairs() { return std::max(1, sm_count() / 2); }
 
 // Weight rows per pair tile.  A tile of 256 leaves pairs idle wherever the tiles are not a multiple of the pairs: [4096, 4096] at 717
-// rows is 48 tiles for 74 pairs, [2560, 10240] at 2048 rows 80.  Any multiple of 16 is a legal tile, so the one with the least
-// estimated time is taken: a 128-byte step of K takes 0.094 us + 0.00073 a row, a launch 3.2 us + 0.009 a row and up to 1.6 where all
+// rows is 48 tiles for 74 pairs, [2560, 10240] at 2048 rows 80.  tcgen05.mma.cta_group::2 with 256 rows takes N in steps of 16 for
+// kind::f8f6f4 and of 32 for kind::i8; of these widths the one with the least estimated time is taken: a 128-byte step of K takes 0.094 us +
+// 0.00073 a row, a launch 3.2 us + 0.009 a row and up to 1.6 where all
 // SMs store their results.  Measured, us, tiles of 256 / the tile taken: [4096, 4096] 717 rows 15.3 / 12.7 (176), [4096, 16384] 717 rows
 // 45.3 / 35.8, [2560, 10240] 1000 rows 29.3 / 19.5 (144), 2048 rows 49.6 / 35.5, [2560, 2560] 2048 rows 16.2 / 13.5, [16384, 4096] 717 rows 38.7 /
 // 35.8 (224).
@@ -281,14 +282,15 @@ static bool t2_forced() {
     static const bool force = std::getenv("RWKVQ_TC2") && std::getenv("RWKVQ_TC2")[0] == 'f';
     return force;
 }
-static T2Tile tc2_tile(int64_t M, int64_t N, int64_t K, int nmat) {
+static T2Tile tc2_tile(int kind, int64_t M, int64_t N, int64_t K, int nmat) {
+    const int step = kind == KIND_I8 ? 32 : 16;
     const char* bn_env = t2_forced() ? std::getenv("RWKVQ_TC2_BN") : nullptr;      // read per call: a test switches tiles in one process
     const int forced = bn_env ? std::atoi(bn_env) : 0;
     const int64_t pairs = t2_grid_pairs(), pt = nmat * ((M + 255) / 256);
     const double kc = (double)((K + kT2Chunk - 1) / kT2Chunk), inv_pairs = 1.0 / (double)pairs;
     T2Tile best{0, 0.};
-    for (int bn = kT2N; bn >= 128; bn -= 16) {                 // on the path of every call: one short division a width where all tiles run at once
-        if (forced >= 128 && forced <= kT2N && forced % 16 == 0 && bn != forced) continue;
+    for (int bn = kT2N; bn >= 128; bn -= step) {                 // on the path of every call: one short division a width where all tiles run at once
+        if (forced >= 128 && forced <= kT2N && forced % step == 0 && bn != forced) continue;
         const int64_t tiles = pt * (int64_t)(((uint32_t)N + (uint32_t)bn - 1) / (uint32_t)bn);      // N < 2^30
         const int64_t waves = tiles <= pairs ? 1 : (tiles + pairs - 1) / pairs;
         const double us = 3.15 + 0.009 * bn + 1.6 * std::min(1.0, (double)tiles * inv_pairs) + (double)waves * kc * (0.094 + 0.000731 * bn);
@@ -313,9 +315,11 @@ bool tc2_eligible(int kind, int64_t M, int64_t N, int64_t K, int nmat, int singl
     const int64_t pairs = t2_grid_pairs();
     const int64_t single = nmat * ((M + 127) / 128) * ((N + single_nb - 1) / single_nb);
     const double kc = (double)((K + kT2Chunk - 1) / kT2Chunk), step1 = single_nb > 128 ? 0.369 : (single_nb > 64 ? 0.218 : 0.193);
-    const double t2 = tc2_tile(M, N, K, nmat).us, t1 = (single_nb > 128 ? 3.3 : (single_nb > 64 ? 4.0 : 3.5)) + (double)((single + 2 * pairs - 1) / (2 * pairs)) * kc * step1;
+    const double t2 = tc2_tile(kind, M, N, K, nmat).us, t1 = (single_nb > 128 ? 3.3 : (single_nb > 64 ? 4.0 : 3.5)) + (double)((single + 2 * pairs - 1) / (2 * pairs)) * kc * step1;
     return t2 <= t1;
 }
+
+int tc2_width(int kind, int64_t M, int64_t N, int64_t K, int nmat) { return tc2_tile(kind, M, N, K, nmat).bn; }
 
 int32_t run_tc2(const Tc2Call& c, int* status, cudaStream_t st, const char* who) {
     Tc2Args a{};
@@ -323,7 +327,7 @@ int32_t run_tc2(const Tc2Call& c, int* status, cudaStream_t st, const char* who)
     a.ffn_amax = c.ffn_amax; a.status = status; a.wait_ns = wait_limit_ns();
     a.ldo = c.ldo; a.ldacc = c.ldacc; a.M = c.M; a.N = c.N; a.K = c.K; a.nmat = c.nmat; a.div_mode = c.div_mode; a.amax_is_amax = c.amax_is_amax; a.flags = c.flags;
     a.kchunks = (c.K + kT2Chunk - 1) / kT2Chunk;
-    a.bn = tc2_tile(c.M, c.N, c.K, c.nmat).bn;
+    a.bn = tc2_tile(c.kind, c.M, c.N, c.K, c.nmat).bn;
     a.ptiles = (c.M + 255) / 256;
     a.qtiles = (c.N + a.bn - 1) / a.bn;
     a.stages = kT2MaxStages;

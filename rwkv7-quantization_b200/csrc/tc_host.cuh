@@ -134,6 +134,7 @@ struct Tc2Call {
     int64_t lda, ldw, ldo, ldacc;
 };
 bool tc2_eligible(int kind, int64_t M, int64_t N, int64_t K, int nmat, int single_nb);
+int tc2_width(int kind, int64_t M, int64_t N, int64_t K, int nmat);      // weight rows per pair tile
 int32_t run_tc2(const Tc2Call& c, int* status, cudaStream_t st, const char* who);
 
 // NVFP4 GEMM for many tokens on CTA pairs (gemm_tc2_nvfp4.cu), and which tiled form these sizes take (0: pairs, else the weight rows

@@ -193,3 +193,28 @@ def test_scratch_sizes_agree_with_the_library():
         for k in (256, 768, 2560, 16384):
             assert abi.linear_nvfp4_scratch_bytes(m, k) == abi.lib().rwkvq_linear_nvfp4_scratch_bytes(m, k)
     assert abi.lib().rwkvq_linear_nvfp4_scratch_bytes(4, 100) == 0
+
+
+def pair_widths():
+    import rwkvq_abi as abi
+    return [(kind, abi.lib().rwkvq_tc_gemm_pair_width(kind, nmat, m, n, k)) for kind in (abi.LINEAR_FP8, abi.LINEAR_INT8) for nmat in (1, 3)
+            for m in (129, 300, 717, 1000, 1500, 2048) for n, k in ((4096, 4096), (2560, 2560), (16384, 4096), (2560, 10240), (1000, 400), (9000, 2064))]
+
+
+def test_pair_tiles_are_instruction_shapes():
+    """tcgen05.mma.cta_group::2 with 256 rows takes N in steps of 16 (FP8) or 32 (INT8): the widths that the plan picks, and every width
+    that its switch asks for."""
+    import subprocess
+    import sys
+    import rwkvq_abi as abi
+    legal = lambda kind, bn: 128 <= bn <= 256 and bn % (32 if kind == abi.LINEAR_INT8 else 16) == 0  # noqa: E731
+    widths = pair_widths()
+    assert all(legal(*w) for w in widths), [w for w in widths if not legal(*w)]
+    assert len({w for w in widths if w[0] == abi.LINEAR_INT8}) > 1      # not one width for all sizes
+    code = f"import os, sys; sys.path[:0] = [{os.path.join(ROOT, 'rwkv7-quantization_b200')!r}, {os.path.dirname(__file__)!r}]\n" \
+           "import test_abi_cpu as t\n" \
+           "for bn in range(112, 273, 8): os.environ['RWKVQ_TC2_BN'] = str(bn); print(t.pair_widths())"
+    out = subprocess.run([sys.executable, "-c", code], check=True, capture_output=True, text=True, env=dict(os.environ, RWKVQ_TC2="force"), timeout=300).stdout
+    forced = [eval(line) for line in out.splitlines()]
+    assert len(forced) == 21 and all(legal(*w) for ws in forced for w in ws)
+    assert {w for w in forced[6] if w[0] == abi.LINEAR_FP8} == {(abi.LINEAR_FP8, 160)} and {w for w in forced[6] if w[0] == abi.LINEAR_INT8} == {(abi.LINEAR_INT8, 160)}
