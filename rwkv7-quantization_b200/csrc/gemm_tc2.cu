@@ -170,6 +170,7 @@ __global__ void __launch_bounds__(kT2Threads, 1) gemm_tc2_kernel(const __grid_co
                     }
                 }
             }
+            if (ok && !(ok = pair_drain_ring(s.empty, rp, a.stages, abort_flag, a.wait_ns))) t2_abort(s, a);
             if (!ok) {      // give copies already in flight a bounded time to land before the CTA's memory is released
                 const unsigned long long t0 = global_ns();
                 while (global_ns() - t0 < 2000000ull) {}

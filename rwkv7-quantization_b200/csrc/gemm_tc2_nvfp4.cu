@@ -132,6 +132,7 @@ __global__ void __launch_bounds__(kN2Threads, 1) gemm_tc2_nvfp4_kernel(const __g
                 }
             }
         }
+        if (ok && !(ok = pair_drain_ring(s.empty, rp, kN2MaxStages, abort_flag, a.wait_ns))) n2_abort(s, a);
         if (!ok) {      // give copies already in flight a bounded time to land before the CTA's memory is released
             const unsigned long long t0 = global_ns();
             while (global_ns() - t0 < 2000000ull) {}

@@ -356,6 +356,14 @@ int32_t rwkvq_nvfp4_pack_scales(const uint8_t* block_scales, int64_t lds, int64_
     return check_launch(who);
 }
 
+// tc_nvfp4_form, or what RWKVQ_NF4_BN (128, 256 or "pair"; read per call: a test switches tiles in one process) asks for
+static int nf_tiled_form(int64_t M, int64_t N, int64_t K) {
+    const char* env = std::getenv("RWKVQ_NF4_BN");
+    const int bn = env ? std::atoi(env) : 0;
+    if (env && env[0] == 'p') return 0;
+    return bn == 128 || bn == 256 ? bn : tc_nvfp4_form(M, N, K);
+}
+
 static int32_t run_tc_nvfp4(const uint8_t* a_codes, int64_t lda, const uint8_t* a_scales_blocked, const float* a_pts,
                             const uint8_t* w_codes, int64_t ldw, const uint8_t* w_scales_blocked, const float* w_tscale,
                             void* out_f16, int64_t ldo, int64_t M, int64_t N, int64_t K, void* workspace, int64_t workspace_bytes,
@@ -373,10 +381,7 @@ static int32_t run_tc_nvfp4(const uint8_t* a_codes, int64_t lda, const uint8_t* 
     if (push == nullptr && tcs_nvfp4_eligible(M, N, K))         // few tokens: K split across a thread-block cluster
         return run_tcs_nvfp4(a_codes, lda, a_scales_blocked, a_pts, w_codes, ldw, w_scales_blocked, w_tscale, (__half*)out_f16, ldo, M, N, K,
                              workspace ? reinterpret_cast<int*>(workspace) + kWsCounterInts : nullptr, (cudaStream_t)stream, who);
-    const char* bn_env = std::getenv("RWKVQ_NF4_BN");          // 128, 256 or "pair"; read per call: a test switches tiles in one process
-    const int forced_bn = bn_env ? std::atoi(bn_env) : 0;
-    const bool forced_pair = bn_env && bn_env[0] == 'p';
-    const int form = forced_pair ? 0 : (forced_bn == 128 || forced_bn == 256 ? forced_bn : tc_nvfp4_form(M, N, K));
+    const int form = nf_tiled_form(M, N, K);
     if (push == nullptr && form == 0)
         return run_tc2_nvfp4(a_codes, lda, a_scales_blocked, a_pts, w_codes, ldw, w_scales_blocked, w_tscale, (__half*)out_f16, ldo, M, N, K,
                              workspace ? reinterpret_cast<int*>(workspace) + kWsCounterInts : nullptr, (cudaStream_t)stream, who);
@@ -401,6 +406,12 @@ static int32_t run_tc_nvfp4(const uint8_t* a_codes, int64_t lda, const uint8_t* 
     if (push)
         return bn == 128 ? launch_nvfp4<128, true>(maps, a, grid, (cudaStream_t)stream, who) : launch_nvfp4<256, true>(maps, a, grid, (cudaStream_t)stream, who);
     return bn == 128 ? launch_nvfp4<128>(maps, a, grid, (cudaStream_t)stream, who) : launch_nvfp4<256>(maps, a, grid, (cudaStream_t)stream, who);
+}
+
+int32_t rwkvq_tc_gemm_nvfp4_form(int64_t M, int64_t N, int64_t K) {
+    if (M <= 0 || N <= 0 || K <= 0 || K % 256) return RWKVQ_E_BADARG;
+    if (tcs_nvfp4_eligible(M, N, K)) return RWKVQ_TC_FORM_CLUSTER;
+    return nf_tiled_form(M, N, K) == 0 ? RWKVQ_TC_FORM_PAIRS : RWKVQ_TC_FORM_TILED;
 }
 
 /* 1 if rwkvq_tc_gemm_nvfp4 runs these sizes on the cluster split-K kernel (few tokens), 0 for the tiled form */

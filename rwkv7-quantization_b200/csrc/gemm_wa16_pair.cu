@@ -29,8 +29,8 @@
 // issuers in the leader CTA, each with every other unit of a step, 4-7 and 8-11 the epilogue of warp 13's and warp 14's units.
 // wfull[] (this CTA's weights) is local; xfull[] (both CTAs' tokens), aready[] (both CTAs' widened weights) and dempty[] live in
 // the leader; empty[] and dfull[] are signalled in both CTAs by a multicast commit.  A slot of widened weights is free when the
-// step kA before it has left the tensor core, which is that step's empty[].  Every wait is bounded; the pair meets before its
-// tensor memory goes.
+// step kA before it has left the tensor core, which is that step's empty[].  Every wait is bounded; the producers wait for the last
+// commits and the pair meets before its tensor memory goes.
 #include <algorithm>
 #include <cstdlib>
 
@@ -204,6 +204,7 @@ __global__ void __launch_bounds__(kP16Threads, 1) gemm_wa16_pair_kernel(const __
                     }
                 }
             }
+            if (ok && !(ok = pair_drain_ring(s.empty, rp, TL::kS, abort_flag, a.wait_ns))) p16_abort(s, a);
             if (!ok) {   // give copies already in flight a bounded time to land before the CTA's memory is released
                 const unsigned long long t0 = global_ns();
                 while (global_ns() - t0 < 2000000ull) {}

@@ -52,6 +52,16 @@ __device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t cluster_add
     asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %1, 0;\n\t@p mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];\n\t}"
                  ::"r"(cluster_addr), "r"(lane) : "memory");
 }
+// The end of a pair's producer warp: waits until every stage of its ring has been released.  A multicast commit arrives in both CTAs
+// on its own time, and the last ones on a stage's barrier release nothing that a later step would wait for: without this a CTA could
+// leave while the peer's commit is still on its way into what is then another CTA's shared memory.  `rp` is the step after the last
+// one; a stage that was never used passes at once (its barrier is in phase 0).  The result is the warp's.
+__device__ __forceinline__ bool pair_drain_ring(uint64_t* empty, RingPos rp, int stages, const volatile int* abort_flag, unsigned long long limit_ns) {
+    bool ok = true;
+#pragma unroll 1
+    for (int i = 0; i < stages && ok; ++i, rp.next(stages)) ok = mbar_wait(&empty[rp.i], rp.phase ^ 1, abort_flag, limit_ns);
+    return __all_sync(0xffffffffu, ok);
+}
 
 }  // namespace tc
 }  // namespace rwkvq
