@@ -498,7 +498,7 @@ struct W16Plan { int NB, slices; bool pair; };
 // [4096, 16384], [2560, 2560], [10240, 2560], [2560, 10240], [1024, 1024] and [4096, 1024] at 8 to 2048 rows: a step (128 k of a tile)
 // takes 0.40 / 0.52 / 0.65 / 0.76 us with 32 / 64 / 96 / 128 tokens on one CTA (INT4: the widened weights and the accumulators share
 // tensor memory's ports with the MMAs) and 0.40 / 0.43 / 0.48 / 0.55 us (INT8: what an SM takes in from L2); on a pair, with 256 weight
-// rows, 0.51 / 0.86 us with 128 / 256 tokens (INT4) and 0.73 us with 256 (INT8); K slices cost 3.4 us for the second launch plus
+// rows, 0.58 / 0.88 us with 128 / 256 tokens (INT4) and 0.73 us with 256 (INT8); K slices cost 3.4 us for the second launch plus
 // the round trip of the partial sums.  Of the forms timed for each size the estimate takes one within 10 % of the best.
 // The register split of the INT4 kernels with 96 and 128 tokens adds up only if a thread starts with 128 registers; a compiler
 // that gives them another number leaves the narrower tiles.  RWKVQ_WA16_MAX_NB lowers the limit (read once).
@@ -516,7 +516,7 @@ static int w16_max_tokens(int fmt) {
 }
 static W16Plan wa16_plan(int fmt, int64_t M, int64_t N, int64_t K) {
     static constexpr double kStep[2][4] = {{400., 520., 650., 760.}, {400., 430., 480., 550.}};      // ns
-    static constexpr double kPairStep[2][2] = {{510., 860.}, {0., 730.}};                            // 0: no such tile
+    static constexpr double kPairStep[2][2] = {{575., 875.}, {0., 730.}};                            // 0: no such tile
     // RWKVQ_WA16_PAIR=0 switches the pairs off, =force uses them wherever they are legal (read once)
     static const char mode = std::getenv("RWKVQ_WA16_PAIR") ? std::getenv("RWKVQ_WA16_PAIR")[0] : 0;
     const int64_t ksteps = (K + kW16K - 1) / kW16K, q4 = (ksteps + 3) / 4;

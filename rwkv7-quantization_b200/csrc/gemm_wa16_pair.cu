@@ -14,6 +14,13 @@
 // (exact), and six of the nine products (zh xh, zh xm, zh xl, zm xh, zm xm, zl xh; the others are below 2^-24 of the whole)
 // are eight k of an MMA, 16 groups a step.  An infinity or NaN has no parts: it is multiplied once, as the highest one.
 //
+// Centred codes.  The two parts cancel where the activations have a mean, and they are added one after the other, so what either
+// loses is lost at its own size, and the tensor core cuts towards zero, always to the same side: with codes 0 to 15 and activations of
+// mean 3 the error of [4096, 16384] against 64 bits was 7.75e-4, of which 6.62e-4 are the rounding to fp16.  So a code goes in as code -
+// 7.5 (2 * code - 15, an exact fp16 integer) and its zero point as zero + 7.5 * scale, the middle of the group's range: 6.62e-4, as
+// with fp32 sums that add both parts group by group.  It costs the widening warps 64 fp16 FMAs a step: 15 ns with 256 tokens, 67 with 128,
+// where they are what a step waits for.  Without zeros (zero = -8 * scale) the codes are centred at 8 and there is no second part.
+//
 // A step is 128 k of one tile; its tokens are units of UN columns with an accumulator each, so that the epilogue adds one unit's
 // group while the tensor core works on others.  What limits a step is less the work (the MMAs of 256 tokens take 1024 clocks) than
 // the roles' own instruction streams and the signals between them: an arrival at the other CTA that orders memory costs 0.4 us
@@ -21,8 +28,8 @@
 // instead of four of 64 from two 0.07, an epilogue at 200 registers that crowds the widening warps 0.1.  Tensor memory: 256
 // columns of accumulators, then kA slots of 64 columns of widened weights; more accumulators and fewer slots change nothing.
 //
-// Measured in a graph, us with the activations' kernel, single CTAs -> pairs.  INT4: [4096, 4096] 200 / 1000 / 2048 rows 21.9 -> 18.6, 56.5 ->
-// 35.4, 105.9 -> 63.0; [16384, 4096] 53.9 -> 33.3, 175.7 -> 121.6, 345.6 -> 218.7; [4096, 16384] 57.0 -> 38.2, 196.0 -> 121.0, 401.0 -> 261.9.
+// Measured in a graph, us with the activations' kernel, single CTAs -> pairs.  INT4: [4096, 4096] 200 / 1000 / 2048 rows 21.4 -> 18.6, 56.2 ->
+// 35.3, 106.8 -> 63.1; [16384, 4096] 53.4 -> 33.2, 177.9 -> 118.5, 356.3 -> 218.1; [4096, 16384] 56.0 -> 38.1, 198.6 -> 122.4, 381.9 -> 248.6.
 // INT8: [4096, 4096] 1000 / 2048 rows 33.7 -> 26.3, 62.5 -> 48.0; [4096, 16384] 122.9 -> 93.1, 259.8 -> 201.6.
 //
 // Roles per CTA (512 threads): warps 0-3 widen (lane quarter = warp), 12 TMA producer, 13 (which owns tensor memory) and 14 MMA
@@ -152,7 +159,7 @@ __global__ void __launch_bounds__(kP16Threads, 1) gemm_wa16_pair_kernel(const __
         const int q4 = (a.ksteps + 3) >> 2;
         it.k0 = (int)((uint32_t)(q4 * it.sl) / (uint32_t)a.slices) * 4;             // below 2^21 * 16
         it.k1 = min((int)((uint32_t)(q4 * (it.sl + 1)) / (uint32_t)a.slices) * 4, a.ksteps);
-        it.nz = kGroup ? (it.k1 - it.k0 + 15) >> 4 : 0;
+        it.nz = kGroup && a.zeros ? (it.k1 - it.k0 + 15) >> 4 : 0;
         return it;
     };
 
@@ -265,7 +272,9 @@ __global__ void __launch_bounds__(kP16Threads, 1) gemm_wa16_pair_kernel(const __
         // ============================== weights: packed -> 16 bits in tensor memory ==============================
         const uint32_t lane_addr = tmem_base + TL::kACol + ((uint32_t)(warp * 32) << 16);
         const int row = warp * 32 + lane;
+        const uint32_t centre = a.zeros ? 15 : 16;
         const uint32_t leader_aready = mapa_u32(smem_u32(&s.aready[0]), 0);
+        const bool vec = (a.groups & 3) == 0;    // host: scales and zeros are 16-byte aligned
         RingPos rp, ap, freed;                   // freed: the step whose MMAs read this slot last
         int slots = TL::kA;
         bool ok = true;
@@ -273,9 +282,9 @@ __global__ void __launch_bounds__(kP16Threads, 1) gemm_wa16_pair_kernel(const __
             const Item it = item_of(t);
             for (int k = it.k0; k < it.k1 + it.nz; ++k, rp.next(TL::kS), ap.next(TL::kA)) {
                 const int st = rp.i;
-                ok = mbar_wait(&s.wfull[st], rp.phase, abort_flag, a.wait_ns);
                 const uint32_t dst = lane_addr + (uint32_t)ap.i * 64;
                 const bool zstep = kGroup && k >= it.k1;
+                ok = mbar_wait(&s.wfull[st], rp.phase, abort_flag, a.wait_ns);
                 if (--slots < 0) {
                     ok = ok && mbar_wait(&s.empty[freed.i], freed.phase, abort_flag, a.wait_ns);
                     freed.next(TL::kS);
@@ -285,18 +294,31 @@ __global__ void __launch_bounds__(kP16Threads, 1) gemm_wa16_pair_kernel(const __
                 tc_fence_after_sync();
                 if (zstep) {
                     griddep_wait();                          // zeros may come from the kernel in front
-                    const int g0 = it.k0 + 16 * (k - it.k1), n = min(it.nt * 256 + (int)rank * 128 + row, a.N - 1);
-                    const float* src = (a.zeros ? a.zeros : a.scales) + (int64_t)n * a.groups;
-                    const float f = a.zeros ? 1.f : -8.f;
+                    const int g0 = it.k0 + 16 * (k - it.k1);
+                    const int64_t at = (int64_t)min(it.nt * 256 + (int)rank * 128 + row, a.N - 1) * a.groups;
 #pragma unroll 1
                     for (int h = 0; h < 2 && g0 + 8 * h < it.k1; ++h) {
+                        float z[8], sc[8];                   // all loads at once: what is past the end is read from the last group
+                        if (vec) {
+#pragma unroll
+                            for (int j = 0; j < 8; j += 4) {
+                                const int g = min(g0 + 8 * h + j, it.k1 - 4);
+                                *reinterpret_cast<float4*>(z + j) = __ldg(reinterpret_cast<const float4*>(a.zeros + at + g));
+                                *reinterpret_cast<float4*>(sc + j) = __ldg(reinterpret_cast<const float4*>(a.scales + at + g));
+                            }
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) {
+                                const int g = min(g0 + 8 * h + j, it.k1 - 1);
+                                z[j] = __ldg(a.zeros + at + g);
+                                sc[j] = __ldg(a.scales + at + g);
+                            }
+                        }
                         uint32_t r[32];
 #pragma unroll
                         for (int j = 0; j < 8; ++j) {
-                            const int g = g0 + 8 * h + j;
-                            const float z = g < it.k1 ? __ldg(src + g) * f : 0.f;
                             // zh zh' | zh' zm | zm zl | 0 0 against xh xm | xl xh' | xm xh' | 0 0 (a primed part is zero beside an infinity or NaN)
-                            const Bf16Parts p = bf16_parts(z);
+                            const Bf16Parts p = bf16_parts(g0 + 8 * h + j < it.k1 ? fmaf(7.5f, sc[j], z[j]) : 0.f);      // of centred codes
                             r[4 * j] = p.h | (p.h1 << 16);
                             r[4 * j + 1] = p.h1 | (p.m << 16);
                             r[4 * j + 2] = p.m | (p.l << 16);
@@ -313,10 +335,10 @@ __global__ void __launch_bounds__(kP16Threads, 1) gemm_wa16_pair_kernel(const __
 #pragma unroll
                             for (int c = 0; c < 2; ++c) {        // 64-byte swizzle: 16-byte piece p of row r sits at p ^ ((r / 2) % 4)
                                 const uint4 v = *reinterpret_cast<const uint4*>(wrow + (((h * 2 + c) ^ ((row >> 1) & 3)) << 4));
-                                widen_nibbles(v.x, r + c * 16, r + c * 16 + 8);
-                                widen_nibbles(v.y, r + c * 16 + 2, r + c * 16 + 10);
-                                widen_nibbles(v.z, r + c * 16 + 4, r + c * 16 + 12);
-                                widen_nibbles(v.w, r + c * 16 + 6, r + c * 16 + 14);
+                                widen_nibbles_centred(v.x, centre, r + c * 16, r + c * 16 + 8);
+                                widen_nibbles_centred(v.y, centre, r + c * 16 + 2, r + c * 16 + 10);
+                                widen_nibbles_centred(v.z, centre, r + c * 16 + 4, r + c * 16 + 12);
+                                widen_nibbles_centred(v.w, centre, r + c * 16 + 6, r + c * 16 + 14);
                             }
                         } else {
 #pragma unroll
@@ -377,13 +399,13 @@ __global__ void __launch_bounds__(kP16Threads, 1) gemm_wa16_pair_kernel(const __
 #pragma unroll
                     for (int n = 0; n < UN / 2; ++n) acc[i][n] = 0;
                 const float* srow = a.scales + (int64_t)min(row, a.N - 1) * a.groups;
-                // scale of group k, or what undoes the factor 2^24 for a step of zero points; three steps under way.  2^24: a code
-                // is widened to a multiple of 2^-24.
-                auto scale_of = [&](int k) { return k < it.k1 ? __ldg(srow + k) : 1.f / 16777216.f; };
+                // scale of group k, or what undoes the factor 2^23 for a step of zero points; three steps under way.  2^23: twice a centred
+                // code is widened to a multiple of 2^-24.
+                auto scale_of = [&](int k) { return k < it.k1 ? __ldg(srow + k) : 1.f / 8388608.f; };
                 float s0 = scale_of(it.k0), s1 = scale_of(it.k0 + 1), s3 = scale_of(it.k0 + 2);
 #pragma unroll 1
                 for (int k = it.k0; k < it.k1 + it.nz && ok; ++k) {
-                    const float sc = s0 * 16777216.f;
+                    const float sc = s0 * 8388608.f;
                     s0 = s1;
                     s1 = s3;
                     s3 = scale_of(k + 3);

@@ -43,6 +43,16 @@ __device__ __forceinline__ void widen_nibbles(uint32_t w, uint32_t* odd, uint32_
     even[0] = w & 0x000F000Fu;
     even[1] = h & 0x000F000Fu;
 }
+// the same of 2 * code - centre, exact (multiples of 2^-24 below 2^-13)
+__device__ __forceinline__ void widen_nibbles_centred(uint32_t w, uint32_t centre, uint32_t* odd, uint32_t* even) {
+    widen_nibbles(w, odd, even);
+    const uint32_t e = 0x80008000u | centre * 0x00010001u, o = 0x80008000u | centre * 0x00100010u;       // - centre * 2^-24, - centre * 2^-20
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        asm("fma.rn.f16x2 %0, %0, %1, %2;" : "+r"(odd[i]) : "r"(0x40004000u), "r"(o));
+        asm("fma.rn.f16x2 %0, %0, %1, %2;" : "+r"(even[i]) : "r"(0x40004000u), "r"(e));
+    }
+}
 __device__ __forceinline__ uint64_t pack2(float lo, float hi) {
     uint64_t r;
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));

@@ -202,3 +202,26 @@ def test_int4_infinite_and_nan_activations_stay_in_their_row(m, n, k):
     ok = [i for i in range(m) if i not in special]
     assert torch.equal(out[ok], want[ok])
     assert not bool(out[special].isfinite().any()) and bool(out[m - 1].isnan().all())
+
+
+@pytest.mark.parametrize("m,n,k", [(600, 4096, 4096), (600, 4096, 16384), (1000, 4096, 2176)])
+def test_int4_scales_and_zeros_that_cancel(m, n, k):
+    """Activations around 8 and zeros of minus the mean weight: the scales' and the zeros' parts of a sum are thousands of times the result.
+    The error before the result is rounded to fp16 may be twice that of fp32 sums that add the two parts group by group."""
+    import rwkvq_abi as abi
+    from int4 import int4_ops, quantize_int4
+    assert abi.lib().rwkvq_tc_gemm_wa16_form(m, n, k, 4) % 1000 in (1000 - 128, 1000 - 256)
+    info = quantize_int4.quantize_to_int4_groupwise(gen(n + k, (n, k), k ** -0.5) * 64, 128)
+    d = {a: b.cuda() if torch.is_tensor(b) else b for a, b in info.items()}
+    u = int4_ops.unpack_int4(d["packed"]).double().reshape(n, k // 128, 128)
+    d["zeros"] = -(d["scales"] * u.mean(2).float())
+    x = (8 + gen(m, (m, k)) * 2.0 ** -5).half().cuda()
+    ref, acc = torch.zeros((m, n), dtype=torch.float64, device="cuda"), torch.zeros((m, n), device="cuda")
+    for g in range(k // 128):
+        xg = x[:, g * 128:(g + 1) * 128].double()
+        for f, v in ((d["scales"][:, g], xg @ u[:, g].t()), (d["zeros"][:, g], xg.sum(1, keepdim=True))):
+            ref += f.double() * v
+            acc += f * v.float()
+    rms = lambda e: float(e.double().square().mean().sqrt())  # noqa: E731
+    err, sums, half = (rms(v.double() - ref) for v in (int4_ops.linear_int4(x, dict(d, qtype="int4_groupwise")), acc, ref.half()))
+    assert err <= 2 * sums + half, (err, sums, half)
