@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(256) wa16_prep_kernel(const uint16_t* __restri
                 if ((threadIdx.x & 15) == 0) {
                     if (xz) {
                         const Bf16Parts p = bf16_parts(sum);
-                        xz[(int64_t)m * groups + (i >> 4)] = make_uint4(p.h | (p.m << 16), p.l | (p.h1 << 16), p.m | (p.h1 << 16), 0u);
+                        xz[(int64_t)m * groups + (i >> 4)] = make_uint4(p.h | (p.m << 16), p.l | (p.h1 << 16), p.m | (p.h1 << 16), p.l | (p.m << 16));
                     } else {
                         xsum[((int64_t)(m / NB) * groups + (i >> 4)) * NB + m % NB] = sum;
                     }

@@ -10,9 +10,10 @@
 // Zero points.  out = sum over groups of scale * (codes . x) + zero * sum(x).  The second part is a product of its own, [rows, groups] x
 // [groups, tokens] in fp32: taken with FMAs it costs the epilogue as much as the scales do, and the group sums, the same for
 // all 32 lanes, come through 128-byte-per-clock shared-memory loads at 16 bytes of use per warp (a third of the step).  So it is done
-// by the tensor core too, after the last group: both fp32 factors are cut into three bf16 parts of 8 mantissa bits each
-// (exact), and six of the nine products (zh xh, zh xm, zh xl, zm xh, zm xm, zl xh; the others are below 2^-24 of the whole)
-// are eight k of an MMA, 16 groups a step.  An infinity or NaN has no parts: it is multiplied once, as the highest one.
+// by the tensor core too, after the last group: both fp32 factors are cut into three bf16 parts of 8 mantissa bits each (exact from
+// 2^-110 up: below, what lies under bf16's 2^-133 is lost), and all products but zl xl, which is below 2^-30 of the whole, are
+// eight k of an MMA, 16 groups a step.  (The parts are cut, not rounded, so zm xl and zl xm each reach 2^-22.)  An infinity or NaN has no
+// parts: it is multiplied once, as the highest one.
 //
 // Centred codes.  The two parts cancel where the activations have a mean, and they are added one after the other, so what either
 // loses is lost at its own size, and the tensor core cuts towards zero, always to the same side: with codes 0 to 15 and activations of
@@ -317,12 +318,12 @@ __global__ void __launch_bounds__(kP16Threads, 1) gemm_wa16_pair_kernel(const __
                         uint32_t r[32];
 #pragma unroll
                         for (int j = 0; j < 8; ++j) {
-                            // zh zh' | zh' zm | zm zl | 0 0 against xh xm | xl xh' | xm xh' | 0 0 (a primed part is zero beside an infinity or NaN)
+                            // zh zh' | zh' zm | zm zl | zm zl against xh xm | xl xh' | xm xh' | xl xm (a primed part is zero beside an infinity or NaN)
                             const Bf16Parts p = bf16_parts(g0 + 8 * h + j < it.k1 ? fmaf(7.5f, sc[j], z[j]) : 0.f);      // of centred codes
                             r[4 * j] = p.h | (p.h1 << 16);
                             r[4 * j + 1] = p.h1 | (p.m << 16);
                             r[4 * j + 2] = p.m | (p.l << 16);
-                            r[4 * j + 3] = 0;
+                            r[4 * j + 3] = p.m | (p.l << 16);
                         }
                         tmem_st32(dst + h * 32, r);
                     }

@@ -93,7 +93,8 @@ inline int32_t w16_map(CUtensorMap* m, const void* ptr, int64_t rows, int64_t ro
     return RWKVQ_OK;
 }
 
-// An fp32 value as three bf16 values of 8 mantissa bits each that add up to it exactly (cut, not rounded: no part overflows).
+// An fp32 value of 2^-110 and more as three bf16 values of 8 mantissa bits each that add up to it exactly (cut, not rounded: no part
+// overflows; of a smaller one what is below bf16's least, 2^-133, is lost).
 // An infinity or NaN is its own highest part and has no others; h1 is the highest part of a finite value only.
 struct Bf16Parts { uint32_t h, h1, m, l; };
 __device__ __forceinline__ Bf16Parts bf16_parts(float v) {

@@ -225,3 +225,23 @@ def test_int4_scales_and_zeros_that_cancel(m, n, k):
     rms = lambda e: float(e.double().square().mean().sqrt())  # noqa: E731
     err, sums, half = (rms(v.double() - ref) for v in (int4_ops.linear_int4(x, dict(d, qtype="int4_groupwise")), acc, ref.half()))
     assert err <= 2 * sums + half, (err, sums, half)
+
+
+def test_int4_zero_points_keep_all_products_of_their_parts():
+    """Zero point of the centred codes and sum of the activations both 1 + 2^-7 - 2^-23 (times a power of two), the values whose lower bf16 parts are
+    largest, against a scale that cancels them exactly.  What is left are errors: half an ulp of the scales' product, the tensor core's
+    sum cut to fp32 (one ulp) and its addends' alignment (one more); without zm xl and zl xm it would be 2^-21 of the product, four ulps."""
+    import rwkvq_abi as abi
+    from int4 import int4_ops
+    m, n, k = 1000, 4096, 256
+    assert abi.lib().rwkvq_tc_gemm_wa16_form(m, n, k, 4) % 1000 in (1000 - 128, 1000 - 256)
+    v = 1 + 2.0 ** -7 - 2.0 ** -23
+    d = {"packed": torch.full((n, k // 2), 0x88, dtype=torch.uint8, device="cuda"), "scales": torch.full((n, 2), 2 * v, device="cuda"),
+         "zeros": torch.full((n, 2), -16 * v, device="cuda"), "group_size": 128, "qtype": "int4_groupwise"}
+    assert float((d["scales"].double() * 8 + d["zeros"].double()).abs().max()) == 0
+    x = torch.zeros((m, k), dtype=torch.float16, device="cuda")
+    x[:, :128] = 65
+    x[:, 0], x[:, 1] = -2.0 ** -10, 66
+    assert float(x.double().sum(1).max()) == v * 2 ** 13
+    y = int4_ops.linear_int4(x, d)
+    assert float(y.abs().max()) <= 2.5 * 2.0 ** -10, float(y.abs().max())
