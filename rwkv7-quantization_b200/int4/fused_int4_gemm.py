@@ -74,7 +74,7 @@ def _groupwise_tc(x, packed, scales, zeros):
         raise RuntimeError("rwkvq: INT4 / INT8 projections run on the GPU only (no CPU fallback)")
     m, dev = x2.shape[0], x2.device
     out = torch.empty((m, n), dtype=torch.float16, device=dev)
-    ws = torch.empty(abi.wa16_workspace_bytes(m, n, k, 4), dtype=torch.uint8, device=dev)
+    ws = torch.empty(abi.wa16_workspace_bytes(m, n, k, 4, dev), dtype=torch.uint8, device=dev)
     abi.call("rwkvq_tc_gemm_int4_group", x2.data_ptr(), abi.dtype_code(x2), k, packed.data_ptr(), packed.stride(0), scales.data_ptr(),
              abi.ptr(zeros), out.data_ptr(), n, m, n, k, ws.data_ptr(), ws.numel(), abi.stream_ptr())
     abi.after_call()

@@ -56,7 +56,7 @@ def _tensor_core(x2, w, scale):
         raise RuntimeError("rwkvq: INT4 / INT8 projections run on the GPU only (no CPU fallback)")
     (m, k), n, dev = x2.shape, w.shape[0], x2.device
     out = torch.empty((m, n), dtype=torch.float16, device=dev)
-    ws = torch.empty(abi.wa16_workspace_bytes(m, n, k, 8), dtype=torch.uint8, device=dev)
+    ws = torch.empty(abi.wa16_workspace_bytes(m, n, k, 8, dev), dtype=torch.uint8, device=dev)
     abi.call("rwkvq_tc_gemm_int8_w8a16", x2.data_ptr(), k, w.data_ptr(), w.stride(0), scale.data_ptr(), out.data_ptr(), n, m, n, k,
              ws.data_ptr(), ws.numel(), abi.stream_ptr())
     abi.after_call()

@@ -406,13 +406,14 @@ def workspace(m: int, n: int, k: int, nmat: int, device) -> torch.Tensor:
 _wa16_need: dict = {}
 
 
-def wa16_workspace_bytes(m: int, n: int, k: int, bits: int) -> int:
-    """rwkvq_tc_gemm_wa16_workspace_bytes, asked once per shape (it estimates every form)."""
-    need = _wa16_need.get((m, n, k, bits))
+def wa16_workspace_bytes(m: int, n: int, k: int, bits: int, device) -> int:
+    """rwkvq_tc_gemm_wa16_workspace_bytes, asked once per shape and device (it estimates every form for the device's SMs)."""
+    key = (m, n, k, bits, device_index(device))
+    need = _wa16_need.get(key)
     if need is None:
         if len(_wa16_need) >= 4096:
             _wa16_need.clear()
-        need = _wa16_need[(m, n, k, bits)] = int(lib().rwkvq_tc_gemm_wa16_workspace_bytes(m, n, k, bits))
+        need = _wa16_need[key] = int(lib().rwkvq_tc_gemm_wa16_workspace_bytes(m, n, k, bits))
     return need
 
 

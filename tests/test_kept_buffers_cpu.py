@@ -36,3 +36,21 @@ def test_superseded_buffers_stay_allocated(monkeypatch, which):
         del buf
     assert len(refs) > 2 and all(r() is not None for r in refs)
     assert sum(b.numel() for b in abi._superseded) <= get(0).numel()
+
+
+def test_weight_only_workspace_is_asked_once_per_shape_and_device(monkeypatch):
+    """The plan behind the size depends on the device's SM count: two unlike devices in one process each get their own."""
+    import torch
+    import rwkvq_abi as abi
+
+    class Lib:
+        asked = 0
+
+        def rwkvq_tc_gemm_wa16_workspace_bytes(self, m, n, k, bits):
+            Lib.asked += 1
+            return 1000 + Lib.asked
+    monkeypatch.setattr(abi, "lib", Lib)
+    monkeypatch.setattr(abi, "_wa16_need", {})
+    d0, d1 = torch.device("cuda", 0), torch.device("cuda", 1)
+    assert [abi.wa16_workspace_bytes(100, 4096, 4096, 4, d) for d in (d0, d1, d0, d1)] == [1001, 1002, 1001, 1002]
+    assert abi.wa16_workspace_bytes(100, 4096, 4096, 8, d0) == 1003
