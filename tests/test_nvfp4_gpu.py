@@ -115,6 +115,8 @@ def test_tensor_core_route(nf, monkeypatch, bn, m, n, k):
     """The tcgen05 block-scaled GEMM (both tile widths and CTA pairs; few and many tiles per CTA) against the oracle and against the GEMV route; ragged M and N."""
     import rwkvq_abi as abi
     monkeypatch.setenv("RWKVQ_NF4_BN", bn)
+    monkeypatch.setenv("RWKVQ_TCS_NF4_MIN_C", "99")     # no size runs on the cluster kernel instead
+    assert abi.lib().rwkvq_tc_gemm_nvfp4_form(m, n, k) == (abi.TC_FORM_PAIRS if bn == "pair" else abi.TC_FORM_TILED)
     w = gen(n * 3 + k, (n, k), (1.0 / k) ** 0.5)
     info = dev(nf.quantize_to_nvfp4(w))
     x = gen(m + 11, (m, k), 1.0, torch.bfloat16)

@@ -134,7 +134,7 @@ def test_results_in_a_column_range(m, n, k, offset):
 
 
 def tile_widths():
-    """Every width of a pair's tile against the widest: halves of an odd number of 16-column pieces, columns past the last tile."""
+    """Every width of a pair's tile (INT8: multiples of 32, the others leave it to the plan) against the widest: halves of an odd number of 16-column pieces, columns past the last tile."""
     import rwkvq_abi as abi
     global SIZES
     sizes = [(129, 1000, 400), (300, 4104, 1040), (517, 2560, 768)]
@@ -142,6 +142,8 @@ def tile_widths():
         want = None
         for bn in range(256, 127, -16):
             os.environ["RWKVQ_TC2_BN"] = str(bn)
+            for (m, n, k), kind in ((s, c) for s in SIZES for c in (abi.LINEAR_FP8, abi.LINEAR_INT8)):
+                assert bn % 32 and kind == abi.LINEAR_INT8 or abi.lib().rwkvq_tc_gemm_pair_width(kind, 1, m, n, k) == bn
             got = results()
             want = got if want is None else want
             assert all(torch.equal(a, b) for a, b in zip(got, want)), (SIZES, bn)
