@@ -1,19 +1,20 @@
-// W8A8 GEMM for many tokens on CTA PAIRS: tcgen05.mma.cta_group::2 (two SMs work on one 256 x 256 tile).
-//
-// Tiles: 256 tokens x bn weight rows (below: bn = 256).
+// W8A8 GEMM for many tokens on CTA PAIRS: tcgen05.mma.cta_group::2 (two SMs work on one tile of 256 tokens x bn weight rows,
+// bn = 128 to 256, see tc2_tile).
 //
 // Why pairs.  With one CTA per 128 x 256 tile (gemm_tc.cu) every 128-byte step of K needs 48 KB of operands from L2
 // per SM for 512 cycles of tensor-core work -- 96 bytes per clock, more than an SM gets from L2, so the tensor pipe
-// idles a third of the time.  In a pair each CTA loads its own 128 token rows and only HALF of the 256 weight rows
-// (32 KB per step per SM, 64 bytes per clock); the MMA issued by the pair's leader reads both halves of the weight
-// tile from the two CTAs' shared memory and accumulates each CTA's 128 x 256 block in that CTA's own tensor memory.
+// idles a third of the time.  In a pair each CTA loads its own 128 token rows and only HALF of the bn weight rows (bn = 256:
+// 32 KB per step per SM, 64 bytes per clock; bn = 128: 24 KB for half the work, 96 again, taken where it fills a wave); the MMA
+// issued by the pair's leader reads both halves of the weight tile from the two CTAs' shared memory and accumulates each CTA's
+// 128 x bn block in that CTA's own tensor memory.
 // No multicast is involved: every TMA load lands in the shared memory of the CTA that issued it.
 //
 // Roles per CTA as in gemm_tc.cu: warp 0 = TMA producer, warp 1 = tensor-memory owner and -- in the leader CTA only --
 // MMA issuer (one elected lane each), warps 2-9 = epilogue (tc_epilogue.cuh).  Barriers: full[] lives in the leader (both producers' bytes are
 // counted there: the loads carry .cta_group::2 and name the leader's barrier), empty[] and tfull[] are signalled in both
 // CTAs at once by a multicast tcgen05.commit, tempty[] of the leader collects the arrivals of both CTAs' epilogue warps.
-// Every wait is bounded; the pair meets at a cluster barrier before the tensor memory is released.
+// Every wait is bounded; the producers wait for the last commits and the pair meets at a cluster barrier before the tensor memory is
+// released.
 #include <algorithm>
 #include <cstdlib>
 
@@ -274,10 +275,10 @@ static int t2_grid_pairs() { return std::max(1, sm_count() / 2); }
 // Weight rows per pair tile.  A tile of 256 leaves pairs idle wherever the tiles are not a multiple of the pairs: [4096, 4096] at 717
 // rows is 48 tiles for 74 pairs, [2560, 10240] at 2048 rows 80.  tcgen05.mma.cta_group::2 with 256 rows takes N in steps of 16 for
 // kind::f8f6f4 and of 32 for kind::i8; of these widths the one with the least estimated time is taken: a 128-byte step of K takes 0.094 us +
-// 0.00073 a row, a launch 3.2 us + 0.009 a row and up to 1.6 where all
-// SMs store their results.  Measured, us, tiles of 256 / the tile taken: [4096, 4096] 717 rows 15.3 / 12.7 (176), [4096, 16384] 717 rows
-// 45.3 / 35.8, [2560, 10240] 1000 rows 29.3 / 19.5 (144), 2048 rows 49.6 / 35.5, [2560, 2560] 2048 rows 16.2 / 13.5, [16384, 4096] 717 rows 38.7 /
-// 35.8 (224).
+// 0.00073 a row, a launch 3.2 us + 0.009 a row and up to 1.6 where all SMs store their results.  Measured, us, tiles of 256 / the tile
+// taken, FP8: [4096, 4096] 717 rows 15.5 / 12.8 (176), [4096, 16384] 717 rows 44.3 / 36.0, [2560, 10240] 1000 rows 29.6 / 19.4 (144), 2048 rows
+// 50.7 / 35.7, [2560, 2560] 2048 rows 16.2 / 13.5, [16384, 4096] 717 rows 36.3 / 35.2 (224).  INT8: 15.1 / 12.8 (192), 42.5 / 34.7, 28.6 / 19.6 (160),
+// 49.8 / 34.4, 15.8 / 12.8, 37.5 / 34.9 (224).
 struct T2Tile { int bn; double us; };
 static bool t2_forced() {
     static const bool force = std::getenv("RWKVQ_TC2") && std::getenv("RWKVQ_TC2")[0] == 'f';
@@ -301,8 +302,8 @@ static T2Tile tc2_tile(int kind, int64_t M, int64_t N, int64_t K, int nmat) {
 }
 // RWKVQ_TC2=0 switches the pairs off, =force uses them wherever they are legal, RWKVQ_TC2_MIN_M raises their first row count (129: below it a pair tile is half empty).
 // Pairs or single CTAs?  The estimate above against that of the single form: 3.3 / 4.0 / 3.5 us and 0.37 / 0.22 / 0.19 a step with 256 / 128 /
-// 64 weight rows per tile.  Measured, us, single / pairs: FP8 [16384, 4096] 384 rows 27.4 / 24.5, 2048 rows 100.3 / 91.4; [4096, 16384] 717 rows 48.6 /
-// 38.6; [4096, 4096] 1000 rows 15.6 / 16.3; [8192, 2048] 384 rows 10.2 / 11.3, 2048 rows 28.3 / 25.3; [2560, 2560] 1500 rows 11.5 / 11.9.
+// 64 weight rows per tile.  Measured, us, single / pairs: FP8 [16384, 4096] 384 rows 26.9 / 24.0, 2048 rows 93.6 / 84.6; [4096, 16384] 717 rows 49.4 /
+// 35.9; [4096, 4096] 1000 rows 15.6 / 16.3; [8192, 2048] 384 rows 10.2 / 11.3, 2048 rows 28.3 / 25.3; [2560, 2560] 1500 rows 11.5 / 11.9.
 bool tc2_eligible(int kind, int64_t M, int64_t N, int64_t K, int nmat, int single_nb) {
     static const int64_t min_m = [] {
         const char* off = std::getenv("RWKVQ_TC2");
